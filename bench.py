@@ -40,7 +40,7 @@ NX = 150
 STEP_BYTES_PER_ELEM, STEP_BYTES_PER_NODE = 364, 152
 KERNEL_BYTES = {"k_force": (80, 48), "k_kinematics": (120, 48), "k_material": (164, 0), "k_node": (0, 104)}
 STATE_FIELDS = ["x", "y", "z", "xd", "yd", "zd", "e", "p", "q", "v", "ss"]
-GEOMETRY_SPLIT = {0: "force geometry formed by k_kinematics and stored for k_force",
+GEOMETRY_SPLIT = {0: "force geometry formed inside k_force",
                   1: "force geometry formed inside k_force"}
 
 

@@ -221,21 +221,19 @@ int lulesh_block_plan(int32_t nx, int32_t blocks_per_edge, int32_t mode, int32_t
                       int32_t* halo_corner_dst);
 
 /* ---- Launch tuning --------------------------------------------------------
- * Threads per block of the four step kernels and the fusion split of the
- * force geometry. lulesh_autotune tries each block-size candidate for one
- * kernel at a time on the live problem (cycles timed with CUDA events),
- * keeps the fastest, then times the other geometry split with its own best
- * force and kinematics blocks and keeps the faster split; it restores the
- * problem's state. No choice changes any result (bitwise). */
+ * Threads per block of the step kernels. lulesh_autotune tries each
+ * block-size candidate of k_node and k_material on the live problem (cycles
+ * timed with CUDA events) and keeps the fastest; it restores the problem's
+ * state. No choice changes any result (bitwise). k_force and k_kinematics run
+ * three threads per element in blocks of 96 and form their geometry
+ * themselves: force_block, kin_block and geometry are checked and handed back
+ * by lulesh_get_tuning, and change nothing. */
 typedef struct {
-  int32_t force_block;   /* k_force: 64, 128 or 256 */
+  int32_t force_block;   /* 64, 128 or 256 (no effect) */
   int32_t node_block;    /* k_node: 128, 256 or 512 */
-  int32_t kin_block;     /* k_kinematics: 64, 128 or 256 */
+  int32_t kin_block;     /* 64, 128 or 256 (no effect) */
   int32_t mat_block;     /* k_material: 64, 128 or 256 */
-  int32_t geometry;      /* where the force kernel's geometry of the positions
-                            (volume derivatives, hourglass modes, node normals)
-                            is formed: 0 by k_kinematics of the cycle before,
-                            stored (408 B per element); 1 inside k_force */
+  int32_t geometry;      /* 0 or 1 (no effect) */
 } lulesh_tuning;
 
 int lulesh_get_tuning(const lulesh_domain* dom, lulesh_tuning* out);

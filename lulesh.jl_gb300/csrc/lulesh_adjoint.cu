@@ -284,14 +284,13 @@ static void set_scalars(lulesh_domain* d, const Scalars5& s) {
   d->sc[LULESH_S_CYCLE] = (double)s.cycle;
 }
 
-// The start of a taped segment: the force kernel's geometry of the current
-// positions, with the first cycle's face normals on its tape and its face
-// diagonals in the set's diag0.
+// The start of a taped segment: the first cycle's face normals on its tape and
+// its face diagonals in the set's diag0.
 static void tape_segment_begin(lulesh_adjoint* a, const CycleTape& first, double* diag0, cudaStream_t s) {
   DevDomain gd = a->dom->dd;
   gd.tapeGeoNext = first.geo;
   gd.tapeDiag = diag0;
-  launch_geometry(gd, s);
+  launch_tape_geometry(gd, s);
 }
 
 // One taped cycle, queued on the stream: the start state to its slot and
@@ -316,9 +315,9 @@ static void tape_cycle(lulesh_adjoint* a, StateBuf& slot, const CycleTape& tp, c
   td.tapeFlags = tp.flags; td.tapeDtc = tp.dtc; td.tapeDth = tp.dth; td.tapeGeo = tp.geo;
   td.tapeKin = tp.kin; td.tapeMat = tp.mat;
   td.tapeGeoNext = next ? next->geo : nullptr;
-  launch_force(td, prm, d->tuning, s);
+  launch_force(td, prm, s);
   launch_node(td, prm, true, d->tuning, s);  // aux: the node kernel stores the accelerations
-  launch_kinematics(td, prm, false, d->tuning, s);
+  launch_kinematics(td, prm, false, s);
   launch_material(td, prm, false, d->tuning, s);
   const int ge = (a->E + kAdjBlock - 1) / kAdjBlock;
   ka_tape_close<<<ge, kAdjBlock, 0, s>>>(tp.dtc, tp.dth, a->E, d->dd.st, rec);
@@ -688,9 +687,9 @@ int lulesh_adj_gradient(lulesh_adjoint* a, int64_t num_cycles, lulesh_adj_result
     ACK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int j = 0; j < K; ++j) {
       launch_time_increment(d->dd.st, 1, prm, s);
-      launch_force(d->dd, prm, d->tuning, s);
+      launch_force(d->dd, prm, s);
       launch_node(d->dd, prm, aux, d->tuning, s);
-      launch_kinematics(d->dd, prm, aux, d->tuning, s);
+      launch_kinematics(d->dd, prm, aux, s);
       launch_material(d->dd, prm, aux, d->tuning, s);
     }
     ACK(cudaStreamEndCapture(s, &g));
@@ -772,11 +771,6 @@ int lulesh_adj_gradient(lulesh_adjoint* a, int64_t num_cycles, lulesh_adj_result
   const int64_t c0 = (int64_t)d->sc[LULESH_S_CYCLE];
   state_to_device_mirror(d);  // no cycle limit: the segments count the cycles
   ACK(cudaMemcpyAsync(d->dd.st, d->hst, sizeof(DevState), cudaMemcpyHostToDevice, s));
-  // the plain segments read the force geometry the kinematics kernel stores;
-  // the taping kernels form their own, so after the gradient (the domain left
-  // at the final state) it has to be formed again
-  ensure_geometry(d);
-  d->geo_valid = false;
   for (int k = 0; k < nplan; ++k) {
     copy_state_from_domain(a, a->ckpts[k], s);
     ACK(cudaMemcpyAsync(a->ckpt_st + k, d->dd.st, sizeof(DevState), cudaMemcpyDeviceToDevice, s));

@@ -68,7 +68,6 @@ inline size_t layout(DevDomain& dd, char* base, int64_t E, int64_t N, bool aux, 
   dd.regElemlist0 = nullptr;
   dd.regOfSlot = nullptr;
   dd.fcx = c.take<double>(nCornerSlot); dd.fcy = c.take<double>(nCornerSlot); dd.fcz = c.take<double>(nCornerSlot);
-  dd.nextGeo = c.take<double>((size_t)kGeoSlots * E);
   dd.tapeGeoNext = nullptr;
   dd.tapeDiag = nullptr;
   dd.st = c.take<DevState>(ninst > 0 ? ninst : 1);

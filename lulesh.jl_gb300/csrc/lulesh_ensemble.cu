@@ -84,7 +84,6 @@ struct lulesh_ensemble {
   std::vector<DevState> init_state;
   cudaGraphExec_t graph = nullptr;
   int64_t graph_key = -1;
-  bool geo_valid = false;  // dd.nextGeo holds the force geometry of the current positions
 };
 
 static double** mutable_node_fields(DevDomain& d, int k) {
@@ -127,9 +126,9 @@ static void drop_graph(lulesh_ensemble* s) {
 
 static void launch_cycle(lulesh_ensemble* s) {
   launch_time_increment(s->dd.st, s->n, s->prm, s->stream);
-  launch_force(s->dd, s->prm, s->tuning, s->stream);
+  launch_force(s->dd, s->prm, s->stream);
   launch_node(s->dd, s->prm, false, s->tuning, s->stream);
-  launch_kinematics(s->dd, s->prm, false, s->tuning, s->stream);
+  launch_kinematics(s->dd, s->prm, false, s->stream);
   launch_material(s->dd, s->prm, false, s->tuning, s->stream);
 }
 
@@ -315,7 +314,6 @@ int lulesh_ens_reset(lulesh_ensemble* s) {
   ECK(cudaSetDevice(s->device));
   int rc = snapshot_copy(s, false);
   if (rc) return rc;
-  s->geo_valid = false;
   return upload_states(s);
 }
 
@@ -340,12 +338,6 @@ int lulesh_ens_run(lulesh_ensemble* s, int64_t num_iters) {
     budget = std::max<int64_t>(budget, num_iters - d.cycle);
   }
   ECK(cudaMemcpyAsync(s->dd.st, s->hst, sizeof(DevState) * s->n, cudaMemcpyHostToDevice, st));
-  // the force kernel's stored geometry (an instance that stopped on an error
-  // keeps its positions until a reset, which clears this)
-  if (!s->geo_valid && s->tuning.geo == 0) {
-    launch_geometry(s->dd, st);
-    s->geo_valid = true;
-  }
   // one graph of the whole run (up to kMaxGraphCycles cycles), kept for the
   // next run of the same length; the run limit lives in the device state and
   // cycles past an instance's stop are no-ops for it
@@ -371,7 +363,6 @@ int lulesh_ens_run(lulesh_ensemble* s, int64_t num_iters) {
     for (int i = 0; i < s->n && all_done; ++i) all_done = s->hst[i].done != 0;
     if (all_done || launched >= budget) break;
   }
-  if (s->tuning.geo != 0) s->geo_valid = false;  // the inline split stores no geometry
   for (int i = 0; i < s->n; ++i) {
     int32_t status, site;
     decode(s->hst[i].status, &status, &site);
@@ -488,7 +479,6 @@ int lulesh_ens_set_tuning(lulesh_ensemble* s, const lulesh_tuning* t) {
   s->tuning.node = t->node_block;
   s->tuning.kin = t->kin_block;
   s->tuning.mat = t->mat_block;
-  if (s->tuning.geo != t->geometry) s->geo_valid = false;
   s->tuning.geo = t->geometry;
   drop_graph(s);
   return LULESH_OK;
@@ -502,7 +492,6 @@ int lulesh_ens_autotune(lulesh_ensemble* s, int32_t cycles, lulesh_tuning* chose
   if (rc) return rc;
   for (int i = 0; i < s->n; ++i) { s->hst[i] = s->init_state[i]; s->hst[i].first = 0; }
   ECK(cudaMemcpyAsync(s->dd.st, s->hst, sizeof(DevState) * s->n, cudaMemcpyHostToDevice, s->stream));
-  launch_geometry(s->dd, s->stream);
   ECK(autotune_blocks(s->dd, s->prm, false, s->n, s->stream, cycles, s->tuning));
   drop_graph(s);
   if ((rc = lulesh_ens_reset(s))) return rc;

@@ -121,9 +121,6 @@ constexpr unsigned long long kInfBits = 0x7FF0000000000000ull;
 constexpr unsigned long long kDtRegisterBits = 0x4415AF1D78B58C40ull;
 __host__ __device__ inline bool dt_registers(unsigned long long acc) { return acc < kDtRegisterBits; }
 
-// doubles per element of DevDomain::nextGeo
-constexpr int kGeoSlots = 51;
-
 // Pointers of one problem's device fields. Element arrays have E entries,
 // node arrays N; corner arrays 8E in corner-major order (c*E + e).
 // A block-partitioned mesh adds ghost slots: the delv arrays hold Eg >= E
@@ -154,12 +151,9 @@ struct DevDomain {
   // region batching (cost model only)
   int* regElemlist0;                          // E, 0-based element ids grouped by region
   int* regOfSlot;                             // E, region rep count per slot
-  // the force kernel's geometry of the current positions, [kGeoSlots][E]
-  // (formed by the kinematics kernel of the cycle before, or by k_geometry)
-  double* nextGeo;
   // taped runs: the next cycle's force tape, where the kinematics kernel (or
-  // k_geometry) writes the face normals of these positions, and at the start
-  // of a taped segment the buffer k_geometry writes their face diagonals to
+  // k_tape_geometry) writes the face normals of these positions, and at the start
+  // of a taped segment the buffer k_tape_geometry writes their face diagonals to
   double* tapeGeoNext;
   double* tapeDiag;
   // corner forces [8][E]

@@ -15,6 +15,7 @@
 // plus k_time_increment (timeIncrement!, src/domain.jl:920-961) for the
 // device-resident run loop.
 #include "lulesh_device.cuh"
+#include "lulesh_fixed_force.cuh"
 #include "lulesh_kernels.h"
 
 namespace lulesh {
@@ -29,21 +30,8 @@ __device__ __forceinline__ bool step_off(const DevState* st) {
 // ---------------------------------------------------------------------------
 // Element geometry at one set of positions
 // ---------------------------------------------------------------------------
-// The force kernel of a cycle sees the positions the kinematics kernel of
-// the cycle before it saw. So the kinematics kernel (or k_geometry, at the
-// start of a run and after the host changed the positions) forms what the
-// force kernel needs from the positions alone and stores it in d.nextGeo
-// ([kGeoSlots][E]), and the force kernel loads it instead of forming it
-// again. Both sides use the functions below, so a stored value is bitwise
-// the one the force kernel would form (the taping force kernel still forms
-// them, for its tape).
-//
-// d.nextGeo slots: 0..23 the volume derivatives of corner n, coordinate k
-// (8k + n, in corner order); 24..35 the hourglass modes of coordinate k
-// (24 + 4k + m, before the 1/(12 determ) scale); 36..47 the node normals of
-// corners 0..3 (36 + 4k + n, before node 0's quirk and the stress scale);
-// 48 and 49 face 0 + face 1's z normal and face 4's y normal (node 0's
-// quirk); 50 the Jacobian determinant of the detJ check.
+// The FP64 forms, of the elements the fixed-point arithmetic does not take
+// (lulesh_fixed.cuh) and of the tapes.
 
 // The 12 face diagonals, two per face in calcElemNodeNormals' argument order
 // p2 - p0, p3 - p1 (src/domain.jl:991-1067). Face f: (2,0,3,1) (5,0,1,4)
@@ -177,22 +165,6 @@ __device__ __forceinline__ void volume_derivatives(const double gU[3][3], const 
   }
 }
 
-__device__ __forceinline__ void store_geometry(double* geo, int E, int e, const double gr[3][8], const double hm[3][4],
-                                               const double B[3][4], double pz01, double ny4, double det) {
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-#pragma unroll
-    for (int n = 0; n < 8; ++n) geo[(8 * k + n) * E + e] = gr[k][n];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) geo[(24 + 4 * k + m) * E + e] = hm[k][m];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) geo[(36 + 4 * k + n) * E + e] = B[k][n];
-  }
-  geo[48 * E + e] = pz01;
-  geo[49 * E + e] = ny4;
-  geo[50 * E + e] = det;
-}
-
 // The force tape's face normals 0..4 of these positions (slots 48 + f,
 // 54 + f, 60 + f), read by the hourglass transpose.
 __device__ __forceinline__ void tape_force_normals(double* tape, int E, int e, const double n[6][3]) {
@@ -215,9 +187,7 @@ __device__ __forceinline__ void tape_diagonals(double* diag, int E, int e, const
     for (int k = 0; k < 3; ++k) diag[(3 * q + k) * E + e] = g[q][k];
 }
 
-// The force kernel's geometry of one element's positions, formed by the same
-// calls in the same order as k_geometry and k_kinematics, so the values are
-// bitwise those they store.
+// The force kernel's geometry of one element's positions.
 __device__ __forceinline__ void force_geometry(const double x[8], const double y[8], const double z[8],
                                                double gr[3][8], double hm[3][4], double B[3][4], double& pz01,
                                                double& ny4, double& det) {
@@ -232,10 +202,9 @@ __device__ __forceinline__ void force_geometry(const double x[8], const double y
   det = jacobian_det(w);
 }
 
-// The stored geometry of the current positions (see above): at the start of
-// a run, after the host changed the positions, and for the ensemble's reset;
-// in a taped run also the first cycle's face diagonals and normals.
-__global__ void __launch_bounds__(kMaxElemBlock) k_geometry(DevDomain d) {
+// At the start of a taped segment: the first cycle's face diagonals and
+// normals on their tapes (later cycles' come from the kinematics kernel).
+__global__ void __launch_bounds__(kMaxElemBlock) k_tape_geometry(DevDomain d) {
   const int E = d.E;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= E) return;
@@ -245,16 +214,10 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_geometry(DevDomain d) {
     const int nd = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, d.st);
     x[c] = LDG(&d.x[nd]); y[c] = LDG(&d.y[nd]); z[c] = LDG(&d.z[nd]);
   }
-  double g[12][3], w[3][3], hm[3][4], n[6][3], B[3][4], pz01, ny4;
-  double U[3][3], gU[3][3], gV[3][3], gW[3][3], gr[3][8];
+  double g[12][3], n[6][3];
   face_diagonals(x, y, z, g);
-  position_walsh(x, y, z, g, w, hm);
 #pragma unroll
   for (int f = 0; f < 5; ++f) face_normal(g, f, n[f]);
-  node_normals(n, B, pz01, ny4);
-  volume_terms(g, U, gU, gV, gW);
-  volume_derivatives(gU, gV, gW, gr);
-  store_geometry(d.nextGeo, E, e, gr, hm, B, pz01, ny4, jacobian_det(w));
   if (d.tapeGeoNext) tape_force_normals(d.tapeGeoNext, E, e, n);
   if (d.tapeDiag) tape_diagonals(d.tapeDiag, E, e, g);
 }
@@ -262,45 +225,33 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_geometry(DevDomain d) {
 // ---------------------------------------------------------------------------
 // k_force
 // ---------------------------------------------------------------------------
-// The geometry of the cycle's positions is loaded from d.nextGeo, or, with
-// GEO_INLINE (the other fusion split, chosen by the autotuner), formed here
-// from the positions (k_kinematics then stores none); the taping variant
-// loads it and adds the volume derivatives, scaled modes and mode sums to
-// the force tape (the diagonals and normals are there already).
-template <int MODE, bool ENS, bool TAPE, bool GEO_INLINE>
-__global__ void __launch_bounds__(kMaxElemBlock) k_force(DevDomain d, Params prm) {
-  const int E = d.E;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  const int inst = ENS ? LULESH_IDX(LDG(&d.elemInst[e]), d.ninst, d.st) : 0;
-  DevState* const st = d.st + inst;
-  if (step_off(st)) return;
-  const double hgcoef = ENS ? LDG(&d.instHg[inst]) : prm.hgcoef;
+// The taped volume derivatives, scaled modes and mode sums of an element.
+template <bool ON>
+struct ForceTape {
+  static constexpr bool on = ON;
+  double* p;  // d.tapeGeo at this element
+  int E;
+  bool live;
+  __device__ void put(int slot, double v) const { if (live) p[slot * E] = v; }
+  __device__ void derivative(int k, int n, double v) const { put(8 * k + n, v); }
+  __device__ void mode(int k, int m, double v) const { put(24 + 4 * k + m, v); }
+  __device__ void sum(int k, int m, double v) const { put(36 + 4 * k + m, v); }
+};
 
+// One element's corner forces in FP64: the elements the fixed-point form does
+// not take (thin, inverted or not finite; it also records the volume errors).
+template <int MODE, bool TAPE>
+__device__ __noinline__ void force_fp64(const DevDomain& d, DevState* st, int e, double hgcoef) {
+  const int E = d.E;
   int nd[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) nd[c] = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, st);
-
   double gr[3][8], hm[3][4], B[3][4], pz01, ny4, det;
-  if (GEO_INLINE) {
+  {
     double x[8], y[8], z[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) { x[c] = LDG(&d.x[nd[c]]); y[c] = LDG(&d.y[nd[c]]); z[c] = LDG(&d.z[nd[c]]); }
     force_geometry(x, y, z, gr, hm, B, pz01, ny4, det);
-  } else {
-    const double* geo = d.nextGeo;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-#pragma unroll
-      for (int n = 0; n < 8; ++n) gr[k][n] = LDG(&geo[(8 * k + n) * E + e]);
-#pragma unroll
-      for (int m = 0; m < 4; ++m) hm[k][m] = LDG(&geo[(24 + 4 * k + m) * E + e]);
-#pragma unroll
-      for (int n = 0; n < 4; ++n) B[k][n] = LDG(&geo[(36 + 4 * k + n) * E + e]);
-    }
-    pz01 = LDG(&geo[48 * E + e]);
-    ny4 = LDG(&geo[49 * E + e]);
-    det = LDG(&geo[50 * E + e]);
   }
   if (le_zero(det)) atomicOr(&st->status, ST_EARLY);
 
@@ -408,6 +359,71 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_force(DevDomain d, Params prm
   }
 }
 
+// Three threads per element, one per coordinate and each in a warp of its own:
+// a block is 32 elements (lulesh_fixed_force.cuh). Bound by the integer pipes
+// (multiply-adds, shifts and logic issue every other cycle and share them:
+// counters 59 % and 46 % of the cycles, no other pipe above 25 %): 0.90 ms per
+// cycle at 150^3, where FP64 took 1.98 ms with the geometry stored by
+// k_kinematics (0.87 ms of that kernel). Seven blocks per SM, 80 registers:
+// six (96 registers) 1.02 ms, five (128) 1.12 ms; below 45^3 the three are
+// alike.
+template <int MODE, bool ENS, bool TAPE>
+__global__ void __launch_bounds__(3 * kFixedElems, 7)
+    k_force(const __grid_constant__ DevDomain d, const __grid_constant__ Params prm) {
+  __shared__ fx::Num column[fx::FS_COUNT * kFixedElems];
+  const int E = d.E;
+  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  // threads past the end repeat the last element and store nothing
+  const int slot = blockIdx.x * kFixedElems + lane;
+  const int e = slot < E ? slot : E - 1;
+  const int inst = ENS ? LULESH_IDX(LDG(&d.elemInst[e]), d.ninst, d.st) : 0;
+  DevState* const st = d.st + inst;
+  const bool live = slot < E && !step_off(st);
+  const double hgcoef = ENS ? LDG(&d.instHg[inst]) : prm.hgcoef;
+  const fx::Slots sh{column + lane, kFixedElems};
+  fx::ForceLane r;
+  const ForceTape<TAPE> tape{TAPE ? d.tapeGeo + e : nullptr, E, live};
+  {
+    const double* const X = k == 0 ? d.x : k == 1 ? d.y : d.z;
+    const double* const U = k == 0 ? d.xd : k == 1 ? d.yd : d.zd;
+    double v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int nd = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, st);
+      r.x[c] = LDG(&X[nd]);
+      v[c] = LDG(&U[nd]);
+    }
+    if (k == 0) {
+      // determ^(-1/3) serves the coefficient (src/domain.jl:1605), its cube
+      // the modes' 1/(12 determ); a volume that is not positive takes neither
+      const double vol = LDG(&d.v[e]);
+      const double rc = inv_cbrt(LDG(&d.volo[e]) * vol);
+      const double coef = gt_zero(hgcoef) ? ((-hgcoef * 0.01) * LDG(&d.ss[e])) * LDG(&d.elemMass[e]) * rc : 0.0;
+      // (a taped element without hourglass forces leaves its tape as it is)
+      const bool take = gt_zero(vol) && !(TAPE && !gt_zero(hgcoef));
+      fx::force_scales(sh, take ? (rc * rc) * (rc * (1.0 / 12.0)) : 0.0, coef);
+    } else if (k == 1) {
+      fx::force_stress(sh, ((-LDG(&d.p[e])) - LDG(&d.q[e])) * 0.125);
+    }
+    fx::force_load(k, sh, v, r);
+  }
+  long long hm[4];
+  __syncthreads();
+  fx::force_diagonals(k, sh, r, hm);
+  __syncthreads();
+  fx::force_products<MODE>(k, sh, r, hm, tape);
+  __syncthreads();
+  fx::force_base(k, sh, r);
+  __syncthreads();
+  if (!live) return;
+  if (r.ok) {
+    double* const out = (k == 0 ? d.fcx : k == 1 ? d.fcy : d.fcz) + e;
+    fx::force_corners(k, sh, r, [&](int n, double f) { out[n * E] = f; }, tape);
+  } else if (k == 0) {
+    force_fp64<MODE, TAPE>(d, st, e, hgcoef);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // k_node
 // ---------------------------------------------------------------------------
@@ -458,9 +474,7 @@ __global__ void __launch_bounds__(kMaxNodeBlock) k_node(DevDomain d, Params prm)
 // ---------------------------------------------------------------------------
 // k_kinematics
 // ---------------------------------------------------------------------------
-// GEO: also store the next force kernel's geometry of these positions
-// (d.nextGeo); without it (the GEO_INLINE split) k_force forms it itself.
-template <bool AUX, bool ENS, bool TAPE, bool GEO>
+template <bool AUX, bool ENS, bool TAPE>
 __global__ void __launch_bounds__(kMaxElemBlock) k_kinematics(DevDomain d, Params prm) {
   const int E = d.E;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -481,8 +495,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_kinematics(DevDomain d, Param
   }
 
   // calcElemVolume (src/utils.jl:36-116) and calcElemCharacteristicLength
-  // (src/domain.jl:1874-1930) from the face diagonals; the next force
-  // kernel's geometry of these positions is stored too.
+  // (src/domain.jl:1874-1930) from the face diagonals.
   double volume, charLength = 0.0;
   double w[3][3];  // first-order Walsh vectors (xi, eta, zeta) of x, y, z
   double cet[3];   // W_zeta x W_xi
@@ -535,15 +548,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_kinematics(DevDomain d, Param
       // the next cycle's face normals, for its hourglass transpose
       if (d.tapeGeoNext) tape_force_normals(d.tapeGeoNext, E, e, n);
     }
-    if (GEO) {
-      double B[3][4], pz01, ny4, gr[3][8];
-      node_normals(n, B, pz01, ny4);
-      volume_derivatives(gU, gV, gW, gr);
-      eta_cofactors(w, cet);
-      store_geometry(d.nextGeo, E, e, gr, hm, B, pz01, ny4, jacobian_det(w, cet));
-    } else {
-      eta_cofactors(w, cet);
-    }
+    eta_cofactors(w, cet);
   }
   const double* wx = w[0];
   const double* wy = w[1];
@@ -662,6 +667,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_kinematics(DevDomain d, Param
     tape_a(1);
   }
 }
+
 
 // ---------------------------------------------------------------------------
 // k_material
@@ -1071,22 +1077,18 @@ __global__ void k_time_increment(DevState* st, int n, Params prm) {
 // ---------------------------------------------------------------------------
 // An ensemble (d.elemInst set) runs the ENS instantiations, which read each
 // element's or node's instance; the plain path runs ENS = false.
-void launch_geometry(const DevDomain& d, cudaStream_t s) {
+void launch_tape_geometry(const DevDomain& d, cudaStream_t s) {
   const int bs = 128;
-  k_geometry<<<(d.E + bs - 1) / bs, bs, 0, s>>>(d);
+  k_tape_geometry<<<(d.E + bs - 1) / bs, bs, 0, s>>>(d);
 }
 
-void launch_force(const DevDomain& d, const Params& prm, const Tuning& t, cudaStream_t s) {
-  const int bs = t.force;
-  const int grid = (d.E + bs - 1) / bs;
-  const bool ens = d.elemInst != nullptr;
-  const bool inl = t.geo != 0 && !d.tapeGeo;  // the taping kernels always use the stored geometry
-#define LULESH_FORCE(M)                                                                            \
-  (ens ? (inl ? k_force<M, true, false, true><<<grid, bs, 0, s>>>(d, prm)                          \
-              : k_force<M, true, false, false><<<grid, bs, 0, s>>>(d, prm))                        \
-       : d.tapeGeo ? k_force<M, false, true, false><<<grid, bs, 0, s>>>(d, prm)                    \
-                   : (inl ? k_force<M, false, false, true><<<grid, bs, 0, s>>>(d, prm)              \
-                          : k_force<M, false, false, false><<<grid, bs, 0, s>>>(d, prm)))
+void launch_force(const DevDomain& d, const Params& prm, cudaStream_t s) {
+  const int bs = 3 * kFixedElems;
+  const int grid = (d.E + kFixedElems - 1) / kFixedElems;
+#define LULESH_FORCE(M)                                                  \
+  (d.elemInst  ? k_force<M, true, false><<<grid, bs, 0, s>>>(d, prm)     \
+   : d.tapeGeo ? k_force<M, false, true><<<grid, bs, 0, s>>>(d, prm)     \
+               : k_force<M, false, false><<<grid, bs, 0, s>>>(d, prm))
   switch (d.mode & 3) {
     case 0: LULESH_FORCE(0); break;
     case 1: LULESH_FORCE(1); break;
@@ -1108,22 +1110,13 @@ void launch_node(const DevDomain& d, const Params& prm, bool aux, const Tuning& 
   else k_node<false, false><<<grid, bs, 0, s>>>(d, prm);
 }
 
-void launch_kinematics(const DevDomain& d, const Params& prm, bool aux, const Tuning& t, cudaStream_t s) {
-  const int bs = t.kin;
+void launch_kinematics(const DevDomain& d, const Params& prm, bool aux, cudaStream_t s) {
+  const int bs = 128;
   const int grid = (d.E + bs - 1) / bs;
-  const bool geo = t.geo == 0;
-  if (d.elemInst) {
-    if (geo) k_kinematics<false, true, false, true><<<grid, bs, 0, s>>>(d, prm);
-    else k_kinematics<false, true, false, false><<<grid, bs, 0, s>>>(d, prm);
-  } else if (d.tapeFlags) {
-    k_kinematics<false, false, true, true><<<grid, bs, 0, s>>>(d, prm);
-  } else if (aux) {
-    if (geo) k_kinematics<true, false, false, true><<<grid, bs, 0, s>>>(d, prm);
-    else k_kinematics<true, false, false, false><<<grid, bs, 0, s>>>(d, prm);
-  } else {
-    if (geo) k_kinematics<false, false, false, true><<<grid, bs, 0, s>>>(d, prm);
-    else k_kinematics<false, false, false, false><<<grid, bs, 0, s>>>(d, prm);
-  }
+  if (d.elemInst) k_kinematics<false, true, false><<<grid, bs, 0, s>>>(d, prm);
+  else if (d.tapeFlags) k_kinematics<false, false, true><<<grid, bs, 0, s>>>(d, prm);
+  else if (aux) k_kinematics<true, false, false><<<grid, bs, 0, s>>>(d, prm);
+  else k_kinematics<false, false, false><<<grid, bs, 0, s>>>(d, prm);
 }
 
 void launch_material(const DevDomain& d, const Params& prm, bool aux, const Tuning& t, cudaStream_t s) {

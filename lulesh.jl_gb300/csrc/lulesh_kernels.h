@@ -12,13 +12,15 @@ namespace lulesh {
 // 255 per thread either way), so the block size is a launch-time choice.
 constexpr int kMaxElemBlock = 256;
 constexpr int kMaxNodeBlock = 512;
+// Elements per block of the kernels that run one thread per element and
+// coordinate: a warp for each coordinate.
+constexpr int kFixedElems = 32;
 
 // Launch configuration chosen by the autotuner (defaults are the block sizes
-// that measured best for the 150^3 problem). `geo` is the fusion split of the
-// force geometry: 0 formed by k_kinematics of the cycle before and stored in
-// DevDomain::nextGeo (fewer FP64 instructions, 816 more bytes per element
-// and cycle), 1 formed inside k_force from the positions. Both give bitwise
-// the same results. The taping kernels of the adjoint always use 0.
+// that measured best for the 150^3 problem). `force`, `kin` and `geo` are the
+// caller's values of lulesh_tuning, kept for lulesh_get_tuning: k_force and
+// k_kinematics run blocks of 3 * kFixedElems threads, and the force geometry is
+// formed in k_force whatever `geo` says.
 struct Tuning {
   int force = 128;
   int node = 256;
@@ -27,12 +29,11 @@ struct Tuning {
   int geo = 0;
 };
 
-// k_geometry: the force kernel's geometry of the current positions (needed
-// before a step whenever the positions did not come from the last step).
-void launch_geometry(const DevDomain& d, cudaStream_t s);
-void launch_force(const DevDomain& d, const Params& prm, const Tuning& t, cudaStream_t s);
+// The first taped cycle's face diagonals and normals.
+void launch_tape_geometry(const DevDomain& d, cudaStream_t s);
+void launch_force(const DevDomain& d, const Params& prm, cudaStream_t s);
 void launch_node(const DevDomain& d, const Params& prm, bool aux, const Tuning& t, cudaStream_t s);
-void launch_kinematics(const DevDomain& d, const Params& prm, bool aux, const Tuning& t, cudaStream_t s);
+void launch_kinematics(const DevDomain& d, const Params& prm, bool aux, cudaStream_t s);
 void launch_material(const DevDomain& d, const Params& prm, bool aux, const Tuning& t, cudaStream_t s);
 void launch_time_increment(DevState* st, int n, const Params& prm, cudaStream_t s);
 

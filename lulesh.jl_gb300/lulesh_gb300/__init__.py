@@ -100,8 +100,8 @@ class Instance(ctypes.Structure):
 
 
 class Tuning(ctypes.Structure):
-    """lulesh_tuning: threads per block of the four step kernels and the
-    geometry split (0 stored by k_kinematics, 1 formed in k_force)."""
+    """lulesh_tuning: threads per block of the step kernels (force_block,
+    kin_block and geometry are kept and change nothing)."""
     _fields_ = [("force_block", ctypes.c_int32), ("node_block", ctypes.c_int32),
                 ("kin_block", ctypes.c_int32), ("mat_block", ctypes.c_int32),
                 ("geometry", ctypes.c_int32)]
