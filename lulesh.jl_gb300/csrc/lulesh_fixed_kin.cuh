@@ -1,0 +1,195 @@
+// Kinematics of one element (volume, characteristic length, velocity
+// divergence, monotonic-Q gradients; src/domain.jl:1874-2320) in the
+// fixed-point arithmetic of lulesh_fixed.cuh, by three threads, one per
+// coordinate, as lulesh_fixed_force.cuh does the forces.
+//
+// A thread converts its coordinate's positions and velocities, forms its
+// component of every cross product and its terms of every dot product; the
+// terms are added in shared memory and the roots and quotients, in FP64, are
+// divided among the three.
+#pragma once
+
+#include "lulesh_fixed.cuh"
+
+namespace lulesh {
+namespace fx {
+
+enum : int {
+  KS_GEO = 0,    // 18 k + q: limbs of diagonal q (12), mean edge (3), half-step edge (3) of coordinate k
+  KS_SUM = 0,    // kSums k + i: coordinate k's terms, over the diagonals once those are read
+  KS_DET = 54,   // k: a term of the Jacobian determinant
+  KS_EXT = 57,   // k: high words of the position and velocity extents
+  KS_MID = 60,   // 1/(64 volume), then the divergence's factor and the divergence
+  KS_COUNT = 63
+};
+// sums over the coordinates
+enum : int {
+  SUM_VOLUME = 0,  // 12 volume over 2^62
+  SUM_FACE = 1,    // 6: squared face vectors over 2^57, force order
+  SUM_AREA = 7,    // 3: squared cross products of the mean edges over 2^57
+  SUM_FLOW = 10,   // 3: those cross products times velocity differences over 2^59
+  SUM_RATE = 13,   // cofactors times velocity differences over 2^61
+  SUM_JAC = 14,    // half-step determinant over 2^59
+  kSums = 15
+};
+static_assert(3 * kSums <= 54, "the sums overlay the diagonals");
+
+// What a thread keeps over the phases: its components (unscaled integers) of
+// the face vectors, the volume's V x W, the edges' cross products, the
+// cofactors, and its velocity differences and edges.
+struct KinLane {
+  double x[8], v[8];
+  int s, sv;
+  bool ok_x, ok;  // positions taken; positions and velocities taken
+  i64 g[12], w[3], vw[3];
+  i64 n[6], gU[3], A[3], C[3];
+  Num half_eta;
+};
+
+// a^2 over 2^57; all four limb products, as the squares of the low limbs do
+// not average out
+LULESH_FX i64 square(Num a) {
+  const i64 h = mulw(a.hi, a.hi), m = mulw(a.hi, a.lo);
+  const u64 l = (u64)mulw(a.lo, a.lo);
+  return shl(h, 7) + ((m + (i64)(l >> 33)) >> 24);
+}
+
+// 1: r.x and r.v hold coordinate k's corner values.
+LULESH_FX void kin_extents(int k, Slots sh, const KinLane& r) {
+  Num m;
+  m.lo = (int)extent_hi(r.x);
+  m.hi = (int)extent_hi(r.v);
+  sh[KS_EXT + k] = m;
+}
+
+// 2: diagonals, mean edges, velocity differences and half-step edges (edge -
+// dt/2 velocity difference, half_dt = dt/2).
+LULESH_FX void kin_edges(int k, Slots sh, double half_dt, KinLane& r) {
+  const Num m0 = sh[KS_EXT], m1 = sh[KS_EXT + 1], m2 = sh[KS_EXT + 2];
+  const int ex = exponent_field(umax(umax((unsigned)m0.lo, (unsigned)m1.lo), (unsigned)m2.lo));
+  int ev = exponent_field(umax(umax((unsigned)m0.hi, (unsigned)m1.hi), (unsigned)m2.hi));
+  r.ok_x = ex >= kMinExtent && ex <= kMaxExtent;
+  const Float T = to_float(half_dt);
+  const bool wild = ev > kMaxSpeed;  // not finite, or far beyond any flow
+  ev = wild ? 0x7ff : imax(ev, kMinSpeed);
+  const int exs = r.ok_x ? ex : 0x7ff;
+  r.s = 1083 - exs;
+  r.sv = 1083 - ev;
+  // dt/2 in units of the edges over those of the velocities, T.m 2^tx: taken
+  // while corners move less than an eighth of the scale's 2^61
+  const int tx = T.k + r.s - r.sv;
+  r.ok = r.ok_x && !wild && tx <= -64 && exponent_field((unsigned)hi_word(half_dt)) != 0x7ff;
+  const Num tau = limbs(T.m >> (r.ok ? imin(-64 - tx, 63) : 63));
+  i64 c[8];
+  LULESH_UNROLL
+  for (int i = 0; i < 8; ++i) c[i] = to_fixed(r.x[i], 8 - exs);
+  diagonals(c, r.g);
+  walsh(c, r.w, nullptr);
+  LULESH_UNROLL
+  for (int i = 0; i < 8; ++i) c[i] = to_fixed(r.v[i], 8 - ev);
+  walsh(c, r.vw, nullptr);
+  const int at = KS_GEO + 18 * k;
+  LULESH_UNROLL
+  for (int q = 0; q < 12; ++q) sh[at + q] = limbs(r.g[q]);
+  LULESH_UNROLL
+  for (int a = 0; a < 3; ++a) {
+    sh[at + 12 + a] = limbs(r.w[a]);
+    const Num h = limbs(r.w[a] - product(limbs(r.vw[a]), tau));
+    sh[at + 15 + a] = h;
+    if (a == 1) r.half_eta = h;
+  }
+}
+
+// 3: component k of the cross products; i1, i2 the slots of the next two
+// coordinates. Reads the diagonals, so a barrier separates it from 4.
+LULESH_FX void kin_products(int k, Slots sh, KinLane& r) {
+  const int i1 = KS_GEO + 18 * (k == 2 ? 0 : k + 1), i2 = KS_GEO + 18 * (k == 0 ? 2 : k - 1);
+  auto cross_k = [&](int a, int b) {
+    return take<0>(mul_minus(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]));
+  };
+  LULESH_UNROLL
+  for (int f = 0; f < 6; ++f) r.n[f] = cross_k(2 * f, 2 * f + 1);
+  // V x W of the three products: (-g7, g0), (g10, -g9), (g4, g2)
+  r.gU[0] = cross_k(0, 7);
+  r.gU[1] = cross_k(9, 10);
+  r.gU[2] = cross_k(4, 2);
+  // eta x zeta, zeta x xi, xi x eta of the mean edges and of the half-step edges
+  r.A[0] = cross_k(13, 14);
+  r.A[1] = cross_k(14, 12);
+  r.A[2] = cross_k(12, 13);
+  r.C[0] = cross_k(16, 17);
+  r.C[1] = cross_k(17, 15);
+  r.C[2] = cross_k(15, 16);
+  sh.put(KS_DET + k, product(limbs(r.w[1]), limbs(r.A[1])));
+}
+
+// 4: coordinate k's terms of the sums.
+LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
+  const int at = KS_SUM + kSums * k;
+  {
+    Acc a = mul(limbs(r.g[1] + r.g[6]), limbs(r.gU[0]));
+    mac(a, limbs(r.g[8] + r.g[11]), limbs(r.gU[1]));
+    mac(a, limbs(r.g[3] + r.g[5]), limbs(r.gU[2]));
+    sh.put(at + SUM_VOLUME, take<2>(a));
+  }
+  LULESH_UNROLL
+  for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square(limbs(r.n[f])));
+  Acc rate;
+  LULESH_UNROLL
+  for (int d = 0; d < 3; ++d) {
+    const Num a = limbs(r.A[d]), u = limbs(r.vw[d]), c = limbs(r.C[d]);
+    sh.put(at + SUM_AREA + d, square(a));
+    // lo*lo too: the velocity difference along one direction can be far below
+    // the extent that sets the scale
+    Acc f = mul(a, u);
+    f.m = mad((int)(mulw(a.lo, u.lo) >> 32), one(), f.m);
+    sh.put(at + SUM_FLOW + d, take<5>(f));
+    if (d == 0) rate = mul(c, u);
+    else mac(rate, c, u);
+  }
+  sh.put(at + SUM_RATE, take<3>(rate));
+  sh.put(at + SUM_JAC, take<5>(mul(r.half_eta, limbs(r.C[1]))));
+}
+
+LULESH_FX i64 kin_sum(Slots sh, int i) {
+  return add(add(sh.get(KS_SUM + i), sh.get(KS_SUM + kSums + i)), sh.get(KS_SUM + 2 * kSums + i));
+}
+
+LULESH_FX i64 kin_determinant(Slots sh) { return sh.get(KS_DET) + sh.get(KS_DET + 1) + sh.get(KS_DET + 2); }
+
+// 5: whether the element is taken (by its determinant and volume too), and the
+// sums in FP64 with their true scales.
+LULESH_FX void kin_accept(Slots sh, KinLane& r) {
+  const bool det = kin_determinant(sh) >= kMinDet;
+  r.ok_x = r.ok_x && det;
+  r.ok = r.ok && det && kin_sum(sh, SUM_VOLUME) >= kMinDet << 4;
+}
+LULESH_FX double kin_volume12(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_VOLUME), 126 - 3 * r.s); }
+// the largest squared face vector and its place in the reference's face order
+// (0, 5, 1, 2, 3, 4 of the force order)
+LULESH_FX double kin_largest_face(Slots sh, const KinLane& r, int& place) {
+  i64 best = kin_sum(sh, SUM_FACE);
+  place = 0;
+  LULESH_UNROLL
+  for (int q = 1; q < 6; ++q) {
+    const i64 a = kin_sum(sh, SUM_FACE + (q == 1 ? 5 : q - 1));
+    if (a > best) {
+      best = a;
+      place = q;
+    }
+  }
+  return to_double(best, 185 - 4 * r.s);
+}
+LULESH_FX double kin_area(Slots sh, const KinLane& r, int d) {
+  return to_double(kin_sum(sh, SUM_AREA + d), 193 - 4 * r.s);
+}
+LULESH_FX double kin_flow(Slots sh, const KinLane& r, int d) {
+  return to_double(kin_sum(sh, SUM_FLOW + d), 129 - 2 * r.s - r.sv);
+}
+LULESH_FX double kin_rate(Slots sh, const KinLane& r) {
+  return to_double(kin_sum(sh, SUM_RATE), 131 - 2 * r.s - r.sv);
+}
+LULESH_FX double kin_jacobian(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_JAC), 129 - 3 * r.s); }
+
+}  // namespace fx
+}  // namespace lulesh

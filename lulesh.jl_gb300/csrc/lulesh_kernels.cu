@@ -16,6 +16,7 @@
 // device-resident run loop.
 #include "lulesh_device.cuh"
 #include "lulesh_fixed_force.cuh"
+#include "lulesh_fixed_kin.cuh"
 #include "lulesh_kernels.h"
 
 namespace lulesh {
@@ -203,23 +204,51 @@ __device__ __forceinline__ void force_geometry(const double x[8], const double y
 }
 
 // At the start of a taped segment: the first cycle's face diagonals and
-// normals on their tapes (later cycles' come from the kinematics kernel).
-__global__ void __launch_bounds__(kMaxElemBlock) k_tape_geometry(DevDomain d) {
+// normals on their tapes, by the phases of k_kinematics, which writes later
+// cycles' (so a segment's first cycle has the bits it has in mid-segment).
+__global__ void __launch_bounds__(3 * kFixedElems) k_tape_geometry(const __grid_constant__ DevDomain d) {
+  __shared__ fx::Num column[fx::KS_COUNT * kFixedElems];
   const int E = d.E;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  double x[8], y[8], z[8];
+  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  const int slot = blockIdx.x * kFixedElems + lane;
+  const int e = slot < E ? slot : E - 1;
+  const fx::Slots sh{column + lane, kFixedElems};
+  fx::KinLane r;
+  const double* const X = k == 0 ? d.x : k == 1 ? d.y : d.z;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    const int nd = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, d.st);
-    x[c] = LDG(&d.x[nd]); y[c] = LDG(&d.y[nd]); z[c] = LDG(&d.z[nd]);
+    r.x[c] = LDG(&X[LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, d.st)]);
+    r.v[c] = 0.0;
   }
-  double g[12][3], n[6][3];
-  face_diagonals(x, y, z, g);
+  fx::kin_extents(k, sh, r);
+  __syncthreads();
+  fx::kin_edges(k, sh, 0.0, r);
+  __syncthreads();
+  fx::kin_products(k, sh, r);
+  __syncthreads();
+  const bool taken = r.ok_x && fx::kin_determinant(sh) >= fx::kMinDet;
+  if (slot >= E) return;
+  if (taken) {
+    if (d.tapeGeoNext)
 #pragma unroll
-  for (int f = 0; f < 5; ++f) face_normal(g, f, n[f]);
-  if (d.tapeGeoNext) tape_force_normals(d.tapeGeoNext, E, e, n);
-  if (d.tapeDiag) tape_diagonals(d.tapeDiag, E, e, g);
+      for (int f = 0; f < 5; ++f) d.tapeGeoNext[(48 + 6 * k + f) * E + e] = fx::to_double(r.n[f], 64 - 2 * r.s);
+    if (d.tapeDiag)
+#pragma unroll
+      for (int q = 0; q < 12; ++q) d.tapeDiag[(3 * q + k) * E + e] = fx::to_double(r.g[q], -r.s);
+  } else if (k == 0) {
+    double x[8], y[8], z[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int nd = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, d.st);
+      x[c] = LDG(&d.x[nd]); y[c] = LDG(&d.y[nd]); z[c] = LDG(&d.z[nd]);
+    }
+    double g[12][3], n[6][3];
+    face_diagonals(x, y, z, g);
+#pragma unroll
+    for (int f = 0; f < 5; ++f) face_normal(g, f, n[f]);
+    if (d.tapeGeoNext) tape_force_normals(d.tapeGeoNext, E, e, n);
+    if (d.tapeDiag) tape_diagonals(d.tapeDiag, E, e, g);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -474,15 +503,12 @@ __global__ void __launch_bounds__(kMaxNodeBlock) k_node(DevDomain d, Params prm)
 // ---------------------------------------------------------------------------
 // k_kinematics
 // ---------------------------------------------------------------------------
-template <bool AUX, bool ENS, bool TAPE>
-__global__ void __launch_bounds__(kMaxElemBlock) k_kinematics(DevDomain d, Params prm) {
+// One element in FP64: what the fixed-point form does not take (thin,
+// inverted or not finite elements; it records the volume error). `geometry`:
+// the tapes of the positions are this function's too.
+template <bool AUX, bool TAPE>
+__device__ __noinline__ void kin_fp64(const DevDomain& d, DevState* st, int e, double dt, bool geometry) {
   const int E = d.E;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  DevState* const st = d.st + (ENS ? LULESH_IDX(LDG(&d.elemInst[e]), d.ninst, d.st) : 0);
-  if (step_off(st)) return;
-  const double dt = st->deltatime;
-
   int nd[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) nd[c] = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, st);
@@ -546,7 +572,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_kinematics(DevDomain d, Param
       d.tapeFlags[e] = (unsigned long long)fidx << TF_FACE_SHIFT;
       d.tapeKin[41 * E + e] = fcx; d.tapeKin[42 * E + e] = fcy; d.tapeKin[43 * E + e] = fcz;
       // the next cycle's face normals, for its hourglass transpose
-      if (d.tapeGeoNext) tape_force_normals(d.tapeGeoNext, E, e, n);
+      if (d.tapeGeoNext && geometry) tape_force_normals(d.tapeGeoNext, E, e, n);
     }
     eta_cofactors(w, cet);
   }
@@ -668,6 +694,137 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_kinematics(DevDomain d, Param
   }
 }
 
+
+// Three threads per element as in k_force (lulesh_fixed_kin.cuh). Bound by the
+// integer pipes: 0.57 ms per cycle at 150^3 (FP64: 1.93 ms without the force
+// geometry). Eight blocks per SM, 80 registers: six (96) 0.67 ms, five (128)
+// 0.77 ms.
+template <bool AUX, bool ENS, bool TAPE>
+__global__ void __launch_bounds__(3 * kFixedElems, 8)
+    k_kinematics(const __grid_constant__ DevDomain d, const __grid_constant__ Params prm) {
+  __shared__ fx::Num column[fx::KS_COUNT * kFixedElems];
+  const int E = d.E;
+  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  // threads past the end repeat the last element and store nothing
+  const int slot = blockIdx.x * kFixedElems + lane;
+  const int e = slot < E ? slot : E - 1;
+  DevState* const st = d.st + (ENS ? LULESH_IDX(LDG(&d.elemInst[e]), d.ninst, d.st) : 0);
+  const bool live = slot < E && !step_off(st);
+  const double dt = st->deltatime;
+  const fx::Slots sh{column + lane, kFixedElems};
+  fx::KinLane r;
+  {
+    const double* const X = k == 0 ? d.x : k == 1 ? d.y : d.z;
+    const double* const U = k == 0 ? d.xd : k == 1 ? d.yd : d.zd;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int nd = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, st);
+      r.x[c] = LDG(&X[nd]);
+      r.v[c] = LDG(&U[nd]);
+    }
+  }
+  fx::kin_extents(k, sh, r);
+  __syncthreads();
+  fx::kin_edges(k, sh, 0.5 * dt, r);
+  __syncthreads();
+  fx::kin_products(k, sh, r);
+  __syncthreads();
+  fx::kin_terms(k, sh, r);
+  __syncthreads();
+  fx::kin_accept(sh, r);
+  // The quotients: each thread forms the volume; coordinate 1 the divergence
+  // and 1/(64 volume), both from one division, coordinate 0 the volume's
+  // change and the characteristic length.
+  const double volume = fx::kin_volume12(sh, r) * (1.0 / 12.0);
+  const double vnew = volume * LDG(&d.inv_volo[e]);
+  const double volq = LDG(&d.volo[e]) * vnew;
+  int face = 0;
+  double rcl = 0.0;
+  auto kin_tape = [&](int slot_, double v) { d.tapeKin[slot_ * E + e] = v; };
+  if (r.ok) {
+    if (k == 1) {
+      const double q64 = fma(64.0, volq, 64.0 * 1.e-36);
+      double inv, norm64;
+      recip2(fx::kin_jacobian(sh, r), q64, inv, norm64);
+      const double vdov = fx::kin_rate(sh, r) * inv;
+      if (live) d.vdov[e] = vdov;
+      sh.put(fx::KS_MID, __double_as_longlong(norm64));
+      if (AUX) {
+        sh.put(fx::KS_MID + 1, __double_as_longlong(inv));
+        sh.put(fx::KS_MID + 2, __double_as_longlong(vdov));
+      }
+      if (TAPE && live) {
+        kin_tape(27, inv);
+        kin_tape(40, norm64);
+      }
+    } else if (k == 0) {
+      // 4*volume/sqrt(max area) with area = 4*|face vector|^2
+      // (src/domain.jl:1874-1930)
+      rcl = rsqrt(fx::kin_largest_face(sh, r, face));
+      if (live) {
+        if (le_zero(vnew)) atomicOr(&st->status, ST_KINEMATICS);
+        d.vnew[e] = vnew;
+        d.delv[e] = vnew - LDG(&d.v[e]);
+        d.arealg[e] = (2.0 * volume) * rcl;
+      }
+      if (TAPE) sh.put(fx::KS_MID + 1, face);
+    }
+  }
+  __syncthreads();
+  if (!live) return;
+  if (r.ok) {
+    // coordinate k also takes direction k (xi, eta, zeta) of the monotonic-Q
+    // gradients (src/domain.jl:2175-2320): with the reference's dxi = W_xi/4
+    // etc., delx = 16*vol/sqrt(|A|^2 + 256*ptiny) and delv = norm/64 *
+    // (A . W(v)) for the cross product A of two Walsh vectors (of the size the
+    // fixed-point form takes, |A|^2 is far above 256*ptiny = 2.56e-34)
+    double* const delx = k == 0 ? d.delx_xi : k == 1 ? d.delx_eta : d.delx_zeta;
+    double* const delv = k == 0 ? d.delv_xi : k == 1 ? d.delv_eta : d.delv_zeta;
+    const double norm64 = __longlong_as_double(sh.get(fx::KS_MID));
+    const double rs = rsqrt(fx::kin_area(sh, r, k));
+    delx[e] = (16.0 * volq) * rs;
+    delv[e] = norm64 * fx::kin_flow(sh, r, k);
+    if (AUX) {
+      double* const dd = k == 0 ? d.dxx : k == 1 ? d.dyy : d.dzz;
+      const double inv = __longlong_as_double(sh.get(fx::KS_MID + 1));
+      const double vdov = __longlong_as_double(sh.get(fx::KS_MID + 2));
+      const double own = fx::to_double(sh.get(fx::KS_SUM + fx::kSums * k + fx::SUM_RATE), 131 - 2 * r.s - r.sv);
+      dd[e] = own * inv - vdov / 3.0;
+    }
+    if (TAPE) {
+      kin_tape(37 + k, rs);
+      if (k == 0) kin_tape(44, rcl);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        kin_tape(3 * k + a, fx::to_double(r.w[a], 2 - r.s));
+        kin_tape(9 + 3 * k + a, fx::to_double(r.vw[a], 2 - r.sv));
+        kin_tape(18 + 3 * a + k, fx::to_double(r.C[a], 68 - 2 * r.s));
+        kin_tape(28 + 3 * a + k, fx::to_double(r.A[a], 68 - 2 * r.s));
+        kin_tape(81 + 3 * a + k, fx::to_double(r.gU[a], 64 - 2 * r.s));
+      }
+      // the 12 diagonals in the order d61 d70 d63 d20 d50 d64 d31 d72 d43 d57
+      // d14 d25 (force-order index, sign)
+      constexpr int gi[12] = {4, 9, 7, 0, 2, 10, 1, 6, 8, 11, 3, 5};
+#pragma unroll
+      for (int q = 0; q < 12; ++q)
+        kin_tape(45 + 3 * q + k, fx::to_double(q == 1 || q == 2 ? -r.g[gi[q]] : r.g[gi[q]], -r.s));
+      // the largest face's cross product in the reference's face order, the
+      // last two faces with reversed diagonals
+      const int place = (int)sh.get(fx::KS_MID + 1);
+      const long long c = place == 0 ? r.n[0] : place == 1 ? r.n[5] : place == 2 ? r.n[1] : place == 3 ? r.n[2]
+                                          : place == 4 ? -r.n[3] : -r.n[4];
+      kin_tape(41 + k, fx::to_double(c, 64 - 2 * r.s));
+      if (k == 0) d.tapeFlags[e] = (unsigned long long)place << TF_FACE_SHIFT;
+    }
+  } else if (k == 0) {
+    kin_fp64<AUX, TAPE>(d, st, e, dt, !r.ok_x);
+  }
+  if (TAPE && d.tapeGeoNext && r.ok_x) {
+    // the next cycle's face normals, for its hourglass transpose
+#pragma unroll
+    for (int f = 0; f < 5; ++f) d.tapeGeoNext[(48 + 6 * k + f) * E + e] = fx::to_double(r.n[f], 64 - 2 * r.s);
+  }
+}
 
 // ---------------------------------------------------------------------------
 // k_material
@@ -1078,8 +1235,7 @@ __global__ void k_time_increment(DevState* st, int n, Params prm) {
 // An ensemble (d.elemInst set) runs the ENS instantiations, which read each
 // element's or node's instance; the plain path runs ENS = false.
 void launch_tape_geometry(const DevDomain& d, cudaStream_t s) {
-  const int bs = 128;
-  k_tape_geometry<<<(d.E + bs - 1) / bs, bs, 0, s>>>(d);
+  k_tape_geometry<<<(d.E + kFixedElems - 1) / kFixedElems, 3 * kFixedElems, 0, s>>>(d);
 }
 
 void launch_force(const DevDomain& d, const Params& prm, cudaStream_t s) {
@@ -1111,8 +1267,8 @@ void launch_node(const DevDomain& d, const Params& prm, bool aux, const Tuning& 
 }
 
 void launch_kinematics(const DevDomain& d, const Params& prm, bool aux, cudaStream_t s) {
-  const int bs = 128;
-  const int grid = (d.E + bs - 1) / bs;
+  const int bs = 3 * kFixedElems;
+  const int grid = (d.E + kFixedElems - 1) / kFixedElems;
   if (d.elemInst) k_kinematics<false, true, false><<<grid, bs, 0, s>>>(d, prm);
   else if (d.tapeFlags) k_kinematics<false, false, true><<<grid, bs, 0, s>>>(d, prm);
   else if (aux) k_kinematics<true, false, false><<<grid, bs, 0, s>>>(d, prm);

@@ -3,6 +3,7 @@
 // run, compared with 113-bit floating point, where every product and sum of
 // these expressions is exact or rounded far below the bounds tested.
 #include "../lulesh.jl_gb300/csrc/lulesh_fixed_force.cuh"
+#include "../lulesh.jl_gb300/csrc/lulesh_fixed_kin.cuh"
 
 #include <cmath>
 #include <cstdlib>
@@ -177,6 +178,107 @@ void check_forces(int mode, int n, const double* pos, const double* vel, const d
     }
     const double scale[4] = {std::fabs(s8) * E * E + std::fabs(coef) * dV, E * E, E * vi12, dV};
     for (int j = 0; j < 4; ++j) err[4 * i + j] = e[j] == 0 ? 0.0 : (double)(e[j] / (Q)scale[j]);
+  }
+}
+
+// Kinematics sums of n elements (pos, vel: [n][3][8]) at half step half_dt.
+// Per element, taken, and err[13 i + j]: errors over the sums' scales (E, dV
+// the largest corner extents): 12 volume over E^3, the largest squared face
+// vector over E^4, the squared edge cross products over 256 E^4 (3), their
+// products with the velocity differences over 64 E^2 dV (3), the cofactor sum
+// over 64 E^2 dV, the half-step determinant over 64 E^3; and of 12 volume and
+// the determinant over their own size; then the largest face's place.
+void check_kinematics(int n, const double* pos, const double* vel, double half_dt, int* taken, double* err) {
+  for (int i = 0; i < n; ++i) {
+    const double(*p)[8] = reinterpret_cast<const double(*)[8]>(pos + 24 * i);
+    const double(*v)[8] = reinterpret_cast<const double(*)[8]>(vel + 24 * i);
+    Num column[KS_COUNT];
+    const Slots sh{column, 1};
+    KinLane r[3];
+    for (int k = 0; k < 3; ++k) {
+      for (int c = 0; c < 8; ++c) {
+        r[k].x[c] = p[k][c];
+        r[k].v[c] = v[k][c];
+      }
+      kin_extents(k, sh, r[k]);
+    }
+    for (int k = 0; k < 3; ++k) kin_edges(k, sh, half_dt, r[k]);
+    for (int k = 0; k < 3; ++k) kin_products(k, sh, r[k]);
+    for (int k = 0; k < 3; ++k) kin_terms(k, sh, r[k]);
+    for (int k = 0; k < 3; ++k) kin_accept(sh, r[k]);
+    if (r[0].ok != r[1].ok || r[0].ok != r[2].ok) std::abort();
+    taken[i] = r[0].ok;
+    if (!taken[i]) continue;
+    int place;
+    const double got[10] = {kin_volume12(sh, r[0]), kin_largest_face(sh, r[0], place),
+                            kin_area(sh, r[0], 0), kin_area(sh, r[0], 1), kin_area(sh, r[0], 2),
+                            kin_flow(sh, r[0], 0), kin_flow(sh, r[0], 1), kin_flow(sh, r[0], 2),
+                            kin_rate(sh, r[0]), kin_jacobian(sh, r[0])};
+    Q want[10];
+    auto d = [&](int k, int a, int b) { return (Q)p[k][a] - p[k][b]; };
+    static const int tv[3][8] = {{3, 1, 7, 2, 6, 3, 2, 0}, {4, 3, 5, 7, 6, 4, 7, 0}, {1, 4, 2, 5, 6, 1, 5, 0}};
+    want[0] = 0;
+    for (int t = 0; t < 3; ++t) {
+      Q U[3], V[3], W[3], c[3];
+      for (int k = 0; k < 3; ++k) {
+        U[k] = d(k, tv[t][0], tv[t][1]) + d(k, tv[t][2], tv[t][3]);
+        V[k] = d(k, tv[t][4], tv[t][5]);
+        W[k] = d(k, tv[t][6], tv[t][7]);
+      }
+      qcross(V, W, c);
+      want[0] += U[0] * c[0] + U[1] * c[1] + U[2] * c[2];
+    }
+    static const int fd[6][4] = {{2, 0, 3, 1}, {6, 4, 5, 7}, {5, 0, 1, 4}, {6, 1, 2, 5}, {7, 2, 3, 6}, {4, 3, 0, 7}};
+    want[1] = 0;
+    Q face[6];
+    for (int q = 0; q < 6; ++q) {
+      Q a[3], b[3], c[3];
+      for (int k = 0; k < 3; ++k) {
+        a[k] = d(k, fd[q][0], fd[q][1]);
+        b[k] = d(k, fd[q][2], fd[q][3]);
+      }
+      qcross(a, b, c);
+      face[q] = c[0] * c[0] + c[1] * c[1] + c[2] * c[2];
+      if (face[q] > want[1]) want[1] = face[q];
+    }
+    Q w[3][3], u[3][3], h[3][3];  // [direction][coordinate]
+    static const int sg[3][8] = {{-1, 1, 1, -1, -1, 1, 1, -1}, {-1, -1, 1, 1, -1, -1, 1, 1}, {-1, -1, -1, -1, 1, 1, 1, 1}};
+    for (int a = 0; a < 3; ++a)
+      for (int k = 0; k < 3; ++k) {
+        w[a][k] = u[a][k] = 0;
+        for (int c = 0; c < 8; ++c) {
+          w[a][k] += sg[a][c] * (Q)p[k][c];
+          u[a][k] += sg[a][c] * (Q)v[k][c];
+        }
+        h[a][k] = w[a][k] - (Q)half_dt * u[a][k];
+      }
+    want[8] = 0;
+    for (int a = 0; a < 3; ++a) {
+      Q A[3], C[3];
+      qcross(w[(a + 1) % 3], w[(a + 2) % 3], A);
+      qcross(h[(a + 1) % 3], h[(a + 2) % 3], C);
+      want[2 + a] = A[0] * A[0] + A[1] * A[1] + A[2] * A[2];
+      want[5 + a] = A[0] * u[a][0] + A[1] * u[a][1] + A[2] * u[a][2];
+      want[8] += C[0] * u[a][0] + C[1] * u[a][1] + C[2] * u[a][2];
+      if (a == 1) want[9] = C[0] * h[1][0] + C[1] * h[1][1] + C[2] * h[1][2];
+    }
+    double E = 0, dV = 0;
+    for (int k = 0; k < 3; ++k)
+      for (int c = 0; c < 8; ++c)
+        for (int b = 0; b < 8; ++b) {
+          E = std::fmax(E, p[k][c] - p[k][b]);
+          dV = std::fmax(dV, v[k][c] - v[k][b]);
+        }
+    const Q E2 = (Q)E * E, flow = 64 * E2 * dV;
+    const Q scale[10] = {E2 * E, E2 * E2, 256 * E2 * E2, 256 * E2 * E2, 256 * E2 * E2, flow, flow, flow, flow, 64 * E2 * E};
+    for (int j = 0; j < 10; ++j) {
+      const Q e = qabs((Q)got[j] - want[j]);
+      err[13 * i + j] = e == 0 ? 0.0 : (double)(e / scale[j]);
+    }
+    err[13 * i + 10] = (double)(qabs((Q)got[0] - want[0]) / qabs(want[0]));
+    err[13 * i + 11] = (double)(qabs((Q)got[9] - want[9]) / qabs(want[9]));
+    // how far the chosen face is from the largest
+    err[13 * i + 12] = (double)((want[1] - face[place]) / want[1]);
   }
 }
 

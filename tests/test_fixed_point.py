@@ -1,4 +1,4 @@
-"""The fixed-point element arithmetic of the force kernel
+"""The fixed-point element arithmetic of the force and kinematics kernels
 (lulesh_fixed*.cuh), the kernels' own functions compiled for the host, against
 113-bit floating point.
 
@@ -54,7 +54,13 @@ def lib(tmp_path_factory):
         L.check_forces(mode, n, _ptr(pos), _ptr(vel), _ptr(scal), _ptr(taken), _ptr(f), _ptr(err))
         return taken.astype(bool), f, err
 
-    L.forces = forces
+    def kinematics(pos, vel, half_dt):
+        n = len(pos)
+        taken, err = np.zeros(n, np.int32), np.zeros((n, 13))
+        L.check_kinematics(n, _ptr(pos), _ptr(vel), ctypes.c_double(half_dt), _ptr(taken), _ptr(err))
+        return taken.astype(bool), err
+
+    L.forces, L.kinematics = forces, kinematics
     return L
 
 
@@ -111,6 +117,33 @@ def test_forces_without_parts(lib):
     assert np.array_equal(lib.forces(0, pos, still, scal)[1], lib.forces(0, pos, still, s)[1])
 
 
+@pytest.mark.parametrize("h", [1.125 / 640, 1.125 / 150, 2.0 ** -7, 0.3, 40.0])
+@pytest.mark.parametrize("jitter,squash,shear", [(0, 1, 0), (1e-9, 1, 0), (0.05, 1, 0), (0.2, 0.6, 0.4), (0.02, 0.2, 0)])
+def test_kinematics(lib, h, jitter, squash, shear):
+    pos, vel, _ = _elements(5, 400, h, jitter, squash, shear)
+    for half_dt in (0.0, h * 1e-6, h * 0.01):
+        taken, err = lib.kinematics(pos, vel, half_dt)
+        assert taken.all() if squash == 1 else taken.any()
+        err = err[taken]
+        assert np.all(err[:, 0] <= 2.0 ** -48) and np.all(err[:, 1:5] <= 2.0 ** -49)
+        assert np.all(err[:, 5:9] <= 2.0 ** -49) and np.all(err[:, 9] <= 2.0 ** -47)
+        assert np.all(err[:, 10] <= 2.0 ** -47) and np.all(err[:, 12] <= 2.0 ** -48)
+
+
+@pytest.mark.parametrize("squash", [0.5, 0.25, 0.125, 0.06, 0.03, 0.015, 0.007])
+def test_thin_elements_are_taken_with_full_accuracy_or_not_at_all(lib, squash):
+    """Over extents through an octave, an element is either left to the FP64
+    form or its volume is good to 2^-47 of itself."""
+    some = 0
+    for h in np.exp2(np.linspace(-7, -6, 9)):
+        pos, vel, scal = _elements(6, 100, h, 0.02 * squash, squash, 0.3)
+        taken, err = lib.kinematics(pos, vel, h * 1e-4)
+        also = lib.forces(0, pos, vel, scal)[0]
+        assert np.all(err[taken][:, 10] <= 2.0 ** -47)
+        some += int(taken.sum()) + int(also.sum())
+    assert some == 0 if squash < 0.01 else some > 0 if squash > 0.1 else True
+
+
 def test_what_is_not_taken(lib):
     """Inverted, flat, tiny, huge and non-finite elements, wild scalars and
     velocities, a step that moves corners by more than the element."""
@@ -128,8 +161,12 @@ def test_what_is_not_taken(lib):
     vel_bad[8, 0, 0] = np.nan
     vel_bad[9, 1, 5] = -np.inf
     vel_bad[10, 2, 5] = 1e140
+    taken, _ = lib.kinematics(bad, vel_bad, 1e-6)
+    assert taken.tolist() == [False] * 11 + [True]
     taken, _, _ = lib.forces(0, bad, vel_bad, scal)
     assert taken.tolist() == [False] * 11 + [True]
+    assert not lib.kinematics(pos, vel, 0.1)[0].any()  # corners move by half a volume's edge and more
+    assert not lib.kinematics(pos, vel, np.nan)[0].any()
     for col, v in ((0, 0.0), (0, -1.0), (0, np.inf), (0, np.nan), (0, 1e-200), (1, np.nan), (1, np.inf), (1, 1e-200),
                    (2, np.nan), (2, -np.inf), (2, 1e200)):
         s = scal.copy()
