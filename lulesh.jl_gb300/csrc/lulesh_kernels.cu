@@ -830,103 +830,122 @@ __global__ void __launch_bounds__(3 * kFixedElems, 8)
 // k_material
 // ---------------------------------------------------------------------------
 
-// One limiter direction, src/domain.jl:2330-2376. `src` reports which value
-// the result is (PHI_*), for the adjoint's tape.
-__device__ __forceinline__ double monoq_phi(double norm, double dm, double dp, const Params& prm, int& src,
-                                            double& t_norm, double& t_dm, double& t_dp) {
-  // norm = 1 / (delv + ptiny) of this direction
-  dm *= norm;
-  dp *= norm;
-  t_norm = norm; t_dm = dm; t_dp = dp;  // kept for the adjoint's tape
-  double phi = 0.5 * (dm + dp);
+// One limiter direction, src/domain.jl:2330-2376, in units of 2 (delv + ptiny):
+// hn = 1 / (2 (delv + ptiny)), dm and dp the neighbours' values, mult2 twice
+// the limiter's multiplier. The comparisons are made before the quotient, with
+// its sign moved to dm and dp, so one product forms the result instead of two
+// and a half. `src` reports which value it is (PHI_*), for the adjoint's tape.
+__device__ __forceinline__ double monoq_phi(double hn, double dm, double dp, const Params& prm, int& src) {
+  const long long sign = __double_as_longlong(hn) & (long long)0x8000000000000000ull;
+  dm = __longlong_as_double(__double_as_longlong(dm) ^ sign);
+  dp = __longlong_as_double(__double_as_longlong(dp) ^ sign);
+  double f = dm + dp;
   src = PHI_MEAN;
-  dm *= prm.monoq_limiter_mult;
-  dp *= prm.monoq_limiter_mult;
+  dm *= prm.monoq_mult2;
+  dp *= prm.monoq_mult2;
   // the comparisons on the integer keys (fkey), with IEEE's outcomes
-  long long kphi = fkey(phi);
+  long long kf = fkey(f);
   const long long km = fkey(dm), kp = fkey(dp);
-  if (km < kphi) { phi = dm; kphi = km; src = PHI_M; }
-  if (kp < kphi) { phi = dp; kphi = kp; src = PHI_P; }
+  if (km < kf) { f = dm; kf = km; src = PHI_M; }
+  if (kp < kf) { f = dp; src = PHI_P; }
+  double phi = f * fabs(hn);
+  long long kphi = fkey(phi);
   if (kphi < 0) { phi = 0.0; kphi = 0; src = PHI_ZERO; }
   if (kphi > prm.k_max_slope) { phi = prm.monoq_max_slope; src = PHI_MAX; }
   return phi;
 }
 
-// Neighbour value for one face of the limiter (the four BC cases).
-__device__ __forceinline__ double monoq_neighbour(const double* dv, unsigned mask, unsigned bits,
-                                                  unsigned symm, unsigned freeb, unsigned comm,
-                                                  int idx, int self, int E, bool& bad) {
+// Element whose value one face of the limiter reads (the four BC cases); -1
+// for the value 0.
+__device__ __forceinline__ int monoq_neighbour(unsigned mask, unsigned bits, unsigned symm, unsigned freeb,
+                                               unsigned comm, int idx, int self, int E, bool& bad) {
   const unsigned c = mask & bits;
   if (c == 0u || c == comm) {
-    if (idx < 0 || idx >= E) { bad = true; return 0.0; }
-    return LDG(&dv[idx]);
+    if (idx < 0 || idx >= E) { bad = true; return -1; }
+    return idx;
   }
-  if (c == symm) return LDG(&dv[self]);
-  if (c == freeb) return 0.0;
-  bad = true;
-  return 0.0;
+  if (c == symm) return self;
+  if (c != freeb) bad = true;
+  return -1;
 }
 
-__device__ __forceinline__ void block_min2(unsigned long long a, unsigned long long b,
-                                           unsigned long long* ga, unsigned long long* gb) {
-  __shared__ unsigned long long sa[32], sb[32];
+// The time constraints of a set of elements: the least Courant candidate (bits
+// of a non-negative double) and the largest |vdov| (likewise). The hydro
+// constraint dvovmax / (|vdov| + 1e-20) (src/domain.jl:3022-3054) falls with
+// |vdov|, and its rounding with it, so the set's least is that of its largest
+// |vdov|: one division for the set.
+struct Limits {
+  unsigned long long courant, rate;
+};
+__device__ __forceinline__ void merge(Limits& a, unsigned long long courant, unsigned long long rate) {
+  a.courant = courant < a.courant ? courant : a.courant;
+  a.rate = rate > a.rate ? rate : a.rate;
+}
+__device__ __forceinline__ void warp_merge(Limits& a) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long ta = __shfl_xor_sync(0xffffffffu, a, o);
-    const unsigned long long tb = __shfl_xor_sync(0xffffffffu, b, o);
-    a = ta < a ? ta : a;
-    b = tb < b ? tb : b;
+    const unsigned long long c = __shfl_xor_sync(0xffffffffu, a.courant, o);
+    const unsigned long long r = __shfl_xor_sync(0xffffffffu, a.rate, o);
+    merge(a, c, r);
   }
+}
+__device__ __forceinline__ double hydro_limit(double rate, const Params& prm) {
+  return prm.dvovmax / (rate + 1.e-20);
+}
+__device__ __forceinline__ void register_limits(const Limits& a, DevState* st, const Params& prm) {
+  if (a.courant != kInfBits) atomicMin(&st->acc_courant, a.courant);
+  if (a.rate != 0ull) {
+    const double h = hydro_limit(__longlong_as_double((long long)a.rate), prm);
+    atomicMin(&st->acc_hydro, (unsigned long long)__double_as_longlong(h));
+  }
+}
+
+// Every thread of the block must call this.
+__device__ __forceinline__ void block_limits(Limits a, DevState* st, const Params& prm) {
+  __shared__ Limits part[32];
+  warp_merge(a);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) { sa[w] = a; sb[w] = b; }
+  if (l == 0) part[w] = a;
   __syncthreads();
   if (w == 0) {
     const int nw = blockDim.x >> 5;
-    a = l < nw ? sa[l] : kInfBits;
-    b = l < nw ? sb[l] : kInfBits;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long ta = __shfl_xor_sync(0xffffffffu, a, o);
-      const unsigned long long tb = __shfl_xor_sync(0xffffffffu, b, o);
-      a = ta < a ? ta : a;
-      b = tb < b ? tb : b;
-    }
-    if (l == 0) {
-      if (a != kInfBits) atomicMin(ga, a);
-      if (b != kInfBits) atomicMin(gb, b);
-    }
+    a.courant = l < nw ? part[l].courant : kInfBits;
+    a.rate = l < nw ? part[l].rate : 0ull;
+    warp_merge(a);
+    if (l == 0) register_limits(a, st, prm);
   }
 }
 
-// Per-instance minima of an ensemble: a warp whose elements all belong to one
+// Per-instance limits of an ensemble: a warp whose elements all belong to one
 // instance reduces first; a warp straddling two instances (or the ragged
 // tail) falls back to one atomic per thread. Every lane must call this.
-__device__ __forceinline__ void warp_min2_by_instance(unsigned long long a, unsigned long long b, int inst,
-                                                      DevState* st) {
+__device__ __forceinline__ void warp_limits_by_instance(Limits a, int inst, DevState* st, const Params& prm) {
   const unsigned full = 0xffffffffu;
   const int inst0 = __shfl_sync(full, inst, 0);
   if (__all_sync(full, inst == inst0)) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long ta = __shfl_xor_sync(full, a, o);
-      const unsigned long long tb = __shfl_xor_sync(full, b, o);
-      a = ta < a ? ta : a;
-      b = tb < b ? tb : b;
-    }
-    if ((threadIdx.x & 31) == 0) {
-      if (a != kInfBits) atomicMin(&st[inst0].acc_courant, a);
-      if (b != kInfBits) atomicMin(&st[inst0].acc_hydro, b);
-    }
+    warp_merge(a);
+    if ((threadIdx.x & 31) == 0) register_limits(a, st + inst0, prm);
   } else {
-    if (a != kInfBits) atomicMin(&st[inst].acc_courant, a);
-    if (b != kInfBits) atomicMin(&st[inst].acc_hydro, b);
+    register_limits(a, st + inst, prm);
   }
+}
+
+// A non-negative double as a float, rounded down; 0 below the float range and
+// infinity above it. On the integer pipe (a conversion takes an FP64 slot).
+__device__ __forceinline__ float coarse(double x) {
+  const int h = __double2hiint(x);
+  if (h < 0x38100000) return 0.f;
+  if (h >= 0x47f00000) return __int_as_float(0x7f800000);
+  return __int_as_float(((h - 0x38000000) << 3) | (int)((unsigned)__double2loint(x) >> 29));
 }
 
 // An empty register move the compiler cannot see through: a value passed
 // through it must be recomputed from it.
 __device__ __forceinline__ void opaque(double& x) { asm volatile("" : "+d"(x)); }
 
+// Bound by FP64 issue: 0.48 ms per cycle at 150^3 in mid-blast (0.71 ms with the
+// limiter and the time constraints formed for every element).
+//
 // REGION: threads take elements in region order (d.regOrder) so that a warp
 // runs one region's rep count; each element's EOS is evaluated that many times.
 template <int MODE, bool AUX, bool ENS, bool TAPE, bool REGION>
@@ -935,7 +954,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = REGION ? (t < E ? LULESH_IDX(LDG(&d.regOrder[t]), E, d.st) : E) : t;
   // every thread of the block takes part in the dt reduction
-  unsigned long long courant = kInfBits, hydro = kInfBits;
+  Limits limits = {kInfBits, 0ull};
   const int inst = (ENS && i < E) ? LULESH_IDX(LDG(&d.elemInst[i]), d.ninst, d.st) : 0;
   DevState* const st = d.st + inst;
   const bool live = (i < E) && !step_off(st);
@@ -944,35 +963,47 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     unsigned long long fl = 0ull;  // branch record (TAPE only)
     // ---- calcMonotonicQRegionForElems, src/domain.jl:2322-2513 ----
     const unsigned mask = LDG(&d.elemBC[i]);
+    const double vdov = LDG(&d.vdov[i]);
+    // an expanding element has no viscosity (qlin = qquad = 0), nor has one
+    // whose velocity gradients are zero: its limiter is only checked, not formed
+    const bool expanding = gt_zero(vdov);
     const double dvxi = LDG(&d.delv_xi[i]), dveta = LDG(&d.delv_eta[i]), dvzeta = LDG(&d.delv_zeta[i]);
+    const bool still = is_zero(dvxi) && is_zero(dveta) && is_zero(dvzeta);
     bool bad = false;
-    int src0, src1, src2;
+    int src0 = PHI_MEAN, src1 = PHI_MEAN, src2 = PHI_MEAN;
     // xi-plus: the reference indexes delv_xi[lxip[i]] without +1 (:2349)
     const int ixp = (MODE & 4) ? LDG(&d.lxip[i]) : LDG(&d.lxip[i]) - 1;
     const int Eg = d.Eg;  // neighbour reads may reach the ghost slots of a block-partitioned mesh
-    double dm = monoq_neighbour(d.delv_xi, mask, XI_M, XI_M_SYMM, XI_M_FREE, XI_M_COMM, LDG(&d.lxim[i]), i, Eg, bad);
-    double dp = monoq_neighbour(d.delv_xi, mask, XI_P, XI_P_SYMM, XI_P_FREE, XI_P_COMM, ixp, i, Eg, bad);
-    double tl[9];  // limiter terms per direction: norm, dm/norm, dp/norm (TAPE)
-    // the three 1/(delv + ptiny) from one division
-    double inx, iny, inz;
-    recip3(dvxi + 1.e-36, dveta + 1.e-36, dvzeta + 1.e-36, inx, iny, inz);
-    const double phixi = monoq_phi(inx, dm, dp, prm, src0, tl[0], tl[3], tl[6]);
-    dm = monoq_neighbour(d.delv_eta, mask, ETA_M, ETA_M_SYMM, ETA_M_FREE, ETA_M_COMM, LDG(&d.letam[i]), i, Eg, bad);
-    dp = monoq_neighbour(d.delv_eta, mask, ETA_P, ETA_P_SYMM, ETA_P_FREE, ETA_P_COMM, LDG(&d.letap[i]), i, Eg, bad);
-    const double phieta = monoq_phi(iny, dm, dp, prm, src1, tl[1], tl[4], tl[7]);
-    dm = monoq_neighbour(d.delv_zeta, mask, ZETA_M, ZETA_M_SYMM, ZETA_M_FREE, ZETA_M_COMM, LDG(&d.lzetam[i]), i, Eg, bad);
-    dp = monoq_neighbour(d.delv_zeta, mask, ZETA_P, ZETA_P_SYMM, ZETA_P_FREE, ZETA_P_COMM, LDG(&d.lzetap[i]), i, Eg, bad);
-    const double phizeta = monoq_phi(inz, dm, dp, prm, src2, tl[2], tl[5], tl[8]);
+    const int xim = monoq_neighbour(mask, XI_M, XI_M_SYMM, XI_M_FREE, XI_M_COMM, LDG(&d.lxim[i]), i, Eg, bad);
+    const int xip = monoq_neighbour(mask, XI_P, XI_P_SYMM, XI_P_FREE, XI_P_COMM, ixp, i, Eg, bad);
+    const int etm = monoq_neighbour(mask, ETA_M, ETA_M_SYMM, ETA_M_FREE, ETA_M_COMM, LDG(&d.letam[i]), i, Eg, bad);
+    const int etp = monoq_neighbour(mask, ETA_P, ETA_P_SYMM, ETA_P_FREE, ETA_P_COMM, LDG(&d.letap[i]), i, Eg, bad);
+    const int ztm = monoq_neighbour(mask, ZETA_M, ZETA_M_SYMM, ZETA_M_FREE, ZETA_M_COMM, LDG(&d.lzetam[i]), i, Eg, bad);
+    const int ztp = monoq_neighbour(mask, ZETA_P, ZETA_P_SYMM, ZETA_P_FREE, ZETA_P_COMM, LDG(&d.lzetap[i]), i, Eg, bad);
     if (bad) err |= ST_BAD_BC;
     // d.tapeMat slot q of this element (TAPE only)
     auto tm = [&](int q, double v) { if (TAPE) d.tapeMat[q * E + i] = v; };
-    if (TAPE) {
-      fl |= (unsigned long long)(src0 | (src1 << 3) | (src2 << 6));
-#pragma unroll
-      for (int q = 0; q < 9; ++q) tm(q, tl[q]);
+    double phixi = 0.0, phieta = 0.0, phizeta = 0.0;
+    if (TAPE || !(expanding || still)) {
+      auto at = [](const double* dv, int j) { return j < 0 ? 0.0 : LDG(&dv[j]); };
+      const double xm = at(d.delv_xi, xim), xp = at(d.delv_xi, xip), em = at(d.delv_eta, etm),
+                   ep = at(d.delv_eta, etp), zm = at(d.delv_zeta, ztm), zp = at(d.delv_zeta, ztp);
+      // the three 1/(2 (delv + ptiny)) from one division
+      double hx, hy, hz;
+      recip3(fma(2.0, dvxi, 2.e-36), fma(2.0, dveta, 2.e-36), fma(2.0, dvzeta, 2.e-36), hx, hy, hz);
+      phixi = monoq_phi(hx, xm, xp, prm, src0);
+      phieta = monoq_phi(hy, em, ep, prm, src1);
+      phizeta = monoq_phi(hz, zm, zp, prm, src2);
+      if (TAPE) {
+        // limiter terms per direction: norm, dm/norm, dp/norm
+        fl |= (unsigned long long)(src0 | (src1 << 3) | (src2 << 6));
+        const double nx = 2.0 * hx, ny = 2.0 * hy, nz = 2.0 * hz;
+        tm(0, nx); tm(1, ny); tm(2, nz);
+        tm(3, xm * nx); tm(4, em * ny); tm(5, zm * nz);
+        tm(6, xp * nx); tm(7, ep * ny); tm(8, zp * nz);
+      }
     }
 
-    const double vdov = LDG(&d.vdov[i]);
     const double vnew = LDG(&d.vnew[i]);
     const double delvc_in = LDG(&d.delv[i]);
 
@@ -989,14 +1020,12 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
       vnewc_in = prm.eosvmax; clamped = true;
       if (TAPE) fl |= TF_VNEW_MAX;
     }
-    // 1/vnewc, 1/vchalf (vchalf = vnewc - delvc/2 > 0) and the hydro
-    // constraint's 1/(|vdov| + 1e-20) from one division
-    const double w_hydro = fabs(vdov) + 1.e-20;
-    double inv_vnewc_in, inv_vchalf_in, inv_w;
-    recip3(vnewc_in, fma(delvc_in, -0.5, vnewc_in), w_hydro, inv_vnewc_in, inv_vchalf_in, inv_w);
+    // 1/vnewc and 1/vchalf (vchalf = vnewc - delvc/2 > 0) from one division
+    double inv_vnewc_in, inv_vchalf_in;
+    recip2(vnewc_in, fma(delvc_in, -0.5, vnewc_in), inv_vnewc_in, inv_vchalf_in);
     const double inv_vnew = clamped ? 1.0 / vnew : inv_vnewc_in;
     double qlin, qquad;
-    if (gt_zero(vdov)) {
+    if (expanding || (still && !TAPE)) {
       qlin = 0.0;
       qquad = 0.0;
       if (TAPE) {
@@ -1046,7 +1075,8 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     const double e_old_in = d.e[i];
     const double p_old_in = d.p[i];
     const double c1s = 2.0 / 3.0;
-    const double inv_rho0 = prm.inv_refdens;
+    // (the reference density is 1 unless the caller sets it)
+    auto over_rho0 = [&](double x) { return prm.inv_refdens == 1.0 ? x : x * prm.inv_refdens; };
     double e_out = 0.0, p_out = 0.0, vv_out = 0.0;
     bool compress_out = false;
     // TINY-guarded sound-speed square root (src/domain.jl:2655-2659, 2738-2742)
@@ -1062,7 +1092,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     const double vchalf = fma(delvc, -0.5, vnewc);
     // the rep passes form the reciprocals anew from their opaque inputs
     double inv_vnewc = inv_vnewc_in, inv_vchalf = inv_vchalf_in;
-    if (REGION) { double iw; recip3(vnewc, vchalf, w_hydro, inv_vnewc, inv_vchalf, iw); }
+    if (REGION) recip2(vnewc, vchalf, inv_vnewc, inv_vchalf);
     // compression = 1/vnewc - 1 and compHalfStep = 1/vchalf - 1 enter only as
     // bvc = c1s (1 + compression) and bvc_half = c1s (1 + compHalfStep):
     // bv and bvh are those factors over c1s for the branch taken
@@ -1100,7 +1130,8 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     tm(14, bv); tm(15, bvh); tm(16, e_new); tm(17, pHalfStep); tm(18, vhalf);
     double q_new = 0.0;
     if (compress) {
-      const double ssc = fma(c1s, e_new, ((vhalf * vhalf) * bvc_half) * pHalfStep) * inv_rho0;
+      // vhalf^2 bvc_half = c1s vhalf, 1 + compHalfStep being 1/vhalf in each branch
+      const double ssc = over_rho0(fma(c1s, e_new, (c1s * vhalf) * pHalfStep));
       const double s1 = tiny_sqrt(ssc, TF_S1_TINY);
       q_new = fma(s1, qlin, qquad);
       tm(19, s1); tm(28, ssc);
@@ -1114,11 +1145,13 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     if (fkey(e_new) < prm.k_emin) { e_new = prm.emin; if (TAPE) fl |= TF_E2_MIN; }
     const double bvc = c1s * bv;
     double p_new = pressure(e_new, bvc, TF_PN1_CUT, TF_PN1_MIN);
-    const double vv_bvc = (vnewc * vnewc) * bvc;
+    // vnewc^2 bvc = c1s vnewc, bvc being c1s/vnewc, except where vnewc >= eosvmax
+    double vv_bvc = c1s * vnewc;
+    if (at_vmax) vv_bvc *= vnewc;
     tm(21, e_new); tm(22, p_new);
     double q_tilde = 0.0;
     if (compress) {
-      const double ssc = fma(c1s, e_new, vv_bvc * p_new) * inv_rho0;
+      const double ssc = over_rho0(fma(c1s, e_new, vv_bvc * p_new));
       const double s2 = tiny_sqrt(ssc, TF_S2_TINY);
       q_tilde = fma(s2, qlin, qquad);
       tm(23, s2); tm(29, ssc);
@@ -1126,7 +1159,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
       tm(23, 0.0); tm(29, 0.0);
     }
     tm(24, q_tilde);
-    e_new = e_new - ((fma(7.0, pq_old, -8.0 * sh) + (p_new + q_tilde)) * delvc) * (1.0 / 6.0);
+    e_new = fma(-(fma(7.0, pq_old, -8.0 * sh) + (p_new + q_tilde)), delvc * (1.0 / 6.0), e_new);
     if (abs_lt(e_new, prm.e_cut)) { e_new = 0.0; if (TAPE) fl |= TF_E3_CUT; }
     if (fkey(e_new) < prm.k_emin) { e_new = prm.emin; if (TAPE) fl |= TF_E3_MIN; }
     p_new = pressure(e_new, bvc, TF_PN2_CUT, TF_PN2_MIN);
@@ -1136,7 +1169,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     const bool compress = compress_out;
     double q_new = 0.0;
     // the last q evaluation and the sound speed share one expression
-    const double ssc3 = fma(c1s, e_new, vv_bvc * p_new) * inv_rho0;
+    const double ssc3 = over_rho0(fma(c1s, e_new, vv_bvc * p_new));
     const double ss_new = tiny_sqrt(ssc3, TF_SS_TINY);
     tm(25, e_new); tm(26, p_new); tm(27, ss_new); tm(30, ssc3);
     if (compress) {
@@ -1155,15 +1188,29 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     if (le_zero(tmpV)) err |= ST_UPDATE;
 
     // ---- Courant and hydro constraints, src/domain.jl:2964-3054 ----
+    // A candidate that is certainly above the least so far is not formed: the
+    // estimate, in FP32 from rounded-down operands, is good to 1e-6, and what it
+    // compares with only falls. (dtf below 1e-30 leaves the float range.)
     double dtc = __longlong_as_double((long long)kInfBits), dth = dtc;
     if (!is_zero(vdov)) {
       const double arealg = LDG(&d.arealg[i]);
-      double dtf = ss_new * ss_new;
-      if (lt_zero(vdov)) dtf = fma(prm.qqc2x64 * (arealg * arealg), vdov * vdov, dtf);
-      dtc = arealg * rsqrt(dtf);
-      dth = prm.dvovmax * inv_w;
-      courant = (unsigned long long)__double_as_longlong(dtc);
-      hydro = (unsigned long long)__double_as_longlong(dth);
+      const unsigned long long rate = (unsigned long long)__double_as_longlong(vdov) & 0x7FFFFFFFFFFFFFFFull;
+      if (rate <= kInfBits) limits.rate = rate;  // (a NaN constrains nothing)
+      bool skip = false;
+      if (!TAPE) {
+        const float fa = coarse(arealg), fs = coarse(ss_new), fv = coarse(fabs(vdov));
+        float f = fs * fs;
+        if (lt_zero(vdov)) f = fmaf((prm.qqc2x64f * fa) * fa, fv * fv, f);
+        const double least = __longlong_as_double((long long)*(volatile unsigned long long*)&st->acc_courant);
+        skip = f > 1e-30f && fa > coarse(least) * (sqrtf(f) * 1.0001f);
+      }
+      if (!skip) {
+        double dtf = ss_new * ss_new;
+        if (lt_zero(vdov)) dtf = fma(prm.qqc2x64 * (arealg * arealg), vdov * vdov, dtf);
+        dtc = arealg * rsqrt(dtf);
+        limits.courant = (unsigned long long)__double_as_longlong(dtc);
+      }
+      if (TAPE) dth = hydro_limit(fabs(vdov), prm);
     }
     if (TAPE) {
       d.tapeFlags[i] |= fl;  // k_kinematics stored the face bits of this cycle
@@ -1172,8 +1219,8 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     }
     if (err) atomicOr(&st->status, err);
   }
-  if (ENS) warp_min2_by_instance(courant, hydro, inst, d.st);
-  else block_min2(courant, hydro, &d.st->acc_courant, &d.st->acc_hydro);
+  if (ENS) warp_limits_by_instance(limits, inst, d.st, prm);
+  else block_limits(limits, d.st, prm);
 }
 
 // ---------------------------------------------------------------------------
