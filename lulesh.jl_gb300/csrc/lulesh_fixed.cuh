@@ -150,6 +150,11 @@ LULESH_FX void mac(Acc& r, Num a, Num b) {
   r.h = mad(a.hi, b.hi, r.h);
   r.m = mad(a.lo, b.hi, mad(a.hi, b.lo, r.m));
 }
+// with lo*lo too, for sums whose terms cancel or are far below their scale
+LULESH_FX void mac_full(Acc& r, Num a, Num b) {
+  mac(r, a, b);
+  r.m = mad((int)(mulw(a.lo, b.lo) >> 32), one(), r.m);
+}
 // a b - c d
 LULESH_FX Acc mul_minus(Num a, Num b, Num c, Num d) {
   Acc r = mul(a, b);
@@ -231,10 +236,10 @@ LULESH_FX Float to_float(double x) {
 // kMinDet: the Jacobian determinant (of the mean edges, which are the extents
 // of an undistorted element) over the cube of the scale's 2^61. An undistorted
 // cube has 2^52 to 2^55 by where its extent lies in [2^60, 2^61); the bound is
-// a volume of 1/8 to 1/64 of the element's bounding box. There the fixed-point
-// volume's error (about 0.6 units of 12 * 2^49) meets that of the FP64
-// expressions, 2^-53.
-constexpr i64 kMinDet = 1ll << 49;
+// a volume of 1/32 to 1/256 of the element's bounding box. There the
+// fixed-point volume's error (0.2 units of 12 * 2^47) meets that of the FP64
+// expressions, 2^-53. A blast's shocked elements hold 0.09 of their boxes.
+constexpr i64 kMinDet = 1ll << 47;
 // extents from 2^-12 (where the guards 1e-36 added to squared areas and to
 // volumes are still below half a unit of them) to 2^40
 constexpr int kMinExtent = 1023 - 12, kMaxExtent = 1023 + 40;

@@ -127,28 +127,28 @@ LULESH_FX void kin_products(int k, Slots sh, KinLane& r) {
 LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
   const int at = KS_SUM + kSums * k;
   {
-    Acc a = mul(limbs(r.g[1] + r.g[6]), limbs(r.gU[0]));
-    mac(a, limbs(r.g[8] + r.g[11]), limbs(r.gU[1]));
-    mac(a, limbs(r.g[3] + r.g[5]), limbs(r.gU[2]));
+    Acc a = {0, 0};
+    mac_full(a, limbs(r.g[1] + r.g[6]), limbs(r.gU[0]));
+    mac_full(a, limbs(r.g[8] + r.g[11]), limbs(r.gU[1]));
+    mac_full(a, limbs(r.g[3] + r.g[5]), limbs(r.gU[2]));
     sh.put(at + SUM_VOLUME, take<2>(a));
   }
   LULESH_UNROLL
   for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square(limbs(r.n[f])));
-  Acc rate;
+  Acc rate = {0, 0};
   LULESH_UNROLL
   for (int d = 0; d < 3; ++d) {
     const Num a = limbs(r.A[d]), u = limbs(r.vw[d]), c = limbs(r.C[d]);
     sh.put(at + SUM_AREA + d, square(a));
-    // lo*lo too: the velocity difference along one direction can be far below
-    // the extent that sets the scale
-    Acc f = mul(a, u);
-    f.m = mad((int)(mulw(a.lo, u.lo) >> 32), one(), f.m);
-    sh.put(at + SUM_FLOW + d, take<5>(f));
-    if (d == 0) rate = mul(c, u);
-    else mac(rate, c, u);
+    Acc flow = {0, 0};
+    mac_full(flow, a, u);
+    sh.put(at + SUM_FLOW + d, take<5>(flow));
+    mac_full(rate, c, u);
   }
   sh.put(at + SUM_RATE, take<3>(rate));
-  sh.put(at + SUM_JAC, take<5>(mul(r.half_eta, limbs(r.C[1]))));
+  Acc jac = {0, 0};
+  mac_full(jac, r.half_eta, limbs(r.C[1]));
+  sh.put(at + SUM_JAC, take<5>(jac));
 }
 
 LULESH_FX i64 kin_sum(Slots sh, int i) {

@@ -15,6 +15,7 @@
 // plus k_time_increment (timeIncrement!, src/domain.jl:920-961) for the
 // device-resident run loop.
 #include "lulesh_device.cuh"
+#include "lulesh_element_fp64.cuh"
 #include "lulesh_fixed_force.cuh"
 #include "lulesh_fixed_kin.cuh"
 #include "lulesh_kernels.h"
@@ -26,229 +27,6 @@ namespace lulesh {
 // stops at its first raised error.
 __device__ __forceinline__ bool step_off(const DevState* st) {
   return (*(volatile const unsigned int*)&st->status) != 0u || (*(volatile const int*)&st->done) != 0;
-}
-
-// ---------------------------------------------------------------------------
-// Element geometry at one set of positions
-// ---------------------------------------------------------------------------
-// The FP64 forms, of the elements the fixed-point arithmetic does not take
-// (lulesh_fixed.cuh) and of the tapes.
-
-// The 12 face diagonals, two per face in calcElemNodeNormals' argument order
-// p2 - p0, p3 - p1 (src/domain.jl:991-1067). Face f: (2,0,3,1) (5,0,1,4)
-// (6,1,2,5) (7,2,3,6) (4,3,0,7) (6,4,5,7), so g = d20 d31 d50 d14 d61 d25
-// d72 d36 d43 d07 d64 d57.
-__device__ __forceinline__ void face_diagonals(const double x[8], const double y[8], const double z[8],
-                                               double g[12][3]) {
-  constexpr int pa[12] = {2, 3, 5, 1, 6, 2, 7, 3, 4, 0, 6, 5};
-  constexpr int pb[12] = {0, 1, 0, 4, 1, 5, 2, 6, 3, 7, 4, 7};
-#pragma unroll
-  for (int q = 0; q < 12; ++q) {
-    g[q][0] = x[pa[q]] - x[pb[q]];
-    g[q][1] = y[pa[q]] - y[pb[q]];
-    g[q][2] = z[pa[q]] - z[pb[q]];
-  }
-}
-
-// Walsh coefficients of the positions: w[k] = the Jacobian columns (xi, eta,
-// zeta) of coordinate k, hm[k] = its hourglass modes (eta*zeta, xi*zeta,
-// xi*eta, xi*eta*zeta; src/domain.jl:1510-1525 without the gamma sums).
-// Face diagonals join corners of one parity, so the three even modes are
-// sums of four of them: eta*zeta = (d64 - d57) - (d20 + d31), xi*zeta =
-// (d07 + d61) - (d43 + d25), xi*eta = (d07 + d61) + (d43 + d25); w and
-// xi*eta*zeta come from the four body diagonals a = p6 - p0, b = p5 - p3,
-// c = p7 - p1, d = p4 - p2: (a+b) - (c+d), (a-b) + (c-d), (a+b) + (c+d) and
-// (a-b) - (c-d). 19 adds per coordinate instead of a 23-add butterfly.
-__device__ __forceinline__ void position_walsh(const double x[8], const double y[8], const double z[8],
-                                               const double g[12][3], double w[3][3], double hm[3][4]) {
-  const double* P[3] = {x, y, z};
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double* v = P[k];
-    const double a = v[6] - v[0], b = v[5] - v[3], c = v[7] - v[1], dd = v[4] - v[2];
-    const double apb = a + b, cpd = c + dd, amb = a - b, cmd = c - dd;
-    w[k][0] = apb - cpd;
-    w[k][1] = amb + cmd;
-    w[k][2] = apb + cpd;
-    hm[k][3] = amb - cmd;
-    hm[k][0] = (g[10][k] - g[11][k]) - (g[0][k] + g[1][k]);
-    const double pp = g[9][k] + g[4][k], qq = g[8][k] + g[5][k];
-    hm[k][1] = pp - qq;
-    hm[k][2] = pp + qq;
-  }
-}
-
-// integrateStressForElems' detJ <= 0 check (src/domain.jl:1101-1105): the
-// sign of 8*(fjxet*cjxet + fjyet*cjyet + fjzet*cjzet) (src/domain.jl:2019),
-// with the eta cofactor column c = W_zeta x W_xi (also the monotonic-Q
-// gradient's eta direction).
-__device__ __forceinline__ void eta_cofactors(const double w[3][3], double c[3]) {
-  cross(w[0][2], w[1][2], w[2][2], w[0][0], w[1][0], w[2][0], c[0], c[1], c[2]);
-}
-__device__ __forceinline__ double jacobian_det(const double w[3][3], const double c[3]) {
-  return fma(w[0][1], c[0], fma(w[1][1], c[1], w[2][1] * c[2]));
-}
-__device__ __forceinline__ double jacobian_det(const double w[3][3]) {
-  double c[3];
-  eta_cofactors(w, c);
-  return jacobian_det(w, c);
-}
-
-// Face f's area vector times -8: the cross product of its two diagonals.
-__device__ __forceinline__ void face_normal(const double g[12][3], int f, double n[3]) {
-  cross(g[2 * f][0], g[2 * f][1], g[2 * f][2], g[2 * f + 1][0], g[2 * f + 1][1], g[2 * f + 1][2], n[0], n[1], n[2]);
-}
-
-// Node normals (calcElemNodeNormals, src/domain.jl:991-1067) of corners 0..3
-// as sums of their three faces' cross products (true B = -Bc/8); node 0
-// without its quirk, for which pz01 and ny4 are returned. The six face
-// normals are the area vectors of a closed surface and sum to zero, and
-// opposite corners touch complementary faces (node 0: faces 0,1,4; node 6:
-// 2,3,5), so corners 6, 7, 4, 5 are minus corners 0, 1, 2, 3 and face 5's
-// normal is never needed.
-__device__ __forceinline__ void node_normals(const double n[6][3], double B[3][4], double& pz01, double& ny4) {
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double p01 = n[0][k] + n[1][k];
-    B[k][0] = p01 + n[4][k];
-    B[k][1] = p01 + n[2][k];
-    B[k][2] = (n[0][k] + n[2][k]) + n[3][k];
-    B[k][3] = (n[0][k] + n[3][k]) + n[4][k];
-    if (k == 2) pz01 = p01;
-  }
-  ny4 = n[4][1];
-}
-
-// calcElemVolume's three triple products U.(V x W) of face diagonals
-// (src/utils.jl:36-116): (d31+d72).(d63 x d20), (d43+d57).(d64 x d70),
-// (d14+d25).(d61 x d50); U[t] and the gradients V x W, W x U, U x V.
-__device__ __forceinline__ void volume_terms(const double g[12][3], double U[3][3], double gU[3][3], double gV[3][3],
-                                             double gW[3][3]) {
-  auto grads = [&](int t, const double V[3], const double W[3]) {
-    cross(V[0], V[1], V[2], W[0], W[1], W[2], gU[t][0], gU[t][1], gU[t][2]);
-    cross(W[0], W[1], W[2], U[t][0], U[t][1], U[t][2], gV[t][0], gV[t][1], gV[t][2]);
-    cross(U[t][0], U[t][1], U[t][2], V[0], V[1], V[2], gW[t][0], gW[t][1], gW[t][2]);
-  };
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    U[0][k] = g[1][k] + g[6][k];
-    U[1][k] = g[8][k] + g[11][k];
-    U[2][k] = g[3][k] + g[5][k];
-  }
-  const double V1[3] = {-g[7][0], -g[7][1], -g[7][2]};
-  grads(0, V1, g[0]);
-  const double W2[3] = {-g[9][0], -g[9][1], -g[9][2]};
-  grads(1, g[10], W2);
-  grads(2, g[4], g[2]);
-}
-
-// calcElemVolumeDerivative (src/domain.jl:1178-1256), times 12, in corner
-// order: its voluDer values are the gradient of 12*volume, the triple
-// products' gradients scattered to their corners (U1 = +3 -1 +7 -2,
-// V1 = +6 -3, W1 = +2 -0; U2 = +4 -3 +5 -7, V2 = +6 -4, W2 = +7 -0;
-// U3 = +1 -4 +2 -5, V3 = +6 -1, W3 = +5 -0). The reference's n-th call
-// stores node owner[n]'s derivative in slot n (slots 1 and 3 exchanged)
-// unless corrected; the force kernel applies that when it reads them.
-__device__ __forceinline__ void volume_derivatives(const double gU[3][3], const double gV[3][3],
-                                                   const double gW[3][3], double gr[3][8]) {
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    // corners 1 and 2, 3 and 7, 4 and 5 share a difference of the U gradients
-    const double t12 = gU[2][k] - gU[0][k], t37 = gU[0][k] - gU[1][k], t45 = gU[1][k] - gU[2][k];
-    gr[k][0] = -((gW[0][k] + gW[1][k]) + gW[2][k]);
-    gr[k][1] = t12 - gV[2][k];
-    gr[k][2] = t12 + gW[0][k];
-    gr[k][3] = t37 - gV[0][k];
-    gr[k][4] = t45 - gV[1][k];
-    gr[k][5] = t45 + gW[2][k];
-    gr[k][6] = (gV[0][k] + gV[1][k]) + gV[2][k];
-    gr[k][7] = t37 + gW[1][k];
-  }
-}
-
-// The force tape's face normals 0..4 of these positions (slots 48 + f,
-// 54 + f, 60 + f), read by the hourglass transpose.
-__device__ __forceinline__ void tape_force_normals(double* tape, int E, int e, const double n[6][3]) {
-#pragma unroll
-  for (int f = 0; f < 5; ++f) {
-    tape[(48 + f) * E + e] = n[f][0];
-    tape[(54 + f) * E + e] = n[f][1];
-    tape[(60 + f) * E + e] = n[f][2];
-  }
-}
-
-// The face diagonals of these positions (slot 3q + k of a [36][E] buffer):
-// at the start of a taped segment, for the position transpose of the run's
-// first cycle (every other cycle's is fused into the kinematics transpose of
-// the cycle before, which reads the kinematics tape).
-__device__ __forceinline__ void tape_diagonals(double* diag, int E, int e, const double g[12][3]) {
-#pragma unroll
-  for (int q = 0; q < 12; ++q)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) diag[(3 * q + k) * E + e] = g[q][k];
-}
-
-// The force kernel's geometry of one element's positions.
-__device__ __forceinline__ void force_geometry(const double x[8], const double y[8], const double z[8],
-                                               double gr[3][8], double hm[3][4], double B[3][4], double& pz01,
-                                               double& ny4, double& det) {
-  double g[12][3], w[3][3], n[6][3], U[3][3], gU[3][3], gV[3][3], gW[3][3];
-  face_diagonals(x, y, z, g);
-  position_walsh(x, y, z, g, w, hm);
-#pragma unroll
-  for (int f = 0; f < 5; ++f) face_normal(g, f, n[f]);
-  node_normals(n, B, pz01, ny4);
-  volume_terms(g, U, gU, gV, gW);
-  volume_derivatives(gU, gV, gW, gr);
-  det = jacobian_det(w);
-}
-
-// At the start of a taped segment: the first cycle's face diagonals and
-// normals on their tapes, by the phases of k_kinematics, which writes later
-// cycles' (so a segment's first cycle has the bits it has in mid-segment).
-__global__ void __launch_bounds__(3 * kFixedElems) k_tape_geometry(const __grid_constant__ DevDomain d) {
-  __shared__ fx::Num column[fx::KS_COUNT * kFixedElems];
-  const int E = d.E;
-  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
-  const int slot = blockIdx.x * kFixedElems + lane;
-  const int e = slot < E ? slot : E - 1;
-  const fx::Slots sh{column + lane, kFixedElems};
-  fx::KinLane r;
-  const double* const X = k == 0 ? d.x : k == 1 ? d.y : d.z;
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    r.x[c] = LDG(&X[LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, d.st)]);
-    r.v[c] = 0.0;
-  }
-  fx::kin_extents(k, sh, r);
-  __syncthreads();
-  fx::kin_edges(k, sh, 0.0, r);
-  __syncthreads();
-  fx::kin_products(k, sh, r);
-  __syncthreads();
-  const bool taken = r.ok_x && fx::kin_determinant(sh) >= fx::kMinDet;
-  if (slot >= E) return;
-  if (taken) {
-    if (d.tapeGeoNext)
-#pragma unroll
-      for (int f = 0; f < 5; ++f) d.tapeGeoNext[(48 + 6 * k + f) * E + e] = fx::to_double(r.n[f], 64 - 2 * r.s);
-    if (d.tapeDiag)
-#pragma unroll
-      for (int q = 0; q < 12; ++q) d.tapeDiag[(3 * q + k) * E + e] = fx::to_double(r.g[q], -r.s);
-  } else if (k == 0) {
-    double x[8], y[8], z[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int nd = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, d.st);
-      x[c] = LDG(&d.x[nd]); y[c] = LDG(&d.y[nd]); z[c] = LDG(&d.z[nd]);
-    }
-    double g[12][3], n[6][3];
-    face_diagonals(x, y, z, g);
-#pragma unroll
-    for (int f = 0; f < 5; ++f) face_normal(g, f, n[f]);
-    if (d.tapeGeoNext) tape_force_normals(d.tapeGeoNext, E, e, n);
-    if (d.tapeDiag) tape_diagonals(d.tapeDiag, E, e, g);
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -267,131 +45,39 @@ struct ForceTape {
   __device__ void sum(int k, int m, double v) const { put(36 + 4 * k + m, v); }
 };
 
-// One element's corner forces in FP64: the elements the fixed-point form does
-// not take (thin, inverted or not finite; it also records the volume errors).
+// The FP64 form, for the elements of a block that the fixed-point form does not
+// take (`mine`); every thread of the block calls it. Out of line: its registers
+// are not the kernel's.
 template <int MODE, bool TAPE>
-__device__ __noinline__ void force_fp64(const DevDomain& d, DevState* st, int e, double hgcoef) {
+__device__ __noinline__ void force_fallback(const DevDomain& d, DevState* st, fx::Num* column, int e, bool mine,
+                                            double hgcoef) {
   const int E = d.E;
-  int nd[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) nd[c] = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, st);
-  double gr[3][8], hm[3][4], B[3][4], pz01, ny4, det;
-  {
-    double x[8], y[8], z[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) { x[c] = LDG(&d.x[nd[c]]); y[c] = LDG(&d.y[nd[c]]); z[c] = LDG(&d.z[nd[c]]); }
-    force_geometry(x, y, z, gr, hm, B, pz01, ny4, det);
-  }
-  if (le_zero(det)) atomicOr(&st->status, ST_EARLY);
-
-  // the reference's slots of the volume derivatives: node 3's in slot 1 and
-  // node 1's in slot 3 unless corrected
-  double dvx[8], dvy[8], dvz[8];
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    const int src = (MODE & 2) ? n : (n == 1 ? 3 : n == 3 ? 1 : n);
-    dvx[n] = gr[0][src]; dvy[n] = gr[1][src]; dvz[n] = gr[2][src];
-  }
-
-  // stress: f = (-sig) * B = (sig/8) * Bc with sig = -p - q; corners 4..7
-  // are minus corners 2, 3, 0, 1, formed before node 0's quirk
-  const double s8 = ((-LDG(&d.p[e])) - LDG(&d.q[e])) * 0.125;
-  double SB[3][4];
-#pragma unroll
-  for (int k = 0; k < 3; ++k)
-#pragma unroll
-    for (int n = 0; n < 4; ++n) SB[k][n] = s8 * B[k][n];
-  double q0y = SB[1][0], q0z = SB[2][0];
-  if (!(MODE & 1)) {
-    // src/domain.jl:1050-1055: node 1 takes face 5's areaY twice, no areaZ
-    q0y = s8 * (B[1][0] + ny4);
-    q0z = s8 * pz01;
-  }
-  // s8*Bc of corner n, component k (n and k are constants after unrolling, so
-  // the sign folds into the instruction that consumes it)
-  auto bstress = [&](int k, int n) -> double {
-    if (n == 0) return k == 0 ? SB[0][0] : k == 1 ? q0y : q0z;
-    if (n < 4) return SB[k][n];
-    return -SB[k][n == 4 ? 2 : n == 5 ? 3 : n == 6 ? 0 : 1];
-  };
-
-  // calcHourglassControlForElems (src/domain.jl:1696-1736): determ = volo*v.
-  const double v = LDG(&d.v[e]);
-  const double determ = LDG(&d.volo[e]) * v;
-  if (le_zero(v)) atomicOr(&st->status, ST_HOURGLASS);
-
-  double fx[8], fy[8], fz[8];
-  if (gt_zero(hgcoef)) {
-    // hourgam (src/domain.jl:1527-1549) with volinv/12 folded into the modes
-    // determ^(-1/3) serves the coefficient, its cube the modes' 1/(12 determ)
-    const double rc = inv_cbrt(determ);
-    const double vi12 = (rc * rc) * (rc * (1.0 / 12.0));
-    double hmx[4], hmy[4], hmz[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) { hmx[m] = hm[0][m] * vi12; hmy[m] = hm[1][m] * vi12; hmz[m] = hm[2][m] * vi12; }
-    if (TAPE) {
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        d.tapeGeo[n * E + e] = dvx[n];
-        d.tapeGeo[(8 + n) * E + e] = dvy[n];
-        d.tapeGeo[(16 + n) * E + e] = dvz[n];
-      }
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        d.tapeGeo[(24 + m) * E + e] = hmx[m];
-        d.tapeGeo[(28 + m) * E + e] = hmy[m];
-        d.tapeGeo[(32 + m) * E + e] = hmz[m];
-      }
-    }
-    double hg[8][4];
-#pragma unroll
-    for (int n = 0; n < 8; ++n)
-#pragma unroll
-      for (int m = 0; m < 4; ++m)
-        hg[n][m] = fma(-dvz[n], hmz[m], fma(-dvy[n], hmy[m], fma(-dvx[n], hmx[m], gamma_nm(n, m))));
-
-    // coefficient = -hgcoef*0.01*ss*mass/cbrt(determ) (src/domain.jl:1605)
-    const double coef = ((-hgcoef * 0.01) * LDG(&d.ss[e])) * LDG(&d.elemMass[e]) * rc;
-
-    // calcElemFBHourglassForce (src/domain.jl:1258-1460), one velocity
-    // component at a time to bound register use.
-    const double* vel[3] = {d.xd, d.yd, d.zd};
-    double* fo[3] = {fx, fy, fz};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      double vv[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) vv[c] = LDG(&vel[k][nd[c]]);
-      double h[4];
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        double s = hg[0][m] * vv[0];
-#pragma unroll
-        for (int n = 1; n < 8; ++n) s = fma(hg[n][m], vv[n], s);
-        if (TAPE) d.tapeGeo[(36 + 4 * k + m) * E + e] = s;
-        h[m] = coef * s;
-      }
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        fo[k][n] = fma(hg[n][0], h[0], fma(hg[n][1], h[1], fma(hg[n][2], h[2], fma(hg[n][3], h[3], bstress(k, n)))));
-      }
-    }
-  } else {
-#pragma unroll
-    for (int n = 0; n < 8; ++n) { fx[n] = bstress(0, n); fy[n] = bstress(1, n); fz[n] = bstress(2, n); }
-  }
+  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  const double* const X = k == 0 ? d.x : k == 1 ? d.y : d.z;
+  const double* const U = k == 0 ? d.xd : k == 1 ? d.yd : d.zd;
+  double x[8], v[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    d.fcx[c * E + e] = fx[c];
-    d.fcy[c * E + e] = fy[c];
-    d.fcz[c * E + e] = fz[c];
+    const int nd = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, st);
+    x[c] = LDG(&X[nd]);
+    v[c] = LDG(&U[nd]);
   }
+  ForceScalars c;
+  c.v = LDG(&d.v[e]);
+  const double rc = inv_cbrt(LDG(&d.volo[e]) * c.v);
+  c.vi12 = (rc * rc) * (rc * (1.0 / 12.0));
+  c.coef = ((-hgcoef * 0.01) * LDG(&d.ss[e])) * LDG(&d.elemMass[e]) * rc;
+  c.s8 = ((-LDG(&d.p[e])) - LDG(&d.q[e])) * 0.125;
+  c.hourglass = gt_zero(hgcoef);
+  double* const out = (k == 0 ? d.fcx : k == 1 ? d.fcy : d.fcz) + e;
+  force_fp64<MODE>(k, RealSlots{reinterpret_cast<double*>(column) + lane, kFixedElems}, x, v, c, mine, st,
+                   [&](int n, double f) { out[n * E] = f; }, ForceTape<TAPE>{TAPE ? d.tapeGeo + e : nullptr, E, true});
 }
 
 // Three threads per element, one per coordinate and each in a warp of its own:
 // a block is 32 elements (lulesh_fixed_force.cuh). Bound by the integer pipes
 // (multiply-adds, shifts and logic issue every other cycle and share them:
-// counters 59 % and 46 % of the cycles, no other pipe above 25 %): 0.90 ms per
+// counters 59 % and 46 % of the cycles, no other pipe above 25 %): 0.91 ms per
 // cycle at 150^3, where FP64 took 1.98 ms with the geometry stored by
 // k_kinematics (0.87 ms of that kernel). Seven blocks per SM, 80 registers:
 // six (96 registers) 1.02 ms, five (128) 1.12 ms; below 45^3 the three are
@@ -408,6 +94,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 7)
   const int inst = ENS ? LULESH_IDX(LDG(&d.elemInst[e]), d.ninst, d.st) : 0;
   DevState* const st = d.st + inst;
   const bool live = slot < E && !step_off(st);
+  if (!__syncthreads_or(live)) return;
   const double hgcoef = ENS ? LDG(&d.instHg[inst]) : prm.hgcoef;
   const fx::Slots sh{column + lane, kFixedElems};
   fx::ForceLane r;
@@ -443,13 +130,14 @@ __global__ void __launch_bounds__(3 * kFixedElems, 7)
   fx::force_products<MODE>(k, sh, r, hm, tape);
   __syncthreads();
   fx::force_base(k, sh, r);
-  __syncthreads();
-  if (!live) return;
-  if (r.ok) {
+  const int others = __syncthreads_or(live && !r.ok);
+  if (live && r.ok) {
     double* const out = (k == 0 ? d.fcx : k == 1 ? d.fcy : d.fcz) + e;
     fx::force_corners(k, sh, r, [&](int n, double f) { out[n * E] = f; }, tape);
-  } else if (k == 0) {
-    force_fp64<MODE, TAPE>(d, st, e, hgcoef);
+  }
+  if (others) {
+    __syncthreads();
+    force_fallback<MODE, TAPE>(d, st, column, e, live && !r.ok, hgcoef);
   }
 }
 
@@ -503,200 +191,182 @@ __global__ void __launch_bounds__(kMaxNodeBlock) k_node(DevDomain d, Params prm)
 // ---------------------------------------------------------------------------
 // k_kinematics
 // ---------------------------------------------------------------------------
-// One element in FP64: what the fixed-point form does not take (thin,
-// inverted or not finite elements; it records the volume error). `geometry`:
-// the tapes of the positions are this function's too.
-template <bool AUX, bool TAPE>
-__device__ __noinline__ void kin_fp64(const DevDomain& d, DevState* st, int e, double dt, bool geometry) {
+// The quotients of the elements marked `mine` from the sums that `get` gives,
+// divided among the three threads: coordinate 1 the divergence and 1/(64
+// volume), both from one division, coordinate 0 the volume's change and the
+// characteristic length, coordinate k direction k of the monotonic-Q gradients.
+// Every thread of the block calls it. Returns the largest face's place (taped
+// runs).
+template <bool AUX, bool TAPE, class Sums>
+__device__ __forceinline__ int kin_quotients(const DevDomain& d, DevState* st, const fx::Slots& sh, int k, int e,
+                                             bool mine, const Sums& get) {
   const int E = d.E;
-  int nd[8];
+  const double volume = get.volume12() * (1.0 / 12.0);
+  const double vnew = volume * LDG(&d.inv_volo[e]);
+  const double volq = LDG(&d.volo[e]) * vnew;
+  double rcl = 0.0;
+  auto tape = [&](int slot, double v) { d.tapeKin[slot * E + e] = v; };
+  if (mine) {
+    if (k == 1) {
+      const double q64 = fma(64.0, volq, 64.0 * 1.e-36);
+      double inv, norm64;
+      recip2(get.jacobian(), q64, inv, norm64);
+      const double vdov = get.rate() * inv;
+      d.vdov[e] = vdov;
+      sh.put(fx::KS_MID, __double_as_longlong(norm64));
+      if (AUX) {
+        sh.put(fx::KS_MID + 1, __double_as_longlong(inv));
+        sh.put(fx::KS_MID + 2, __double_as_longlong(vdov));
+      }
+      if (TAPE) {
+        tape(27, inv);
+        tape(40, norm64);
+      }
+    } else if (k == 0) {
+      // 4*volume/sqrt(max area) with area = 4*|face vector|^2
+      // (src/domain.jl:1874-1930)
+      int place;
+      rcl = rsqrt(get.face(place));
+      if (le_zero(vnew)) atomicOr(&st->status, ST_KINEMATICS);
+      d.vnew[e] = vnew;
+      d.delv[e] = vnew - LDG(&d.v[e]);
+      d.arealg[e] = (2.0 * volume) * rcl;
+      if (TAPE) sh.put(fx::KS_MID + 1, place);
+    }
+  }
+  __syncthreads();
+  if (!mine) return 0;
+  // src/domain.jl:2175-2320; with the reference's dxi = W_xi/4 etc.: delx =
+  // 16*vol/sqrt(|A|^2 + 256*ptiny) and delv = norm/64 * (A . W(v)) for the cross
+  // product A of two Walsh vectors
+  double* const delx = k == 0 ? d.delx_xi : k == 1 ? d.delx_eta : d.delx_zeta;
+  double* const delv = k == 0 ? d.delv_xi : k == 1 ? d.delv_eta : d.delv_zeta;
+  const double norm64 = __longlong_as_double(sh.get(fx::KS_MID));
+  const double rs = rsqrt(get.area(k));
+  delx[e] = (16.0 * volq) * rs;
+  delv[e] = norm64 * get.flow(k);
+  if (AUX) {
+    double* const dd = k == 0 ? d.dxx : k == 1 ? d.dyy : d.dzz;
+    const double inv = __longlong_as_double(sh.get(fx::KS_MID + 1));
+    const double vdov = __longlong_as_double(sh.get(fx::KS_MID + 2));
+    dd[e] = get.own_rate(k) * inv - vdov / 3.0;
+  }
+  if (!TAPE) return 0;
+  const int place = (int)sh.get(fx::KS_MID + 1);
+  tape(37 + k, rs);
+  if (k == 0) {
+    tape(44, rcl);
+    d.tapeFlags[e] = (unsigned long long)place << TF_FACE_SHIFT;
+  }
+  return place;
+}
+
+// Coordinate k's taped components; t gives them as doubles. The 12 diagonals
+// in the order d61 d70 d63 d20 d50 d64 d31 d72 d43 d57 d14 d25 (force-order
+// index, sign), the largest face's vector in the reference's face order, the
+// last two faces with reversed diagonals.
+template <class Taped>
+__device__ __forceinline__ void kin_tape(const DevDomain& d, int k, int e, int place, const Taped& t) {
+  const int E = d.E;
+  auto put = [&](int slot, double v) { d.tapeKin[slot * E + e] = v; };
 #pragma unroll
-  for (int c = 0; c < 8; ++c) nd[c] = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, st);
-  double x[8], y[8], z[8];
+  for (int a = 0; a < 3; ++a) {
+    put(3 * k + a, t.w(a));
+    put(9 + 3 * k + a, t.vw(a));
+    put(18 + 3 * a + k, t.C(a));
+    put(28 + 3 * a + k, t.A(a));
+    put(81 + 3 * a + k, t.gU(a));
+  }
+  constexpr int gi[12] = {4, 9, 7, 0, 2, 10, 1, 6, 8, 11, 3, 5};
+#pragma unroll
+  for (int q = 0; q < 12; ++q) put(45 + 3 * q + k, q == 1 || q == 2 ? -t.g(gi[q]) : t.g(gi[q]));
+  const double c = place == 0 ? t.n(0) : place == 1 ? t.n(5) : place == 2 ? t.n(1) : place == 3 ? t.n(2)
+                                    : place == 4 ? -t.n(3) : -t.n(4);
+  put(41 + k, c);
+}
+
+// The next cycle's face normals, for its hourglass transpose.
+template <class Taped>
+__device__ __forceinline__ void kin_tape_next(const DevDomain& d, int k, int e, const Taped& t) {
+#pragma unroll
+  for (int f = 0; f < 5; ++f) d.tapeGeoNext[(48 + 6 * k + f) * d.E + e] = t.n(f);
+}
+
+struct FixedSums {
+  const fx::Slots& sh;
+  const fx::KinLane& r;
+  __device__ double volume12() const { return fx::kin_volume12(sh, r); }
+  __device__ double face(int& place) const { return fx::kin_largest_face(sh, r, place); }
+  // (of the size the fixed-point form takes, |A|^2 is far above 256*ptiny)
+  __device__ double area(int k) const { return fx::kin_area(sh, r, k); }
+  __device__ double flow(int k) const { return fx::kin_flow(sh, r, k); }
+  __device__ double rate() const { return fx::kin_rate(sh, r); }
+  __device__ double jacobian() const { return fx::kin_jacobian(sh, r); }
+  __device__ double own_rate(int k) const {
+    return fx::to_double(sh.get(fx::KS_SUM + fx::kSums * k + fx::SUM_RATE), 131 - 2 * r.s - r.sv);
+  }
+};
+struct FixedTaped {
+  const fx::KinLane& r;
+  __device__ double w(int a) const { return fx::to_double(r.w[a], 2 - r.s); }
+  __device__ double vw(int a) const { return fx::to_double(r.vw[a], 2 - r.sv); }
+  __device__ double C(int a) const { return fx::to_double(r.C[a], 68 - 2 * r.s); }
+  __device__ double A(int a) const { return fx::to_double(r.A[a], 68 - 2 * r.s); }
+  __device__ double gU(int a) const { return fx::to_double(r.gU[a], 64 - 2 * r.s); }
+  __device__ double g(int q) const { return fx::to_double(r.g[q], -r.s); }
+  __device__ double n(int f) const { return fx::to_double(r.n[f], 64 - 2 * r.s); }
+};
+struct RealSums {
+  const KinSums& s;
+  __device__ double volume12() const { return s.volume12; }
+  __device__ double face(int& place) const { place = s.place; return s.face; }
+  __device__ double area(int) const { return s.area; }
+  __device__ double flow(int) const { return s.flow; }
+  __device__ double rate() const { return s.rate; }
+  __device__ double jacobian() const { return s.jacobian; }
+  __device__ double own_rate(int) const { return s.own_rate; }
+};
+struct RealTaped {
+  const KinTaped& t;
+  __device__ double w(int a) const { return t.w[a]; }
+  __device__ double vw(int a) const { return t.vw[a]; }
+  __device__ double C(int a) const { return t.C[a]; }
+  __device__ double A(int a) const { return t.A[a]; }
+  __device__ double gU(int a) const { return t.gU[a]; }
+  __device__ double g(int q) const { return t.g[q]; }
+  __device__ double n(int f) const { return t.n[f]; }
+};
+
+// The FP64 form, for the elements of a block that the fixed-point form does not
+// take (`mine`); every thread of the block calls it. `geometry`: the next
+// cycle's normals are its too (they depend on the positions alone, and the
+// fixed-point form takes those of an element whose velocities it refuses).
+template <bool AUX, bool TAPE>
+__device__ __noinline__ void kin_fallback(const DevDomain& d, DevState* st, fx::Num* column, int e, bool mine,
+                                          bool geometry, double dt) {
+  const int E = d.E;
+  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  const double* const X = k == 0 ? d.x : k == 1 ? d.y : d.z;
+  const double* const U = k == 0 ? d.xd : k == 1 ? d.yd : d.zd;
+  double x[8], v[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    x[c] = LDG(&d.x[nd[c]]);
-    y[c] = LDG(&d.y[nd[c]]);
-    z[c] = LDG(&d.z[nd[c]]);
+    const int nd = LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, st);
+    x[c] = LDG(&X[nd]);
+    v[c] = LDG(&U[nd]);
   }
-
-  // calcElemVolume (src/utils.jl:36-116) and calcElemCharacteristicLength
-  // (src/domain.jl:1874-1930) from the face diagonals.
-  double volume, charLength = 0.0;
-  double w[3][3];  // first-order Walsh vectors (xi, eta, zeta) of x, y, z
-  double cet[3];   // W_zeta x W_xi
-  {
-    double g[12][3], hm[3][4], n[6][3], U[3][3], gU[3][3], gV[3][3], gW[3][3];
-    face_diagonals(x, y, z, g);
-    position_walsh(x, y, z, g, w, hm);
-    volume_terms(g, U, gU, gV, gW);
-    auto triple_t = [&](int t) { return fma(U[t][0], gU[t][0], fma(U[t][1], gU[t][1], U[t][2] * gU[t][2])); };
-    volume = ((triple_t(0) + triple_t(1)) + triple_t(2)) * (1.0 / 12.0);
-#pragma unroll
-    for (int f = 0; f < 6; ++f) face_normal(g, f, n[f]);
-    if (TAPE) {
-      // the 12 diagonals in the order d61 d70 d63 d20 d50 d64 d31 d72 d43 d57
-      // d14 d25 (force-order index, sign) and the V x W factors
-      constexpr int gi[12] = {4, 9, 7, 0, 2, 10, 1, 6, 8, 11, 3, 5};
-      constexpr int gs[12] = {1, -1, -1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
-#pragma unroll
-      for (int q = 0; q < 12; ++q)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) d.tapeKin[(45 + 3 * q + k) * E + e] = gs[q] < 0 ? -g[gi[q]][k] : g[gi[q]][k];
-#pragma unroll
-      for (int t = 0; t < 3; ++t)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) d.tapeKin[(81 + 3 * t + k) * E + e] = gU[t][k];
-    }
-    // areaFace (src/domain.jl:1874-1891): with f, g = a -/+ b for the face
-    // diagonals a, b, |f|^2|g|^2 - (f.g)^2 = |f x g|^2 = 4 |a x b|^2; the 4
-    // is folded into arealg below. The reference's faces in order are the
-    // force order's 0, 5, 1, 2, 3, 4, the last two with reversed diagonals
-    // (so minus those cross products).
-    int fidx = 0;
-    double fcx = 0.0, fcy = 0.0, fcz = 0.0;  // the largest face's cross product (TAPE)
-    constexpr int ff[6] = {0, 5, 1, 2, 3, 4};
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      const double* c = n[ff[q]];
-      // area4 >= +0 and charLength too: their bit patterns order them
-      const double area4 = fma(c[0], c[0], fma(c[1], c[1], c[2] * c[2]));
-      if (TAPE && (q == 0 || __double_as_longlong(area4) > __double_as_longlong(charLength))) {
-        const bool neg = q >= 4;
-        fidx = q;
-        fcx = neg ? -c[0] : c[0]; fcy = neg ? -c[1] : c[1]; fcz = neg ? -c[2] : c[2];
-      }
-      charLength = max_nonneg(area4, charLength);
-    }
-    if (TAPE) {
-      d.tapeFlags[e] = (unsigned long long)fidx << TF_FACE_SHIFT;
-      d.tapeKin[41 * E + e] = fcx; d.tapeKin[42 * E + e] = fcy; d.tapeKin[43 * E + e] = fcz;
-      // the next cycle's face normals, for its hourglass transpose
-      if (d.tapeGeoNext && geometry) tape_force_normals(d.tapeGeoNext, E, e, n);
-    }
-    eta_cofactors(w, cet);
-  }
-  const double* wx = w[0];
-  const double* wy = w[1];
-  const double* wz = w[2];
-  const double vnew = volume * LDG(&d.inv_volo[e]);
-  if (le_zero(vnew)) atomicOr(&st->status, ST_KINEMATICS);
-  d.vnew[e] = vnew;
-  d.delv[e] = vnew - LDG(&d.v[e]);
-  // 4*volume/sqrt(max area) with area = 4*area4
-  {
-    const double rcl = rsqrt(charLength);
-    d.arealg[e] = (2.0 * volume) * rcl;
-    if (TAPE) d.tapeKin[44 * E + e] = rcl;
-  }
-
-  // Velocity gradient trace at the half-step position (src/domain.jl:2128-2158)
-  double vxw[3], vyw[3], vzw[3];
-  {
-    double v8[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) v8[c] = LDG(&d.xd[nd[c]]);
-    walsh1(v8, vxw);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) v8[c] = LDG(&d.yd[nd[c]]);
-    walsh1(v8, vyw);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) v8[c] = LDG(&d.zd[nd[c]]);
-    walsh1(v8, vzw);
-  }
-  if (TAPE) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      d.tapeKin[a * E + e] = wx[a]; d.tapeKin[(3 + a) * E + e] = wy[a]; d.tapeKin[(6 + a) * E + e] = wz[a];
-      d.tapeKin[(9 + a) * E + e] = vxw[a]; d.tapeKin[(12 + a) * E + e] = vyw[a]; d.tapeKin[(15 + a) * E + e] = vzw[a];
-    }
-  }
-  // 1/det of the velocity gradient and 1/(64 vol + 64 ptiny) of the Q
-  // gradients come from one division
-  const double volq = LDG(&d.volo[e]) * vnew;
-  const double q64 = fma(64.0, volq, 64.0 * 1.e-36);
-  double inv, norm64;
-  {
-    const double dt2 = -0.5 * dt;
-    double F[3][3];  // F[k][a]: coordinate k, direction a (xi, eta, zeta)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      F[0][a] = fma(dt2, vxw[a], wx[a]);
-      F[1][a] = fma(dt2, vyw[a], wy[a]);
-      F[2][a] = fma(dt2, vzw[a], wz[a]);
-    }
-    // cofactors (src/domain.jl:1976-1987)
-    const double Cxxi = fma(F[1][1], F[2][2], -(F[2][1] * F[1][2]));
-    const double Cxet = fma(F[2][0], F[1][2], -(F[1][0] * F[2][2]));
-    const double Cxze = fma(F[1][0], F[2][1], -(F[2][0] * F[1][1]));
-    const double Cyxi = fma(F[2][1], F[0][2], -(F[0][1] * F[2][2]));
-    const double Cyet = fma(F[0][0], F[2][2], -(F[2][0] * F[0][2]));
-    const double Cyze = fma(F[2][0], F[0][1], -(F[0][0] * F[2][1]));
-    const double Czxi = fma(F[0][1], F[1][2], -(F[1][1] * F[0][2]));
-    const double Czet = fma(F[1][0], F[0][2], -(F[0][0] * F[1][2]));
-    const double Czze = fma(F[0][0], F[1][1], -(F[1][0] * F[0][1]));
-    const double det = fma(F[0][1], Cxet, fma(F[1][1], Cyet, F[2][1] * Czet));
-    const double d1 = fma(Cxxi, vxw[0], fma(Cxet, vxw[1], Cxze * vxw[2]));
-    const double d2 = fma(Cyxi, vyw[0], fma(Cyet, vyw[1], Cyze * vyw[2]));
-    const double d3 = fma(Czxi, vzw[0], fma(Czet, vzw[1], Czze * vzw[2]));
-    recip2(det, q64, inv, norm64);
-    const double vdov = ((d1 + d2) + d3) * inv;
-    d.vdov[e] = vdov;
-    if (TAPE) {
-      // cofactor columns C_xi, C_eta, C_zeta (x, y, z each), then 1/det
-      const double cof[9] = {Cxxi, Cyxi, Czxi, Cxet, Cyet, Czet, Cxze, Cyze, Czze};
-#pragma unroll
-      for (int q = 0; q < 9; ++q) d.tapeKin[(18 + q) * E + e] = cof[q];
-      d.tapeKin[27 * E + e] = inv;
-    }
-    if (AUX) {
-      const double third = vdov / 3.0;
-      d.dxx[e] = d1 * inv - third;
-      d.dyy[e] = d2 * inv - third;
-      d.dzz[e] = d3 * inv - third;
-    }
-  }
-
-  // calcMonotonicQGradientsForElems (src/domain.jl:2175-2320). With the
-  // reference's dxi = W_xi/4 etc.: delx = 16*vol/sqrt(|A|^2 + 256*ptiny) and
-  // delv = norm/64 * (A . W(v)) for the cross product A of two Walsh vectors.
-  {
-    const double ptiny = 1.e-36;
-    const double vol = volq;
-    const double vol16 = 16.0 * vol;
-    double ax, ay, az, rs;
-    // taped per direction d (xi, eta, zeta): the cross product A and 1/|A|
-    auto tape_a = [&](int dir) {
-      if (TAPE) {
-        d.tapeKin[(28 + 3 * dir) * E + e] = ax; d.tapeKin[(29 + 3 * dir) * E + e] = ay;
-        d.tapeKin[(30 + 3 * dir) * E + e] = az; d.tapeKin[(37 + dir) * E + e] = rs;
-      }
-    };
-    if (TAPE) d.tapeKin[40 * E + e] = norm64;
-    // zeta: xi x eta
-    cross(wx[0], wy[0], wz[0], wx[1], wy[1], wz[1], ax, ay, az);
-    rs = rsqrt(fma(ax, ax, fma(ay, ay, fma(az, az, 256.0 * ptiny))));
-    d.delx_zeta[e] = vol16 * rs;
-    d.delv_zeta[e] = norm64 * fma(ax, vxw[2], fma(ay, vyw[2], az * vzw[2]));
-    tape_a(2);
-    // xi: eta x zeta
-    cross(wx[1], wy[1], wz[1], wx[2], wy[2], wz[2], ax, ay, az);
-    rs = rsqrt(fma(ax, ax, fma(ay, ay, fma(az, az, 256.0 * ptiny))));
-    d.delx_xi[e] = vol16 * rs;
-    d.delv_xi[e] = norm64 * fma(ax, vxw[0], fma(ay, vyw[0], az * vzw[0]));
-    tape_a(0);
-    // eta: zeta x xi (formed for the detJ check)
-    ax = cet[0]; ay = cet[1]; az = cet[2];
-    rs = rsqrt(fma(ax, ax, fma(ay, ay, fma(az, az, 256.0 * ptiny))));
-    d.delx_eta[e] = vol16 * rs;
-    d.delv_eta[e] = norm64 * fma(ax, vxw[1], fma(ay, vyw[1], az * vzw[1]));
-    tape_a(1);
+  KinSums sums;
+  KinTaped t;
+  kin_fp64(k, RealSlots{reinterpret_cast<double*>(column) + lane, kFixedElems}, x, v, dt, sums, t);
+  const int place = kin_quotients<AUX, TAPE>(d, st, fx::Slots{column + lane, kFixedElems}, k, e, mine, RealSums{sums});
+  if (TAPE && mine) {
+    kin_tape(d, k, e, place, RealTaped{t});
+    if (d.tapeGeoNext && geometry) kin_tape_next(d, k, e, RealTaped{t});
   }
 }
 
-
 // Three threads per element as in k_force (lulesh_fixed_kin.cuh). Bound by the
-// integer pipes: 0.57 ms per cycle at 150^3 (FP64: 1.93 ms without the force
+// integer pipes: 0.58 ms per cycle at 150^3 (FP64: 1.93 ms without the force
 // geometry). Eight blocks per SM, 80 registers: six (96) 0.67 ms, five (128)
 // 0.77 ms.
 template <bool AUX, bool ENS, bool TAPE>
@@ -710,6 +380,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 8)
   const int e = slot < E ? slot : E - 1;
   DevState* const st = d.st + (ENS ? LULESH_IDX(LDG(&d.elemInst[e]), d.ninst, d.st) : 0);
   const bool live = slot < E && !step_off(st);
+  if (!__syncthreads_or(live)) return;
   const double dt = st->deltatime;
   const fx::Slots sh{column + lane, kFixedElems};
   fx::KinLane r;
@@ -732,98 +403,67 @@ __global__ void __launch_bounds__(3 * kFixedElems, 8)
   fx::kin_terms(k, sh, r);
   __syncthreads();
   fx::kin_accept(sh, r);
-  // The quotients: each thread forms the volume; coordinate 1 the divergence
-  // and 1/(64 volume), both from one division, coordinate 0 the volume's
-  // change and the characteristic length.
-  const double volume = fx::kin_volume12(sh, r) * (1.0 / 12.0);
-  const double vnew = volume * LDG(&d.inv_volo[e]);
-  const double volq = LDG(&d.volo[e]) * vnew;
-  int face = 0;
-  double rcl = 0.0;
-  auto kin_tape = [&](int slot_, double v) { d.tapeKin[slot_ * E + e] = v; };
-  if (r.ok) {
-    if (k == 1) {
-      const double q64 = fma(64.0, volq, 64.0 * 1.e-36);
-      double inv, norm64;
-      recip2(fx::kin_jacobian(sh, r), q64, inv, norm64);
-      const double vdov = fx::kin_rate(sh, r) * inv;
-      if (live) d.vdov[e] = vdov;
-      sh.put(fx::KS_MID, __double_as_longlong(norm64));
-      if (AUX) {
-        sh.put(fx::KS_MID + 1, __double_as_longlong(inv));
-        sh.put(fx::KS_MID + 2, __double_as_longlong(vdov));
-      }
-      if (TAPE && live) {
-        kin_tape(27, inv);
-        kin_tape(40, norm64);
-      }
-    } else if (k == 0) {
-      // 4*volume/sqrt(max area) with area = 4*|face vector|^2
-      // (src/domain.jl:1874-1930)
-      rcl = rsqrt(fx::kin_largest_face(sh, r, face));
-      if (live) {
-        if (le_zero(vnew)) atomicOr(&st->status, ST_KINEMATICS);
-        d.vnew[e] = vnew;
-        d.delv[e] = vnew - LDG(&d.v[e]);
-        d.arealg[e] = (2.0 * volume) * rcl;
-      }
-      if (TAPE) sh.put(fx::KS_MID + 1, face);
-    }
+  const int others = __syncthreads_or(live && !r.ok);
+  const int place = kin_quotients<AUX, TAPE>(d, st, sh, k, e, live && r.ok, FixedSums{sh, r});
+  if (TAPE && live) {
+    if (r.ok) kin_tape(d, k, e, place, FixedTaped{r});
+    if (d.tapeGeoNext && r.ok_x) kin_tape_next(d, k, e, FixedTaped{r});
   }
+  if (others) {
+    __syncthreads();
+    kin_fallback<AUX, TAPE>(d, st, column, e, live && !r.ok, !r.ok_x, dt);
+  }
+}
+
+// At the start of a taped segment: the first cycle's face diagonals and
+// normals on their tapes, by the phases of k_kinematics, which writes later
+// cycles' (so a segment's first cycle has the bits it has in mid-segment).
+__global__ void __launch_bounds__(3 * kFixedElems) k_tape_geometry(const __grid_constant__ DevDomain d) {
+  __shared__ fx::Num column[fx::KS_COUNT * kFixedElems];
+  const int E = d.E;
+  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  const int slot = blockIdx.x * kFixedElems + lane;
+  const int e = slot < E ? slot : E - 1;
+  const fx::Slots sh{column + lane, kFixedElems};
+  fx::KinLane r;
+  const double* const X = k == 0 ? d.x : k == 1 ? d.y : d.z;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    r.x[c] = LDG(&X[LULESH_IDX(LDG(&d.nodelist[c * E + e]), d.N, d.st)]);
+    r.v[c] = 0.0;
+  }
+  fx::kin_extents(k, sh, r);
   __syncthreads();
+  fx::kin_edges(k, sh, 0.0, r);
+  __syncthreads();
+  fx::kin_products(k, sh, r);
+  __syncthreads();
+  const bool taken = r.ok_x && fx::kin_determinant(sh) >= fx::kMinDet;
+  const bool live = slot < E;
+  double g[12], n[5];
+#pragma unroll
+  for (int q = 0; q < 12; ++q) g[q] = fx::to_double(r.g[q], -r.s);
+#pragma unroll
+  for (int f = 0; f < 5; ++f) n[f] = fx::to_double(r.n[f], 64 - 2 * r.s);
+  if (__syncthreads_or(live && !taken)) {
+    KinSums sums;
+    KinTaped t;
+    double v[8] = {};
+    kin_fp64(k, RealSlots{reinterpret_cast<double*>(column) + lane, kFixedElems}, r.x, v, 0.0, sums, t);
+    if (!taken) {
+#pragma unroll
+      for (int q = 0; q < 12; ++q) g[q] = t.g[q];
+#pragma unroll
+      for (int f = 0; f < 5; ++f) n[f] = t.n[f];
+    }
+  }
   if (!live) return;
-  if (r.ok) {
-    // coordinate k also takes direction k (xi, eta, zeta) of the monotonic-Q
-    // gradients (src/domain.jl:2175-2320): with the reference's dxi = W_xi/4
-    // etc., delx = 16*vol/sqrt(|A|^2 + 256*ptiny) and delv = norm/64 *
-    // (A . W(v)) for the cross product A of two Walsh vectors (of the size the
-    // fixed-point form takes, |A|^2 is far above 256*ptiny = 2.56e-34)
-    double* const delx = k == 0 ? d.delx_xi : k == 1 ? d.delx_eta : d.delx_zeta;
-    double* const delv = k == 0 ? d.delv_xi : k == 1 ? d.delv_eta : d.delv_zeta;
-    const double norm64 = __longlong_as_double(sh.get(fx::KS_MID));
-    const double rs = rsqrt(fx::kin_area(sh, r, k));
-    delx[e] = (16.0 * volq) * rs;
-    delv[e] = norm64 * fx::kin_flow(sh, r, k);
-    if (AUX) {
-      double* const dd = k == 0 ? d.dxx : k == 1 ? d.dyy : d.dzz;
-      const double inv = __longlong_as_double(sh.get(fx::KS_MID + 1));
-      const double vdov = __longlong_as_double(sh.get(fx::KS_MID + 2));
-      const double own = fx::to_double(sh.get(fx::KS_SUM + fx::kSums * k + fx::SUM_RATE), 131 - 2 * r.s - r.sv);
-      dd[e] = own * inv - vdov / 3.0;
-    }
-    if (TAPE) {
-      kin_tape(37 + k, rs);
-      if (k == 0) kin_tape(44, rcl);
+  if (d.tapeGeoNext)
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        kin_tape(3 * k + a, fx::to_double(r.w[a], 2 - r.s));
-        kin_tape(9 + 3 * k + a, fx::to_double(r.vw[a], 2 - r.sv));
-        kin_tape(18 + 3 * a + k, fx::to_double(r.C[a], 68 - 2 * r.s));
-        kin_tape(28 + 3 * a + k, fx::to_double(r.A[a], 68 - 2 * r.s));
-        kin_tape(81 + 3 * a + k, fx::to_double(r.gU[a], 64 - 2 * r.s));
-      }
-      // the 12 diagonals in the order d61 d70 d63 d20 d50 d64 d31 d72 d43 d57
-      // d14 d25 (force-order index, sign)
-      constexpr int gi[12] = {4, 9, 7, 0, 2, 10, 1, 6, 8, 11, 3, 5};
+    for (int f = 0; f < 5; ++f) d.tapeGeoNext[(48 + 6 * k + f) * E + e] = n[f];
+  if (d.tapeDiag)
 #pragma unroll
-      for (int q = 0; q < 12; ++q)
-        kin_tape(45 + 3 * q + k, fx::to_double(q == 1 || q == 2 ? -r.g[gi[q]] : r.g[gi[q]], -r.s));
-      // the largest face's cross product in the reference's face order, the
-      // last two faces with reversed diagonals
-      const int place = (int)sh.get(fx::KS_MID + 1);
-      const long long c = place == 0 ? r.n[0] : place == 1 ? r.n[5] : place == 2 ? r.n[1] : place == 3 ? r.n[2]
-                                          : place == 4 ? -r.n[3] : -r.n[4];
-      kin_tape(41 + k, fx::to_double(c, 64 - 2 * r.s));
-      if (k == 0) d.tapeFlags[e] = (unsigned long long)place << TF_FACE_SHIFT;
-    }
-  } else if (k == 0) {
-    kin_fp64<AUX, TAPE>(d, st, e, dt, !r.ok_x);
-  }
-  if (TAPE && d.tapeGeoNext && r.ok_x) {
-    // the next cycle's face normals, for its hourglass transpose
-#pragma unroll
-    for (int f = 0; f < 5; ++f) d.tapeGeoNext[(48 + 6 * k + f) * E + e] = fx::to_double(r.n[f], 64 - 2 * r.s);
-  }
+    for (int q = 0; q < 12; ++q) d.tapeDiag[(3 * q + k) * E + e] = g[q];
 }
 
 // ---------------------------------------------------------------------------
