@@ -44,7 +44,7 @@ struct ForceScalars {
 // value), tape and errors as in the fixed-point phases.
 template <int MODE, class Out, class Tape>
 __device__ __forceinline__ void force_fp64(int k, const RealSlots& sh, const double x[8], const double v[8],
-                                           const ForceScalars& c, bool mine, DevState* st, Out out, Tape tape) {
+                                           const ForceScalars& c, bool mine, unsigned* status, Out out, Tape tape) {
   using namespace fx;
   const int at = FS_GEO + 18 * k, i1 = FS_GEO + 18 * (k == 2 ? 0 : k + 1), i2 = FS_GEO + 18 * (k == 0 ? 2 : k - 1);
   double hm[4], w1;
@@ -104,8 +104,8 @@ __device__ __forceinline__ void force_fp64(int k, const RealSlots& sh, const dou
   }
   __syncthreads();
   if (mine && k == 0) {
-    if (le_zero(sh[FS_DET] + sh[FS_DET + 1] + sh[FS_DET + 2])) atomicOr(&st->status, ST_EARLY);
-    if (le_zero(c.v)) atomicOr(&st->status, ST_HOURGLASS);
+    if (le_zero(sh[FS_DET] + sh[FS_DET + 1] + sh[FS_DET + 2])) atomicOr(status, ST_EARLY);
+    if (le_zero(c.v)) atomicOr(status, ST_HOURGLASS);
   }
 #pragma unroll
   for (int j = 0; j < 11; ++j) {

@@ -70,7 +70,7 @@ __device__ __noinline__ void force_fallback(const DevDomain& d, DevState* st, fx
   c.s8 = ((-LDG(&d.p[e])) - LDG(&d.q[e])) * 0.125;
   c.hourglass = gt_zero(hgcoef);
   double* const out = (k == 0 ? d.fcx : k == 1 ? d.fcy : d.fcz) + e;
-  force_fp64<MODE>(k, RealSlots{reinterpret_cast<double*>(column) + lane, kFixedElems}, x, v, c, mine, st,
+  force_fp64<MODE>(k, RealSlots{reinterpret_cast<double*>(column) + lane, kFixedElems}, x, v, c, mine, &st->status,
                    [&](int n, double f) { out[n * E] = f; }, ForceTape<TAPE>{TAPE ? d.tapeGeo + e : nullptr, E, true});
 }
 
