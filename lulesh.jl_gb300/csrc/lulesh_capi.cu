@@ -520,9 +520,10 @@ int lulesh_lagrange_leapfrog(lulesh_domain* d) {
   const Params prm = make_params(d);
   state_to_device_mirror(d);
   int rc;
-  if ((rc = h2d(d->dd.st, d->hst, 1, d->stream))) return rc;
+  launch_put_state(d->dd.st, *d->hst, d->stream);
   if ((rc = launch_step(d, prm, false, d->timing))) return rc;
-  if ((rc = d2h(d->hst, d->dd.st, 1, d->stream))) return rc;
+  launch_get_state(d->dd.st, d->hst, d->stream);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(d->stream));
   if (d->timing && (rc = collect_times(d))) return rc;
   state_from_device_mirror(d);
@@ -538,7 +539,7 @@ int lulesh_run(lulesh_domain* d, int64_t num_iters, lulesh_scalars* out) {
   d->hst->num_iters = num_iters;
   int rc;
   cudaStream_t s = d->stream;
-  if ((rc = h2d(d->dd.st, d->hst, 1, s))) return rc;
+  launch_put_state(d->dd.st, *d->hst, s);
   // cycles the loop can still take: the first always runs, later ones while cycle < num_iters
   const int64_t cyc0 = d->cycle_i();
   const int64_t budget = std::max<int64_t>(1, num_iters - cyc0);
@@ -584,7 +585,8 @@ int lulesh_run(lulesh_domain* d, int64_t num_iters, lulesh_scalars* out) {
         CK(cudaGraphLaunch(d->graph, s));
         launched += kGraphCycles;
       }
-      if ((rc = d2h(d->hst, d->dd.st, 1, s))) return rc;
+      launch_get_state(d->dd.st, d->hst, s);
+      CK(cudaGetLastError());
       CK(cudaStreamSynchronize(s));
     } while (!d->hst->done && launched < budget);
   }

@@ -1043,6 +1043,22 @@ void launch_material(const DevDomain& d, const Params& prm, bool aux, const Tuni
 #undef LULESH_MAT
 }
 
+// One problem's step state to and from the device by kernels of the cycle's
+// chain: a copy of 96 bytes goes through the copy engine, which waits for the
+// kernel before it to flush and holds up the one after it.
+__global__ void k_put_state(DevState* st, DevState value) {
+  wait_for_last_kernel();
+  if (threadIdx.x == 0) *st = value;
+}
+__global__ void k_get_state(const DevState* st, DevState* host) {
+  wait_for_last_kernel();
+  if (threadIdx.x == 0) *host = *st;
+}
+void launch_put_state(DevState* st, const DevState& value, cudaStream_t s) { launch(k_put_state, 1, 32, s, st, value); }
+void launch_get_state(const DevState* st, DevState* pinned, cudaStream_t s) {
+  launch(k_get_state, 1, 32, s, st, pinned);
+}
+
 void launch_time_increment(DevState* st, int n, const Params& prm, cudaStream_t s) {
   launch(k_time_increment, (n + 127) / 128, 128, s, st, n, prm);
 }

@@ -36,6 +36,9 @@ void launch_node(const DevDomain& d, const Params& prm, bool aux, const Tuning& 
 void launch_kinematics(const DevDomain& d, const Params& prm, bool aux, cudaStream_t s);
 void launch_material(const DevDomain& d, const Params& prm, bool aux, const Tuning& t, cudaStream_t s);
 void launch_time_increment(DevState* st, int n, const Params& prm, cudaStream_t s);
+// One problem's step state to the device, and to pinned host memory.
+void launch_put_state(DevState* st, const DevState& value, cudaStream_t s);
+void launch_get_state(const DevState* st, DevState* pinned, cudaStream_t s);
 
 // Picks block sizes for the four step kernels by timing them on the live
 // problem (lulesh_tune.cu); the state advances, so callers save and restore it.
