@@ -304,8 +304,8 @@ static void tape_cycle(lulesh_adjoint* a, StateBuf& slot, const CycleTape& tp, c
   lulesh_domain* d = a->dom;
   const Params prm = make_params(d);
   const int nmax = std::max(a->E, a->N);
-  ka_tape_begin<<<(nmax + kAdjBlock - 1) / kAdjBlock, kAdjBlock, 0, s>>>(domain_set(a), buf_set(slot), a->E, a->N,
-                                                                        d->dd.st, rec, prm);
+  launch(ka_tape_begin, (nmax + kAdjBlock - 1) / kAdjBlock, kAdjBlock, s, domain_set(a), buf_set(slot), a->E, a->N,
+         d->dd.st, rec, prm);
   DevDomain td = d->dd;
   td.vnew = tp.vnew; td.delv = tp.delv; td.arealg = tp.arealg; td.vdov = tp.vdov;
   td.delv_xi = tp.dv[0]; td.delv_eta = tp.dv[1]; td.delv_zeta = tp.dv[2];
@@ -320,7 +320,7 @@ static void tape_cycle(lulesh_adjoint* a, StateBuf& slot, const CycleTape& tp, c
   launch_kinematics(td, prm, false, s);
   launch_material(td, prm, false, d->tuning, s);
   const int ge = (a->E + kAdjBlock - 1) / kAdjBlock;
-  ka_tape_close<<<ge, kAdjBlock, 0, s>>>(tp.dtc, tp.dth, a->E, d->dd.st, rec);
+  launch(ka_tape_close, ge, kAdjBlock, s, tp.dtc, tp.dth, a->E, d->dd.st, rec);
 }
 
 static void set_cycle_pointers(lulesh_adjoint* a, const StateBuf& s0, const StateBuf& s1, const CycleTape& t) {
@@ -345,19 +345,20 @@ static void reverse_cycle(lulesh_adjoint* a, const CycleRec* rec, cudaStream_t s
   lulesh_domain* d = a->dom;
   const Params prm = make_params(d);
   const int ge = (a->E + kAdjBlock - 1) / kAdjBlock, gn = (a->N + kAdjBlock - 1) / kAdjBlock;
+  const int g3 = (a->E + kFixedElems - 1) / kFixedElems, b3 = 3 * kFixedElems;  // one thread per coordinate
   const int mode = d->dd.mode;
   const double irho0 = 1.0 / prm.refdens;
-  if (mode & 4) ka_material<4><<<ge, kAdjBlock, 0, s>>>(a->ad, prm, irho0, rec, a->dsc);
-  else ka_material<0><<<ge, kAdjBlock, 0, s>>>(a->ad, prm, irho0, rec, a->dsc);
+  if (mode & 4) launch(ka_material<4>, ge, kAdjBlock, s, a->ad, prm, irho0, rec, a->dsc);
+  else launch(ka_material<0>, ge, kAdjBlock, s, a->ad, prm, irho0, rec, a->dsc);
   const double hg = d->sc[LULESH_S_HGCOEF];
   // ka_kinematics also gathers the limiter's neighbour reads and does the
   // position transpose of the next cycle's k_force; ka_node gathers the
   // corners; ka_hourglass leaves this cycle's force terms for the
   // ka_kinematics of the cycle before (or ka_force_geo after the first cycle)
-#define LULESH_KA_CYCLE(M)                                            \
-  ka_kinematics<M><<<ge, kAdjBlock, 0, s>>>(a->ad, rec);              \
-  ka_node<<<gn, kAdjBlock, 0, s>>>(a->ad, rec);                       \
-  ka_hourglass<M><<<ge, kAdjBlock, 0, s>>>(a->ad, hg)
+#define LULESH_KA_CYCLE(M)                            \
+  launch(ka_kinematics<M>, g3, b3, s, a->ad, rec);    \
+  launch(ka_node, gn, kAdjBlock, s, a->ad, rec);      \
+  launch(ka_hourglass<M>, g3, b3, s, a->ad, hg)
   switch (mode & 3) {
     case 0: LULESH_KA_CYCLE(0); break;
     case 1: LULESH_KA_CYCLE(1); break;
@@ -365,7 +366,7 @@ static void reverse_cycle(lulesh_adjoint* a, const CycleRec* rec, cudaStream_t s
     default: LULESH_KA_CYCLE(3); break;
   }
 #undef LULESH_KA_CYCLE
-  ka_cycle_close<<<1, kCloseBlock, 0, s>>>(a->ad, ge, gn, rec, a->dsc, prm);
+  launch(ka_cycle_close, 1, kCloseBlock, s, a->ad, g3, gn, rec, a->dsc, prm);
 }
 
 // Position transpose of the run's first cycle's k_force (the last one the
@@ -467,7 +468,8 @@ int lulesh_adj_create(lulesh_domain* dom, double radius, int32_t checkpoint_ever
   if ((rc = alloc_set(a, a->allocs, a->sets[0]))) return fail(rc);
   if ((rc = alloc_state(a, a->final_state))) return fail(rc);
   AdjDev& ad = a->ad;
-  const int ge = (E + kAdjBlock - 1) / kAdjBlock, gn = (N + kAdjBlock - 1) / kAdjBlock;
+  const int gn = (N + kAdjBlock - 1) / kAdjBlock;
+  const int g3 = (E + kFixedElems - 1) / kFixedElems;
   if ((rc = dalloc(a, &ad.lx, N)) || (rc = dalloc(a, &ad.ly, N)) || (rc = dalloc(a, &ad.lz, N)) ||
       (rc = dalloc(a, &ad.lxd, N)) || (rc = dalloc(a, &ad.lyd, N)) || (rc = dalloc(a, &ad.lzd, N)) ||
       (rc = dalloc(a, &ad.lfx, N)) || (rc = dalloc(a, &ad.lfy, N)) || (rc = dalloc(a, &ad.lfz, N)) ||
@@ -478,8 +480,8 @@ int lulesh_adj_create(lulesh_domain* dom, double radius, int32_t checkpoint_ever
       (rc = dalloc(a, &ad.cV, 24 * (size_t)E)) || (rc = dalloc(a, &ad.fX, 24 * (size_t)E)) ||
       (rc = dalloc(a, &ad.fV, 24 * (size_t)E)) || (rc = dalloc(a, &ad.sLdv, 24 * (size_t)E)) ||
       (rc = dalloc(a, &ad.sLU, 15 * (size_t)E)) || (rc = dalloc(a, &ad.sLhm, 12 * (size_t)E)) ||
-      (rc = dalloc(a, &ad.part_dt, std::max(ge, gn))) ||
-      (rc = dalloc(a, &ad.part_dtn, gn)) || (rc = dalloc(a, &ad.part_hg, ge)) || (rc = dalloc(a, &a->scal, 4)) ||
+      (rc = dalloc(a, &ad.part_dt, std::max(g3, gn))) ||
+      (rc = dalloc(a, &ad.part_dtn, gn)) || (rc = dalloc(a, &ad.part_hg, g3)) || (rc = dalloc(a, &a->scal, 4)) ||
       (rc = dalloc(a, &a->dsc, 1)) || (rc = dalloc(a, &a->we, E)) || (rc = dalloc(a, &a->wn, N)) ||
       (rc = dalloc(a, &a->fx_s, N)) || (rc = dalloc(a, &a->fy_s, N)) || (rc = dalloc(a, &a->fz_s, N)))
     return fail(rc);

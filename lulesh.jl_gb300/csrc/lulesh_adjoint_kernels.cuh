@@ -16,6 +16,9 @@
 #include <climits>
 
 #include "lulesh_device.cuh"
+#include "lulesh_fixed_force.cuh"
+#include "lulesh_kernels.h"
+#include "lulesh_launch.cuh"
 
 namespace lulesh {
 
@@ -90,6 +93,16 @@ __device__ __forceinline__ void block_sum_to(double v, double* out) {
   if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
+// The same for a block of one thread per element and coordinate.
+__device__ __forceinline__ void block_sum3_to(double v, double* out) {
+  __shared__ double part[3];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) out[blockIdx.x] = (part[0] + part[1]) + part[2];
+}
+
 struct V3 {
   double x, y, z;
 };
@@ -126,6 +139,7 @@ __global__ void __launch_bounds__(kAdjBlock, 4) ka_material(AdjDev a, Params prm
   const int E = a.E;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= E) return;
+  wait_for_last_kernel();
   // the cycle's Courant/hydro minima pass their adjoint to the element that
   // attained them
   const int argmin_c = rec->argmin_c, argmin_h = rec->argmin_h;
@@ -313,6 +327,13 @@ __global__ void __launch_bounds__(kAdjBlock, 4) ka_material(AdjDev a, Params prm
   for (int d = 0; d < 3; ++d) {
     const int src = (int)((fl >> (3 * d)) & 7ull);
     double Ldm = 0.0, Ldp = 0.0;
+    if (qzero) {  // the limiter was not used
+      a.lnb[(2 * d) * E + i] = 0.0;
+      a.lnb[(2 * d + 1) * E + i] = 0.0;
+      a.ldv[d][i] = 0.0;
+      a.ldx[d][i] = 0.0;
+      continue;
+    }
     if (src == PHI_MEAN) { Ldm = 0.5 * Lphi[d]; Ldp = 0.5 * Lphi[d]; }
     else if (src == PHI_M) Ldm = prm.monoq_limiter_mult * Lphi[d];
     else if (src == PHI_P) Ldp = prm.monoq_limiter_mult * Lphi[d];
@@ -369,231 +390,226 @@ __device__ __forceinline__ void walsh_modes_t(const double t[4], double out[8]) 
 // Hessian-vector product merges with this cycle's volume gradient, and its
 // stress terms add to the same face-diagonal adjoints, scattered once.
 // ---------------------------------------------------------------------------
-template <int MODE>
-__global__ void __launch_bounds__(kAdjBlock, 3) ka_kinematics(AdjDev a, const CycleRec* rec) {
-  const int E = a.E;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  const double dt = rec->dt;
-  double Ldt = 0.0;
-  if (e < E) {
-    // forward values from the kinematics kernel's tape (slots: see tapeKin)
-    auto tk = [&](int q) { return a.kin[q * E + e]; };
+//
+// Three threads per element, one per coordinate and each in a warp of its own,
+// as in the forward kernels: a thread forms its component of every product,
+// and what a cross product needs of the other components is in shared memory.
+// Every cross product adds onto its target in two FMAs.
+enum : int {
+  // per coordinate: mean edges, half-step edges, tape's 12 diagonals, U vectors,
+  // the differences of dL/ddv along V and W, the stress faces' terms; then the
+  // adjoints of the edges' cross products and of the cofactors, Lv12 U + dU and
+  // the characteristic face's term
+  KA_W = 0, KA_F = 3, KA_D = 6, KA_U = 18, KA_DV = 21, KA_DW = 24, KA_LN = 27,
+  KA_LA = 32, KA_LC = 35, KA_A = 38, KA_LF = 41, KA_COMP = 42,
+  // per direction d: 2 Ls2, Ldv norm64, Ldv, its part of Lvol; 3 k + d: dot terms
+  KA_DIR = 3 * KA_COMP, KA_DOT = KA_DIR + 12, KA_COUNT = KA_DOT + 9
+};
 
-    const double vnew = a.vnew[e], volo = a.volo[e];
-    double Lvnew = a.lvnew[e] + a.ldelv[e];
-    a.lv[e] -= a.ldelv[e];  // delv = vnew - v
-    // Walsh vectors of positions and velocities
-    V3 W[3], VW[3];
+template <int MODE>
+__global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, const CycleRec* rec) {
+  __shared__ double column[KA_COUNT * kFixedElems];
+  const int E = a.E;
+  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  const int slot = blockIdx.x * kFixedElems + lane;
+  const bool live = slot < E;
+  const int e = live ? slot : E - 1;  // threads past the end repeat the last element and store nothing
+  wait_for_last_kernel();
+  const double dt = rec->dt;
+  auto sh = [&](int i) -> double& { return column[i * kFixedElems + lane]; };
+  const int own = KA_COMP * k, c1 = KA_COMP * (k == 2 ? 0 : k + 1), c2 = KA_COMP * (k == 0 ? 2 : k - 1);
+  // component k of (slot p) x (slot q), added to y
+  auto add_cross = [&](double y, int p, int q) {
+    return fma(sh(c1 + p), sh(c2 + q), fma(-sh(c2 + p), sh(c1 + q), y));
+  };
+  // forward values from the kinematics kernel's tape (slots: see tapeKin)
+  auto tk = [&](int q) { return a.kin[q * E + e]; };
+
+  const double vnew = a.vnew[e], volo = a.volo[e], inv_volo = a.inv_volo[e];
+  const double vol = volo * vnew, norm64 = tk(40);  // norm64 = 1/(64 vol + 64 ptiny)
+  const double inv = tk(27), lvdov = a.lvdov[e];
+  const double Ls = lvdov * inv, Ldet = -lvdov * a.vdov[e] * inv;
+  const double ldelv = a.ldelv[e], Lar = a.larealg[e], lvnew_in = a.lvnew[e];
+  if (live && k == 0) a.lv[e] -= ldelv;  // delv = vnew - v
+  double A[3], VW[3], C[3], dU[3];
+  {
+    // direction k: limiter reads of this element's delv by its neighbours
+    // (inverse neighbour list, fixed order) join its own delv adjoint
+    double Ldv = a.ldv[k][e];
+    for (int j = a.nbStart[e]; j < a.nbStart[e + 1]; ++j) {
+      const int ent = a.nbList[j];
+      if (((ent / E) >> 1) == k) Ldv += a.lnb[ent];
+    }
+    const double rs = tk(37 + k);  // 1/sqrt(|A|^2 + 256 ptiny)
+    const double t = a.ldx[k][e] * 16.0 * rs;
+    sh(KA_DIR + k) = -(t * vol) * (rs * rs);  // 2 Ls2, Ls2 = Ldx 16 vol (-1/2) rs^3
+    sh(KA_DIR + 3 + k) = Ldv * norm64;
+    sh(KA_DIR + 6 + k) = Ldv;
+    sh(KA_DIR + 9 + k) = t;
+    const double dt2 = -0.5 * dt;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      W[d] = v3(tk(d), tk(3 + d), tk(6 + d));
-      VW[d] = v3(tk(9 + d), tk(12 + d), tk(15 + d));
+      const double w = tk(3 * k + d);
+      VW[d] = tk(9 + 3 * k + d);
+      A[d] = tk(28 + 3 * d + k);
+      C[d] = tk(18 + 3 * d + k);
+      sh(own + KA_W + d) = w;
+      sh(own + KA_F + d) = fma(dt2, VW[d], w);
+      sh(KA_DOT + 3 * k + d) = A[d] * VW[d];
     }
-    V3 LW[3] = {v3(0, 0, 0), v3(0, 0, 0), v3(0, 0, 0)}, LVW[3] = {v3(0, 0, 0), v3(0, 0, 0), v3(0, 0, 0)};
-    // ---- monotonic-Q gradients ----
-    {
-      const double vol = volo * vnew;
-      const double norm64 = tk(40);  // 1/(64 vol + 64 ptiny)
-      double Lvol = 0.0, Lnorm64 = 0.0;
-      // limiter reads of this element's delv by its neighbours (inverse
-      // neighbour list, fixed order) join its own delv adjoints
-      double Ldvs[3] = {a.ldv[0][e], a.ldv[1][e], a.ldv[2][e]};
-      for (int j = a.nbStart[e]; j < a.nbStart[e + 1]; ++j) {
-        const int ent = a.nbList[j];
-        const int dir = (ent / E) >> 1;
-        const double v = a.lnb[ent];
-        if (dir == 0) Ldvs[0] += v;
-        else if (dir == 1) Ldvs[1] += v;
-        else Ldvs[2] += v;
-      }
-      // direction d uses A = P x Q and velocity vector VW[d]
-      const int Pi[3] = {1, 2, 0}, Qi[3] = {2, 0, 1};
+    // the 12 diagonals of the new positions: d61 d70 d63 d20 d50 d64 d31 d72
+    // d43 d57 d14 d25
+    double g[12];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const V3 P = W[Pi[d]], Q = W[Qi[d]];
-        const V3 A = v3(tk(28 + 3 * d), tk(29 + 3 * d), tk(30 + 3 * d));  // P x Q
-        const double rs = tk(37 + d);  // 1/sqrt(|A|^2 + 256 ptiny)
-        const double Ldx = a.ldx[d][e], Ldv = Ldvs[d];
-        Lvol += Ldx * 16.0 * rs;
-        const double Ls2 = Ldx * 16.0 * vol * (-0.5) * rs * rs * rs;
-        V3 LA = v3(2.0 * A.x * Ls2, 2.0 * A.y * Ls2, 2.0 * A.z * Ls2);
-        const double dot = vdot(A, VW[d]);
-        Lnorm64 += Ldv * dot;
-        vaxpy(LA, Ldv * norm64, VW[d]);
-        vaxpy(LVW[d], Ldv * norm64, A);
-        vadd(LW[Pi[d]], vcross(Q, LA));
-        vadd(LW[Qi[d]], vcross(LA, P));
-      }
-      Lvol += Lnorm64 * (-64.0 * norm64 * norm64);
-      Lvnew += Lvol * volo;
+    for (int q = 0; q < 12; ++q) {
+      g[q] = tk(45 + 3 * q + k);
+      sh(own + KA_D + q) = g[q];
     }
-    // ---- velocity-gradient trace at the half step ----
-    {
-      const double dt2 = -0.5 * dt;
-      V3 F[3];
+    sh(own + KA_U) = g[6] + g[7];
+    sh(own + KA_U + 1) = g[8] + g[9];
+    sh(own + KA_U + 2) = g[10] + g[11];
+    // The next cycle's force kernel used the gradient of 12*volume (its
+    // voluDer, dv): G = dL/ddv (zero before the first transposed cycle; the
+    // faithful slots 1 and 3 swapped back) makes its transpose the
+    // Hessian-vector product of the same triple products along G; dU, dV, dW
+    // are the differences of G along U, V, W.
+    double G[8];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        F[d] = v3(fma(dt2, VW[d].x, W[d].x), fma(dt2, VW[d].y, W[d].y), fma(dt2, VW[d].z, W[d].z));
-      }
-      // cofactor columns C0 = F1 x F2, C1 = F2 x F0, C2 = F0 x F1 and 1/det
-      const V3 C0 = v3(tk(18), tk(19), tk(20)), C1 = v3(tk(21), tk(22), tk(23)), C2 = v3(tk(24), tk(25), tk(26));
-      const double inv = tk(27);
-      const double vdov = a.vdov[e];
-      const double Ls = a.lvdov[e] * inv;
-      const double Ldet = -a.lvdov[e] * vdov * inv;
-      V3 LC[3];
-      LC[0] = v3(Ls * VW[0].x, Ls * VW[0].y, Ls * VW[0].z);
-      LC[1] = v3(Ls * VW[1].x, Ls * VW[1].y, Ls * VW[1].z);
-      LC[2] = v3(Ls * VW[2].x, Ls * VW[2].y, Ls * VW[2].z);
-      vaxpy(LVW[0], Ls, C0);
-      vaxpy(LVW[1], Ls, C1);
-      vaxpy(LVW[2], Ls, C2);
-      vaxpy(LC[1], Ldet, F[1]);
-      V3 LF[3] = {v3(0, 0, 0), v3(0, 0, 0), v3(0, 0, 0)};
-      vaxpy(LF[1], Ldet, C1);
-      // C0 = F1 x F2, C1 = F2 x F0, C2 = F0 x F1
-      vadd(LF[1], vcross(F[2], LC[0])); vadd(LF[2], vcross(LC[0], F[1]));
-      vadd(LF[2], vcross(F[0], LC[1])); vadd(LF[0], vcross(LC[1], F[2]));
-      vadd(LF[0], vcross(F[1], LC[2])); vadd(LF[1], vcross(LC[2], F[0]));
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        vadd(LW[d], LF[d]);
-        vaxpy(LVW[d], dt2, LF[d]);
-        Ldt += -0.5 * vdot(LF[d], VW[d]);
-      }
+    for (int c = 0; c < 8; ++c) {
+      const int src = (MODE & 2) ? c : c == 1 ? 3 : c == 3 ? 1 : c;
+      G[c] = a.sLdv[(k * 8 + src) * E + e];
     }
-    // Walsh transposes; the position corners start from the next cycle's
-    // hourglass-mode transpose Gamma^T dL/dhm
-    double LX[3][8], LV[3][8];
+    dU[0] = (G[3] - G[1]) + (G[7] - G[2]);
+    dU[1] = (G[4] - G[3]) + (G[5] - G[7]);
+    dU[2] = (G[1] - G[4]) + (G[2] - G[5]);
+    sh(own + KA_DV) = G[6] - G[3];
+    sh(own + KA_DV + 1) = G[6] - G[4];
+    sh(own + KA_DV + 2) = G[6] - G[1];
+    sh(own + KA_DW) = G[2] - G[0];
+    sh(own + KA_DW + 1) = G[7] - G[0];
+    sh(own + KA_DW + 2) = G[5] - G[0];
+    // The next cycle's stress force: face f's normal d1 x d2 with LN = s8 LU_f
+    // gives d1 the adjoint d2 x LN and d2 the adjoint LN x d1; s8 from this
+    // cycle's end state.
+    const double s8 = ((-a.p1[e]) - a.q1[e]) * 0.125;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      double t[4];
-#pragma unroll
-      for (int m = 0; m < 4; ++m) t[m] = a.sLhm[(k * 4 + m) * E + e];
-      walsh_modes_t(t, LX[k]);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) LV[k][c] = 0.0;
-    }
-    {
-      const double lwx[3] = {LW[0].x, LW[1].x, LW[2].x}, lwy[3] = {LW[0].y, LW[1].y, LW[2].y},
-                   lwz[3] = {LW[0].z, LW[1].z, LW[2].z};
-      walsh1_t(lwx, LX[0]); walsh1_t(lwy, LX[1]); walsh1_t(lwz, LX[2]);
-      const double lvx[3] = {LVW[0].x, LVW[1].x, LVW[2].x}, lvy[3] = {LVW[0].y, LVW[1].y, LVW[2].y},
-                   lvz[3] = {LVW[0].z, LVW[1].z, LVW[2].z};
-      walsh1_t(lvx, LV[0]); walsh1_t(lvy, LV[1]); walsh1_t(lvz, LV[2]);
-    }
-    // the velocity corners, plus the hourglass velocity corners of the cycle
-    // after this one
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int c = 0; c < 8; ++c) a.cV[(k * 8 + c) * E + e] = LV[k][c] + a.fV[(k * 8 + c) * E + e];
-    // ---- volume and characteristic length, and the position transpose of
-    //      the next cycle's k_force (same positions, same face diagonals) ----
-    {
-      // the 12 diagonals of the new positions are on the tape in the order
-      // d61 d70 d63 d20 d50 d64 d31 d72 d43 d57 d14 d25
-      auto dg = [&](int q) { return v3(tk(45 + 3 * q), tk(46 + 3 * q), tk(47 + 3 * q)); };
-      const double volume = vnew * volo;  // vnew = volume / volo
-      // characteristic length from the face the tape recorded: its diagonals
-      // fa, fb (kinematics face order (d20, d31) (d64, d57) (d50, d14)
-      // (d61, d25) (d72, d63) (d43, d70))
-      const int f = (int)((a.flags[e] >> TF_FACE_SHIFT) & 7ull);
-      const int qa = f == 0 ? 3 : f == 1 ? 5 : f == 2 ? 4 : f == 3 ? 0 : f == 4 ? 7 : 8;
-      const int qb = f == 0 ? 6 : f == 1 ? 9 : f == 2 ? 10 : f == 3 ? 11 : f == 4 ? 2 : 1;
-      const V3 nf = v3(tk(41), tk(42), tk(43));  // fa x fb
-      const double rsc = tk(44);                  // 1/|fa x fb|
-      const double Lar = a.larealg[e];
-      double Lvolume = Lar * 2.0 * rsc + Lvnew * a.inv_volo[e];
-      const double Lcl = Lar * 2.0 * volume * (-0.5) * rsc * rsc * rsc;
-      const V3 Ln = v3(2.0 * nf.x * Lcl, 2.0 * nf.y * Lcl, 2.0 * nf.z * Lcl);
-      const V3 Lfa = vcross(dg(qb), Ln), Lfb = vcross(Ln, dg(qa));
-      const double Lv12 = Lvolume * (1.0 / 12.0);
-      // The next cycle's force kernel used the gradient of 12*volume (its
-      // voluDer, dv): G = dL/ddv (zero before the first transposed cycle;
-      // the faithful slots 1 and 3 swapped back) makes its transpose the
-      // Hessian-vector product of the same triple products along G. With
-      // this cycle's Lv12 * gradient: dL/dU = Lv12 (V x W) + dV x W + V x dW,
-      // dL/dV = W x (Lv12 U + dU) + dW x U, dL/dW = (Lv12 U + dU) x V + U x dV,
-      // dU, dV, dW the differences of G along U, V, W (V x W is taped).
-      double G[3][8];
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) G[j][c] = a.sLdv[(j * 8 + c) * E + e];
-      if (!(MODE & 2)) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) { const double t = G[j][1]; G[j][1] = G[j][3]; G[j][3] = t; }
-      }
-      auto gd = [&](int p, int q) { return v3(G[0][p] - G[0][q], G[1][p] - G[1][q], G[2][p] - G[2][q]); };
-      auto triple_t = [&](const V3& U, const V3& V, const V3& W, const V3& gUt, const V3& dU, const V3& dV,
-                          const V3& dW, V3& LUa, V3& LUb, V3& LVd, V3& LWd) {
-        V3 A = dU; vaxpy(A, Lv12, U);
-        V3 gU = vcross(dV, W); vadd(gU, vcross(V, dW)); vaxpy(gU, Lv12, gUt);
-        V3 gV = vcross(W, A); vadd(gV, vcross(dW, U));
-        V3 gW = vcross(A, V); vadd(gW, vcross(U, dV));
-        vadd(LUa, gU); vadd(LUb, gU); vadd(LVd, gV); vadd(LWd, gW);
-      };
-      // The next cycle's stress force: face f's normal d1 x d2 (its
-      // diagonals, force order: faces (d20, d31) (d50, d14) (d61, d25)
-      // (d72, d36) (d43, d07), d36 = -d63, d07 = -d70) with LN = s8 LU_f
-      // gives d1 the adjoint d2 x LN and d2 the adjoint LN x d1; s8 from
-      // this cycle's end state.
-      const double s8 = ((-a.p1[e]) - a.q1[e]) * 0.125;
-      auto LN = [&](int fc) {
-        return v3(s8 * a.sLU[(fc * 3) * E + e], s8 * a.sLU[(fc * 3 + 1) * E + e], s8 * a.sLU[(fc * 3 + 2) * E + e]);
-      };
-      auto put = [&](const V3& L, int p, int q) {
-        LX[0][p] += L.x; LX[1][p] += L.y; LX[2][p] += L.z;
-        LX[0][q] -= L.x; LX[1][q] -= L.y; LX[2][q] -= L.z;
-      };
-      const V3 z0 = v3(0, 0, 0);
-      // Each triple product's four diagonals take adjoints from it, from two
-      // or one of the stress faces and possibly the characteristic face, and
-      // from nothing else: three disjoint groups, each scattered once.
-      {  // (d31 + d72).(d63 x d20), faces 0 and 3, characteristic faces 0 and 4
-        const V3 d63 = dg(2), d20 = dg(3), d31 = dg(6), d72 = dg(7);
-        V3 L63 = z0, L20 = z0, L31 = z0, L72 = z0;
-        V3 U = d31; vadd(U, d72);
-        V3 dU = gd(3, 1); vadd(dU, gd(7, 2));
-        triple_t(U, d63, d20, v3(tk(81), tk(82), tk(83)), dU, gd(6, 3), gd(2, 0), L31, L72, L63, L20);
-        { const V3 n = LN(0); vadd(L20, vcross(d31, n)); vadd(L31, vcross(n, d20)); }
-        { const V3 n = LN(3); vadd(L72, vcross(n, d63)); vadd(L63, vcross(d72, n)); }
-        if (f == 0) { vadd(L20, Lfa); vadd(L31, Lfb); }
-        else if (f == 4) { vadd(L72, Lfa); vadd(L63, Lfb); }
-        put(L63, 6, 3); put(L20, 2, 0); put(L31, 3, 1); put(L72, 7, 2);
-      }
-      {  // (d43 + d57).(d64 x d70), face 4, characteristic faces 1 and 5
-        const V3 d70 = dg(1), d64 = dg(5), d43 = dg(8), d57 = dg(9);
-        V3 L70 = z0, L64 = z0, L43 = z0, L57 = z0;
-        V3 U = d43; vadd(U, d57);
-        V3 dU = gd(4, 3); vadd(dU, gd(5, 7));
-        triple_t(U, d64, d70, v3(tk(84), tk(85), tk(86)), dU, gd(6, 4), gd(7, 0), L43, L57, L64, L70);
-        { const V3 n = LN(4); vadd(L43, vcross(n, d70)); vadd(L70, vcross(d43, n)); }
-        if (f == 1) { vadd(L64, Lfa); vadd(L57, Lfb); }
-        else if (f == 5) { vadd(L43, Lfa); vadd(L70, Lfb); }
-        put(L70, 7, 0); put(L64, 6, 4); put(L43, 4, 3); put(L57, 5, 7);
-      }
-      {  // (d14 + d25).(d61 x d50), faces 1 and 2, characteristic faces 2 and 3
-        const V3 d61 = dg(0), d50 = dg(4), d14 = dg(10), d25 = dg(11);
-        V3 L61 = z0, L50 = z0, L14 = z0, L25 = z0;
-        V3 U = d14; vadd(U, d25);
-        V3 dU = gd(1, 4); vadd(dU, gd(2, 5));
-        triple_t(U, d61, d50, v3(tk(87), tk(88), tk(89)), dU, gd(6, 1), gd(5, 0), L14, L25, L61, L50);
-        { const V3 n = LN(1); vadd(L50, vcross(d14, n)); vadd(L14, vcross(n, d50)); }
-        { const V3 n = LN(2); vadd(L61, vcross(d25, n)); vadd(L25, vcross(n, d61)); }
-        if (f == 2) { vadd(L50, Lfa); vadd(L14, Lfb); }
-        else if (f == 3) { vadd(L61, Lfa); vadd(L25, Lfb); }
-        put(L61, 6, 1); put(L50, 5, 0); put(L14, 1, 4); put(L25, 2, 5);
-      }
-    }
-    // the position corners
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int c = 0; c < 8; ++c) a.cX[(k * 8 + c) * E + e] = LX[k][c];
+    for (int f = 0; f < 5; ++f) sh(own + KA_LN + f) = s8 * a.sLU[(3 * f + k) * E + e];
   }
-  block_sum_to(Ldt, a.part_dt);
+  __syncthreads();
+  // ---- scalars of the volume, and the adjoints that crosses take ----
+  double Lvnew = lvnew_in + ldelv, Lv12;
+  double LVW[3], LF[3];
+  {
+    double Lvol = 0.0, Lnorm64 = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double dot = (sh(KA_DOT + d) + sh(KA_DOT + 3 + d)) + sh(KA_DOT + 6 + d);
+      Lvol += sh(KA_DIR + 9 + d);
+      Lnorm64 = fma(sh(KA_DIR + 6 + d), dot, Lnorm64);
+      const double ldn = sh(KA_DIR + 3 + d);
+      sh(own + KA_LA + d) = fma(A[d], sh(KA_DIR + d), ldn * VW[d]);
+      LVW[d] = fma(ldn, A[d], Ls * C[d]);
+      // velocity-gradient trace: cofactor columns C and 1/det
+      sh(own + KA_LC + d) = d == 1 ? fma(Ldet, sh(own + KA_F + 1), Ls * VW[1]) : Ls * VW[d];
+    }
+    Lvol = fma(Lnorm64, -64.0 * norm64 * norm64, Lvol);
+    Lvnew = fma(Lvol, volo, Lvnew);
+    // characteristic length from the face the tape recorded
+    const double rsc = tk(44);  // 1/|fa x fb|
+    Lv12 = fma(Lar * 2.0, rsc, Lvnew * inv_volo) * (1.0 / 12.0);
+    // 2 Lcl, Lcl = Lar 2 volume (-1/2) rsc^3
+    sh(own + KA_LF) = tk(41 + k) * (-2.0 * (Lar * vol) * (rsc * rsc * rsc));
+#pragma unroll
+    for (int t = 0; t < 3; ++t) sh(own + KA_A + t) = fma(Lv12, sh(own + KA_U + t), dU[t]);
+  }
+  __syncthreads();
+  double Ldt = 0.0;
+  // ---- positions' and velocities' edges ----
+  double LW[3] = {0.0, 0.0, 0.0};
+  {
+    // direction d uses A = P x Q
+    constexpr int Pi[3] = {1, 2, 0}, Qi[3] = {2, 0, 1};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      LW[Pi[d]] = add_cross(LW[Pi[d]], KA_W + Qi[d], KA_LA + d);
+      LW[Qi[d]] = add_cross(LW[Qi[d]], KA_LA + d, KA_W + Pi[d]);
+    }
+    // C0 = F1 x F2, C1 = F2 x F0, C2 = F0 x F1
+    LF[0] = add_cross(add_cross(0.0, KA_LC + 1, KA_F + 2), KA_F + 1, KA_LC + 2);
+    LF[1] = add_cross(add_cross(Ldet * C[1], KA_F + 2, KA_LC), KA_LC + 2, KA_F);
+    LF[2] = add_cross(add_cross(0.0, KA_LC, KA_F + 1), KA_F, KA_LC + 1);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      LW[d] += LF[d];
+      LVW[d] = fma(-0.5 * dt, LF[d], LVW[d]);
+      Ldt = fma(LF[d], VW[d], Ldt);
+    }
+    Ldt *= -0.5;
+  }
+  // the velocity corners (the Walsh transpose), plus the hourglass velocity
+  // corners of the cycle after this one
+  {
+    const double p = LVW[0] + LVW[2], q = LVW[2] - LVW[0];
+    const double La = p + LVW[1], Lb = p - LVW[1], Lc = q + LVW[1], Ld = q - LVW[1];
+    const double LV[8] = {-La, -Lc, -Ld, -Lb, Ld, Lb, La, Lc};
+    if (live)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) a.cV[(k * 8 + c) * E + e] = LV[c] + a.fV[(k * 8 + c) * E + e];
+  }
+  // ---- volume and characteristic length, and the position transpose of the
+  //      next cycle's k_force (same positions, same face diagonals) ----
+  // dL/dU = Lv12 (V x W) + dV x W + V x dW, dL/dV = W x A + dW x U, dL/dW =
+  // A x V + U x dV with A = Lv12 U + dU (V x W is taped)
+  double L[12];
+  {
+    constexpr int iv[3] = {2, 5, 0}, iw[3] = {3, 1, 4}, ua[3] = {6, 8, 10}, ub[3] = {7, 9, 11};
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      const double gU = add_cross(add_cross(Lv12 * tk(81 + 3 * t + k), KA_DV + t, KA_D + iw[t]), KA_D + iv[t], KA_DW + t);
+      L[ua[t]] = gU;
+      L[ub[t]] = gU;
+      L[iv[t]] = add_cross(add_cross(0.0, KA_D + iw[t], KA_A + t), KA_DW + t, KA_U + t);
+      L[iw[t]] = add_cross(add_cross(0.0, KA_A + t, KA_D + iv[t]), KA_U + t, KA_DV + t);
+    }
+    // stress faces (d20, d31) (d50, d14) (d61, d25) (d72, d36) (d43, d07),
+    // d36 = -d63, d07 = -d70
+    L[3] = add_cross(L[3], KA_D + 6, KA_LN);
+    L[6] = add_cross(L[6], KA_LN, KA_D + 3);
+    L[4] = add_cross(L[4], KA_D + 10, KA_LN + 1);
+    L[10] = add_cross(L[10], KA_LN + 1, KA_D + 4);
+    L[0] = add_cross(L[0], KA_D + 11, KA_LN + 2);
+    L[11] = add_cross(L[11], KA_LN + 2, KA_D);
+    L[7] = add_cross(L[7], KA_LN + 3, KA_D + 2);
+    L[2] = add_cross(L[2], KA_D + 7, KA_LN + 3);
+    L[8] = add_cross(L[8], KA_LN + 4, KA_D + 1);
+    L[1] = add_cross(L[1], KA_D + 8, KA_LN + 4);
+    // characteristic face: diagonals fa, fb in the kinematics face order (d20,
+    // d31) (d64, d57) (d50, d14) (d61, d25) (d72, d63) (d43, d70)
+    const int f = (int)((a.flags[e] >> TF_FACE_SHIFT) & 7ull);
+    if (f == 0) { L[3] = add_cross(L[3], KA_D + 6, KA_LF); L[6] = add_cross(L[6], KA_LF, KA_D + 3); }
+    else if (f == 1) { L[5] = add_cross(L[5], KA_D + 9, KA_LF); L[9] = add_cross(L[9], KA_LF, KA_D + 5); }
+    else if (f == 2) { L[4] = add_cross(L[4], KA_D + 10, KA_LF); L[10] = add_cross(L[10], KA_LF, KA_D + 4); }
+    else if (f == 3) { L[0] = add_cross(L[0], KA_D + 11, KA_LF); L[11] = add_cross(L[11], KA_LF, KA_D); }
+    else if (f == 4) { L[7] = add_cross(L[7], KA_D + 2, KA_LF); L[2] = add_cross(L[2], KA_LF, KA_D + 7); }
+    else { L[8] = add_cross(L[8], KA_D + 1, KA_LF); L[1] = add_cross(L[1], KA_LF, KA_D + 8); }
+  }
+  // the position corners: the next cycle's hourglass-mode transpose Gamma^T
+  // dL/dhm, the edges' Walsh transpose, and the diagonals
+  double LX[8];
+  {
+    double t[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) t[m] = a.sLhm[(k * 4 + m) * E + e];
+    walsh_modes_t(t, LX);
+    walsh1_t(LW, LX);
+    constexpr int pp[12] = {6, 7, 6, 2, 5, 6, 3, 7, 4, 5, 1, 2}, pq[12] = {1, 0, 3, 0, 0, 4, 1, 2, 3, 7, 4, 5};
+#pragma unroll
+    for (int q = 0; q < 12; ++q) { LX[pp[q]] += L[q]; LX[pq[q]] -= L[q]; }
+  }
+  if (live)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) a.cX[(k * 8 + c) * E + e] = LX[c];
+  block_sum3_to(live ? Ldt : 0.0, a.part_dt);
 }
 
 // Sums the force corner buffers into node adjoints (added to what is there):
@@ -620,6 +636,7 @@ __global__ void __launch_bounds__(kAdjBlock) ka_gather_corners(AdjDev a) {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kAdjBlock) ka_node(AdjDev a, const CycleRec* rec) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  wait_for_last_kernel();
   const double dt = rec->dt;
   double Ldt = 0.0;
   if (i < a.N) {
@@ -672,29 +689,6 @@ __global__ void __launch_bounds__(kAdjBlock) ka_node(AdjDev a, const CycleRec* r
 // positions).
 // ---------------------------------------------------------------------------
 
-// The 8 volume derivatives (times 12) of one coordinate pair, in the forward
-// kernel's slot order: dv_x uses (ey, ez), dv_y (ex, ez), dv_z (ey, ex) with
-// the sign pattern of each.
-template <int MODE>
-__device__ __forceinline__ void volu_der(const double ex[12], const double ey[12], const double ez[12],
-                                         double dv[3][8]) {
-  constexpr int pe[8][6] = {{5, 3, 4, 8, 7, 9}, {3, 0, 2, 9, 6, 11}, {0, 1, 7, 11, 4, 10},
-                            {1, 5, 6, 10, 2, 8}, {10, 11, 7, 1, 4, 0}, {11, 9, 2, 0, 6, 3},
-                            {9, 8, 4, 3, 7, 5}, {8, 10, 6, 5, 2, 1}};
-  constexpr int owner[8] = {0, 3, 2, 1, 4, 5, 6, 7};
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    const int p12 = pe[n][0], p01 = pe[n][1], p04 = pe[n][2], p34 = pe[n][3], p25 = pe[n][4], p35 = pe[n][5];
-    const int slot = (MODE & 2) ? owner[n] : n;
-    dv[0][slot] = fma(ey[p12], ez[p01], fma(-ey[p01], ez[p12], fma(ey[p04], ez[p34],
-                  fma(-ey[p34], ez[p04], fma(-ey[p25], ez[p35], ey[p35] * ez[p25])))));
-    dv[1][slot] = fma(-ex[p12], ez[p01], fma(ex[p01], ez[p12], fma(-ex[p04], ez[p34],
-                  fma(ex[p34], ez[p04], fma(ex[p25], ez[p35], -(ex[p35] * ez[p25]))))));
-    dv[2][slot] = fma(-ey[p12], ex[p01], fma(ey[p01], ex[p12], fma(-ey[p04], ex[p34],
-                  fma(ey[p34], ex[p04], fma(ey[p25], ex[p35], -(ey[p35] * ex[p25]))))));
-  }
-}
-
 // Hourglass transpose. With hg[n][m] = gamma[n][m] - sum_j dv_j[n] hms_j[m]
 // (hms = the modes over 12*determ), S_k = hg^T V_k, T_k = hg^T lf_k (lf the
 // force adjoints) and coef the hourglass coefficient, the forward force is
@@ -704,202 +698,261 @@ __device__ __forceinline__ void volu_der(const double ex[12], const double ey[12
 //   dL/dhms_j = -coef sum_k (S_k (lf_k . dv_j) + T_k (V_k . dv_j)),
 //   dL/dcoef  = sum_k S_k . T_k,
 // where hg^T u = Gamma(u) - sum_j hms_j (dv_j . u): 3x3 dot-product tables
-// replace the 8x4 matrices hg and dL/dhg. Three blocks per SM (168
-// registers, a few spilled) run faster than two without spills: the
-// transpose is partly latency-bound at 48^3.
+// replace the 8x4 matrices hg and dL/dhg.
+//
+// Three threads per element, one per coordinate k of V and lf. The 8-corner
+// sums D_k, C_k and the modes of lf_k run on the integer pipes: derivatives
+// share one scale per coordinate, velocities and force adjoints enter by their
+// differences to corner 0 (the derivatives sum to zero over the corners, the
+// modes' signs do too). dL/ddv is formed up to the same constant for every
+// corner, which the differences it is used by do not see.
+enum : int {
+  HA_DV = 0,                 // 8 j + c: limbs of the volume derivatives of coordinate j
+  HA_V = 24, HA_L = 48,      // 8 k + c: velocities and force adjoints
+  HA_HMS = 72,               // 4 j + m
+  HA_P = 84,                 // 12 k + 4 j + m: coordinate k's part of P_j[m]
+  HA_NA = 120, HA_NB = 129,  // 3 k + j
+  HA_DVK = 138,              // j: the derivatives' exponent, and whether they are in range
+  HA_COEF = 141,             // coef, -coef vi12
+  HA_SUM = 143,              // k: S_k . T_k; 3 + j: P_j . hms_j; 6 + k: normals' part of the stress
+  HA_COUNT = 152
+};
+
+// Corner differences u[c] - u[0] below 2^59, c = 1..7, with their scale's
+// exponent; false for values that are not finite.
+__device__ __forceinline__ bool corner_differences(const double u[8], fx::i64 d[8], int& s) {
+  int ev = fx::exponent_field(fx::extent_hi(u));
+  // (all zero, or in range)
+  const bool ok = ev == 0 || (ev >= fx::kMinSpeed && ev <= fx::kMaxSpeed);
+  ev = ok ? fx::imax(ev, fx::kMinSpeed) : 0x7ff;
+  s = 1081 - ev;
+  const fx::i64 u0 = fx::to_fixed(u[0], 6 - ev);
+  d[0] = 0;
+#pragma unroll
+  for (int c = 1; c < 8; ++c) d[c] = fx::sub(fx::to_fixed(u[c], 6 - ev), u0);
+  return ok;
+}
+
 template <int MODE>
-__global__ void __launch_bounds__(kAdjBlock, 3) ka_hourglass(AdjDev a, double hgcoef) {
+__global__ void __launch_bounds__(3 * kFixedElems, 6) ka_hourglass(AdjDev a, double hgcoef) {
+  __shared__ double column[HA_COUNT * kFixedElems];
   const int E = a.E;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  const int slot = blockIdx.x * kFixedElems + lane;
+  const bool live = slot < E;
+  const int e = live ? slot : E - 1;  // threads past the end repeat the last element and store nothing
+  auto sh = [&](int i) -> double& { return column[i * kFixedElems + lane]; };
+  auto num = [&](int i) -> fx::Num& { return reinterpret_cast<fx::Num*>(column)[i * kFixedElems + lane]; };
+  const double* const V = k == 0 ? a.xd0 : k == 1 ? a.yd0 : a.zd0;
+  const double* const Lf = k == 0 ? a.lfx : k == 1 ? a.lfy : a.lfz;
+  int nd[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) nd[c] = a.nodelist[c * E + e];
+  wait_for_last_kernel();
+  double lf[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) lf[c] = Lf[nd[c]];
   double Lhg_coef = 0.0;
-  if (e < E) {
-    int nd[8];
+  if (!(hgcoef > 0.0)) {
+    if (live) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) nd[c] = a.nodelist[c * E + e];
-    if (!(hgcoef > 0.0)) {
+      for (int c = 0; c < 8; ++c) { a.fV[(k * 8 + c) * E + e] = 0.0; a.sLdv[(k * 8 + c) * E + e] = 0.0; }
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
+      for (int m = 0; m < 4; ++m) a.sLhm[(k * 4 + m) * E + e] = 0.0;
+    }
+  } else {
+    double inv_det = 0.0, vi12 = 0.0, ss = 0.0, mass = 0.0, r = 0.0;  // thread 0
+    double S[4], v[8], dv[8];
+    {
+      // the forward kernel's volume derivatives, scaled modes and mode sums
 #pragma unroll
-        for (int c = 0; c < 8; ++c) { a.fV[(k * 8 + c) * E + e] = 0.0; a.sLdv[(k * 8 + c) * E + e] = 0.0; }
+      for (int c = 0; c < 8; ++c) dv[c] = a.geo[(k * 8 + c) * E + e];
 #pragma unroll
-      for (int k = 0; k < 12; ++k) a.sLhm[k * E + e] = 0.0;
-    } else {
-      const double* Vp[3] = {a.xd0, a.yd0, a.zd0};
-      const double* Lf[3] = {a.lfx, a.lfy, a.lfz};
-      // the forward kernel's volume derivatives and scaled modes, from the tape
-      double hms[3][4], dv[3][8];
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) dv[j][c] = a.geo[(j * 8 + c) * E + e];
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) hms[j][m] = a.geo[(24 + j * 4 + m) * E + e];
-      const double determ = a.volo[e] * a.v0[e];
-      const double inv_det = 1.0 / determ;
-      const double vi12 = inv_det * (1.0 / 12.0);
-      const double ss = a.ss0[e], mass = a.elemMass[e];
-      const double r = inv_cbrt(determ);
-      const double c0 = -hgcoef * 0.01;
-      const double coef = ((c0 * ss) * mass) * r;
-      // S_k (taped), D[k][j] = V_k . dv_j and T_k, C[k][j] = lf_k . dv_j
-      double S[3][4], T[3][4], D[3][3], C[3][3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        double u[8], w2[4], w1[3];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) S[k][m] = a.geo[(36 + 4 * k + m) * E + e];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) u[c] = Vp[k][nd[c]];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          double s = dv[j][0] * u[0];
-#pragma unroll
-          for (int c = 1; c < 8; ++c) s = fma(dv[j][c], u[c], s);
-          D[k][j] = s;
-        }
-#pragma unroll
-        for (int c = 0; c < 8; ++c) u[c] = Lf[k][nd[c]];
-        walsh7(u, w1, w2);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          double s = dv[j][0] * u[0];
-#pragma unroll
-          for (int c = 1; c < 8; ++c) s = fma(dv[j][c], u[c], s);
-          C[k][j] = s;
-        }
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-          T[k][m] = fma(-hms[2][m], C[k][2], fma(-hms[1][m], C[k][1], fma(-hms[0][m], C[k][0], w2[m])));
+      for (int m = 0; m < 4; ++m) {
+        sh(HA_HMS + 4 * k + m) = a.geo[(24 + 4 * k + m) * E + e];
+        S[m] = a.geo[(36 + 4 * k + m) * E + e];
       }
-      double Lcoef = 0.0;
+      unsigned top = 0;
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
+      for (int c = 0; c < 8; ++c) {
+        v[c] = V[nd[c]];
+        sh(HA_V + 8 * k + c) = v[c];
+        sh(HA_L + 8 * k + c) = lf[c];
+        top = fx::umax(top, (unsigned)fx::hi_word(dv[c]) & 0x7fffffffu);
+      }
+      // below 2^60
+      int ed = fx::exponent_field(top);
+      const bool ok = ed == 0 || (ed >= fx::kMinSpeed && ed <= fx::kMaxSpeed);
+      ed = ok ? fx::imax(ed, fx::kMinSpeed) : 0x7ff;
 #pragma unroll
-        for (int m = 0; m < 4; ++m) Lcoef = fma(S[k][m], T[k][m], Lcoef);
-      // A[k][j] = S_k . hms_j, B[k][j] = T_k . hms_j
-      double A[3][3], B[3][3];
+      for (int c = 0; c < 8; ++c) num(HA_DV + 8 * k + c) = fx::limbs(fx::to_fixed(dv[c], 7 - ed));
+      fx::Num x;
+      x.lo = 1082 - ed;
+      x.hi = ok;
+      num(HA_DVK + k) = x;
+      if (k == 0) {
+        const double determ = a.volo[e] * a.v0[e];
+        inv_det = 1.0 / determ;
+        vi12 = inv_det * (1.0 / 12.0);
+        ss = a.ss0[e];
+        mass = a.elemMass[e];
+        r = inv_cbrt(determ);
+        const double coef = ((-hgcoef * 0.01 * ss) * mass) * r;
+        sh(HA_COEF) = coef;
+        sh(HA_COEF + 1) = -coef * vi12;
+      }
+    }
+    __syncthreads();
+    // D[j] = V . dv_j, C[j] = lf . dv_j, w2 = the modes of lf
+    double D[3], C[3], w2[4];
+    {
+      fx::i64 dl[8], du[8];
+      int sl, su;
+      const bool okl = corner_differences(lf, dl, sl), oku = corner_differences(v, du, su);
+      const bool ok = okl && oku && (num(HA_DVK).hi & num(HA_DVK + 1).hi & num(HA_DVK + 2).hi);
+      if (ok) {
+        fx::Num nl[8], nu[8];
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
+        for (int c = 1; c < 8; ++c) { nl[c] = fx::limbs(dl[c]); nu[c] = fx::limbs(du[c]); }
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          A[k][j] = fma(S[k][0], hms[j][0], fma(S[k][1], hms[j][1], fma(S[k][2], hms[j][2], S[k][3] * hms[j][3])));
-          B[k][j] = fma(T[k][0], hms[j][0], fma(T[k][1], hms[j][1], fma(T[k][2], hms[j][2], T[k][3] * hms[j][3])));
-        }
-      // dL/dhms_j = -coef P_j with P_j[m] the dot products below; dL/dhm_j =
-      // vi12 dL/dhms_j (hms = vi12 hm); dL/dvi12 = sum_j dL/dhms_j . hms_j / vi12
-      double Pvi = 0.0;  // sum_j P_j . hms_j
-      {
-        const double ncv = -coef * vi12;
+          fx::Acc x = fx::mul(num(HA_DV + 8 * j + 1), nu[1]), y = fx::mul(num(HA_DV + 8 * j + 1), nl[1]);
 #pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-          for (int m = 0; m < 4; ++m) {
-            const double P = fma(S[0][m], C[0][j], fma(S[1][m], C[1][j], fma(S[2][m], C[2][j],
-                             fma(T[0][m], D[0][j], fma(T[1][m], D[1][j], T[2][m] * D[2][j])))));
-            Pvi = fma(P, hms[j][m], Pvi);
-            a.sLhm[(j * 4 + m) * E + e] = ncv * P;
+          for (int c = 2; c < 8; ++c) {
+            const fx::Num g = num(HA_DV + 8 * j + c);
+            fx::mac(x, g, nu[c]);
+            fx::mac(y, g, nl[c]);
           }
-      }
-      const double Lvi12 = -coef * Pvi;
-      // the coefficient folded into the tables: nA = -coef A, nB = -coef B
-      double nA[3][3], nB[3][3];
+          const int sd = num(HA_DVK + j).lo;
+          D[j] = fx::to_double(fx::take<3>(x), 61 - sd - su);
+          C[j] = fx::to_double(fx::take<3>(y), 61 - sd - sl);
+        }
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
+        for (int m = 0; m < 4; ++m) {
+          fx::i64 t = 0;
 #pragma unroll
-        for (int j = 0; j < 3; ++j) { nA[k][j] = -coef * A[k][j]; nB[k][j] = -coef * B[k][j]; }
-      // dL/dV_k = coef (Gamma^T T_k - sum_j dv_j B[k][j]) = Gamma^T (coef T_k) + sum_j dv_j nB[k][j]
+          for (int c = 1; c < 8; ++c) t += (fx::kGammaSigns >> (4 * c + m)) & 1u ? -dl[c] : dl[c];
+          w2[m] = fx::to_double(t, -sl);
+        }
+      } else {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        double cT[4], q[8];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) cT[m] = coef * T[k][m];
-        walsh_modes_t(cT, q);
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          a.fV[(k * 8 + c) * E + e] = fma(dv[2][c], nB[k][2], fma(dv[1][c], nB[k][1], fma(dv[0][c], nB[k][0], q[c])));
-      }
-      // dL/ddv_j = -coef sum_k (lf_k A[k][j] + V_k B[k][j]) = sum_k (lf_k nA[k][j] + V_k nB[k][j])
-      {
-        double Ldv[3][8];
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-          for (int c = 0; c < 8; ++c) Ldv[j][c] = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
+        for (int j = 0; j < 3; ++j) {
+          D[j] = C[j] = 0.0;
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            const double lf = Lf[k][nd[c]], vv = Vp[k][nd[c]];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) Ldv[j][c] = fma(lf, nA[k][j], fma(vv, nB[k][j], Ldv[j][c]));
+            const double g = a.geo[(j * 8 + c) * E + e];
+            D[j] = fma(g, v[c], D[j]);
+            C[j] = fma(g, lf[c], C[j]);
           }
         }
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-          for (int c = 0; c < 8; ++c) a.sLdv[(j * 8 + c) * E + e] = Ldv[j][c];
+        double w1[3];
+        walsh7(lf, w1, w2);
       }
+    }
+    const double coef = sh(HA_COEF);
+    // T = hg^T lf, A[j] = S . hms_j, B[j] = T . hms_j
+    double T[4], Lcoef = 0.0, nA[3], nB[3];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      T[m] = fma(-sh(HA_HMS + 8 + m), C[2], fma(-sh(HA_HMS + 4 + m), C[1], fma(-sh(HA_HMS + m), C[0], w2[m])));
+      Lcoef = fma(S[m], T[m], Lcoef);
+    }
+    sh(HA_SUM + k) = Lcoef;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      double x = 0.0, y = 0.0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const double h = sh(HA_HMS + 4 * j + m);
+        x = fma(S[m], h, x);
+        y = fma(T[m], h, y);
+        sh(HA_P + 12 * k + 4 * j + m) = fma(S[m], C[j], T[m] * D[j]);
+      }
+      // the coefficient folded into the tables
+      nA[j] = -coef * x;
+      nB[j] = -coef * y;
+      sh(HA_NA + 3 * k + j) = nA[j];
+      sh(HA_NB + 3 * k + j) = nB[j];
+    }
+    // dL/dV = coef (Gamma^T T - sum_j dv_j B[j]) = Gamma^T (coef T) + sum_j dv_j nB[j]
+    {
+      double cT[4], q[8];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) cT[m] = coef * T[m];
+      walsh_modes_t(cT, q);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        double f = q[c];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) f = fma(a.geo[(j * 8 + c) * E + e], nB[j], f);
+        if (live) a.fV[(k * 8 + c) * E + e] = f;
+      }
+    }
+    __syncthreads();
+    // coordinate k as the derivatives' j. dL/dhms_j = -coef P_j with P_j[m] the
+    // sums below; dL/dhm_j = vi12 dL/dhms_j (hms = vi12 hm); dL/dvi12 = sum_j
+    // dL/dhms_j . hms_j / vi12
+    double Pvi = 0.0;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const double P = (sh(HA_P + 4 * k + m) + sh(HA_P + 12 + 4 * k + m)) + sh(HA_P + 24 + 4 * k + m);
+      Pvi = fma(P, sh(HA_HMS + 4 * k + m), Pvi);
+      if (live) a.sLhm[(k * 4 + m) * E + e] = sh(HA_COEF + 1) * P;
+    }
+    sh(HA_SUM + 3 + k) = Pvi;
+    // dL/ddv_j = -coef sum_k (lf_k A[k][j] + V_k B[k][j]) = sum_k (lf_k nA[k][j] + V_k nB[k][j])
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      double t = 0.0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        t = fma(sh(HA_L + 8 * q + c), sh(HA_NA + 3 * q + k), fma(sh(HA_V + 8 * q + c), sh(HA_NB + 3 * q + k), t));
+      if (live) a.sLdv[(k * 8 + c) * E + e] = t;
+    }
+    __syncthreads();
+    if (live && k == 0) {
       // coef = c0 ss mass determ^(-1/3), vi12 = 1/(12 determ), determ = volo v
-      a.lss[e] += Lcoef * c0 * mass * r;
-      Lhg_coef = Lcoef * (-0.01) * ss * mass * r;
-      const double Ldeterm = (Lcoef * c0 * ss * mass * (-1.0 / 3.0) * r - Lvi12) * inv_det;
+      const double c0 = -hgcoef * 0.01;
+      const double Lc = (sh(HA_SUM) + sh(HA_SUM + 1)) + sh(HA_SUM + 2);
+      const double Lvi12 = -coef * ((sh(HA_SUM + 3) + sh(HA_SUM + 4)) + sh(HA_SUM + 5));
+      a.lss[e] += Lc * c0 * mass * r;
+      Lhg_coef = Lc * (-0.01) * ss * mass * r;
+      const double Ldeterm = (Lc * c0 * ss * mass * (-1.0 / 3.0) * r - Lvi12) * inv_det;
       a.lv[e] += Ldeterm * a.volo[e];
     }
-    // stress part of the force, f = s8 * B with s8 = (-p - q)/8. The forward
-    // forms B0..B3 from faces 0-4 (node n's three face cross products) and
-    // the opposite corners as B6 = -B0, B7 = -B1, B4 = -B2, B5 = -B3 (the face
-    // normals of a closed surface sum to zero), so face 5 carries no adjoint:
-    // sum_n lf_n . B_n = sum_f N_f . LU_f. The face terms LU go to sLU for
-    // the position transpose; p and q get -1/8 sum_f N_f . LU_f here, before
-    // the material transpose of the cycle before reads them.
-    {
-      const double* Lf[3] = {a.lfx, a.lfy, a.lfz};
+  }
+  // stress part of the force, f = s8 * B with s8 = (-p - q)/8. The forward
+  // forms B0..B3 from faces 0-4 (node n's three face cross products) and
+  // the opposite corners as B6 = -B0, B7 = -B1, B4 = -B2, B5 = -B3 (the face
+  // normals of a closed surface sum to zero), so face 5 carries no adjoint:
+  // sum_n lf_n . B_n = sum_f N_f . LU_f. The face terms LU go to sLU for
+  // the position transpose; p and q get -1/8 sum_f N_f . LU_f here, before
+  // the material transpose of the cycle before reads them.
+  {
+    // w_n = lf_n - lf_opposite(n) for the corners 0..3 (opposites 6, 7, 4, 5),
+    // which touch faces {0,1,4} {0,1,2} {0,2,3} {0,3,4}
+    const double w0 = lf[0] - lf[6], w1 = lf[1] - lf[7], w2 = lf[2] - lf[4], w3 = lf[3] - lf[5];
+    const double w01 = w0 + w1, w23 = w2 + w3;
+    double LU[5] = {w01 + w23, w01, w1 + w2, w23, w0 + w3};
+    // src/domain.jl:1050-1055: node 1 (corner 0) takes face 5's areaY twice
+    // and no areaZ; its opposite corner has the plain sum
+    if (!(MODE & 1) && k != 0) LU[4] += k == 1 ? lf[0] : -lf[0];
+    double part = 0.0;
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
       // face normals 0..4 (the forward's cross products, from the tape)
-      V3 N[5];
-#pragma unroll
-      for (int f = 0; f < 5; ++f) N[f] = v3(a.geo[(48 + f) * E + e], a.geo[(54 + f) * E + e], a.geo[(60 + f) * E + e]);
-      auto lfv = [&](int n) { return v3(Lf[0][nd[n]], Lf[1][nd[n]], Lf[2][nd[n]]); };
-      // w_n = lf_n - lf_opposite(n) for the corners 0..3 (opposites 6, 7, 4, 5)
-      const V3 lf0 = lfv(0);
-      V3 w0 = lf0, w1 = lfv(1), w2 = lfv(2), w3 = lfv(3);
-      {
-        const V3 o0 = lfv(6), o1 = lfv(7), o2 = lfv(4), o3 = lfv(5);
-        w0.x -= o0.x; w0.y -= o0.y; w0.z -= o0.z;
-        w1.x -= o1.x; w1.y -= o1.y; w1.z -= o1.z;
-        w2.x -= o2.x; w2.y -= o2.y; w2.z -= o2.z;
-        w3.x -= o3.x; w3.y -= o3.y; w3.z -= o3.z;
-      }
-      // corners 0..3 touch faces {0,1,4} {0,1,2} {0,2,3} {0,3,4}
-      V3 w01 = w0; vadd(w01, w1);
-      V3 w23 = w2; vadd(w23, w3);
-      V3 LU[5];
-      LU[0] = w01; vadd(LU[0], w23);
-      LU[1] = w01;
-      LU[2] = w1; vadd(LU[2], w2);
-      LU[3] = w23;
-      LU[4] = w0; vadd(LU[4], w3);
-      if (!(MODE & 1)) {
-        // src/domain.jl:1050-1055: node 1 (corner 0) takes face 5's areaY twice
-        // and no areaZ; its opposite corner has the plain sum
-        LU[4].y += lf0.y;
-        LU[4].z -= lf0.z;
-      }
-      double Ls8 = 0.0;
-#pragma unroll
-      for (int f = 0; f < 5; ++f) {
-        Ls8 += vdot(N[f], LU[f]);
-        a.sLU[(f * 3) * E + e] = LU[f].x;
-        a.sLU[(f * 3 + 1) * E + e] = LU[f].y;
-        a.sLU[(f * 3 + 2) * E + e] = LU[f].z;
-      }
-      const double Lpq = -0.125 * Ls8;
+      part = fma(a.geo[(48 + 6 * k + f) * E + e], LU[f], part);
+      if (live) a.sLU[(3 * f + k) * E + e] = LU[f];
+    }
+    sh(HA_SUM + 6 + k) = part;
+    __syncthreads();
+    if (live && k == 1) {
+      const double Lpq = -0.125 * ((sh(HA_SUM + 6) + sh(HA_SUM + 7)) + sh(HA_SUM + 8));
       a.lp[e] += Lpq;
       a.lq[e] += Lpq;
     }
   }
-  block_sum_to(Lhg_coef, a.part_hg);
+  block_sum3_to(Lhg_coef, a.part_hg);
 }
 
 // Position transpose of one element's k_force, added into LX:
@@ -1085,6 +1138,7 @@ __host__ __device__ inline void time_increment_reverse(const CycleRec& r, const 
 constexpr int kCloseBlock = 256;
 __global__ void __launch_bounds__(kCloseBlock) ka_cycle_close(AdjDev a, int ge, int gn, const CycleRec* rec,
                                                                AdjScal* sc, Params prm) {
+  wait_for_last_kernel();
   double t_kin = 0.0, t_node = 0.0, t_hg = 0.0;
   for (int j = threadIdx.x; j < ge; j += kCloseBlock) { t_kin += a.part_dt[j]; t_hg += a.part_hg[j]; }
   for (int j = threadIdx.x; j < gn; j += kCloseBlock) t_node += a.part_dtn[j];
@@ -1144,6 +1198,7 @@ __global__ void __launch_bounds__(kAdjBlock) ka_copy_state(StateSet src, StateSe
 // makes the cycle a no-op (done / status, which the step kernels check).
 __global__ void __launch_bounds__(kAdjBlock) ka_tape_begin(StateSet src, StateSet dst, int E, int N, DevState* st,
                                                             CycleRec* rec, Params prm) {
+  wait_for_last_kernel();
   copy_state_at(blockIdx.x * blockDim.x + threadIdx.x, src, dst, E, N);
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   if (st->status != 0u || st->done) return;
@@ -1175,6 +1230,7 @@ __global__ void __launch_bounds__(kAdjBlock) ka_tape_begin(StateSet src, StateSe
 // scan keeps, src/domain.jl:3003-3008 and :3041-3046).
 __global__ void __launch_bounds__(kAdjBlock) ka_tape_close(const double* dtc, const double* dth, int E,
                                                             const DevState* st, CycleRec* rec) {
+  wait_for_last_kernel();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned long long bc = st->acc_courant, bh = st->acc_hydro;
   if (i == 0) {
