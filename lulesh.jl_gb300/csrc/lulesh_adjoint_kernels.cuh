@@ -373,9 +373,10 @@ __device__ __forceinline__ void walsh1_t(const double Lw[3], double L[8]) {
 
 // Transpose of the hourglass mode transform: out[n] = sum_m gamma[n][m] t[m]
 // (12 adds).
-__device__ __forceinline__ void walsh_modes_t(const double t[4], double out[8]) {
-  const double cm = t[2] - t[3], cp = t[2] + t[3];
-  const double s = t[0] + t[1], d = t[0] - t[1];
+template <class T>
+__device__ __forceinline__ void walsh_modes_t(const T t[4], T out[8]) {
+  const T cm = t[2] - t[3], cp = t[2] + t[3];
+  const T s = t[0] + t[1], d = t[0] - t[1];
   out[0] = s + cm; out[1] = d - cm; out[2] = cm - s; out[3] = -d - cm;
   out[4] = cp - s; out[5] = -d - cp; out[6] = s + cp; out[7] = d - cp;
 }
@@ -700,15 +701,17 @@ __global__ void __launch_bounds__(kAdjBlock) ka_node(AdjDev a, const CycleRec* r
 // where hg^T u = Gamma(u) - sum_j hms_j (dv_j . u): 3x3 dot-product tables
 // replace the 8x4 matrices hg and dL/dhg.
 //
-// Three threads per element, one per coordinate k of V and lf. The 8-corner
-// sums D_k, C_k and the modes of lf_k run on the integer pipes: derivatives
-// share one scale per coordinate, velocities and force adjoints enter by their
-// differences to corner 0 (the derivatives sum to zero over the corners, the
-// modes' signs do too). dL/ddv is formed up to the same constant for every
-// corner, which the differences it is used by do not see.
+// Three threads per element, one per coordinate k of V and lf. The sums over
+// the 8 corners and onto them run on the integer pipes: derivatives share one
+// scale per coordinate, velocities and force adjoints enter by their differences
+// to corner 0 (the derivatives sum to zero over the corners, the modes' signs do
+// too). dL/ddv is formed up to the same constant for every corner, which the
+// differences it is used by do not see. A sum of products with coefficients of
+// different size takes the largest term's unit, the others' mantissas shifted.
 enum : int {
   HA_DV = 0,                 // 8 j + c: limbs of the volume derivatives of coordinate j
-  HA_V = 24, HA_L = 48,      // 8 k + c: velocities and force adjoints
+  HA_V = 24, HA_L = 48,      // 8 k + c: limbs of the corner differences of the velocities and force
+                             // adjoints, in place of corner 0 their exponent and whether they are in range
   HA_HMS = 72,               // 4 j + m
   HA_P = 84,                 // 12 k + 4 j + m: coordinate k's part of P_j[m]
   HA_NA = 120, HA_NB = 129,  // 3 k + j
@@ -718,23 +721,31 @@ enum : int {
   HA_COUNT = 152
 };
 
-// Corner differences u[c] - u[0] below 2^59, c = 1..7, with their scale's
-// exponent; false for values that are not finite.
-__device__ __forceinline__ bool corner_differences(const double u[8], fx::i64 d[8], int& s) {
+// Limbs of the corner differences u[c] - u[0], c = 1..7, below 2^59, and in
+// place of corner 0 their scale's exponent and whether they are in range.
+template <class Put>
+__device__ __forceinline__ void corner_differences(const double u[8], Put put) {
   int ev = fx::exponent_field(fx::extent_hi(u));
   // (all zero, or in range)
   const bool ok = ev == 0 || (ev >= fx::kMinSpeed && ev <= fx::kMaxSpeed);
   ev = ok ? fx::imax(ev, fx::kMinSpeed) : 0x7ff;
-  s = 1081 - ev;
+  fx::Num x;
+  x.lo = 1081 - ev;
+  x.hi = ok;
+  put(0, x);
   const fx::i64 u0 = fx::to_fixed(u[0], 6 - ev);
-  d[0] = 0;
 #pragma unroll
-  for (int c = 1; c < 8; ++c) d[c] = fx::sub(fx::to_fixed(u[c], 6 - ev), u0);
-  return ok;
+  for (int c = 1; c < 8; ++c) put(c, fx::limbs(fx::sub(fx::to_fixed(u[c], 6 - ev), u0)));
 }
 
+// A coefficient's mantissa in the unit 2^u of a sum, its own unit being 2^e.
+__device__ __forceinline__ fx::i64 in_unit(const fx::Float& f, int e, int u) { return f.m >> fx::imin(u - e, 63); }
+// Whether a sum is in range: coefficients at most 2^400 (so not infinities or
+// NaN, top their largest exponent), and a unit whose values are doubles or none.
+__device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && (u < -2000 || u >= -950); }
+
 template <int MODE>
-__global__ void __launch_bounds__(3 * kFixedElems, 6) ka_hourglass(AdjDev a, double hgcoef) {
+__global__ void __launch_bounds__(3 * kFixedElems, 5) ka_hourglass(AdjDev a, double hgcoef) {
   __shared__ double column[HA_COUNT * kFixedElems];
   const int E = a.E;
   const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
@@ -776,10 +787,10 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_hourglass(AdjDev a, dou
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         v[c] = V[nd[c]];
-        sh(HA_V + 8 * k + c) = v[c];
-        sh(HA_L + 8 * k + c) = lf[c];
         top = fx::umax(top, (unsigned)fx::hi_word(dv[c]) & 0x7fffffffu);
       }
+      corner_differences(v, [&](int c, fx::Num x) { num(HA_V + 8 * k + c) = x; });
+      corner_differences(lf, [&](int c, fx::Num x) { num(HA_L + 8 * k + c) = x; });
       // below 2^60
       int ed = fx::exponent_field(top);
       const bool ok = ed == 0 || (ed >= fx::kMinSpeed && ed <= fx::kMaxSpeed);
@@ -804,50 +815,47 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_hourglass(AdjDev a, dou
     }
     __syncthreads();
     // D[j] = V . dv_j, C[j] = lf . dv_j, w2 = the modes of lf
+    const bool ok = num(HA_DVK).hi & num(HA_DVK + 1).hi & num(HA_DVK + 2).hi & num(HA_V).hi & num(HA_V + 8).hi &
+                    num(HA_V + 16).hi & num(HA_L).hi & num(HA_L + 8).hi & num(HA_L + 16).hi;
     double D[3], C[3], w2[4];
-    {
-      fx::i64 dl[8], du[8];
-      int sl, su;
-      const bool okl = corner_differences(lf, dl, sl), oku = corner_differences(v, du, su);
-      const bool ok = okl && oku && (num(HA_DVK).hi & num(HA_DVK + 1).hi & num(HA_DVK + 2).hi);
-      if (ok) {
-        fx::Num nl[8], nu[8];
+    if (ok) {
+      const int su = num(HA_V + 8 * k).lo, sl = num(HA_L + 8 * k).lo;
 #pragma unroll
-        for (int c = 1; c < 8; ++c) { nl[c] = fx::limbs(dl[c]); nu[c] = fx::limbs(du[c]); }
+      for (int j = 0; j < 3; ++j) {
+        fx::Acc x = fx::mul(num(HA_DV + 8 * j + 1), num(HA_V + 8 * k + 1));
+        fx::Acc y = fx::mul(num(HA_DV + 8 * j + 1), num(HA_L + 8 * k + 1));
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          fx::Acc x = fx::mul(num(HA_DV + 8 * j + 1), nu[1]), y = fx::mul(num(HA_DV + 8 * j + 1), nl[1]);
-#pragma unroll
-          for (int c = 2; c < 8; ++c) {
-            const fx::Num g = num(HA_DV + 8 * j + c);
-            fx::mac(x, g, nu[c]);
-            fx::mac(y, g, nl[c]);
-          }
-          const int sd = num(HA_DVK + j).lo;
-          D[j] = fx::to_double(fx::take<3>(x), 61 - sd - su);
-          C[j] = fx::to_double(fx::take<3>(y), 61 - sd - sl);
+        for (int c = 2; c < 8; ++c) {
+          fx::mac(x, num(HA_DV + 8 * j + c), num(HA_V + 8 * k + c));
+          fx::mac(y, num(HA_DV + 8 * j + c), num(HA_L + 8 * k + c));
         }
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          fx::i64 t = 0;
-#pragma unroll
-          for (int c = 1; c < 8; ++c) t += (fx::kGammaSigns >> (4 * c + m)) & 1u ? -dl[c] : dl[c];
-          w2[m] = fx::to_double(t, -sl);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          D[j] = C[j] = 0.0;
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const double g = a.geo[(j * 8 + c) * E + e];
-            D[j] = fma(g, v[c], D[j]);
-            C[j] = fma(g, lf[c], C[j]);
-          }
-        }
-        double w1[3];
-        walsh7(lf, w1, w2);
+        const int sd = num(HA_DVK + j).lo;
+        D[j] = fx::to_double(fx::take<3>(x), 61 - sd - su);
+        C[j] = fx::to_double(fx::take<3>(y), 61 - sd - sl);
       }
+      fx::i64 t[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int c = 1; c < 8; ++c) {
+        const fx::Num x = num(HA_L + 8 * k + c);
+        const fx::i64 d = fx::shl((fx::i64)x.hi, 32) + x.lo;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) t[m] += (fx::kGammaSigns >> (4 * c + m)) & 1u ? -d : d;
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) w2[m] = fx::to_double(t[m], -sl);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        D[j] = C[j] = 0.0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const double g = a.geo[(j * 8 + c) * E + e];
+          D[j] = fma(g, v[c], D[j]);
+          C[j] = fma(g, lf[c], C[j]);
+        }
+      }
+      double w1[3];
+      walsh7(lf, w1, w2);
     }
     const double coef = sh(HA_COEF);
     // T = hg^T lf, A[j] = S . hms_j, B[j] = T . hms_j
@@ -876,16 +884,50 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_hourglass(AdjDev a, dou
     }
     // dL/dV = coef (Gamma^T T - sum_j dv_j B[j]) = Gamma^T (coef T) + sum_j dv_j nB[j]
     {
-      double cT[4], q[8];
+      double cT[4];
 #pragma unroll
       for (int m = 0; m < 4; ++m) cT[m] = coef * T[m];
-      walsh_modes_t(cT, q);
+      // products over 2^62 below 2^60.6, the modes' mantissas over 4
+      fx::Float fT[4], fB[3];
+      int u = fx::kNoExponent, top = u;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        double f = q[c];
+      for (int m = 0; m < 4; ++m) {
+        fT[m] = fx::to_float(cT[m]);
+        top = fx::imax(top, fT[m].k);
+        u = fx::imax(u, fT[m].k + 2);
+      }
 #pragma unroll
-        for (int j = 0; j < 3; ++j) f = fma(a.geo[(j * 8 + c) * E + e], nB[j], f);
-        if (live) a.fV[(k * 8 + c) * E + e] = f;
+      for (int j = 0; j < 3; ++j) {
+        fB[j] = fx::to_float(nB[j]);
+        top = fx::imax(top, fB[j].k);
+        fB[j].k += 62 - num(HA_DVK + j).lo;
+        u = fx::imax(u, fB[j].k);
+      }
+      if (ok && good_sum(top, u)) {
+        fx::Num B[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) B[j] = fx::limbs(in_unit(fB[j], fB[j].k, u));
+        fx::i64 t[4], q[8];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) t[m] = in_unit(fT[m], fT[m].k, u);
+        walsh_modes_t(t, q);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          fx::Acc x = fx::mul(num(HA_DV + c), B[0]);
+          fx::mac(x, num(HA_DV + 8 + c), B[1]);
+          fx::mac(x, num(HA_DV + 16 + c), B[2]);
+          if (live) a.fV[(k * 8 + c) * E + e] = fx::to_double(fx::take<2>(x) + q[c], u);
+        }
+      } else {
+        double q[8];
+        walsh_modes_t(cT, q);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          double f = q[c];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) f = fma(a.geo[(j * 8 + c) * E + e], nB[j], f);
+          if (live) a.fV[(k * 8 + c) * E + e] = f;
+        }
       }
     }
     __syncthreads();
@@ -901,13 +943,50 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_hourglass(AdjDev a, dou
     }
     sh(HA_SUM + 3 + k) = Pvi;
     // dL/ddv_j = -coef sum_k (lf_k A[k][j] + V_k B[k][j]) = sum_k (lf_k nA[k][j] + V_k nB[k][j])
+    {
+      fx::Float fA[3], fB[3];
+      int u = fx::kNoExponent, top = u;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      double t = 0.0;
+      for (int q = 0; q < 3; ++q) {
+        fA[q] = fx::to_float(sh(HA_NA + 3 * q + k));
+        fB[q] = fx::to_float(sh(HA_NB + 3 * q + k));
+        top = fx::imax(top, fx::imax(fA[q].k, fB[q].k));
+        fA[q].k += 61 - num(HA_L + 8 * q).lo;
+        fB[q].k += 61 - num(HA_V + 8 * q).lo;
+        u = fx::imax(u, fx::imax(fA[q].k, fB[q].k));
+      }
+      if (ok && good_sum(top, u)) {
+        fx::Num A[3], B[3];
 #pragma unroll
-      for (int q = 0; q < 3; ++q)
-        t = fma(sh(HA_L + 8 * q + c), sh(HA_NA + 3 * q + k), fma(sh(HA_V + 8 * q + c), sh(HA_NB + 3 * q + k), t));
-      if (live) a.sLdv[(k * 8 + c) * E + e] = t;
+        for (int q = 0; q < 3; ++q) {
+          A[q] = fx::limbs(in_unit(fA[q], fA[q].k, u));
+          B[q] = fx::limbs(in_unit(fB[q], fB[q].k, u));
+        }
+        if (live) a.sLdv[(k * 8) * E + e] = 0.0;
+#pragma unroll
+        for (int c = 1; c < 8; ++c) {
+          fx::Acc x = fx::mul(num(HA_L + c), A[0]);
+          fx::mac(x, num(HA_V + c), B[0]);
+#pragma unroll
+          for (int q = 1; q < 3; ++q) {
+            fx::mac(x, num(HA_L + 8 * q + c), A[q]);
+            fx::mac(x, num(HA_V + 8 * q + c), B[q]);
+          }
+          if (live) a.sLdv[(k * 8 + c) * E + e] = fx::to_double(fx::take<3>(x), u);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const int n = a.nodelist[c * E + e];
+          const double l3[3] = {a.lfx[n], a.lfy[n], a.lfz[n]};
+          const double v3_[3] = {a.xd0[n], a.yd0[n], a.zd0[n]};
+          double t = 0.0;
+#pragma unroll
+          for (int q = 0; q < 3; ++q)
+            t = fma(l3[q], sh(HA_NA + 3 * q + k), fma(v3_[q], sh(HA_NB + 3 * q + k), t));
+          if (live) a.sLdv[(k * 8 + c) * E + e] = t;
+        }
+      }
     }
     __syncthreads();
     if (live && k == 0) {

@@ -64,3 +64,34 @@ def test_thin_and_ordinary_elements_match_oracle(gpu_lib, oracle_mod, mode, nx, 
         assert_fields(g, o, STEP_F64 + AUX_F64, where=f"step {step}")
     g.close()
     o.close()
+
+
+@pytest.mark.parametrize("nx", [2, 3, 6])
+@pytest.mark.parametrize("mode", [0, 7])
+def test_adjoint_forms_agree(gpu_lib, mode, nx):
+    """The reverse sweep is linear in its seeds, and seeds of 2^-700 or 2^480
+    are outside what its integer sums take (2^-400 to 2^400): the FP64 form's
+    gradients, scaled back exactly, against the integer form's. 2 cycles of 8
+    dependent sums of at most 64 terms, rounded to 2^-53 of partial sums up to
+    2^8 times the largest gradient of the field."""
+    tol = 2 * 8 * 64 * 2.0 ** -53 * 2 ** 8
+    rng = np.random.default_rng(0xE8 + nx)
+    fields = ("x", "y", "z", "xd", "yd", "zd", "e", "p", "q", "v", "ss")
+    out = []
+    state = seeds = None
+    for scale in (0, -700, 480):
+        g = gpu_lib.Domain(gpu_lib.LuleshProblem(nx=nx, mode=mode))
+        if state is None:
+            state = g.e + 1e4 * (1.0 + rng.random(g.numElem))
+            seeds = {f: rng.standard_normal(g.field(f).size) * (rng.random(g.field(f).size) < 0.7) for f in fields}
+        g.e = state
+        gpu_lib.run(g, 3)
+        adj = gpu_lib.Adjoint(g, checkpoint_every=1)
+        for f in fields:
+            adj.set_seed(f, seeds[f] * 2.0 ** scale)
+        adj.gradient(2)
+        out.append({f: adj.grad(f) * 2.0 ** -scale for f in fields})
+        adj.close()
+    for other in out[1:]:
+        for f in fields:
+            assert np.abs(other[f] - out[0][f]).max() <= tol * np.abs(out[0][f]).max(), f
