@@ -362,9 +362,10 @@ __global__ void __launch_bounds__(kAdjBlock, 4) ka_material(AdjDev a, Params prm
 
 // Transpose of walsh1: adds dL/dv of the 8 corner values for the adjoints
 // Lw of the three coefficients (through the body diagonals, 14 adds).
-__device__ __forceinline__ void walsh1_t(const double Lw[3], double L[8]) {
-  const double p = Lw[0] + Lw[2], q = Lw[2] - Lw[0];
-  const double La = p + Lw[1], Lb = p - Lw[1], Lc = q + Lw[1], Ld = q - Lw[1];
+template <class T>
+__device__ __forceinline__ void walsh1_t(const T Lw[3], T L[8]) {
+  const T p = Lw[0] + Lw[2], q = Lw[2] - Lw[0];
+  const T La = p + Lw[1], Lb = p - Lw[1], Lc = q + Lw[1], Ld = q - Lw[1];
   L[6] += La; L[0] -= La;
   L[5] += Lb; L[3] -= Lb;
   L[7] += Lc; L[1] -= Lc;
@@ -381,6 +382,17 @@ __device__ __forceinline__ void walsh_modes_t(const T t[4], T out[8]) {
   out[4] = cp - s; out[5] = -d - cp; out[6] = s + cp; out[7] = d - cp;
 }
 
+// to_fixed rounded towards zero, so that zeros of both signs give zero: where no
+// adjoint has come to an element yet, its sums stay exact zeros.
+__device__ __forceinline__ fx::i64 to_fixed0(double x, int bias) {
+  return fx::sub(fx::to_fixed(x, bias), (fx::i64)(fx::hi_word(x) >> 31));
+}
+// A coefficient's mantissa in the unit 2^u of a sum, its own unit being 2^e.
+__device__ __forceinline__ fx::i64 in_unit(const fx::Float& f, int e, int u) { return f.m >> fx::imin(u - e, 63); }
+// Whether a sum is in range: coefficients at most 2^400 (so not infinities or
+// NaN, top their largest exponent), and a unit whose values are doubles or none.
+__device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && (u < -2000 || u >= -950); }
+
 // ---------------------------------------------------------------------------
 // ka_kinematics: transpose of k_kinematics (volume, characteristic length,
 // velocity-gradient trace, monotonic-Q gradients), into the corner buffers.
@@ -395,16 +407,29 @@ __device__ __forceinline__ void walsh_modes_t(const T t[4], T out[8]) {
 // Three threads per element, one per coordinate and each in a warp of its own,
 // as in the forward kernels: a thread forms its component of every product,
 // and what a cross product needs of the other components is in shared memory.
-// Every cross product adds onto its target in two FMAs.
+//
+// The crosses onto the face diagonals, all of a diagonal (or a sum of two) and
+// an adjoint vector, and the sums onto the position corners run on the integer
+// pipes. Diagonals are scaled by their coordinate's extent 2^-sg[k], adjoint
+// vectors by 2^-(sg[k] + common), so that both products of a cross have one
+// unit; what else joins the corners (edges, modes, V x W) enters as mantissas
+// in the largest term's unit. Elements of sizes or adjoints out of range take
+// the crosses in doubles, the diagonals from the tape.
+// What bounds it: integer and FP64 issue together. At 48^3 173 us with the
+// crosses and corner sums on the FP64 pipe (87 % busy), 116 us so (78 %); a
+// gradient of 40 cycles at 48^3 21.7 -> 20.0 ms, of 24 cycles at 15^3 2.81 ->
+// 2.73. Six blocks per SM (96 registers; 147 slots are the most six can have)
+// against five and seven: 20.04, 20.37, 20.18 ms.
 enum : int {
   // per coordinate: mean edges, half-step edges, tape's 12 diagonals, U vectors,
-  // the differences of dL/ddv along V and W, the stress faces' terms; then the
-  // adjoints of the edges' cross products and of the cofactors, Lv12 U + dU and
-  // the characteristic face's term
-  KA_W = 0, KA_F = 3, KA_D = 6, KA_U = 18, KA_DV = 21, KA_DW = 24, KA_LN = 27,
-  KA_LA = 32, KA_LC = 35, KA_A = 38, KA_LF = 41, KA_COMP = 42,
-  // per direction d: 2 Ls2, Ldv norm64, Ldv, its part of Lvol; 3 k + d: dot terms
-  KA_DIR = 3 * KA_COMP, KA_DOT = KA_DIR + 12, KA_COUNT = KA_DOT + 9
+  // the differences of dL/ddv along V and W, the faces' terms (by the face's
+  // first diagonal), Lv12 U + dU; then the adjoints of the edges' cross products
+  // and of the cofactors
+  KA_W = 0, KA_F = 3, KA_D = 6, KA_U = 18, KA_DV = 21, KA_DW = 24, KA_LN = 27, KA_A = 33,
+  KA_LA = 36, KA_LC = 39, KA_COMP = 42,
+  // per direction d: 2 Ls2, Ldv norm64, its part of Lvol; 3 k + d: dot terms; per
+  // coordinate sg and the largest scale its adjoint vectors take
+  KA_DIR = 3 * KA_COMP, KA_DOT = KA_DIR + 9, KA_EXP = KA_DOT + 9, KA_COUNT = KA_EXP + 3
 };
 
 template <int MODE>
@@ -418,6 +443,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   wait_for_last_kernel();
   const double dt = rec->dt;
   auto sh = [&](int i) -> double& { return column[i * kFixedElems + lane]; };
+  auto num = [&](int i) -> fx::Num& { return reinterpret_cast<fx::Num*>(column)[i * kFixedElems + lane]; };
   const int own = KA_COMP * k, c1 = KA_COMP * (k == 2 ? 0 : k + 1), c2 = KA_COMP * (k == 0 ? 2 : k - 1);
   // component k of (slot p) x (slot q), added to y
   auto add_cross = [&](double y, int p, int q) {
@@ -432,7 +458,9 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   const double Ls = lvdov * inv, Ldet = -lvdov * a.vdov[e] * inv;
   const double ldelv = a.ldelv[e], Lar = a.larealg[e], lvnew_in = a.lvnew[e];
   if (live && k == 0) a.lv[e] -= ldelv;  // delv = vnew - v
-  double A[3], VW[3], C[3], dU[3];
+  double A[3], VW[3], C[3], U[3], dU[3];
+  unsigned top = 0;  // high word of the largest adjoint vector component
+  bool ok;           // extent in range
   {
     // direction k: limiter reads of this element's delv by its neighbours
     // (inverse neighbour list, fixed order) join its own delv adjoint
@@ -445,8 +473,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     const double t = a.ldx[k][e] * 16.0 * rs;
     sh(KA_DIR + k) = -(t * vol) * (rs * rs);  // 2 Ls2, Ls2 = Ldx 16 vol (-1/2) rs^3
     sh(KA_DIR + 3 + k) = Ldv * norm64;
-    sh(KA_DIR + 6 + k) = Ldv;
-    sh(KA_DIR + 9 + k) = t;
+    sh(KA_DIR + 6 + k) = t;
     const double dt2 = -0.5 * dt;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -464,11 +491,23 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
 #pragma unroll
     for (int q = 0; q < 12; ++q) {
       g[q] = tk(45 + 3 * q + k);
-      sh(own + KA_D + q) = g[q];
+      top = fx::umax(top, (unsigned)fx::hi_word(g[q]) & 0x7fffffffu);
     }
-    sh(own + KA_U) = g[6] + g[7];
-    sh(own + KA_U + 1) = g[8] + g[9];
-    sh(own + KA_U + 2) = g[10] + g[11];
+    const int eg = fx::exponent_field(top);
+    top = 0;
+    ok = eg >= fx::kMinExtent && eg <= fx::kMaxExtent;
+    num(KA_EXP + k).lo = 1081 - eg;  // below 2^59
+    fx::i64 x[12];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+      x[q] = fx::to_fixed(g[q], 6 - eg);
+      num(own + KA_D + q) = fx::limbs(x[q]);
+    }
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      U[t] = g[6 + 2 * t] + g[7 + 2 * t];
+      num(own + KA_U + t) = fx::limbs(fx::add(x[6 + 2 * t], x[7 + 2 * t]));
+    }
     // The next cycle's force kernel used the gradient of 12*volume (its
     // voluDer, dv): G = dL/ddv (zero before the first transposed cycle; the
     // faithful slots 1 and 3 swapped back) makes its transpose the
@@ -483,47 +522,81 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     dU[0] = (G[3] - G[1]) + (G[7] - G[2]);
     dU[1] = (G[4] - G[3]) + (G[5] - G[7]);
     dU[2] = (G[1] - G[4]) + (G[2] - G[5]);
-    sh(own + KA_DV) = G[6] - G[3];
-    sh(own + KA_DV + 1) = G[6] - G[4];
-    sh(own + KA_DV + 2) = G[6] - G[1];
-    sh(own + KA_DW) = G[2] - G[0];
-    sh(own + KA_DW + 1) = G[7] - G[0];
-    sh(own + KA_DW + 2) = G[5] - G[0];
+    auto put = [&](int i, double y) {
+      top = fx::umax(top, (unsigned)fx::hi_word(y) & 0x7fffffffu);
+      sh(own + i) = y;
+    };
+    put(KA_DV, G[6] - G[3]);
+    put(KA_DV + 1, G[6] - G[4]);
+    put(KA_DV + 2, G[6] - G[1]);
+    put(KA_DW, G[2] - G[0]);
+    put(KA_DW + 1, G[7] - G[0]);
+    put(KA_DW + 2, G[5] - G[0]);
     // The next cycle's stress force: face f's normal d1 x d2 with LN = s8 LU_f
     // gives d1 the adjoint d2 x LN and d2 the adjoint LN x d1; s8 from this
-    // cycle's end state.
+    // cycle's end state. Faces (d20, d31) (d50, d14) (d61, d25) (d72, d36) (d43,
+    // d07) with d36 = -d63, d07 = -d70, the adjoint pairs of the last two turned.
     const double s8 = ((-a.p1[e]) - a.q1[e]) * 0.125;
+    constexpr int at[5] = {3, 4, 0, 2, 1};
 #pragma unroll
-    for (int f = 0; f < 5; ++f) sh(own + KA_LN + f) = s8 * a.sLU[(3 * f + k) * E + e];
+    for (int f = 0; f < 5; ++f) put(KA_LN + at[f], s8 * a.sLU[(3 * f + k) * E + e]);
+    sh(own + KA_LN + 5) = 0.0;  // the face (d64, d57), of the characteristic length alone
   }
   __syncthreads();
   // ---- scalars of the volume, and the adjoints that crosses take ----
   double Lvnew = lvnew_in + ldelv, Lv12;
   double LVW[3], LF[3];
   {
-    double Lvol = 0.0, Lnorm64 = 0.0;
+    double Lvol = 0.0, Lnorm64 = 0.0;  // the latter times norm64
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const double dot = (sh(KA_DOT + d) + sh(KA_DOT + 3 + d)) + sh(KA_DOT + 6 + d);
-      Lvol += sh(KA_DIR + 9 + d);
-      Lnorm64 = fma(sh(KA_DIR + 6 + d), dot, Lnorm64);
+      Lvol += sh(KA_DIR + 6 + d);
       const double ldn = sh(KA_DIR + 3 + d);
+      Lnorm64 = fma(ldn, dot, Lnorm64);
       sh(own + KA_LA + d) = fma(A[d], sh(KA_DIR + d), ldn * VW[d]);
       LVW[d] = fma(ldn, A[d], Ls * C[d]);
       // velocity-gradient trace: cofactor columns C and 1/det
       sh(own + KA_LC + d) = d == 1 ? fma(Ldet, sh(own + KA_F + 1), Ls * VW[1]) : Ls * VW[d];
     }
-    Lvol = fma(Lnorm64, -64.0 * norm64 * norm64, Lvol);
+    Lvol = fma(Lnorm64, -64.0 * norm64, Lvol);
     Lvnew = fma(Lvol, volo, Lvnew);
     // characteristic length from the face the tape recorded
     const double rsc = tk(44);  // 1/|fa x fb|
     Lv12 = fma(Lar * 2.0, rsc, Lvnew * inv_volo) * (1.0 / 12.0);
-    // 2 Lcl, Lcl = Lar 2 volume (-1/2) rsc^3
-    sh(own + KA_LF) = tk(41 + k) * (-2.0 * (Lar * vol) * (rsc * rsc * rsc));
+    // 2 Lcl, Lcl = Lar 2 volume (-1/2) rsc^3, joins the terms of its face: in the
+    // kinematics face order (d20, d31) (d64, d57) (d50, d14) (d61, d25) (d72, d63)
+    // (d43, d70)
+    const double lf = tk(41 + k) * (-2.0 * (Lar * vol) * (rsc * rsc * rsc));
+    const int f = (int)((a.flags[e] >> TF_FACE_SHIFT) & 7ull);
+    const int at = KA_LN + ((0x120453 >> (4 * f)) & 15);
+    const double ln = sh(own + at) + (f < 4 ? lf : -lf);
+    sh(own + at) = ln;
+    top = fx::umax(top, (unsigned)fx::hi_word(ln) & 0x7fffffffu);
 #pragma unroll
-    for (int t = 0; t < 3; ++t) sh(own + KA_A + t) = fma(Lv12, sh(own + KA_U + t), dU[t]);
+    for (int t = 0; t < 3; ++t) {
+      const double y = fma(Lv12, U[t], dU[t]);
+      sh(own + KA_A + t) = y;
+      top = fx::umax(top, (unsigned)fx::hi_word(y) & 0x7fffffffu);
+    }
+    int ea = fx::exponent_field(top);
+    ok = ok && (top == 0 || (ea >= fx::kMinSpeed && ea <= fx::kMaxSpeed));
+    num(KA_EXP + k).hi = ok ? 1081 - fx::imax(ea, fx::kMinSpeed) : fx::kNoExponent;  // below 2^59
   }
   __syncthreads();
+  // scales: of an adjoint vector's component j sg[j] + common, of a cross's
+  // component k uc
+  int uc;
+  {
+    const fx::Num x0 = num(KA_EXP), x1 = num(KA_EXP + 1), x2 = num(KA_EXP + 2);
+    ok = fx::imin(x0.hi, fx::imin(x1.hi, x2.hi)) != fx::kNoExponent;
+    const int common = fx::imin(x0.hi - x0.lo, fx::imin(x1.hi - x1.lo, x2.hi - x2.lo));
+    const int sg = k == 0 ? x0.lo : k == 1 ? x1.lo : x2.lo;
+    uc = 61 - (x0.lo + x1.lo + x2.lo - sg + common);
+    if (ok)
+#pragma unroll
+      for (int q = KA_DV; q < KA_LA; ++q) num(own + q) = fx::limbs(to_fixed0(sh(own + q), sg + common - 1075));
+  }
   double Ldt = 0.0;
   // ---- positions' and velocities' edges ----
   double LW[3] = {0.0, 0.0, 0.0};
@@ -560,52 +633,111 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   // ---- volume and characteristic length, and the position transpose of the
   //      next cycle's k_force (same positions, same face diagonals) ----
   // dL/dU = Lv12 (V x W) + dV x W + V x dW, dL/dV = W x A + dW x U, dL/dW =
-  // A x V + U x dV with A = Lv12 U + dU (V x W is taped)
-  double L[12];
-  {
-    constexpr int iv[3] = {2, 5, 0}, iw[3] = {3, 1, 4}, ua[3] = {6, 8, 10}, ub[3] = {7, 9, 11};
+  // A x V + U x dV with A = Lv12 U + dU (V x W is taped). U, V, W of triple t:
+  // diagonals 6 + 2 t and 7 + 2 t, iv, iw; the partner of diagonal q in its face
+  constexpr int iv[3] = {2, 5, 0}, iw[3] = {3, 1, 4}, partner[12] = {11, 8, 7, 6, 10, 9, 3, 2, 1, 5, 4, 0};
+  // corners a diagonal runs from and to
+  constexpr int pp[12] = {6, 7, 6, 2, 5, 6, 3, 7, 4, 5, 1, 2}, pq[12] = {1, 0, 3, 0, 0, 4, 1, 2, 3, 7, 4, 5};
+  double vw[3], tm[4], LX[8];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) vw[t] = Lv12 * tk(81 + 3 * t + k);
+  // the next cycle's hourglass modes
+#pragma unroll
+  for (int m = 0; m < 4; ++m) tm[m] = a.sLhm[(k * 4 + m) * E + e];
+  __syncthreads();
+  bool summed = false;
+  if (ok) {
+    struct Cross { fx::Acc p, n; };
+    auto first = [&](int i, int j) {
+      Cross r;
+      r.p = fx::mul(num(c1 + i), num(c2 + j));
+      r.n = fx::mul(num(c2 + i), num(c1 + j));
+      return r;
+    };
+    auto plus = [&](Cross& r, int i, int j) {
+      fx::mac(r.p, num(c1 + i), num(c2 + j));
+      fx::mac(r.n, num(c2 + i), num(c1 + j));
+    };
+    auto value = [&](const Cross& r) {
+      fx::Acc d;
+      d.h = r.p.h - r.n.h;
+      d.m = r.p.m - r.n.m;
+      return fx::take<3>(d);
+    };
+    fx::i64 X[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // below 3 2^60
+    auto onto = [&](int q, fx::i64 y) { X[pp[q]] += y; X[pq[q]] -= y; };
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
-      const double gU = add_cross(add_cross(Lv12 * tk(81 + 3 * t + k), KA_DV + t, KA_D + iw[t]), KA_D + iv[t], KA_DW + t);
-      L[ua[t]] = gU;
-      L[ub[t]] = gU;
-      L[iv[t]] = add_cross(add_cross(0.0, KA_D + iw[t], KA_A + t), KA_DW + t, KA_U + t);
-      L[iw[t]] = add_cross(add_cross(0.0, KA_A + t, KA_D + iv[t]), KA_U + t, KA_DV + t);
+      const int v = iv[t], w = iw[t];
+      Cross r = first(KA_DV + t, KA_D + w);
+      plus(r, KA_D + v, KA_DW + t);
+      const fx::i64 gU = value(r);
+#pragma unroll
+      for (int q = 6 + 2 * t; q < 8 + 2 * t; ++q) onto(q, gU + value(first(KA_LN + partner[q], KA_D + partner[q])));
+      r = first(KA_D + w, KA_A + t);
+      plus(r, KA_DW + t, KA_U + t);
+      plus(r, KA_D + partner[v], KA_LN + v);
+      onto(v, value(r));
+      r = first(KA_A + t, KA_D + v);
+      plus(r, KA_U + t, KA_DV + t);
+      plus(r, KA_D + partner[w], KA_LN + w);
+      onto(w, value(r));
     }
-    // stress faces (d20, d31) (d50, d14) (d61, d25) (d72, d36) (d43, d07),
-    // d36 = -d63, d07 = -d70
-    L[3] = add_cross(L[3], KA_D + 6, KA_LN);
-    L[6] = add_cross(L[6], KA_LN, KA_D + 3);
-    L[4] = add_cross(L[4], KA_D + 10, KA_LN + 1);
-    L[10] = add_cross(L[10], KA_LN + 1, KA_D + 4);
-    L[0] = add_cross(L[0], KA_D + 11, KA_LN + 2);
-    L[11] = add_cross(L[11], KA_LN + 2, KA_D);
-    L[7] = add_cross(L[7], KA_LN + 3, KA_D + 2);
-    L[2] = add_cross(L[2], KA_D + 7, KA_LN + 3);
-    L[8] = add_cross(L[8], KA_LN + 4, KA_D + 1);
-    L[1] = add_cross(L[1], KA_D + 8, KA_LN + 4);
-    // characteristic face: diagonals fa, fb in the kinematics face order (d20,
-    // d31) (d64, d57) (d50, d14) (d61, d25) (d72, d63) (d43, d70)
-    const int f = (int)((a.flags[e] >> TF_FACE_SHIFT) & 7ull);
-    if (f == 0) { L[3] = add_cross(L[3], KA_D + 6, KA_LF); L[6] = add_cross(L[6], KA_LF, KA_D + 3); }
-    else if (f == 1) { L[5] = add_cross(L[5], KA_D + 9, KA_LF); L[9] = add_cross(L[9], KA_LF, KA_D + 5); }
-    else if (f == 2) { L[4] = add_cross(L[4], KA_D + 10, KA_LF); L[10] = add_cross(L[10], KA_LF, KA_D + 4); }
-    else if (f == 3) { L[0] = add_cross(L[0], KA_D + 11, KA_LF); L[11] = add_cross(L[11], KA_LF, KA_D); }
-    else if (f == 4) { L[7] = add_cross(L[7], KA_D + 2, KA_LF); L[2] = add_cross(L[2], KA_LF, KA_D + 7); }
-    else { L[8] = add_cross(L[8], KA_D + 1, KA_LF); L[1] = add_cross(L[1], KA_LF, KA_D + 8); }
+    // the other terms' mantissas below 2^58, ten to a corner
+    fx::Float f[10];
+    int top = fx::kNoExponent;
+#pragma unroll
+    for (int q = 0; q < 10; ++q) {
+      f[q] = fx::to_float(q < 3 ? vw[q] : q < 6 ? LW[q - 3] : tm[q - 6]);
+      top = fx::imax(top, f[q].k);
+    }
+    const int u = fx::imax(uc, top + 3);
+    summed = good_sum(top, u);
+    if (summed) {
+      fx::i64 i[10], y[8];
+#pragma unroll
+      for (int q = 0; q < 10; ++q) i[q] = in_unit(f[q], f[q].k, u);
+      const fx::i64 t[4] = {i[6], i[7], i[8], i[9]}, w[3] = {i[3], i[4], i[5]};
+      walsh_modes_t(t, y);
+      walsh1_t(w, y);
+#pragma unroll
+      for (int q = 6; q < 12; ++q) { y[pp[q]] += i[(q - 6) / 2]; y[pq[q]] -= i[(q - 6) / 2]; }
+      const int down = fx::imin(u - uc, 63);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) LX[c] = fx::to_double((X[c] >> down) + y[c], u);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) LX[c] = fx::to_double(X[c], uc);
+    }
+  } else {
+    const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+    auto at = [&](int j, int i) {
+      if (i >= KA_DV) return sh(KA_COMP * j + i);
+      auto d = [&](int q) { return a.kin[(45 + 3 * q + j) * E + e]; };
+      return i < KA_U ? d(i - KA_D) : d(6 + 2 * (i - KA_U)) + d(7 + 2 * (i - KA_U));
+    };
+    auto plus = [&](double y, int i, int j) { return fma(at(k1, i), at(k2, j), fma(-at(k2, i), at(k1, j), y)); };
+#pragma unroll
+    for (int c = 0; c < 8; ++c) LX[c] = 0.0;
+    auto onto = [&](int q, double y) { LX[pp[q]] += y; LX[pq[q]] -= y; };
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      const int v = iv[t], w = iw[t];
+      const double gU = plus(plus(0.0, KA_DV + t, KA_D + w), KA_D + v, KA_DW + t);
+#pragma unroll
+      for (int q = 6 + 2 * t; q < 8 + 2 * t; ++q) onto(q, plus(gU, KA_LN + partner[q], KA_D + partner[q]));
+      onto(v, plus(plus(plus(0.0, KA_D + w, KA_A + t), KA_DW + t, KA_U + t), KA_D + partner[v], KA_LN + v));
+      onto(w, plus(plus(plus(0.0, KA_A + t, KA_D + v), KA_U + t, KA_DV + t), KA_D + partner[w], KA_LN + w));
+    }
   }
-  // the position corners: the next cycle's hourglass-mode transpose Gamma^T
-  // dL/dhm, the edges' Walsh transpose, and the diagonals
-  double LX[8];
-  {
-    double t[4];
+  if (!summed) {
+    double y[8];
+    walsh_modes_t(tm, y);
+    walsh1_t(LW, y);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) t[m] = a.sLhm[(k * 4 + m) * E + e];
-    walsh_modes_t(t, LX);
-    walsh1_t(LW, LX);
-    constexpr int pp[12] = {6, 7, 6, 2, 5, 6, 3, 7, 4, 5, 1, 2}, pq[12] = {1, 0, 3, 0, 0, 4, 1, 2, 3, 7, 4, 5};
+    for (int q = 6; q < 12; ++q) { y[pp[q]] += vw[(q - 6) / 2]; y[pq[q]] -= vw[(q - 6) / 2]; }
 #pragma unroll
-    for (int q = 0; q < 12; ++q) { LX[pp[q]] += L[q]; LX[pq[q]] -= L[q]; }
+    for (int c = 0; c < 8; ++c) LX[c] += y[c];
   }
   if (live)
 #pragma unroll
@@ -707,7 +839,13 @@ __global__ void __launch_bounds__(kAdjBlock) ka_node(AdjDev a, const CycleRec* r
 // to corner 0 (the derivatives sum to zero over the corners, the modes' signs do
 // too). dL/ddv is formed up to the same constant for every corner, which the
 // differences it is used by do not see. A sum of products with coefficients of
-// different size takes the largest term's unit, the others' mantissas shifted.
+// different size takes the largest term's unit, the others' mantissas shifted. Values
+// outside 2^-400..2^400, infinities and NaN take the same sums in doubles, from
+// the tape.
+// What bounds it: integer and FP64 issue together. At 48^3 155 us with every
+// sum on the FP64 pipe (81 % busy), 116 us so (77 %); a gradient of 40 cycles at 48^3 went from 22.9 to 21.7 ms by this form, of 24 cycles at
+// 15^3 from 2.97 to 2.93 ms. Five blocks per SM (128 registers, no spills)
+// against six and seven: 21.63, 21.71, 21.78 ms.
 enum : int {
   HA_DV = 0,                 // 8 j + c: limbs of the volume derivatives of coordinate j
   HA_V = 24, HA_L = 48,      // 8 k + c: limbs of the corner differences of the velocities and force
@@ -733,16 +871,10 @@ __device__ __forceinline__ void corner_differences(const double u[8], Put put) {
   x.lo = 1081 - ev;
   x.hi = ok;
   put(0, x);
-  const fx::i64 u0 = fx::to_fixed(u[0], 6 - ev);
+  const fx::i64 u0 = to_fixed0(u[0], 6 - ev);
 #pragma unroll
-  for (int c = 1; c < 8; ++c) put(c, fx::limbs(fx::sub(fx::to_fixed(u[c], 6 - ev), u0)));
+  for (int c = 1; c < 8; ++c) put(c, fx::limbs(fx::sub(to_fixed0(u[c], 6 - ev), u0)));
 }
-
-// A coefficient's mantissa in the unit 2^u of a sum, its own unit being 2^e.
-__device__ __forceinline__ fx::i64 in_unit(const fx::Float& f, int e, int u) { return f.m >> fx::imin(u - e, 63); }
-// Whether a sum is in range: coefficients at most 2^400 (so not infinities or
-// NaN, top their largest exponent), and a unit whose values are doubles or none.
-__device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && (u < -2000 || u >= -950); }
 
 template <int MODE>
 __global__ void __launch_bounds__(3 * kFixedElems, 5) ka_hourglass(AdjDev a, double hgcoef) {
