@@ -688,8 +688,7 @@ int lulesh_adj_gradient(lulesh_adjoint* a, int64_t num_cycles, lulesh_adj_result
     cudaGraph_t g;
     ACK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int j = 0; j < K; ++j) {
-      launch_time_increment(d->dd.st, 1, prm, s);
-      launch_force(d->dd, prm, s);
+      launch_force(d->dd, prm, s, true);
       launch_node(d->dd, prm, aux, d->tuning, s);
       launch_kinematics(d->dd, prm, aux, s);
       launch_material(d->dd, prm, aux, d->tuning, s);

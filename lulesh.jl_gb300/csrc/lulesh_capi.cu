@@ -96,6 +96,7 @@ void lulesh::state_to_device_mirror(lulesh_domain* d) {
   s->done = 0;
   s->num_iters = LLONG_MAX;  // no cycle limit unless a run sets one
   s->first = 1;
+  s->force_status = 0;
 }
 
 void lulesh::state_from_device_mirror(lulesh_domain* d) {
@@ -215,14 +216,16 @@ static int launch_step(lulesh_domain* d, const Params& prm, bool with_time_incre
     d->ring_used += 1;
   }
   if (ev) cudaEventRecord(ev[0], s);
-  if (with_time_increment) {
+  // k_force takes the time step along, unless each is to be timed by itself
+  const bool with_force = with_time_increment && !timed;
+  if (with_time_increment && !with_force) {
     TraceRange r("timeIncrement!");
     launch_time_increment(d->dd.st, 1, prm, s);
   }
   if (ev) cudaEventRecord(ev[1], s);
   {
-    TraceRange r("calcForceForNodes");
-    launch_force(d->dd, prm, s);
+    TraceRange r(with_force ? "timeIncrement! + calcForceForNodes" : "calcForceForNodes");
+    launch_force(d->dd, prm, s, with_force);
   }
   if (ev) cudaEventRecord(ev[2], s);
   {

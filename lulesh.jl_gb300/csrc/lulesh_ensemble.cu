@@ -125,8 +125,7 @@ static void drop_graph(lulesh_ensemble* s) {
 }
 
 static void launch_cycle(lulesh_ensemble* s) {
-  launch_time_increment(s->dd.st, s->n, s->prm, s->stream);
-  launch_force(s->dd, s->prm, s->stream);
+  launch_force(s->dd, s->prm, s->stream, true);
   launch_node(s->dd, s->prm, false, s->tuning, s->stream);
   launch_kinematics(s->dd, s->prm, false, s->stream);
   launch_material(s->dd, s->prm, false, s->tuning, s->stream);
@@ -254,7 +253,7 @@ int lulesh_ens_create(const lulesh_instance* instances, int32_t n, int32_t mode,
     DevState& st = s->init_state[i];
     std::memset(&st, 0, sizeof(st));
     st.time = 0.0; st.deltatime = m.deltatime; st.dtcourant = 1e20; st.dthydro = 1e20; st.cycle = 0;
-    st.acc_courant = kInfBits; st.acc_hydro = kInfBits; st.status = 0; st.done = 0; st.first = 1;
+    st.acc_courant = kInfBits; st.acc_hydro = kInfBits; st.status = 0; st.done = 0; st.first = 1; st.force_status = 0;
     st.num_iters = LLONG_MAX;
   };
   {
@@ -334,6 +333,7 @@ int lulesh_ens_run(lulesh_ensemble* s, int64_t num_iters) {
     d.acc_hydro = kInfBits;
     if (d.status == 0u) d.done = 0;
     d.first = 1;
+    d.force_status = 0;
     d.num_iters = num_iters;
     budget = std::max<int64_t>(budget, num_iters - d.cycle);
   }

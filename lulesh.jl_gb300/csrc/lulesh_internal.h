@@ -105,13 +105,15 @@ inline void finish_params(Params& p) {
 // Device-resident step state. acc_* are running minima (bit patterns of
 // non-negative doubles, so an unsigned min is the FP min) filled by the
 // material kernel and folded into dtcourant/dthydro by timeIncrement.
-struct DevState {
+struct alignas(16) DevState {
   double time, deltatime, dtcourant, dthydro;
   long long cycle;
   unsigned long long acc_courant, acc_hydro;
-  unsigned int status;
-  int done;             // device run loop: 1 once stoptime/num_iters/error is reached
   long long num_iters;   // device run loop: stop once cycle >= num_iters (after the first)
+  // (these three in one load)
+  alignas(16) unsigned int status;
+  int done;             // device run loop: 1 once stoptime/num_iters/error is reached
+  unsigned int force_status;  // what k_force found while the cycle's time step ran beside it
   long long first;       // device run loop: 1 before the first cycle of a run call
 };
 

@@ -27,8 +27,32 @@ namespace lulesh {
 // device run loop) recorded an error or finished the run, as the reference
 // stops at its first raised error.
 __device__ __forceinline__ bool step_off(const DevState* st) {
-  return (*(volatile const unsigned int*)&st->status) != 0u || (*(volatile const int*)&st->done) != 0;
+  const uint2 f = __ldcv(reinterpret_cast<const uint2*>(&st->status));
+  return (f.x | f.y) != 0u;
 }
+
+// timeIncrement! of one problem in the device run loop.
+__device__ void advance_time(DevState* st, const Params& prm) {
+  if (st->done) return;
+  if (st->status) { st->done = 1; return; }
+  // fold the previous step's minima (src/domain.jl:3012-3014, 3050-3052)
+  if (dt_registers(st->acc_courant)) st->dtcourant = __longlong_as_double((long long)st->acc_courant);
+  if (dt_registers(st->acc_hydro)) st->dthydro = __longlong_as_double((long long)st->acc_hydro);
+  st->acc_courant = kInfBits;
+  st->acc_hydro = kInfBits;
+  // examples/benchmark.jl:82-98: while time < stoptime ... break if cycle >= num_iters
+  if (!(st->time < prm.stoptime) || (!st->first && st->cycle >= st->num_iters)) { st->done = 1; return; }
+  st->first = 0;
+  double time = st->time, dt = st->deltatime;
+  long long cycle = st->cycle;
+  time_increment(time, dt, cycle, st->dtcourant, st->dthydro, prm);
+  st->time = time;
+  st->deltatime = dt;
+  st->cycle = cycle;
+}
+
+// blocks of k_force that run the time steps of n problems
+__host__ __device__ constexpr int time_blocks(int n) { return (n + 3 * kFixedElems - 1) / (3 * kFixedElems); }
 
 // ---------------------------------------------------------------------------
 // k_force
@@ -50,8 +74,8 @@ struct ForceTape {
 // take (`mine`); every thread of the block calls it. Out of line: its registers
 // are not the kernel's.
 template <int MODE, bool TAPE>
-__device__ __noinline__ void force_fallback(const DevDomain& d, DevState* st, fx::Num* column, int e, bool mine,
-                                            double hgcoef) {
+__device__ __noinline__ void force_fallback(const DevDomain& d, DevState* st, unsigned* status, fx::Num* column, int e,
+                                            bool mine, double hgcoef) {
   const int E = d.E;
   const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
   const double* const X = k == 0 ? d.x : k == 1 ? d.y : d.z;
@@ -71,7 +95,7 @@ __device__ __noinline__ void force_fallback(const DevDomain& d, DevState* st, fx
   c.s8 = ((-d.p[e]) - d.q[e]) * 0.125;
   c.hourglass = gt_zero(hgcoef);
   double* const out = (k == 0 ? d.fcx : k == 1 ? d.fcy : d.fcz) + e;
-  force_fp64<MODE>(k, RealSlots{reinterpret_cast<double*>(column) + lane, kFixedElems}, x, v, c, mine, &st->status,
+  force_fp64<MODE>(k, RealSlots{reinterpret_cast<double*>(column) + lane, kFixedElems}, x, v, c, mine, status,
                    [&](int n, double f) { out[n * E] = f; }, ForceTape<TAPE>{TAPE ? d.tapeGeo + e : nullptr, E, true});
 }
 
@@ -83,12 +107,30 @@ __device__ __noinline__ void force_fallback(const DevDomain& d, DevState* st, fx
 // k_kinematics (0.87 ms of that kernel). Seven blocks per SM, 80 registers:
 // six (96 registers) 1.02 ms, five (128) 1.12 ms; below 45^3 the three are
 // alike.
-template <int MODE, bool ENS, bool TAPE>
+//
+// TIME: the cycle's timeIncrement! runs here too, by blocks of its own after
+// the elements'; the forces need neither dt nor time. The element blocks may
+// see the problem's done flag of before or after: a cycle it ends leaves
+// nothing but the corner forces, which nobody reads. An error they find waits in
+// force_status until k_node knows whether the cycle takes place. A launch less
+// per cycle: 25.8 -> 22.7 us at 8^3, 40.2 -> 35.3 at 30^3, 2139 -> 2137 at 150^3,
+// with the flags read in one load (one by one, past the first-level cache,
+// k_node's third flag cost 12 us at 150^3).
+template <int MODE, bool ENS, bool TAPE, bool TIME>
 __global__ void __launch_bounds__(3 * kFixedElems, 7)
     k_force(const __grid_constant__ DevDomain d, const __grid_constant__ Params prm) {
   __shared__ fx::Num column[fx::FS_COUNT * kFixedElems];
   const int E = d.E;
   const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
+  if (TIME) {
+    const int block = blockIdx.x - (E + kFixedElems - 1) / kFixedElems;
+    if (block >= 0) {
+      const int problem = block * (3 * kFixedElems) + threadIdx.x;
+      wait_for_last_kernel();
+      if (problem < d.ninst) advance_time(d.st + problem, prm);
+      return;
+    }
+  }
   // threads past the end repeat the last element and store nothing
   const int slot = blockIdx.x * kFixedElems + lane;
   const int e = slot < E ? slot : E - 1;
@@ -141,7 +183,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 7)
   }
   if (others) {
     __syncthreads();
-    force_fallback<MODE, TAPE>(d, st, column, e, live && !r.ok, hgcoef);
+    force_fallback<MODE, TAPE>(d, st, TIME ? &st->force_status : &st->status, column, e, live && !r.ok, hgcoef);
   }
 }
 
@@ -158,8 +200,14 @@ __global__ void __launch_bounds__(kMaxNodeBlock) k_node(DevDomain d, Params prm)
   const double im = LDG(&d.inv_nodalMass[i]);
   const int first = s < t ? LDG(&d.cornerList[s]) : 0;
   wait_for_last_kernel();
-  if (step_off(st)) return;
+  const uint4 flags = __ldcv(reinterpret_cast<const uint4*>(&st->status));  // status, done, force_status
   const double dt = st->deltatime;
+  if (flags.x | flags.y) return;
+  // what a k_force that ran beside the time step found
+  if (flags.z) {
+    atomicOr(&st->status, flags.z);
+    return;
+  }
 #ifdef LULESH_CHECK
   // the node's corner range must lie within the corner list; an empty one reads nothing
   if (s < 0 || t < s || t > d.nCornerList) { atomicOr(&st->status, ST_INDEX); t = s; }
@@ -908,25 +956,6 @@ __global__ void k_halo_delv(DevDomain d) {
 // ---------------------------------------------------------------------------
 // k_time_increment (device run loop): one thread per problem
 // ---------------------------------------------------------------------------
-__device__ void advance_time(DevState* st, const Params& prm) {
-  if (st->done) return;
-  if (st->status) { st->done = 1; return; }
-  // fold the previous step's minima (src/domain.jl:3012-3014, 3050-3052)
-  if (dt_registers(st->acc_courant)) st->dtcourant = __longlong_as_double((long long)st->acc_courant);
-  if (dt_registers(st->acc_hydro)) st->dthydro = __longlong_as_double((long long)st->acc_hydro);
-  st->acc_courant = kInfBits;
-  st->acc_hydro = kInfBits;
-  // examples/benchmark.jl:82-98: while time < stoptime ... break if cycle >= num_iters
-  if (!(st->time < prm.stoptime) || (!st->first && st->cycle >= st->num_iters)) { st->done = 1; return; }
-  st->first = 0;
-  double time = st->time, dt = st->deltatime;
-  long long cycle = st->cycle;
-  time_increment(time, dt, cycle, st->dtcourant, st->dthydro, prm);
-  st->time = time;
-  st->deltatime = dt;
-  st->cycle = cycle;
-}
-
 __global__ void k_time_increment(DevState* st, int n, Params prm) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   wait_for_last_kernel();
@@ -949,13 +978,16 @@ void launch_tape_geometry(const DevDomain& d, cudaStream_t s) {
   k_tape_geometry<<<(d.E + kFixedElems - 1) / kFixedElems, 3 * kFixedElems, 0, s>>>(d);
 }
 
-void launch_force(const DevDomain& d, const Params& prm, cudaStream_t s) {
+void launch_force(const DevDomain& d, const Params& prm, cudaStream_t s, bool time) {
   const int bs = 3 * kFixedElems;
   const int grid = (d.E + kFixedElems - 1) / kFixedElems;
-#define LULESH_FORCE(M)                                                  \
-  (d.elemInst  ? launch(k_force<M, true, false>, grid, bs, s, d, prm)     \
-   : d.tapeGeo ? launch(k_force<M, false, true>, grid, bs, s, d, prm)     \
-               : launch(k_force<M, false, false>, grid, bs, s, d, prm))
+  const int with = grid + time_blocks(d.ninst);
+#define LULESH_FORCE(M)                                                            \
+  (time ? (d.elemInst ? launch(k_force<M, true, false, true>, with, bs, s, d, prm)  \
+                      : launch(k_force<M, false, false, true>, with, bs, s, d, prm)) \
+   : d.elemInst ? launch(k_force<M, true, false, false>, grid, bs, s, d, prm)       \
+   : d.tapeGeo  ? launch(k_force<M, false, true, false>, grid, bs, s, d, prm)       \
+                : launch(k_force<M, false, false, false>, grid, bs, s, d, prm))
   switch (d.mode & 3) {
     case 0: LULESH_FORCE(0); break;
     case 1: LULESH_FORCE(1); break;

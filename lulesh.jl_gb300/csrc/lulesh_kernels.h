@@ -31,7 +31,9 @@ struct Tuning {
 
 // The first taped cycle's face diagonals and normals.
 void launch_tape_geometry(const DevDomain& d, cudaStream_t s);
-void launch_force(const DevDomain& d, const Params& prm, cudaStream_t s);
+// with time: the cycle's time step too, in place of launch_time_increment (not
+// while taping)
+void launch_force(const DevDomain& d, const Params& prm, cudaStream_t s, bool time = false);
 void launch_node(const DevDomain& d, const Params& prm, bool aux, const Tuning& t, cudaStream_t s);
 void launch_kinematics(const DevDomain& d, const Params& prm, bool aux, cudaStream_t s);
 void launch_material(const DevDomain& d, const Params& prm, bool aux, const Tuning& t, cudaStream_t s);
