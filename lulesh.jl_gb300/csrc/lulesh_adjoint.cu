@@ -358,7 +358,7 @@ static void reverse_cycle(lulesh_adjoint* a, const CycleRec* rec, cudaStream_t s
 #define LULESH_KA_CYCLE(M)                            \
   launch(ka_kinematics<M>, g3, b3, s, a->ad, rec);    \
   launch(ka_node, gn, kAdjBlock, s, a->ad, rec);      \
-  launch(ka_hourglass<M>, g3, b3, s, a->ad, hg)
+  launch(ka_hourglass<M>, g3 + 1, b3, s, a->ad, hg, gn, rec, a->dsc, prm)
   switch (mode & 3) {
     case 0: LULESH_KA_CYCLE(0); break;
     case 1: LULESH_KA_CYCLE(1); break;
@@ -366,7 +366,6 @@ static void reverse_cycle(lulesh_adjoint* a, const CycleRec* rec, cudaStream_t s
     default: LULESH_KA_CYCLE(3); break;
   }
 #undef LULESH_KA_CYCLE
-  launch(ka_cycle_close, 1, kCloseBlock, s, a->ad, g3, gn, rec, a->dsc, prm);
 }
 
 // Position transpose of the run's first cycle's k_force (the last one the
@@ -810,6 +809,8 @@ int lulesh_adj_gradient(lulesh_adjoint* a, int64_t num_cycles, lulesh_adj_result
   const Scalars5 final_sc = get_scalars(d);
   // ---- reverse sweep ----
   ACK(cudaMemsetAsync(a->dsc, 0, sizeof(AdjScal), s));
+  const int g3 = (a->E + kFixedElems - 1) / kFixedElems;
+  ACK(cudaMemsetAsync(a->ad.part_hg, 0, sizeof(double) * (size_t)g3, s));
   // the force-transpose inputs the first transposed cycle's ka_kinematics
   // reads (no cycle after it): zero
   ACK(cudaMemsetAsync(a->ad.fV, 0, 24 * sizeof(double) * (size_t)a->E, s));
@@ -871,14 +872,15 @@ int lulesh_adj_gradient(lulesh_adjoint* a, int64_t num_cycles, lulesh_adj_result
     ka_gather_corners<<<(a->N + kAdjBlock - 1) / kAdjBlock, kAdjBlock, 0, s>>>(a->ad);
   }
   copy_state_to_domain(a, a->final_state, s);
-  AdjScal hsc;
-  ACK(cudaMemcpyAsync(&hsc, a->dsc, sizeof(AdjScal), cudaMemcpyDeviceToHost, s));
+  ka_sum<<<1, kAdjBlock, 0, s>>>(a->ad.part_hg, g3, a->scal);
+  double grad_hgcoef;
+  ACK(cudaMemcpyAsync(&grad_hgcoef, a->scal, sizeof(double), cudaMemcpyDeviceToHost, s));
   ACK(cudaStreamSynchronize(s));
   set_scalars(d, final_sc);
   state_to_device_mirror(d);
   ACK(cudaMemcpy(d->dd.st, d->hst, sizeof(DevState), cudaMemcpyHostToDevice));
   auto t2 = std::chrono::steady_clock::now();
-  out.grad_hgcoef = hsc.Lhg;
+  out.grad_hgcoef = grad_hgcoef;
   out.sweep = plan;
   out.forward_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
   out.reverse_ms = std::chrono::duration<double, std::milli>(t2 - t1).count();

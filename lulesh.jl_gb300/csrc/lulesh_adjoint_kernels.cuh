@@ -34,7 +34,7 @@ struct CycleRec {
 
 // Adjoints of the Domain scalars carried from cycle to cycle.
 struct AdjScal {
-  double Ltime, Ldt, Ldtc, Ldth, Lhg;
+  double Ltime, Ldt, Ldtc, Ldth;
 };
 
 // The 11 state fields (x y z xd yd zd e p q v ss) of one stored state.
@@ -76,7 +76,7 @@ struct AdjDev {
   double *cX, *cV;                            // [3][8][E] kinematics corner buffers
   double *fX, *fV;                            // [3][8][E] force corner buffers: the first cycle's position
                                               // transpose; each cycle's hourglass velocity corners
-  double *part_dt, *part_dtn, *part_hg;       // per-block partial sums (kinematics, node, force)
+  double *part_dt, *part_dtn, *part_hg;       // per-block partial sums (kinematics, node; hourglass over the cycles)
   double *sLdv, *sLhm;                        // [3][8][E], [3][4][E]: hourglass -> geometry
   double* sLU;                                // [5][3][E]: the stress force's face terms (hourglass -> geometry)
 };
@@ -815,6 +815,86 @@ __global__ void __launch_bounds__(kAdjBlock) ka_node(AdjDev a, const CycleRec* r
   block_sum_to(Ldt, a.part_dtn);
 }
 
+// Transpose of timeIncrement! (src/domain.jl:920-961) for the recorded
+// inputs: Ldt is the adjoint of the new deltatime; adds to the adjoints of
+// the previous time, deltatime, dtcourant and dthydro along the branch taken.
+__host__ __device__ inline void time_increment_reverse(const CycleRec& r, const Params& prm, double Ldt,
+                                                       double& Ltime, double& Ldt_prev, double& Ldtc,
+                                                       double& Ldth) {
+  double targetdt = prm.stoptime - r.time_prev;
+  double dt_pre = r.dt_prev;
+  int which = 0, rb = 0;
+  bool mb = false;
+  const bool adaptive = prm.dtfixed <= 0.0 && r.cycle_prev != 0;
+  if (adaptive) {
+    const double olddt = r.dt_prev;
+    double gnewdt = (double)INFINITY;
+    if (r.dtc_in < gnewdt) { gnewdt = r.dtc_in / 2.0; which = 1; }
+    if (r.dth_in < gnewdt) { gnewdt = r.dth_in * 2.0 / 3.0; which = 2; }
+    double newdt = gnewdt;
+    const double ratio = newdt / olddt;
+    if (ratio >= 1.0) {
+      if (ratio < prm.deltatimemultlb) { newdt = olddt; rb = 1; }
+      else if (ratio > prm.deltatimemultub) { newdt = olddt * prm.deltatimemultub; rb = 2; }
+    }
+    if (!(newdt != newdt) && (prm.dtmax != prm.dtmax || prm.dtmax < newdt)) { newdt = prm.dtmax; mb = true; }
+    dt_pre = newdt;
+  }
+  bool t1 = false;
+  if (dt_pre < targetdt && targetdt < 4.0 * dt_pre / 3.0) { targetdt = 2.0 * dt_pre / 3.0; t1 = true; }
+  const bool t2 = targetdt < dt_pre;
+  double Lpre = 0.0;
+  if (t2) {
+    if (t1) Lpre += (2.0 / 3.0) * Ldt;
+    else Ltime += -Ldt;  // dt = stoptime - time
+  } else {
+    Lpre += Ldt;
+  }
+  if (!adaptive) { Ldt_prev += Lpre; return; }
+  if (mb) return;
+  if (rb == 1) { Ldt_prev += Lpre; return; }
+  if (rb == 2) { Ldt_prev += prm.deltatimemultub * Lpre; return; }
+  if (which == 1) Ldtc += 0.5 * Lpre;
+  else if (which == 2) Ldth += (2.0 / 3.0) * Lpre;
+}
+
+// Closes the transpose of one cycle's time (one block of 3 kFixedElems threads):
+// sums the kernels' partial adjoints of dt in a fixed order (each thread its
+// strided share of both, a warp tree, then the warps in order), then transposes
+// time += dt and timeIncrement! on the carried scalar adjoints.
+__device__ __noinline__ void cycle_close(const AdjDev& a, int ge, int gn, const CycleRec* rec, AdjScal* sc,
+                                         const Params& prm) {
+  constexpr int kBlock = 3 * kFixedElems;
+  double t_kin = 0.0, t_node = 0.0;
+  for (int j = threadIdx.x; j < ge; j += kBlock) t_kin += a.part_dt[j];
+  for (int j = threadIdx.x; j < gn; j += kBlock) t_node += a.part_dtn[j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    t_kin += __shfl_down_sync(0xffffffffu, t_kin, o);
+    t_node += __shfl_down_sync(0xffffffffu, t_node, o);
+  }
+  __shared__ double wsum[2][kBlock / 32];
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) { wsum[0][w] = t_kin; wsum[1][w] = t_node; }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double s_kin = wsum[0][0], s_node = wsum[1][0];
+#pragma unroll
+  for (int k = 1; k < kBlock / 32; ++k) { s_kin += wsum[0][k]; s_node += wsum[1][k]; }
+  const CycleRec r = *rec;
+  AdjScal v = *sc;
+  // a minimum the cycle did not reach leaves the scalar as it was
+  double Ldtc_prev = r.active_c ? 0.0 : v.Ldtc, Ldth_prev = r.active_h ? 0.0 : v.Ldth;
+  // time_n = time_{n-1} + dt_n
+  const double Ldt_tot = v.Ldt + (s_kin + s_node) + v.Ltime;
+  double Ldt_prev = 0.0;
+  time_increment_reverse(r, prm, Ldt_tot, v.Ltime, Ldt_prev, Ldtc_prev, Ldth_prev);
+  v.Ldt = Ldt_prev;
+  v.Ldtc = Ldtc_prev;
+  v.Ldth = Ldth_prev;
+  *sc = v;
+}
+
 // ---------------------------------------------------------------------------
 // Transpose of k_force, in two kernels: ka_hourglass (the FB hourglass force
 // onto the velocities, ss, v, hgcoef and the two geometric factors) and
@@ -846,6 +926,10 @@ __global__ void __launch_bounds__(kAdjBlock) ka_node(AdjDev a, const CycleRec* r
 // sum on the FP64 pipe (81 % busy), 116 us so (77 %); a gradient of 40 cycles at 48^3 went from 22.9 to 21.7 ms by this form, of 24 cycles at
 // 15^3 from 2.97 to 2.93 ms. Five blocks per SM (128 registers, no spills)
 // against six and seven: 21.63, 21.71, 21.78 ms.
+//
+// The last block closes the cycle's time beside the elements (nothing here reads
+// it). As a launch of one block it took 10 us of the chain at 48^3; a gradient of
+// 40 cycles 19.80 -> 19.35 ms without it, of 24 cycles at 15^3 2.78 -> 2.65.
 enum : int {
   HA_DV = 0,                 // 8 j + c: limbs of the volume derivatives of coordinate j
   HA_V = 24, HA_L = 48,      // 8 k + c: limbs of the corner differences of the velocities and force
@@ -877,9 +961,15 @@ __device__ __forceinline__ void corner_differences(const double u[8], Put put) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(3 * kFixedElems, 5) ka_hourglass(AdjDev a, double hgcoef) {
+__global__ void __launch_bounds__(3 * kFixedElems, 5)
+    ka_hourglass(AdjDev a, double hgcoef, int gn, const CycleRec* rec, AdjScal* sc, Params prm) {
   __shared__ double column[HA_COUNT * kFixedElems];
   const int E = a.E;
+  if (blockIdx.x == gridDim.x - 1) {
+    wait_for_last_kernel();
+    cycle_close(a, gridDim.x - 1, gn, rec, sc, prm);
+    return;
+  }
   const int lane = threadIdx.x % kFixedElems, k = threadIdx.x / kFixedElems;
   const int slot = blockIdx.x * kFixedElems + lane;
   const bool live = slot < E;
@@ -1163,7 +1253,12 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5) ka_hourglass(AdjDev a, dou
       a.lq[e] += Lpq;
     }
   }
-  block_sum3_to(Lhg_coef, a.part_hg);
+  // the block's sum over the cycles so far
+  if (k == 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) Lhg_coef += __shfl_down_sync(0xffffffffu, Lhg_coef, o);
+    if (lane == 0) a.part_hg[blockIdx.x] += Lhg_coef;
+  }
 }
 
 // Position transpose of one element's k_force, added into LX:
@@ -1297,89 +1392,6 @@ __device__ double block_fixed_sum(const double* part, int n) {
 __global__ void __launch_bounds__(kAdjBlock) ka_sum(const double* part, int n, double* out) {
   const double s = block_fixed_sum<kAdjBlock>(part, n);
   if (threadIdx.x == 0) *out = s;
-}
-
-// Transpose of timeIncrement! (src/domain.jl:920-961) for the recorded
-// inputs: Ldt is the adjoint of the new deltatime; adds to the adjoints of
-// the previous time, deltatime, dtcourant and dthydro along the branch taken.
-__host__ __device__ inline void time_increment_reverse(const CycleRec& r, const Params& prm, double Ldt,
-                                                       double& Ltime, double& Ldt_prev, double& Ldtc,
-                                                       double& Ldth) {
-  double targetdt = prm.stoptime - r.time_prev;
-  double dt_pre = r.dt_prev;
-  int which = 0, rb = 0;
-  bool mb = false;
-  const bool adaptive = prm.dtfixed <= 0.0 && r.cycle_prev != 0;
-  if (adaptive) {
-    const double olddt = r.dt_prev;
-    double gnewdt = (double)INFINITY;
-    if (r.dtc_in < gnewdt) { gnewdt = r.dtc_in / 2.0; which = 1; }
-    if (r.dth_in < gnewdt) { gnewdt = r.dth_in * 2.0 / 3.0; which = 2; }
-    double newdt = gnewdt;
-    const double ratio = newdt / olddt;
-    if (ratio >= 1.0) {
-      if (ratio < prm.deltatimemultlb) { newdt = olddt; rb = 1; }
-      else if (ratio > prm.deltatimemultub) { newdt = olddt * prm.deltatimemultub; rb = 2; }
-    }
-    if (!(newdt != newdt) && (prm.dtmax != prm.dtmax || prm.dtmax < newdt)) { newdt = prm.dtmax; mb = true; }
-    dt_pre = newdt;
-  }
-  bool t1 = false;
-  if (dt_pre < targetdt && targetdt < 4.0 * dt_pre / 3.0) { targetdt = 2.0 * dt_pre / 3.0; t1 = true; }
-  const bool t2 = targetdt < dt_pre;
-  double Lpre = 0.0;
-  if (t2) {
-    if (t1) Lpre += (2.0 / 3.0) * Ldt;
-    else Ltime += -Ldt;  // dt = stoptime - time
-  } else {
-    Lpre += Ldt;
-  }
-  if (!adaptive) { Ldt_prev += Lpre; return; }
-  if (mb) return;
-  if (rb == 1) { Ldt_prev += Lpre; return; }
-  if (rb == 2) { Ldt_prev += prm.deltatimemultub * Lpre; return; }
-  if (which == 1) Ldtc += 0.5 * Lpre;
-  else if (which == 2) Ldth += (2.0 / 3.0) * Lpre;
-}
-
-// Closes the transpose of one cycle (one block): sums the kernels' partial
-// adjoints of dt and hgcoef in a fixed order (each thread its strided share
-// of all three, a warp tree, then the warps in order), then transposes
-// time += dt and timeIncrement! on the carried scalar adjoints.
-constexpr int kCloseBlock = 256;
-__global__ void __launch_bounds__(kCloseBlock) ka_cycle_close(AdjDev a, int ge, int gn, const CycleRec* rec,
-                                                               AdjScal* sc, Params prm) {
-  wait_for_last_kernel();
-  double t_kin = 0.0, t_node = 0.0, t_hg = 0.0;
-  for (int j = threadIdx.x; j < ge; j += kCloseBlock) { t_kin += a.part_dt[j]; t_hg += a.part_hg[j]; }
-  for (int j = threadIdx.x; j < gn; j += kCloseBlock) t_node += a.part_dtn[j];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    t_kin += __shfl_down_sync(0xffffffffu, t_kin, o);
-    t_node += __shfl_down_sync(0xffffffffu, t_node, o);
-    t_hg += __shfl_down_sync(0xffffffffu, t_hg, o);
-  }
-  __shared__ double wsum[3][kCloseBlock / 32];
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) { wsum[0][w] = t_kin; wsum[1][w] = t_node; wsum[2][w] = t_hg; }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  double s_kin = wsum[0][0], s_node = wsum[1][0], s_hg = wsum[2][0];
-#pragma unroll
-  for (int k = 1; k < kCloseBlock / 32; ++k) { s_kin += wsum[0][k]; s_node += wsum[1][k]; s_hg += wsum[2][k]; }
-  const CycleRec r = *rec;
-  AdjScal v = *sc;
-  v.Lhg += s_hg;
-  // a minimum the cycle did not reach leaves the scalar as it was
-  double Ldtc_prev = r.active_c ? 0.0 : v.Ldtc, Ldth_prev = r.active_h ? 0.0 : v.Ldth;
-  // time_n = time_{n-1} + dt_n
-  const double Ldt_tot = v.Ldt + (s_kin + s_node) + v.Ltime;
-  double Ldt_prev = 0.0;
-  time_increment_reverse(r, prm, Ldt_tot, v.Ltime, Ldt_prev, Ldtc_prev, Ldth_prev);
-  v.Ldt = Ldt_prev;
-  v.Ldtc = Ldtc_prev;
-  v.Ldth = Ldth_prev;
-  *sc = v;
 }
 
 // Copies the 11 state fields (node fields n < N, element fields n < E).
