@@ -112,10 +112,6 @@ __device__ __forceinline__ V3 vcross(const V3& a, const V3& b) {
   cross(a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z);
   return c;
 }
-__device__ __forceinline__ double vdot(const V3& a, const V3& b) { return fma(a.x, b.x, fma(a.y, b.y, a.z * b.z)); }
-__device__ __forceinline__ void vaxpy(V3& y, double a, const V3& x) {
-  y.x = fma(a, x.x, y.x); y.y = fma(a, x.y, y.y); y.z = fma(a, x.z, y.z);
-}
 __device__ __forceinline__ void vadd(V3& y, const V3& x) { y.x += x.x; y.y += x.y; y.z += x.z; }
 
 // Resolved limiter neighbour: the element whose delv is read (self for a

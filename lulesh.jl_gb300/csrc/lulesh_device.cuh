@@ -1,10 +1,12 @@
 // Device-side element and node arithmetic of the LagrangeLeapFrog step.
 //
 // Every function restates a reference expression in a form with fewer FP64
-// instructions (GB300 issues about two FP64 instructions per clock per SM,
-// so the FP64 instruction count, not HBM, bounds this step). The
-// reformulations are exact in real arithmetic and differ from the
-// reference's left-to-right evaluation only by rounding:
+// instructions (GB300 issues about two FP64 instructions per clock per SM; the
+// geometry and the hourglass forces, two thirds of the step's arithmetic, run on
+// the integer pipes for that reason, lulesh_fixed.cuh, and in these forms where
+// that does not take an element). The reformulations are exact in real
+// arithmetic and differ from the reference's left-to-right evaluation only by
+// rounding:
 //  * the shape-function Jacobian columns (src/domain.jl:1964-1974) and the
 //    monotonic-Q gradients (src/domain.jl:2244-2254) are the first-order
 //    Walsh coefficients of the 8 corner values, taken through the four body
@@ -18,8 +20,8 @@
 //    each other (the face normals of a closed surface sum to zero);
 //  * a face's area vector (sumElemFaceNormal, src/domain.jl:971-989) is
 //    -(d1 x d2)/8 for the face's two diagonals d1, d2;
-//  * voluDer (src/domain.jl:1178-1211) only ever sums the 12 hex edges, so
-//    the 36 edge sums are formed once per element;
+//  * the eight voluDer calls (src/domain.jl:1178-1211) are the gradient of
+//    calcElemVolume's three triple products of face diagonals;
 //  * the velocity-gradient trace (src/domain.jl:2023-2081, 2156-2158) is
 //    trace(C^T W(v)) / det, with C the cofactors of the Jacobian and W(v) the
 //    Walsh coefficients of the velocities;
@@ -48,18 +50,6 @@ namespace lulesh {
 #else
 #define LULESH_IDX(i, n, st) (i)
 #endif
-
-// gamma[n][m] of calcFBHourglassForceForElems, src/domain.jl:1490-1499.
-__device__ __forceinline__ double gamma_nm(int n, int m) {
-  // column m is the Walsh function eta*zeta, xi*zeta, xi*eta, xi*eta*zeta
-  // over the corner signs xi = (-,+,+,-,-,+,+,-), eta = (-,-,+,+,-,-,+,+),
-  // zeta = (-,-,-,-,+,+,+,+).
-  const int xs = ((n == 1) | (n == 2) | (n == 5) | (n == 6)) ? 1 : -1;
-  const int es = ((n == 2) | (n == 3) | (n == 6) | (n == 7)) ? 1 : -1;
-  const int zs = (n >= 4) ? 1 : -1;
-  const int v = (m == 0) ? es * zs : (m == 1) ? xs * zs : (m == 2) ? xs * es : xs * es * zs;
-  return (double)v;
-}
 
 // First-order Walsh coefficients (xi, eta, zeta) of 8 corner values through
 // the four body diagonals: 11 FP64 adds.
@@ -118,12 +108,6 @@ __device__ __forceinline__ bool lt_zero(double a) { return fkey(a) < 0; }  // a 
 __device__ __forceinline__ bool is_zero(double a) {                         // a == 0.0
   return (__double_as_longlong(a) & 0x7FFFFFFFFFFFFFFFll) == 0;
 }
-// max of two non-negative doubles (+0 included) by their bit patterns
-__device__ __forceinline__ double max_nonneg(double a, double b) {
-  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-  return __longlong_as_double(x > y ? x : y);
-}
-
 // x^(-1/3) for x > 0 in six FP64 instructions: a single-precision seed y0
 // refined by one second-order Householder step. With e = 1 - x y0^3 the
 // exact value is y0 (1 - e)^(-1/3) = y0 (1 + e/3 + 2e^2/9 + 14e^3/81 + ...);

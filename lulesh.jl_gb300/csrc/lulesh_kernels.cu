@@ -1,5 +1,7 @@
-// The LagrangeLeapFrog step as four sm_103a kernels (one thread per element
-// or node, FP64 throughout):
+// The LagrangeLeapFrog step as four sm_103a kernels. k_force and k_kinematics
+// run three threads per element, one per coordinate, on 64-bit fixed-point
+// numbers (lulesh_fixed.cuh; elements these do not take in FP64), k_node and
+// k_material one thread per node or element in FP64:
 //   k_force      calcVolumeForceForElems: stress integration + FB hourglass,
 //                one 8-corner force triple per element corner
 //                (src/domain.jl:963-1762)
@@ -12,8 +14,8 @@
 //                applyMaterialPropertiesForElems/evalEOSForElems +
 //                updateVolumesForElems + Courant/hydro dt minima
 //                (src/domain.jl:2322-3064)
-// plus k_time_increment (timeIncrement!, src/domain.jl:920-961) for the
-// device-resident run loop.
+// plus timeIncrement! (src/domain.jl:920-961) for the device-resident run loop,
+// in blocks of k_force or as k_time_increment.
 #include "lulesh_device.cuh"
 #include "lulesh_element_fp64.cuh"
 #include "lulesh_fixed_force.cuh"
