@@ -93,16 +93,6 @@ __device__ __forceinline__ void block_sum_to(double v, double* out) {
   if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
-// The same for a block of one thread per element and coordinate.
-__device__ __forceinline__ void block_sum3_to(double v, double* out) {
-  __shared__ double part[3];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) out[blockIdx.x] = (part[0] + part[1]) + part[2];
-}
-
 struct V3 {
   double x, y, z;
 };
@@ -415,7 +405,9 @@ __device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && 
 // crosses and corner sums on the FP64 pipe (87 % busy), 116 us so (78 %); a
 // gradient of 40 cycles at 48^3 21.7 -> 20.0 ms, of 24 cycles at 15^3 2.81 ->
 // 2.73. Six blocks per SM (96 registers; 147 slots are the most six can have)
-// against five and seven: 20.04, 20.37, 20.18 ms.
+// against five and seven: 20.04, 20.37, 20.18 ms. The volume's scalars in one
+// thread instead of all three (a barrier more) and the velocity corners on the
+// integer pipes: 19.52 -> 18.91 ms, 2.65 -> 2.61.
 enum : int {
   // per coordinate: mean edges, half-step edges, tape's 12 diagonals, U vectors,
   // the differences of dL/ddv along V and W, the faces' terms (by the face's
@@ -539,31 +531,37 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     sh(own + KA_LN + 5) = 0.0;  // the face (d64, d57), of the characteristic length alone
   }
   __syncthreads();
-  // ---- scalars of the volume, and the adjoints that crosses take ----
-  double Lvnew = lvnew_in + ldelv, Lv12;
+  // ---- the edges' adjoints; in thread 0 the scalars of the volume ----
   double LVW[3], LF[3];
-  {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double ldn = sh(KA_DIR + 3 + d);
+    sh(own + KA_LA + d) = fma(A[d], sh(KA_DIR + d), ldn * VW[d]);
+    LVW[d] = fma(ldn, A[d], Ls * C[d]);
+    // velocity-gradient trace: cofactor columns C and 1/det
+    sh(own + KA_LC + d) = d == 1 ? fma(Ldet, sh(own + KA_F + 1), Ls * VW[1]) : Ls * VW[d];
+  }
+  if (k == 0) {
     double Lvol = 0.0, Lnorm64 = 0.0;  // the latter times norm64
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const double dot = (sh(KA_DOT + d) + sh(KA_DOT + 3 + d)) + sh(KA_DOT + 6 + d);
       Lvol += sh(KA_DIR + 6 + d);
-      const double ldn = sh(KA_DIR + 3 + d);
-      Lnorm64 = fma(ldn, dot, Lnorm64);
-      sh(own + KA_LA + d) = fma(A[d], sh(KA_DIR + d), ldn * VW[d]);
-      LVW[d] = fma(ldn, A[d], Ls * C[d]);
-      // velocity-gradient trace: cofactor columns C and 1/det
-      sh(own + KA_LC + d) = d == 1 ? fma(Ldet, sh(own + KA_F + 1), Ls * VW[1]) : Ls * VW[d];
+      Lnorm64 = fma(sh(KA_DIR + 3 + d), (sh(KA_DOT + d) + sh(KA_DOT + 3 + d)) + sh(KA_DOT + 6 + d), Lnorm64);
     }
     Lvol = fma(Lnorm64, -64.0 * norm64, Lvol);
-    Lvnew = fma(Lvol, volo, Lvnew);
+    const double Lvnew = fma(Lvol, volo, lvnew_in + ldelv);
     // characteristic length from the face the tape recorded
     const double rsc = tk(44);  // 1/|fa x fb|
-    Lv12 = fma(Lar * 2.0, rsc, Lvnew * inv_volo) * (1.0 / 12.0);
-    // 2 Lcl, Lcl = Lar 2 volume (-1/2) rsc^3, joins the terms of its face: in the
-    // kinematics face order (d20, d31) (d64, d57) (d50, d14) (d61, d25) (d72, d63)
-    // (d43, d70)
-    const double lf = tk(41 + k) * (-2.0 * (Lar * vol) * (rsc * rsc * rsc));
+    sh(KA_DOT) = fma(Lar * 2.0, rsc, Lvnew * inv_volo) * (1.0 / 12.0);
+    // 2 Lcl, Lcl = Lar 2 volume (-1/2) rsc^3
+    sh(KA_DOT + 1) = -2.0 * (Lar * vol) * (rsc * rsc * rsc);
+  }
+  __syncthreads();
+  const double Lv12 = sh(KA_DOT);
+  {
+    // the characteristic length joins the terms of its face: in the kinematics
+    // face order (d20, d31) (d64, d57) (d50, d14) (d61, d25) (d72, d63) (d43, d70)
+    const double lf = tk(41 + k) * sh(KA_DOT + 1);
     const int f = (int)((a.flags[e] >> TF_FACE_SHIFT) & 7ull);
     const int at = KA_LN + ((0x120453 >> (4 * f)) & 15);
     const double ln = sh(own + at) + (f < 4 ? lf : -lf);
@@ -578,20 +576,6 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     int ea = fx::exponent_field(top);
     ok = ok && (top == 0 || (ea >= fx::kMinSpeed && ea <= fx::kMaxSpeed));
     num(KA_EXP + k).hi = ok ? 1081 - fx::imax(ea, fx::kMinSpeed) : fx::kNoExponent;  // below 2^59
-  }
-  __syncthreads();
-  // scales: of an adjoint vector's component j sg[j] + common, of a cross's
-  // component k uc
-  int uc;
-  {
-    const fx::Num x0 = num(KA_EXP), x1 = num(KA_EXP + 1), x2 = num(KA_EXP + 2);
-    ok = fx::imin(x0.hi, fx::imin(x1.hi, x2.hi)) != fx::kNoExponent;
-    const int common = fx::imin(x0.hi - x0.lo, fx::imin(x1.hi - x1.lo, x2.hi - x2.lo));
-    const int sg = k == 0 ? x0.lo : k == 1 ? x1.lo : x2.lo;
-    uc = 61 - (x0.lo + x1.lo + x2.lo - sg + common);
-    if (ok)
-#pragma unroll
-      for (int q = KA_DV; q < KA_LA; ++q) num(own + q) = fx::limbs(to_fixed0(sh(own + q), sg + common - 1075));
   }
   double Ldt = 0.0;
   // ---- positions' and velocities' edges ----
@@ -614,17 +598,51 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
       LVW[d] = fma(-0.5 * dt, LF[d], LVW[d]);
       Ldt = fma(LF[d], VW[d], Ldt);
     }
-    Ldt *= -0.5;
+    sh(KA_DIR + k) = live ? -0.5 * Ldt : 0.0;
+  }
+  __syncthreads();
+  // scales: of an adjoint vector's component j sg[j] + common, of a cross's
+  // component k uc
+  int uc;
+  {
+    const fx::Num x0 = num(KA_EXP), x1 = num(KA_EXP + 1), x2 = num(KA_EXP + 2);
+    ok = fx::imin(x0.hi, fx::imin(x1.hi, x2.hi)) != fx::kNoExponent;
+    const int common = fx::imin(x0.hi - x0.lo, fx::imin(x1.hi - x1.lo, x2.hi - x2.lo));
+    const int sg = k == 0 ? x0.lo : k == 1 ? x1.lo : x2.lo;
+    uc = 61 - (x0.lo + x1.lo + x2.lo - sg + common);
+    if (ok)
+#pragma unroll
+      for (int q = KA_DV; q < KA_LA; ++q) num(own + q) = fx::limbs(to_fixed0(sh(own + q), sg + common - 1075));
   }
   // the velocity corners (the Walsh transpose), plus the hourglass velocity
   // corners of the cycle after this one
   {
-    const double p = LVW[0] + LVW[2], q = LVW[2] - LVW[0];
-    const double La = p + LVW[1], Lb = p - LVW[1], Lc = q + LVW[1], Ld = q - LVW[1];
-    const double LV[8] = {-La, -Lc, -Ld, -Lb, Ld, Lb, La, Lc};
-    if (live)
+    fx::Float f[11];  // LVW, then the corners: mantissas below 2^59, four to a corner
+    int top = fx::kNoExponent;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) a.cV[(k * 8 + c) * E + e] = LV[c] + a.fV[(k * 8 + c) * E + e];
+    for (int q = 0; q < 11; ++q) {
+      f[q] = fx::to_float(q < 3 ? LVW[q] : a.fV[(k * 8 + q - 3) * E + e]);
+      top = fx::imax(top, f[q].k);
+    }
+    const int u = top + 2;
+    if (good_sum(top, u)) {
+      fx::i64 y[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) y[c] = in_unit(f[3 + c], f[3 + c].k, u);
+      const fx::i64 w[3] = {in_unit(f[0], f[0].k, u), in_unit(f[1], f[1].k, u), in_unit(f[2], f[2].k, u)};
+      walsh1_t(w, y);
+      if (live)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) a.cV[(k * 8 + c) * E + e] = fx::to_double(y[c], u);
+    } else {
+      double y[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) y[c] = a.fV[(k * 8 + c) * E + e];
+      walsh1_t(LVW, y);
+      if (live)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) a.cV[(k * 8 + c) * E + e] = y[c];
+    }
   }
   // ---- volume and characteristic length, and the position transpose of the
   //      next cycle's k_force (same positions, same face diagonals) ----
@@ -738,7 +756,12 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   if (live)
 #pragma unroll
     for (int c = 0; c < 8; ++c) a.cX[(k * 8 + c) * E + e] = LX[c];
-  block_sum3_to(live ? Ldt : 0.0, a.part_dt);
+  if (k == 2) {
+    double Ldt = (sh(KA_DIR) + sh(KA_DIR + 1)) + sh(KA_DIR + 2);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) Ldt += __shfl_down_sync(0xffffffffu, Ldt, o);
+    if (lane == 0) a.part_dt[blockIdx.x] = Ldt;
+  }
 }
 
 // Sums the force corner buffers into node adjoints (added to what is there):
