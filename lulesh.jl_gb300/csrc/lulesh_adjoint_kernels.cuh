@@ -394,29 +394,30 @@ __device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && 
 // as in the forward kernels: a thread forms its component of every product,
 // and what a cross product needs of the other components is in shared memory.
 //
-// The crosses onto the face diagonals, all of a diagonal (or a sum of two) and
-// an adjoint vector, and the sums onto the position corners run on the integer
-// pipes. Diagonals are scaled by their coordinate's extent 2^-sg[k], adjoint
-// vectors by 2^-(sg[k] + common), so that both products of a cross have one
-// unit; what else joins the corners (edges, modes, V x W) enters as mantissas
-// in the largest term's unit. Elements of sizes or adjoints out of range take
-// the crosses in doubles, the diagonals from the tape.
-// What bounds it: integer and FP64 issue together. At 48^3 173 us with the
-// crosses and corner sums on the FP64 pipe (87 % busy), 116 us so (78 %); a
-// gradient of 40 cycles at 48^3 21.7 -> 20.0 ms, of 24 cycles at 15^3 2.81 ->
-// 2.73. Six blocks per SM (96 registers; 147 slots are the most six can have)
-// against five and seven: 20.04, 20.37, 20.18 ms. The volume's scalars in one
-// thread instead of all three (a barrier more) and the velocity corners on the
-// integer pipes: 19.52 -> 18.91 ms, 2.65 -> 2.61.
+// The crosses onto the edges and the face diagonals, all of an edge, a diagonal
+// (or a sum of two) and an adjoint vector, and the sums onto the position corners
+// run on the integer pipes. Edges and diagonals are scaled by their coordinate's
+// extent 2^-sg[k], adjoint vectors by 2^-(sg[k] + common), so that both products
+// of a cross have one unit; what else joins the corners (edges, modes, V x W)
+// enters as mantissas in the largest term's unit. Elements of sizes or adjoints
+// out of range take the crosses in doubles, the positions' part from the tape.
+// Bound by FP64 issue (350 slots per element, the pipe 71 % busy; ALU 29 %,
+// multiply-adds 16 %). At 48^3 173 us with the crosses and corner sums on the FP64
+// pipe (87 % busy), 116 us so; a gradient of 40 cycles at 48^3 21.7 -> 20.0 ms, of
+// 24 cycles at 15^3 2.81 -> 2.73. Six blocks per SM (96 registers; 148 slots are
+// the most six can have) against five and seven: 20.04, 20.37, 20.18 ms. The
+// volume's scalars in one thread instead of all three (a barrier more) and the
+// velocity corners on the integer pipes: 101 us, 19.52 -> 18.91 ms, 2.65 -> 2.61;
+// the edges' crosses there too: 95 us, 18.61 -> 18.29, 2.60 -> 2.60.
 enum : int {
-  // per coordinate: mean edges, half-step edges, tape's 12 diagonals, U vectors,
+  // per coordinate: mean edges, half-step edges, 12 diagonals, U vectors (limbs),
   // the differences of dL/ddv along V and W, the faces' terms (by the face's
   // first diagonal), Lv12 U + dU; then the adjoints of the edges' cross products
-  // and of the cofactors
+  // and of the cofactors (doubles, then limbs)
   KA_W = 0, KA_F = 3, KA_D = 6, KA_U = 18, KA_DV = 21, KA_DW = 24, KA_LN = 27, KA_A = 33,
   KA_LA = 36, KA_LC = 39, KA_COMP = 42,
   // per direction d: 2 Ls2, Ldv norm64, its part of Lvol; 3 k + d: dot terms; per
-  // coordinate sg and the largest scale its adjoint vectors take
+  // coordinate sg and the largest scales its adjoint vectors take
   KA_DIR = 3 * KA_COMP, KA_DOT = KA_DIR + 9, KA_EXP = KA_DOT + 9, KA_COUNT = KA_EXP + 3
 };
 
@@ -433,10 +434,6 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   auto sh = [&](int i) -> double& { return column[i * kFixedElems + lane]; };
   auto num = [&](int i) -> fx::Num& { return reinterpret_cast<fx::Num*>(column)[i * kFixedElems + lane]; };
   const int own = KA_COMP * k, c1 = KA_COMP * (k == 2 ? 0 : k + 1), c2 = KA_COMP * (k == 0 ? 2 : k - 1);
-  // component k of (slot p) x (slot q), added to y
-  auto add_cross = [&](double y, int p, int q) {
-    return fma(sh(c1 + p), sh(c2 + q), fma(-sh(c2 + p), sh(c1 + q), y));
-  };
   // forward values from the kinematics kernel's tape (slots: see tapeKin)
   auto tk = [&](int q) { return a.kin[q * E + e]; };
 
@@ -446,9 +443,10 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   const double Ls = lvdov * inv, Ldet = -lvdov * a.vdov[e] * inv;
   const double ldelv = a.ldelv[e], Lar = a.larealg[e], lvnew_in = a.lvnew[e];
   if (live && k == 0) a.lv[e] -= ldelv;  // delv = vnew - v
-  double A[3], VW[3], C[3], U[3], dU[3];
+  double A[3], VW[3], C[3], U[3], dU[3], F1;
   unsigned top = 0;  // high word of the largest adjoint vector component
   bool ok;           // extent in range
+  int sg;            // its scale
   {
     // direction k: limiter reads of this element's delv by its neighbours
     // (inverse neighbour list, fixed order) join its own delv adjoint
@@ -463,16 +461,19 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     sh(KA_DIR + 3 + k) = Ldv * norm64;
     sh(KA_DIR + 6 + k) = t;
     const double dt2 = -0.5 * dt;
+    double W[3], F[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const double w = tk(3 * k + d);
       VW[d] = tk(9 + 3 * k + d);
       A[d] = tk(28 + 3 * d + k);
       C[d] = tk(18 + 3 * d + k);
-      sh(own + KA_W + d) = w;
-      sh(own + KA_F + d) = fma(dt2, VW[d], w);
+      W[d] = w;
+      F[d] = fma(dt2, VW[d], w);
+      top = fx::umax(top, fx::umax((unsigned)fx::hi_word(W[d]) & 0x7fffffffu, (unsigned)fx::hi_word(F[d]) & 0x7fffffffu));
       sh(KA_DOT + 3 * k + d) = A[d] * VW[d];
     }
+    F1 = F[1];
     // the 12 diagonals of the new positions: d61 d70 d63 d20 d50 d64 d31 d72
     // d43 d57 d14 d25
     double g[12];
@@ -484,7 +485,12 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     const int eg = fx::exponent_field(top);
     top = 0;
     ok = eg >= fx::kMinExtent && eg <= fx::kMaxExtent;
-    num(KA_EXP + k).lo = 1081 - eg;  // below 2^59
+    sg = 1081 - eg;  // below 2^59
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      num(own + KA_W + d) = fx::limbs(fx::to_fixed(W[d], 6 - eg));
+      num(own + KA_F + d) = fx::limbs(fx::to_fixed(F[d], 6 - eg));
+    }
     fx::i64 x[12];
 #pragma unroll
     for (int q = 0; q < 12; ++q) {
@@ -532,14 +538,25 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   }
   __syncthreads();
   // ---- the edges' adjoints; in thread 0 the scalars of the volume ----
-  double LVW[3], LF[3];
+  double LVW[3], LA[3], LC[3];
+  {
+    unsigned ta = 0, tc = 0;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double ldn = sh(KA_DIR + 3 + d);
-    sh(own + KA_LA + d) = fma(A[d], sh(KA_DIR + d), ldn * VW[d]);
-    LVW[d] = fma(ldn, A[d], Ls * C[d]);
-    // velocity-gradient trace: cofactor columns C and 1/det
-    sh(own + KA_LC + d) = d == 1 ? fma(Ldet, sh(own + KA_F + 1), Ls * VW[1]) : Ls * VW[d];
+    for (int d = 0; d < 3; ++d) {
+      const double ldn = sh(KA_DIR + 3 + d);
+      LA[d] = fma(A[d], sh(KA_DIR + d), ldn * VW[d]);
+      LVW[d] = fma(ldn, A[d], Ls * C[d]);
+      // velocity-gradient trace: cofactor columns C and 1/det
+      LC[d] = d == 1 ? fma(Ldet, F1, Ls * VW[1]) : Ls * VW[d];
+      ta = fx::umax(ta, (unsigned)fx::hi_word(LA[d]) & 0x7fffffffu);
+      tc = fx::umax(tc, (unsigned)fx::hi_word(LC[d]) & 0x7fffffffu);
+    }
+    // the scale of below 2^59, plus 512; 0: out of range
+    auto limit = [&](unsigned t) {
+      const int x = fx::exponent_field(t);
+      return ok && (t == 0 || (x >= fx::kMinSpeed && x <= fx::kMaxSpeed)) ? 1081 - fx::imax(x, fx::kMinSpeed) + 512 : 0;
+    };
+    num(KA_EXP + k).lo = (sg & 0xff) | limit(ta) << 8 | limit(tc) << 20;
   }
   if (k == 0) {
     double Lvol = 0.0, Lnorm64 = 0.0;  // the latter times norm64
@@ -577,28 +594,31 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     ok = ok && (top == 0 || (ea >= fx::kMinSpeed && ea <= fx::kMaxSpeed));
     num(KA_EXP + k).hi = ok ? 1081 - fx::imax(ea, fx::kMinSpeed) : fx::kNoExponent;  // below 2^59
   }
-  double Ldt = 0.0;
-  // ---- positions' and velocities' edges ----
-  double LW[3] = {0.0, 0.0, 0.0};
+  // the edges' adjoints in their units
+  bool ok_edges;
+  int uA, uC;
   {
-    // direction d uses A = P x Q
-    constexpr int Pi[3] = {1, 2, 0}, Qi[3] = {2, 0, 1};
+    const int x0 = num(KA_EXP).lo, x1 = num(KA_EXP + 1).lo, x2 = num(KA_EXP + 2).lo;
+    auto least = [&](int shift) {
+      const int a0 = (x0 >> shift) & 0xfff, a1 = (x1 >> shift) & 0xfff, a2 = (x2 >> shift) & 0xfff;
+      return fx::imin(a0, fx::imin(a1, a2)) == 0
+                 ? fx::kNoExponent
+                 : fx::imin(a0 - (x0 & 0xff), fx::imin(a1 - (x1 & 0xff), a2 - (x2 & 0xff))) - 512;
+    };
+    const int cA = least(8), cC = least(20), both = (x0 & 0xff) + (x1 & 0xff) + (x2 & 0xff) - sg;
+    ok_edges = fx::imin(cA, cC) != fx::kNoExponent;
+    uA = 61 - (both + cA);
+    uC = 61 - (both + cC);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      LW[Pi[d]] = add_cross(LW[Pi[d]], KA_W + Qi[d], KA_LA + d);
-      LW[Qi[d]] = add_cross(LW[Qi[d]], KA_LA + d, KA_W + Pi[d]);
+      if (ok_edges) {
+        num(own + KA_LA + d) = fx::limbs(to_fixed0(LA[d], sg + cA - 1075));
+        num(own + KA_LC + d) = fx::limbs(to_fixed0(LC[d], sg + cC - 1075));
+      } else {
+        sh(own + KA_LA + d) = LA[d];
+        sh(own + KA_LC + d) = LC[d];
+      }
     }
-    // C0 = F1 x F2, C1 = F2 x F0, C2 = F0 x F1
-    LF[0] = add_cross(add_cross(0.0, KA_LC + 1, KA_F + 2), KA_F + 1, KA_LC + 2);
-    LF[1] = add_cross(add_cross(Ldet * C[1], KA_F + 2, KA_LC), KA_LC + 2, KA_F);
-    LF[2] = add_cross(add_cross(0.0, KA_LC, KA_F + 1), KA_F, KA_LC + 1);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      LW[d] += LF[d];
-      LVW[d] = fma(-0.5 * dt, LF[d], LVW[d]);
-      Ldt = fma(LF[d], VW[d], Ldt);
-    }
-    sh(KA_DIR + k) = live ? -0.5 * Ldt : 0.0;
   }
   __syncthreads();
   // scales: of an adjoint vector's component j sg[j] + common, of a cross's
@@ -607,12 +627,70 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   {
     const fx::Num x0 = num(KA_EXP), x1 = num(KA_EXP + 1), x2 = num(KA_EXP + 2);
     ok = fx::imin(x0.hi, fx::imin(x1.hi, x2.hi)) != fx::kNoExponent;
-    const int common = fx::imin(x0.hi - x0.lo, fx::imin(x1.hi - x1.lo, x2.hi - x2.lo));
-    const int sg = k == 0 ? x0.lo : k == 1 ? x1.lo : x2.lo;
-    uc = 61 - (x0.lo + x1.lo + x2.lo - sg + common);
+    const int s0 = x0.lo & 0xff, s1 = x1.lo & 0xff, s2 = x2.lo & 0xff;
+    const int common = fx::imin(x0.hi - s0, fx::imin(x1.hi - s1, x2.hi - s2));
+    uc = 61 - (s0 + s1 + s2 - sg + common);
     if (ok)
 #pragma unroll
       for (int q = KA_DV; q < KA_LA; ++q) num(own + q) = fx::limbs(to_fixed0(sh(own + q), sg + common - 1075));
+  }
+  // component k of sums of (slot i) x (slot j)
+  struct Cross { fx::Acc p, n; };
+  auto first = [&](int i, int j) {
+    Cross r;
+    r.p = fx::mul(num(c1 + i), num(c2 + j));
+    r.n = fx::mul(num(c2 + i), num(c1 + j));
+    return r;
+  };
+  auto plus = [&](Cross& r, int i, int j) {
+    fx::mac(r.p, num(c1 + i), num(c2 + j));
+    fx::mac(r.n, num(c2 + i), num(c1 + j));
+  };
+  auto value = [&](const Cross& r) {
+    fx::Acc d;
+    d.h = r.p.h - r.n.h;
+    d.m = r.p.m - r.n.m;
+    return fx::take<3>(d);
+  };
+  // the same in doubles, the positions' slots from the tape
+  const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+  auto at = [&](int j, int i) {
+    if (i >= KA_DV) return sh(KA_COMP * j + i);
+    auto t = [&](int q) { return a.kin[q * E + e]; };
+    if (i < KA_F) return t(3 * j + i - KA_W);
+    if (i < KA_D) return fma(-0.5 * dt, t(9 + 3 * j + i - KA_F), t(3 * j + i - KA_F));
+    auto d = [&](int q) { return t(45 + 3 * q + j); };
+    return i < KA_U ? d(i - KA_D) : d(6 + 2 * (i - KA_U)) + d(7 + 2 * (i - KA_U));
+  };
+  auto add_cross = [&](double y, int i, int j) { return fma(at(k1, i), at(k2, j), fma(-at(k2, i), at(k1, j), y)); };
+  // ---- positions' and velocities' edges: direction d uses A = P x Q, P and Q the
+  //      edges after it; C0 = F1 x F2, C1 = F2 x F0, C2 = F0 x F1 ----
+  double LW[3], LF[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int b = (i + 1) % 3, c = (i + 2) % 3;  // P of c, Q of b
+    if (ok_edges) {
+      Cross r = first(KA_W + b, KA_LA + c);
+      plus(r, KA_LA + b, KA_W + c);
+      LW[i] = fx::to_double(value(r), uA);
+      r = first(KA_F + b, KA_LC + c);
+      plus(r, KA_LC + b, KA_F + c);
+      LF[i] = fx::to_double(value(r), uC);
+    } else {
+      LW[i] = add_cross(add_cross(0.0, KA_W + b, KA_LA + c), KA_LA + b, KA_W + c);
+      LF[i] = add_cross(add_cross(0.0, KA_F + b, KA_LC + c), KA_LC + b, KA_F + c);
+    }
+  }
+  LF[1] = fma(Ldet, C[1], LF[1]);
+  {
+    double Ldt = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      LW[d] += LF[d];
+      LVW[d] = fma(-0.5 * dt, LF[d], LVW[d]);
+      Ldt = fma(LF[d], VW[d], Ldt);
+    }
+    sh(KA_DIR + k) = live ? -0.5 * Ldt : 0.0;
   }
   // the velocity corners (the Walsh transpose), plus the hourglass velocity
   // corners of the cycle after this one
@@ -661,23 +739,6 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   __syncthreads();
   bool summed = false;
   if (ok) {
-    struct Cross { fx::Acc p, n; };
-    auto first = [&](int i, int j) {
-      Cross r;
-      r.p = fx::mul(num(c1 + i), num(c2 + j));
-      r.n = fx::mul(num(c2 + i), num(c1 + j));
-      return r;
-    };
-    auto plus = [&](Cross& r, int i, int j) {
-      fx::mac(r.p, num(c1 + i), num(c2 + j));
-      fx::mac(r.n, num(c2 + i), num(c1 + j));
-    };
-    auto value = [&](const Cross& r) {
-      fx::Acc d;
-      d.h = r.p.h - r.n.h;
-      d.m = r.p.m - r.n.m;
-      return fx::take<3>(d);
-    };
     fx::i64 X[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // below 3 2^60
     auto onto = [&](int q, fx::i64 y) { X[pp[q]] += y; X[pq[q]] -= y; };
 #pragma unroll
@@ -724,24 +785,17 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
       for (int c = 0; c < 8; ++c) LX[c] = fx::to_double(X[c], uc);
     }
   } else {
-    const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
-    auto at = [&](int j, int i) {
-      if (i >= KA_DV) return sh(KA_COMP * j + i);
-      auto d = [&](int q) { return a.kin[(45 + 3 * q + j) * E + e]; };
-      return i < KA_U ? d(i - KA_D) : d(6 + 2 * (i - KA_U)) + d(7 + 2 * (i - KA_U));
-    };
-    auto plus = [&](double y, int i, int j) { return fma(at(k1, i), at(k2, j), fma(-at(k2, i), at(k1, j), y)); };
 #pragma unroll
     for (int c = 0; c < 8; ++c) LX[c] = 0.0;
     auto onto = [&](int q, double y) { LX[pp[q]] += y; LX[pq[q]] -= y; };
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
       const int v = iv[t], w = iw[t];
-      const double gU = plus(plus(0.0, KA_DV + t, KA_D + w), KA_D + v, KA_DW + t);
+      const double gU = add_cross(add_cross(0.0, KA_DV + t, KA_D + w), KA_D + v, KA_DW + t);
 #pragma unroll
-      for (int q = 6 + 2 * t; q < 8 + 2 * t; ++q) onto(q, plus(gU, KA_LN + partner[q], KA_D + partner[q]));
-      onto(v, plus(plus(plus(0.0, KA_D + w, KA_A + t), KA_DW + t, KA_U + t), KA_D + partner[v], KA_LN + v));
-      onto(w, plus(plus(plus(0.0, KA_A + t, KA_D + v), KA_U + t, KA_DV + t), KA_D + partner[w], KA_LN + w));
+      for (int q = 6 + 2 * t; q < 8 + 2 * t; ++q) onto(q, add_cross(gU, KA_LN + partner[q], KA_D + partner[q]));
+      onto(v, add_cross(add_cross(add_cross(0.0, KA_D + w, KA_A + t), KA_DW + t, KA_U + t), KA_D + partner[v], KA_LN + v));
+      onto(w, add_cross(add_cross(add_cross(0.0, KA_A + t, KA_D + v), KA_U + t, KA_DV + t), KA_D + partner[w], KA_LN + w));
     }
   }
   if (!summed) {
@@ -941,10 +995,11 @@ __device__ __noinline__ void cycle_close(const AdjDev& a, int ge, int gn, const 
 // different size takes the largest term's unit, the others' mantissas shifted. Values
 // outside 2^-400..2^400, infinities and NaN take the same sums in doubles, from
 // the tape.
-// What bounds it: integer and FP64 issue together. At 48^3 155 us with every
-// sum on the FP64 pipe (81 % busy), 116 us so (77 %); a gradient of 40 cycles at 48^3 went from 22.9 to 21.7 ms by this form, of 24 cycles at
-// 15^3 from 2.97 to 2.93 ms. Five blocks per SM (128 registers, no spills)
-// against six and seven: 21.63, 21.71, 21.78 ms.
+// Bound by FP64 issue (451 slots per element, the pipe 76 % busy; ALU 18 %,
+// multiply-adds 10 %). At 48^3 155 us with every sum on the FP64 pipe (81 %
+// busy), 113 us so; a gradient of 40 cycles at 48^3 went from 22.9 to 21.7 ms by
+// this form, of 24 cycles at 15^3 from 2.97 to 2.93 ms. Five blocks per SM (128
+// registers, no spills) against six and seven: 21.63, 21.71, 21.78 ms.
 //
 // The last block closes the cycle's time beside the elements (nothing here reads
 // it). As a launch of one block it took 10 us of the chain at 48^3; a gradient of
