@@ -15,8 +15,8 @@
 // The forward sweep runs as lulesh_run does (CUDA graphs, dt on the device);
 // the recompute and the transpose of a segment are queued without any host
 // synchronisation. With two tape sets (when they fit), segment k-1 is
-// recomputed on a second stream while segment k is transposed: the FP64-bound
-// forward kernels fill the SMs the latency-bound transposes leave idle.
+// recomputed on a second stream while segment k is transposed: the forward
+// kernels fill what the transposes leave idle.
 // The handle is left at its final state. Every derivative is that of the
 // branches the forward run took.
 #include <cuda_runtime.h>
