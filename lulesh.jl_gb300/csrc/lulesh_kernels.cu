@@ -642,8 +642,9 @@ __device__ __forceinline__ float coarse(double x) {
 // through it must be recomputed from it.
 __device__ __forceinline__ void opaque(double& x) { asm volatile("" : "+d"(x)); }
 
-// Bound by FP64 issue: 0.48 ms per cycle at 150^3 in mid-blast (0.71 ms with the
-// limiter and the time constraints formed for every element).
+// Bound by FP64 issue (pipe 82 % busy): 0.48 ms per cycle at 150^3 in mid-blast
+// (0.71 ms with the limiter and the time constraints formed for every element);
+// over a run's first 200 cycles 0.36 ms, 0.75 before.
 //
 // REGION: threads take elements in region order (d.regOrder) so that a warp
 // runs one region's rep count; each element's EOS is evaluated that many times.
