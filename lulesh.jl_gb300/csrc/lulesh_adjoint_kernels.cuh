@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kAdjBlock, 4) ka_material(AdjDev a, Params prm
   ip[2] = limiter_index(mask, ZETA_P, ZETA_P_SYMM, ZETA_P_FREE, ZETA_P_COMM, a.lzetap[i], i, E);
 
   // forward values from the material kernel's tape (slots: see tapeMat)
-  auto tm = [&](int q) { return a.mat[q * E + i]; };
+  auto tm = [&](int q) { return a.mat[row(q, E, i)]; };
   double self[3], norm[3], tdm[3], tdp[3], phi[3], delx[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -314,8 +314,8 @@ __global__ void __launch_bounds__(kAdjBlock, 4) ka_material(AdjDev a, Params prm
     const int src = (int)((fl >> (3 * d)) & 7ull);
     double Ldm = 0.0, Ldp = 0.0;
     if (qzero) {  // the limiter was not used
-      a.lnb[(2 * d) * E + i] = 0.0;
-      a.lnb[(2 * d + 1) * E + i] = 0.0;
+      a.lnb[row(2 * d, E, i)] = 0.0;
+      a.lnb[row(2 * d + 1, E, i)] = 0.0;
       a.ldv[d][i] = 0.0;
       a.ldx[d][i] = 0.0;
       continue;
@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(kAdjBlock, 4) ka_material(AdjDev a, Params prm
     double sm = 0.0, sp = 0.0;
     if (im[d] == i) Lself[d] += Lm; else if (im[d] >= 0) sm = Lm;
     if (ip[d] == i) Lself[d] += Lp; else if (ip[d] >= 0) sp = Lp;
-    a.lnb[(2 * d) * E + i] = sm;
-    a.lnb[(2 * d + 1) * E + i] = sp;
+    a.lnb[row(2 * d, E, i)] = sm;
+    a.lnb[row(2 * d + 1, E, i)] = sp;
     a.ldv[d][i] = Lself[d];
     a.ldx[d][i] = Ldx[d];
   }
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   auto num = [&](int i) -> fx::Num& { return reinterpret_cast<fx::Num*>(column)[i * kFixedElems + lane]; };
   const int own = KA_COMP * k, c1 = KA_COMP * (k == 2 ? 0 : k + 1), c2 = KA_COMP * (k == 0 ? 2 : k - 1);
   // forward values from the kinematics kernel's tape (slots: see tapeKin)
-  auto tk = [&](int q) { return a.kin[q * E + e]; };
+  auto tk = [&](int q) { return a.kin[row(q, E, e)]; };
 
   const double vnew = a.vnew[e], volo = a.volo[e], inv_volo = a.inv_volo[e];
   const double vol = volo * vnew, norm64 = tk(40);  // norm64 = 1/(64 vol + 64 ptiny)
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       const int src = (MODE & 2) ? c : c == 1 ? 3 : c == 3 ? 1 : c;
-      G[c] = a.sLdv[(k * 8 + src) * E + e];
+      G[c] = a.sLdv[row(k * 8 + src, E, e)];
     }
     dU[0] = (G[3] - G[1]) + (G[7] - G[2]);
     dU[1] = (G[4] - G[3]) + (G[5] - G[7]);
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     const double s8 = ((-a.p1[e]) - a.q1[e]) * 0.125;
     constexpr int at[5] = {3, 4, 0, 2, 1};
 #pragma unroll
-    for (int f = 0; f < 5; ++f) put(KA_LN + at[f], s8 * a.sLU[(3 * f + k) * E + e]);
+    for (int f = 0; f < 5; ++f) put(KA_LN + at[f], s8 * a.sLU[row(3 * f + k, E, e)]);
     sh(own + KA_LN + 5) = 0.0;  // the face (d64, d57), of the characteristic length alone
   }
   __syncthreads();
@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
   auto at = [&](int j, int i) {
     if (i >= KA_DV) return sh(KA_COMP * j + i);
-    auto t = [&](int q) { return a.kin[q * E + e]; };
+    auto t = [&](int q) { return a.kin[row(q, E, e)]; };
     if (i < KA_F) return t(3 * j + i - KA_W);
     if (i < KA_D) return fma(-0.5 * dt, t(9 + 3 * j + i - KA_F), t(3 * j + i - KA_F));
     auto d = [&](int q) { return t(45 + 3 * q + j); };
@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     int top = fx::kNoExponent;
 #pragma unroll
     for (int q = 0; q < 11; ++q) {
-      f[q] = fx::to_float(q < 3 ? LVW[q] : a.fV[(k * 8 + q - 3) * E + e]);
+      f[q] = fx::to_float(q < 3 ? LVW[q] : a.fV[row(k * 8 + q - 3, E, e)]);
       top = fx::imax(top, f[q].k);
     }
     const int u = top + 2;
@@ -711,15 +711,15 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
       walsh1_t(w, y);
       if (live)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) a.cV[(k * 8 + c) * E + e] = fx::to_double(y[c], u);
+        for (int c = 0; c < 8; ++c) a.cV[row(k * 8 + c, E, e)] = fx::to_double(y[c], u);
     } else {
       double y[8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) y[c] = a.fV[(k * 8 + c) * E + e];
+      for (int c = 0; c < 8; ++c) y[c] = a.fV[row(k * 8 + c, E, e)];
       walsh1_t(LVW, y);
       if (live)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) a.cV[(k * 8 + c) * E + e] = y[c];
+        for (int c = 0; c < 8; ++c) a.cV[row(k * 8 + c, E, e)] = y[c];
     }
   }
   // ---- volume and characteristic length, and the position transpose of the
@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   for (int t = 0; t < 3; ++t) vw[t] = Lv12 * tk(81 + 3 * t + k);
   // the next cycle's hourglass modes
 #pragma unroll
-  for (int m = 0; m < 4; ++m) tm[m] = a.sLhm[(k * 4 + m) * E + e];
+  for (int m = 0; m < 4; ++m) tm[m] = a.sLhm[row(k * 4 + m, E, e)];
   __syncthreads();
   bool summed = false;
   if (ok) {
@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
   }
   if (live)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) a.cX[(k * 8 + c) * E + e] = LX[c];
+    for (int c = 0; c < 8; ++c) a.cX[row(k * 8 + c, E, e)] = LX[c];
   if (k == 2) {
     double Ldt = (sh(KA_DIR) + sh(KA_DIR + 1)) + sh(KA_DIR + 2);
 #pragma unroll
@@ -1063,9 +1063,9 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
   if (!(hgcoef > 0.0)) {
     if (live) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) { a.fV[(k * 8 + c) * E + e] = 0.0; a.sLdv[(k * 8 + c) * E + e] = 0.0; }
+      for (int c = 0; c < 8; ++c) { a.fV[row(k * 8 + c, E, e)] = 0.0; a.sLdv[row(k * 8 + c, E, e)] = 0.0; }
 #pragma unroll
-      for (int m = 0; m < 4; ++m) a.sLhm[(k * 4 + m) * E + e] = 0.0;
+      for (int m = 0; m < 4; ++m) a.sLhm[row(k * 4 + m, E, e)] = 0.0;
     }
   } else {
     double inv_det = 0.0, vi12 = 0.0, ss = 0.0, mass = 0.0, r = 0.0;  // thread 0
@@ -1073,11 +1073,11 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
     {
       // the forward kernel's volume derivatives, scaled modes and mode sums
 #pragma unroll
-      for (int c = 0; c < 8; ++c) dv[c] = a.geo[(k * 8 + c) * E + e];
+      for (int c = 0; c < 8; ++c) dv[c] = a.geo[row(k * 8 + c, E, e)];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        sh(HA_HMS + 4 * k + m) = a.geo[(24 + 4 * k + m) * E + e];
-        S[m] = a.geo[(36 + 4 * k + m) * E + e];
+        sh(HA_HMS + 4 * k + m) = a.geo[row(24 + 4 * k + m, E, e)];
+        S[m] = a.geo[row(36 + 4 * k + m, E, e)];
       }
       unsigned top = 0;
 #pragma unroll
@@ -1145,7 +1145,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
         D[j] = C[j] = 0.0;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          const double g = a.geo[(j * 8 + c) * E + e];
+          const double g = a.geo[row(j * 8 + c, E, e)];
           D[j] = fma(g, v[c], D[j]);
           C[j] = fma(g, lf[c], C[j]);
         }
@@ -1212,7 +1212,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
           fx::Acc x = fx::mul(num(HA_DV + c), B[0]);
           fx::mac(x, num(HA_DV + 8 + c), B[1]);
           fx::mac(x, num(HA_DV + 16 + c), B[2]);
-          if (live) a.fV[(k * 8 + c) * E + e] = fx::to_double(fx::take<2>(x) + q[c], u);
+          if (live) a.fV[row(k * 8 + c, E, e)] = fx::to_double(fx::take<2>(x) + q[c], u);
         }
       } else {
         double q[8];
@@ -1221,8 +1221,8 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
         for (int c = 0; c < 8; ++c) {
           double f = q[c];
 #pragma unroll
-          for (int j = 0; j < 3; ++j) f = fma(a.geo[(j * 8 + c) * E + e], nB[j], f);
-          if (live) a.fV[(k * 8 + c) * E + e] = f;
+          for (int j = 0; j < 3; ++j) f = fma(a.geo[row(j * 8 + c, E, e)], nB[j], f);
+          if (live) a.fV[row(k * 8 + c, E, e)] = f;
         }
       }
     }
@@ -1235,7 +1235,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
     for (int m = 0; m < 4; ++m) {
       const double P = (sh(HA_P + 4 * k + m) + sh(HA_P + 12 + 4 * k + m)) + sh(HA_P + 24 + 4 * k + m);
       Pvi = fma(P, sh(HA_HMS + 4 * k + m), Pvi);
-      if (live) a.sLhm[(k * 4 + m) * E + e] = sh(HA_COEF + 1) * P;
+      if (live) a.sLhm[row(k * 4 + m, E, e)] = sh(HA_COEF + 1) * P;
     }
     sh(HA_SUM + 3 + k) = Pvi;
     // dL/ddv_j = -coef sum_k (lf_k A[k][j] + V_k B[k][j]) = sum_k (lf_k nA[k][j] + V_k nB[k][j])
@@ -1258,7 +1258,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
           A[q] = fx::limbs(in_unit(fA[q], fA[q].k, u));
           B[q] = fx::limbs(in_unit(fB[q], fB[q].k, u));
         }
-        if (live) a.sLdv[(k * 8) * E + e] = 0.0;
+        if (live) a.sLdv[row(k * 8, E, e)] = 0.0;
 #pragma unroll
         for (int c = 1; c < 8; ++c) {
           fx::Acc x = fx::mul(num(HA_L + c), A[0]);
@@ -1268,7 +1268,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
             fx::mac(x, num(HA_L + 8 * q + c), A[q]);
             fx::mac(x, num(HA_V + 8 * q + c), B[q]);
           }
-          if (live) a.sLdv[(k * 8 + c) * E + e] = fx::to_double(fx::take<3>(x), u);
+          if (live) a.sLdv[row(k * 8 + c, E, e)] = fx::to_double(fx::take<3>(x), u);
         }
       } else {
 #pragma unroll
@@ -1280,7 +1280,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
 #pragma unroll
           for (int q = 0; q < 3; ++q)
             t = fma(l3[q], sh(HA_NA + 3 * q + k), fma(v3_[q], sh(HA_NB + 3 * q + k), t));
-          if (live) a.sLdv[(k * 8 + c) * E + e] = t;
+          if (live) a.sLdv[row(k * 8 + c, E, e)] = t;
         }
       }
     }
@@ -1316,8 +1316,8 @@ __global__ void __launch_bounds__(3 * kFixedElems, 5)
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
       // face normals 0..4 (the forward's cross products, from the tape)
-      part = fma(a.geo[(48 + 6 * k + f) * E + e], LU[f], part);
-      if (live) a.sLU[(3 * f + k) * E + e] = LU[f];
+      part = fma(a.geo[row(48 + 6 * k + f, E, e)], LU[f], part);
+      if (live) a.sLU[row(3 * f + k, E, e)] = LU[f];
     }
     sh(HA_SUM + 6 + k) = part;
     __syncthreads();
@@ -1356,7 +1356,7 @@ __device__ __forceinline__ void force_geo_t(const AdjDev& a, int e, const V3 dgs
   for (int k = 0; k < 3; ++k) {
     double t[4], q[8];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) t[m] = a.sLhm[(k * 4 + m) * E + e];
+    for (int m = 0; m < 4; ++m) t[m] = a.sLhm[row(k * 4 + m, E, e)];
     walsh_modes_t(t, q);
 #pragma unroll
     for (int c = 0; c < 8; ++c) LX[k][c] = q[c];
@@ -1369,7 +1369,7 @@ __device__ __forceinline__ void force_geo_t(const AdjDev& a, int e, const V3 dgs
 #pragma unroll
     for (int j = 0; j < 3; ++j)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) G[j][c] = a.sLdv[(j * 8 + c) * E + e];
+      for (int c = 0; c < 8; ++c) G[j][c] = a.sLdv[row(j * 8 + c, E, e)];
     if (!(MODE & 2)) {
       // the faithful forward stores node 3's derivative in slot 1 and node 1's in slot 3
 #pragma unroll
@@ -1409,7 +1409,7 @@ __device__ __forceinline__ void force_geo_t(const AdjDev& a, int e, const V3 dgs
   {
     V3 LU[5];
 #pragma unroll
-    for (int f = 0; f < 5; ++f) LU[f] = v3(a.sLU[(f * 3) * E + e], a.sLU[(f * 3 + 1) * E + e], a.sLU[(f * 3 + 2) * E + e]);
+    for (int f = 0; f < 5; ++f) LU[f] = v3(a.sLU[row(f * 3, E, e)], a.sLU[row(f * 3 + 1, E, e)], a.sLU[row(f * 3 + 2, E, e)]);
     auto face_t = [&](int f, const V3& d1, const V3& d2, int p0, int p1, int p2, int p3) {
       const V3 LN = v3(s8 * LU[f].x, s8 * LU[f].y, s8 * LU[f].z);
       const V3 L1 = vcross(d2, LN), L2 = vcross(LN, d1);
@@ -1434,14 +1434,14 @@ __global__ void __launch_bounds__(kAdjBlock, 3) ka_force_geo(AdjDev a) {
   if (e >= E) return;
   V3 dgs[12];
 #pragma unroll
-  for (int q = 0; q < 12; ++q) dgs[q] = v3(a.diag0[(3 * q) * E + e], a.diag0[(3 * q + 1) * E + e], a.diag0[(3 * q + 2) * E + e]);
+  for (int q = 0; q < 12; ++q) dgs[q] = v3(a.diag0[row(3 * q, E, e)], a.diag0[row(3 * q + 1, E, e)], a.diag0[row(3 * q + 2, E, e)]);
   const double s8 = ((-a.p0[e]) - a.q0[e]) * 0.125;
   double LX[3][8];
   force_geo_t<MODE>(a, e, dgs, s8, LX);
 #pragma unroll
   for (int k = 0; k < 3; ++k)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) a.fX[(k * 8 + c) * E + e] = LX[k][c];
+    for (int c = 0; c < 8; ++c) a.fX[row(k * 8 + c, E, e)] = LX[k][c];
 }
 
 // Sum of `n` partials in a fixed order by one block of BS threads; every

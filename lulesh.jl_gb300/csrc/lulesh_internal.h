@@ -1,6 +1,7 @@
 // Internal structures of the GB300 LagrangeLeapFrog library.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <cuda_runtime.h>
@@ -126,6 +127,14 @@ constexpr unsigned long long kInfBits = 0x7FF0000000000000ull;
 // (and NaNs, whose patterns lie above +inf) the unsigned order is the FP order.
 constexpr unsigned long long kDtRegisterBits = 0x4415AF1D78B58C40ull;
 __host__ __device__ inline bool dt_registers(unsigned long long acc) { return acc < kDtRegisterBits; }
+
+// Entry of element e in row `slot` of a [slots][E] array. The tapes have up to 90
+// rows and the adjoint's corner buffers 24: past 2^31 entries from 288^3 and 448^3
+// elements on. (The arrays of 8 rows stay below it: nx <= 640.)
+// Unsigned 32-bit factors: one wide multiply-add.
+__host__ __device__ inline size_t row(int slot, int E, int e) {
+  return (size_t)(unsigned)slot * (unsigned)E + (unsigned)e;
+}
 
 // Pointers of one problem's device fields. Element arrays have E entries,
 // node arrays N; corner arrays 8E in corner-major order (c*E + e).

@@ -66,7 +66,7 @@ struct ForceTape {
   double* p;  // d.tapeGeo at this element
   int E;
   bool live;
-  __device__ void put(int slot, double v) const { if (live) p[slot * E] = v; }
+  __device__ void put(int slot, double v) const { if (live) p[row(slot, E, 0)] = v; }
   __device__ void derivative(int k, int n, double v) const { put(8 * k + n, v); }
   __device__ void mode(int k, int m, double v) const { put(24 + 4 * k + m, v); }
   __device__ void sum(int k, int m, double v) const { put(36 + 4 * k + m, v); }
@@ -261,7 +261,7 @@ __device__ __forceinline__ int kin_quotients(const DevDomain& d, DevState* st, c
   const double vnew = volume * LDG(&d.inv_volo[e]);
   const double volq = LDG(&d.volo[e]) * vnew;
   double rcl = 0.0;
-  auto tape = [&](int slot, double v) { d.tapeKin[slot * E + e] = v; };
+  auto tape = [&](int slot, double v) { d.tapeKin[row(slot, E, e)] = v; };
   if (mine) {
     if (k == 1) {
       const double q64 = fma(64.0, volq, 64.0 * 1.e-36);
@@ -324,7 +324,7 @@ __device__ __forceinline__ int kin_quotients(const DevDomain& d, DevState* st, c
 template <class Taped>
 __device__ __forceinline__ void kin_tape(const DevDomain& d, int k, int e, int place, const Taped& t) {
   const int E = d.E;
-  auto put = [&](int slot, double v) { d.tapeKin[slot * E + e] = v; };
+  auto put = [&](int slot, double v) { d.tapeKin[row(slot, E, e)] = v; };
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     put(3 * k + a, t.w(a));
@@ -345,7 +345,7 @@ __device__ __forceinline__ void kin_tape(const DevDomain& d, int k, int e, int p
 template <class Taped>
 __device__ __forceinline__ void kin_tape_next(const DevDomain& d, int k, int e, const Taped& t) {
 #pragma unroll
-  for (int f = 0; f < 5; ++f) d.tapeGeoNext[(48 + 6 * k + f) * d.E + e] = t.n(f);
+  for (int f = 0; f < 5; ++f) d.tapeGeoNext[row(48 + 6 * k + f, d.E, e)] = t.n(f);
 }
 
 struct FixedSums {
@@ -519,10 +519,10 @@ __global__ void __launch_bounds__(3 * kFixedElems) k_tape_geometry(const __grid_
   if (!live) return;
   if (d.tapeGeoNext)
 #pragma unroll
-    for (int f = 0; f < 5; ++f) d.tapeGeoNext[(48 + 6 * k + f) * E + e] = n[f];
+    for (int f = 0; f < 5; ++f) d.tapeGeoNext[row(48 + 6 * k + f, E, e)] = n[f];
   if (d.tapeDiag)
 #pragma unroll
-    for (int q = 0; q < 12; ++q) d.tapeDiag[(3 * q + k) * E + e] = g[q];
+    for (int q = 0; q < 12; ++q) d.tapeDiag[row(3 * q + k, E, e)] = g[q];
 }
 
 // ---------------------------------------------------------------------------
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     int src0 = PHI_MEAN, src1 = PHI_MEAN, src2 = PHI_MEAN;
     if (bad) err |= ST_BAD_BC;
     // d.tapeMat slot q of this element (TAPE only)
-    auto tm = [&](int q, double v) { if (TAPE) d.tapeMat[q * E + i] = v; };
+    auto tm = [&](int q, double v) { if (TAPE) d.tapeMat[row(q, E, i)] = v; };
     double phixi = 0.0, phieta = 0.0, phizeta = 0.0;
     if (TAPE || !(expanding || still)) {
       auto at = [](const double* dv, int j) { return j < 0 ? 0.0 : dv[j]; };
