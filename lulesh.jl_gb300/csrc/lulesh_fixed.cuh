@@ -162,6 +162,13 @@ LULESH_FX Acc mul_minus(Num a, Num b, Num c, Num d) {
   r.m -= mad(c.lo, d.hi, mulw(c.hi, d.lo));
   return r;
 }
+// the same with lo*lo too
+LULESH_FX Acc mul_minus_full(Num a, Num b, Num c, Num d) {
+  Acc r = mul_minus(a, b, c, d);
+  r.m = mad((int)(mulw(a.lo, b.lo) >> 32), one(), r.m);
+  r.m -= mulw(c.lo, d.lo) >> 32;
+  return r;
+}
 // the accumulated sum over 2^(64 - B), rounded down (a rounding addend would
 // cost two moves; what it would save, half a unit, is below the dropped lo*lo)
 template <int B>
@@ -169,6 +176,18 @@ LULESH_FX i64 take(Acc a) {
   return B == 0 ? mad((int)(a.m >> 32), one(), a.h) : shl(a.h, B) + (a.m >> (32 - B));
 }
 LULESH_FX i64 product(Num a, Num b) { return take<0>(mul(a, b)); }
+// How far |x| < 2^61 can be shifted left and stay below 2^61, at most 29 (from
+// the high word alone).
+LULESH_FX int room(i64 x) {
+  const int h = (int)(x >> 32);
+  return imax(leading_zeros((unsigned)(h ^ (h >> 31))) - 3, 0);
+}
+// The accumulated sum over 2^(64 - B), B as large as it stays below 2^61 with:
+// a component far below the others of its vector keeps its bits.
+LULESH_FX i64 take_all(Acc a, int& B) {
+  B = room(take<0>(a));
+  return shl(a.h, B) + (a.m >> (32 - B));
+}
 // --- conversions ------------------------------------------------------------
 // Exponent field of a bound on the extent of eight doubles, from their high
 // words: max - min with the low words rounded outwards. NaN and infinities

@@ -27,19 +27,23 @@ enum : int {
   SUM_VOLUME = 0,  // 12 volume over 2^62
   SUM_FACE = 1,    // 6: squared face vectors over 2^57, force order
   SUM_AREA = 7,    // 3: squared cross products of the mean edges over 2^57
-  SUM_FLOW = 10,   // 3: those cross products times velocity differences over 2^59
-  SUM_RATE = 13,   // cofactors times velocity differences over 2^61
+  SUM_FLOW = 10,   // 3: those cross products times velocity differences
+  SUM_RATE = 13,   // cofactors times velocity differences
   SUM_JAC = 14,    // half-step determinant over 2^59
-  kSums = 15
+  SUM_EXPO = 15,   // (16 bits each) exponents of the three flows and the rate
+  kSums = 16
 };
+// exponent of a term that is exactly zero
+constexpr int kNoTerm = -16384;
 static_assert(3 * kSums <= 54, "the sums overlay the diagonals");
 
 // What a thread keeps over the phases: its components (unscaled integers) of
-// the face vectors, the volume's V x W, the edges' cross products, the
-// cofactors, and its velocity differences and edges.
+// the face vectors, the volume's V x W, the edges' cross products (over
+// 2^(64 - up)), the cofactors (over 2^62), and its velocity differences and edges.
 struct KinLane {
   double x[8], v[8];
-  int s, sv;
+  int s, sv;  // scales of the positions and of this coordinate's velocities
+  int up[3];
   bool ok_x, ok;  // positions taken; positions and velocities taken
   i64 g[12], w[3], vw[3];
   i64 n[6], gU[3], A[3], C[3];
@@ -63,22 +67,25 @@ LULESH_FX void kin_extents(int k, Slots sh, const KinLane& r) {
 }
 
 // 2: diagonals, mean edges, velocity differences and half-step edges (edge -
-// dt/2 velocity difference, half_dt = dt/2).
+// dt/2 velocity difference, half_dt = dt/2). Each coordinate's velocities have
+// their own scale: in flow along one axis the others' differences, which alone
+// make up the monotonic-Q gradients across it, are as small as they please.
 LULESH_FX void kin_edges(int k, Slots sh, double half_dt, KinLane& r) {
   const Num m0 = sh[KS_EXT], m1 = sh[KS_EXT + 1], m2 = sh[KS_EXT + 2];
   const int ex = exponent_field(umax(umax((unsigned)m0.lo, (unsigned)m1.lo), (unsigned)m2.lo));
-  int ev = exponent_field(umax(umax((unsigned)m0.hi, (unsigned)m1.hi), (unsigned)m2.hi));
+  const int fastest = exponent_field(umax(umax((unsigned)m0.hi, (unsigned)m1.hi), (unsigned)m2.hi));
   r.ok_x = ex >= kMinExtent && ex <= kMaxExtent;
   const Float T = to_float(half_dt);
-  const bool wild = ev > kMaxSpeed;  // not finite, or far beyond any flow
-  ev = wild ? 0x7ff : imax(ev, kMinSpeed);
+  const bool wild = fastest > kMaxSpeed;  // not finite, or far beyond any flow
+  const int ev = wild ? 0x7ff : imax(exponent_field((unsigned)(k == 0 ? m0 : k == 1 ? m1 : m2).hi), kMinSpeed);
   const int exs = r.ok_x ? ex : 0x7ff;
   r.s = 1083 - exs;
   r.sv = 1083 - ev;
   // dt/2 in units of the edges over those of the velocities, T.m 2^tx: taken
   // while corners move less than an eighth of the scale's 2^61
   const int tx = T.k + r.s - r.sv;
-  r.ok = r.ok_x && !wild && tx <= -64 && exponent_field((unsigned)hi_word(half_dt)) != 0x7ff;
+  r.ok = r.ok_x && !wild && T.k + r.s - 1083 + imax(fastest, kMinSpeed) <= -64 &&
+         exponent_field((unsigned)hi_word(half_dt)) != 0x7ff;
   const Num tau = limbs(T.m >> (r.ok ? imin(-64 - tx, 63) : 63));
   i64 c[8];
   LULESH_UNROLL
@@ -114,13 +121,13 @@ LULESH_FX void kin_products(int k, Slots sh, KinLane& r) {
   r.gU[1] = cross_k(9, 10);
   r.gU[2] = cross_k(4, 2);
   // eta x zeta, zeta x xi, xi x eta of the mean edges and of the half-step edges
-  r.A[0] = cross_k(13, 14);
-  r.A[1] = cross_k(14, 12);
-  r.A[2] = cross_k(12, 13);
-  r.C[0] = cross_k(16, 17);
-  r.C[1] = cross_k(17, 15);
-  r.C[2] = cross_k(15, 16);
-  sh.put(KS_DET + k, product(limbs(r.w[1]), limbs(r.A[1])));
+  LULESH_UNROLL
+  for (int d = 0; d < 3; ++d) {
+    const int a = 12 + (d + 1) % 3, b = 12 + (d + 2) % 3;
+    r.A[d] = take_all(mul_minus_full(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]), r.up[d]);
+    r.C[d] = take<2>(mul_minus(sh[i1 + a + 3], sh[i2 + b + 3], sh[i2 + a + 3], sh[i1 + b + 3]));
+  }
+  sh.put(KS_DET + k, product(limbs(r.w[1]), limbs(r.A[1] >> r.up[1])));
 }
 
 // 4: coordinate k's terms of the sums.
@@ -135,24 +142,51 @@ LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
   }
   LULESH_UNROLL
   for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square(limbs(r.n[f])));
+  // The terms of a sum with velocities differ in scale by coordinate: each is
+  // brought to 2^60 and carries its exponent, and the sum takes the largest's.
+  int e[4];
+  auto put_term = [&](int i, i64 t, int shift, int& expo) {
+    const int c = room(t);
+    sh.put(at + i, shl(t, c));
+    expo = t != 0 ? -(r.sv + shift + c) : kNoTerm;
+  };
   Acc rate = {0, 0};
   LULESH_UNROLL
   for (int d = 0; d < 3; ++d) {
-    const Num a = limbs(r.A[d]), u = limbs(r.vw[d]), c = limbs(r.C[d]);
-    sh.put(at + SUM_AREA + d, square(a));
+    const Num u = limbs(r.vw[d]), c = limbs(r.C[d]);
+    sh.put(at + SUM_AREA + d, square(limbs(r.A[d] >> r.up[d])));
     Acc flow = {0, 0};
-    mac_full(flow, a, u);
-    sh.put(at + SUM_FLOW + d, take<5>(flow));
+    mac_full(flow, limbs(r.A[d]), u);
+    put_term(SUM_FLOW + d, take<3>(flow), r.up[d], e[d]);
     mac_full(rate, c, u);
   }
-  sh.put(at + SUM_RATE, take<3>(rate));
+  put_term(SUM_RATE, take<1>(rate), 0, e[3]);
+  Num x;
+  x.lo = (e[0] & 0xffff) | (int)((unsigned)e[1] << 16);
+  x.hi = (e[2] & 0xffff) | (int)((unsigned)e[3] << 16);
+  sh[at + SUM_EXPO] = x;
   Acc jac = {0, 0};
   mac_full(jac, r.half_eta, limbs(r.C[1]));
-  sh.put(at + SUM_JAC, take<5>(jac));
+  sh.put(at + SUM_JAC, take<3>(jac));
 }
 
 LULESH_FX i64 kin_sum(Slots sh, int i) {
   return add(add(sh.get(KS_SUM + i), sh.get(KS_SUM + kSums + i)), sh.get(KS_SUM + 2 * kSums + i));
+}
+
+// the exponent of coordinate j's term of flow i, or of the rate (i = 3)
+LULESH_FX int kin_expo(Slots sh, int j, int i) {
+  const Num x = sh[KS_SUM + kSums * j + SUM_EXPO];
+  const int w = i < 2 ? x.lo : x.hi;
+  return i & 1 ? w >> 16 : (int)(short)w;
+}
+// the sum of those terms, times 2^k
+LULESH_FX double kin_aligned(Slots sh, int sum, int i, int k) {
+  const int e0 = kin_expo(sh, 0, i), e1 = kin_expo(sh, 1, i), e2 = kin_expo(sh, 2, i);
+  const int top = imax(e0, imax(e1, e2));
+  const i64 t = (sh.get(KS_SUM + sum) >> imin(top - e0, 63)) + (sh.get(KS_SUM + kSums + sum) >> imin(top - e1, 63)) +
+                (sh.get(KS_SUM + 2 * kSums + sum) >> imin(top - e2, 63));
+  return to_double(t, k + top);
 }
 
 LULESH_FX i64 kin_determinant(Slots sh) { return sh.get(KS_DET) + sh.get(KS_DET + 1) + sh.get(KS_DET + 2); }
@@ -184,10 +218,12 @@ LULESH_FX double kin_area(Slots sh, const KinLane& r, int d) {
   return to_double(kin_sum(sh, SUM_AREA + d), 193 - 4 * r.s);
 }
 LULESH_FX double kin_flow(Slots sh, const KinLane& r, int d) {
-  return to_double(kin_sum(sh, SUM_FLOW + d), 129 - 2 * r.s - r.sv);
+  return kin_aligned(sh, SUM_FLOW + d, d, 131 - 2 * r.s);
 }
-LULESH_FX double kin_rate(Slots sh, const KinLane& r) {
-  return to_double(kin_sum(sh, SUM_RATE), 131 - 2 * r.s - r.sv);
+LULESH_FX double kin_rate(Slots sh, const KinLane& r) { return kin_aligned(sh, SUM_RATE, 3, 131 - 2 * r.s); }
+// coordinate k's part of it
+LULESH_FX double kin_own_rate(Slots sh, const KinLane& r, int k) {
+  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 131 - 2 * r.s + kin_expo(sh, k, 3));
 }
 LULESH_FX double kin_jacobian(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_JAC), 129 - 3 * r.s); }
 

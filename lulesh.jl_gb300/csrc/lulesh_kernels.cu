@@ -358,16 +358,14 @@ struct FixedSums {
   __device__ double flow(int k) const { return fx::kin_flow(sh, r, k); }
   __device__ double rate() const { return fx::kin_rate(sh, r); }
   __device__ double jacobian() const { return fx::kin_jacobian(sh, r); }
-  __device__ double own_rate(int k) const {
-    return fx::to_double(sh.get(fx::KS_SUM + fx::kSums * k + fx::SUM_RATE), 131 - 2 * r.s - r.sv);
-  }
+  __device__ double own_rate(int k) const { return fx::kin_own_rate(sh, r, k); }
 };
 struct FixedTaped {
   const fx::KinLane& r;
   __device__ double w(int a) const { return fx::to_double(r.w[a], 2 - r.s); }
   __device__ double vw(int a) const { return fx::to_double(r.vw[a], 2 - r.sv); }
-  __device__ double C(int a) const { return fx::to_double(r.C[a], 68 - 2 * r.s); }
-  __device__ double A(int a) const { return fx::to_double(r.A[a], 68 - 2 * r.s); }
+  __device__ double C(int a) const { return fx::to_double(r.C[a], 66 - 2 * r.s); }
+  __device__ double A(int a) const { return fx::to_double(r.A[a], 68 - r.up[a] - 2 * r.s); }
   __device__ double gU(int a) const { return fx::to_double(r.gU[a], 64 - 2 * r.s); }
   __device__ double g(int q) const { return fx::to_double(r.g[q], -r.s); }
   __device__ double n(int f) const { return fx::to_double(r.n[f], 64 - 2 * r.s); }

@@ -1,0 +1,188 @@
+// Host harness of the kinematics' fixed-point sums (lulesh_fixed_kin.cuh) beside
+// the FP64 expressions the kernels had and still have for the elements the
+// fixed-point form does not take (kin_fp64 in lulesh_element_fp64.cuh), both
+// against 113-bit floating point.
+#include "../lulesh.jl_gb300/csrc/lulesh_fixed_kin.cuh"
+
+#include <cmath>
+#include <cstdlib>
+
+#if defined(__x86_64__)
+typedef __float128 Q;
+#else
+typedef long double Q;  // binary128 on aarch64
+#endif
+
+namespace {
+using namespace lulesh::fx;
+
+Q qabs(Q a) { return a < 0 ? -a : a; }
+
+// kin_fp64's sums: 12 volume, the largest squared face vector, areas, flows,
+// rate, determinant.
+void fp64_sums(const double p[3][8], const double v[3][8], double half_dt, double out[10]) {
+  static const int pa[12] = {2, 3, 5, 1, 6, 2, 7, 3, 4, 0, 6, 5}, pb[12] = {0, 1, 0, 4, 1, 5, 2, 6, 3, 7, 4, 7};
+  auto walsh = [](const double x[8], double w[3]) {
+    const double a = x[6] - x[0], b = x[5] - x[3], c = x[7] - x[1], d = x[4] - x[2];
+    const double apb = a + b, cpd = c + d;
+    w[0] = apb - cpd;
+    w[1] = (a - b) + (c - d);
+    w[2] = apb + cpd;
+  };
+  double g[3][12], w[3][3], u[3][3], h[3][3], t[3][15];
+  for (int k = 0; k < 3; ++k) {
+    for (int q = 0; q < 12; ++q) g[k][q] = p[k][pa[q]] - p[k][pb[q]];
+    walsh(p[k], w[k]);
+    walsh(v[k], u[k]);
+    for (int a = 0; a < 3; ++a) h[k][a] = std::fma(-half_dt, u[k][a], w[k][a]);
+  }
+  for (int k = 0; k < 3; ++k) {
+    const int i = (k + 1) % 3, j = (k + 2) % 3;
+    auto cr = [&](const double a1, const double b2, const double a2, const double b1) { return std::fma(a1, b2, -a2 * b1); };
+    auto gc = [&](int a, int b) { return cr(g[i][a], g[j][b], g[j][a], g[i][b]); };
+    t[k][0] = std::fma(g[k][1] + g[k][6], gc(0, 7),
+                       std::fma(g[k][8] + g[k][11], gc(9, 10), (g[k][3] + g[k][5]) * gc(4, 2)));
+    for (int f = 0; f < 6; ++f) t[k][1 + f] = gc(2 * f, 2 * f + 1) * gc(2 * f, 2 * f + 1);
+    double C[3];
+    for (int a = 0; a < 3; ++a) {
+      const int b = (a + 1) % 3, c = (a + 2) % 3;
+      const double A = cr(w[i][b], w[j][c], w[j][b], w[i][c]);
+      C[a] = cr(h[i][b], h[j][c], h[j][b], h[i][c]);
+      t[k][7 + a] = A * A;
+      t[k][10 + a] = A * u[k][a];
+    }
+    t[k][13] = std::fma(C[0], u[k][0], std::fma(C[1], u[k][1], C[2] * u[k][2]));
+    t[k][14] = h[k][1] * C[1];
+  }
+  auto sum = [&](int q) { return (t[0][q] + t[1][q]) + t[2][q]; };
+  out[0] = sum(0);
+  out[1] = 0;
+  for (int f = 0; f < 6; ++f) out[1] = std::fmax(out[1], sum(1 + f));
+  for (int j = 2; j < 10; ++j) out[j] = sum(5 + j);
+}
+
+// c = a x b, and p the sums of its products' magnitudes
+void cross(const Q a[3], const Q b[3], Q c[3], Q p[3]) {
+  for (int k = 0; k < 3; ++k) {
+    const Q s = a[(k + 1) % 3] * b[(k + 2) % 3], t = a[(k + 2) % 3] * b[(k + 1) % 3];
+    c[k] = s - t;
+    p[k] = qabs(s) + qabs(t);
+  }
+}
+}  // namespace
+
+extern "C" {
+
+// Sums of n elements (pos, vel: [n][3][8]) at half step half_dt: per element
+// taken, and for sum j (12 volume, the largest squared face vector, the squared
+// edge cross products (3), their products with the velocity differences (3), the
+// cofactor sum, the half-step determinant) want[10 i + j], the errors of the fixed-point
+// form and of the FP64 form, and the sum of the magnitudes of its products.
+// (Sums with velocities take 4 of the coordinate's velocity extent for a
+// difference, the size of its four body diagonals.)
+void check_sizes(int n, const double* pos, const double* vel, double half_dt, int* taken, double* want, double* fixed,
+                 double* fp64, double* size) {
+  for (int i = 0; i < n; ++i) {
+    const double(*p)[8] = reinterpret_cast<const double(*)[8]>(pos + 24 * i);
+    const double(*v)[8] = reinterpret_cast<const double(*)[8]>(vel + 24 * i);
+    Num column[KS_COUNT];
+    const Slots sh{column, 1};
+    KinLane r[3];
+    for (int k = 0; k < 3; ++k) {
+      for (int c = 0; c < 8; ++c) {
+        r[k].x[c] = p[k][c];
+        r[k].v[c] = v[k][c];
+      }
+      kin_extents(k, sh, r[k]);
+    }
+    for (int k = 0; k < 3; ++k) kin_edges(k, sh, half_dt, r[k]);
+    for (int k = 0; k < 3; ++k) kin_products(k, sh, r[k]);
+    for (int k = 0; k < 3; ++k) kin_terms(k, sh, r[k]);
+    for (int k = 0; k < 3; ++k) kin_accept(sh, r[k]);
+    if (r[0].ok != r[1].ok || r[0].ok != r[2].ok) std::abort();
+    taken[i] = r[0].ok;
+    if (!taken[i]) continue;
+    int place;
+    const double got[10] = {kin_volume12(sh, r[0]), kin_largest_face(sh, r[0], place),
+                            kin_area(sh, r[0], 0), kin_area(sh, r[0], 1), kin_area(sh, r[0], 2),
+                            kin_flow(sh, r[0], 0), kin_flow(sh, r[0], 1), kin_flow(sh, r[0], 2),
+                            kin_rate(sh, r[0]), kin_jacobian(sh, r[0])};
+    Q w[10], s[10];
+    for (int j = 0; j < 10; ++j) w[j] = s[j] = 0;
+    auto d = [&](int k, int a, int b) { return (Q)p[k][a] - p[k][b]; };
+    static const int tv[3][8] = {{3, 1, 7, 2, 6, 3, 2, 0}, {4, 3, 5, 7, 6, 4, 7, 0}, {1, 4, 2, 5, 6, 1, 5, 0}};
+    for (int t = 0; t < 3; ++t) {
+      Q U[3], V[3], W[3], c[3], m[3];
+      for (int k = 0; k < 3; ++k) {
+        U[k] = d(k, tv[t][0], tv[t][1]) + d(k, tv[t][2], tv[t][3]);
+        V[k] = d(k, tv[t][4], tv[t][5]);
+        W[k] = d(k, tv[t][6], tv[t][7]);
+      }
+      cross(V, W, c, m);
+      for (int k = 0; k < 3; ++k) {
+        w[0] += U[k] * c[k];
+        s[0] += qabs(U[k]) * m[k];
+      }
+    }
+    static const int fd[6][4] = {{2, 0, 3, 1}, {6, 4, 5, 7}, {5, 0, 1, 4}, {6, 1, 2, 5}, {7, 2, 3, 6}, {4, 3, 0, 7}};
+    for (int q = 0; q < 6; ++q) {
+      Q a[3], b[3], c[3], m[3], f = 0, g = 0;
+      for (int k = 0; k < 3; ++k) {
+        a[k] = d(k, fd[q][0], fd[q][1]);
+        b[k] = d(k, fd[q][2], fd[q][3]);
+      }
+      cross(a, b, c, m);
+      for (int k = 0; k < 3; ++k) {
+        f += c[k] * c[k];
+        g += qabs(c[k]) * m[k];
+      }
+      if (f > w[1]) {
+        w[1] = f;
+        s[1] = g;
+      }
+    }
+    Q e[3][3], u[3][3], h[3][3], dV[3];  // [direction][coordinate]
+    static const int sg[3][8] = {{-1, 1, 1, -1, -1, 1, 1, -1}, {-1, -1, 1, 1, -1, -1, 1, 1}, {-1, -1, -1, -1, 1, 1, 1, 1}};
+    for (int k = 0; k < 3; ++k) {
+      dV[k] = 0;
+      for (int c = 0; c < 8; ++c)
+        for (int b = 0; b < 8; ++b)
+          if ((Q)v[k][c] - v[k][b] > dV[k]) dV[k] = (Q)v[k][c] - v[k][b];
+      for (int a = 0; a < 3; ++a) {
+        e[a][k] = u[a][k] = 0;
+        for (int c = 0; c < 8; ++c) {
+          e[a][k] += sg[a][c] * (Q)p[k][c];
+          u[a][k] += sg[a][c] * (Q)v[k][c];
+        }
+        h[a][k] = e[a][k] - (Q)half_dt * u[a][k];
+      }
+    }
+    for (int a = 0; a < 3; ++a) {
+      Q A[3], Am[3], C[3], Cm[3];
+      cross(e[(a + 1) % 3], e[(a + 2) % 3], A, Am);
+      cross(h[(a + 1) % 3], h[(a + 2) % 3], C, Cm);
+      for (int k = 0; k < 3; ++k) {
+        w[2 + a] += A[k] * A[k];
+        s[2 + a] += qabs(A[k]) * Am[k];
+        w[5 + a] += A[k] * u[a][k];
+        s[5 + a] += Am[k] * 4 * dV[k];
+        w[8] += C[k] * u[a][k];
+        s[8] += Cm[k] * 4 * dV[k];
+        if (a == 1) {
+          w[9] += C[k] * h[1][k];
+          s[9] += Cm[k] * qabs(h[1][k]);
+        }
+      }
+    }
+    double plain[10];
+    fp64_sums(p, v, half_dt, plain);
+    for (int j = 0; j < 10; ++j) {
+      want[10 * i + j] = (double)w[j];
+      fixed[10 * i + j] = (double)qabs((Q)got[j] - w[j]);
+      fp64[10 * i + j] = (double)qabs((Q)plain[j] - w[j]);
+      size[10 * i + j] = (double)s[j];
+    }
+  }
+}
+
+}  // extern "C"

@@ -1,0 +1,65 @@
+"""The kinematics' fixed-point sums (lulesh_fixed_kin.cuh) beside the FP64
+expressions they took the place of, both against 113-bit floating point: over a
+group of elements the largest error, relative to the sum of the magnitudes of the
+sum's products, may not be larger than that of the FP64 expressions by more than
+2^-52 (a result rounded to a double, 2^-53 of the sum, and as much again for
+cuts at 2^-56 and below). A bound over the element's box cannot see a direction,
+or a velocity component, far below the others.
+"""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+CUBE = np.array([[0, 1, 1, 0, 0, 1, 1, 0], [0, 0, 1, 1, 0, 0, 1, 1], [0, 0, 0, 0, 1, 1, 1, 1]], float)
+
+
+@pytest.fixture(scope="module")
+def sums(tmp_path_factory):
+    cxx = os.environ.get("CXX") or shutil.which("g++")
+    so = str(tmp_path_factory.mktemp("sizes") / "sizes.so")
+    subprocess.run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off",
+                    os.path.join(ROOT, "tests", "fixed_sizes_check.cpp"), "-o", so], check=True)
+    lib = ctypes.CDLL(so)
+
+    def run(pos, vel, half_dt):
+        n = len(pos)
+        taken = np.zeros(n, np.int32)
+        out = [np.zeros((n, 10)) for _ in range(4)]
+        lib.check_sizes(n, *(a.ctypes.data_as(ctypes.c_void_p) for a in (pos, vel)), ctypes.c_double(half_dt),
+                        *(a.ctypes.data_as(ctypes.c_void_p) for a in (taken, *out)))
+        return taken.astype(bool), *out  # want, errors of the fixed-point and the FP64 form, size
+    return run
+
+
+def _elements(seed, n, h, jitter, squash=1.0, axis=2, ratio=1.0):
+    """n elements on a mesh of spacing h, jittered and squashed along an axis;
+    velocities whose differences along x are 1/ratio those of y and z."""
+    r = np.random.default_rng(seed)
+    e = CUBE + jitter * r.uniform(-1, 1, (n, 3, 8))
+    e[:, axis] *= squash
+    pos = np.ascontiguousarray(h * (np.floor(r.uniform(0, 1 / h, (n, 3, 1))) + e))
+    vel = r.uniform(-1, 1, (n, 3, 8))
+    vel[:, 1:] *= ratio
+    return pos, np.ascontiguousarray(vel)
+
+
+def _no_further_off(fixed, fp64, size, which):
+    for j in which:
+        assert (fixed[:, j] / size[:, j]).max() <= (fp64[:, j] / size[:, j]).max() + 2.0 ** -52, j
+
+
+@pytest.mark.parametrize("h", [1.125 / 150, 2.0 ** -7, 0.3])
+@pytest.mark.parametrize("jitter", [0.0, 1e-6, 0.05])
+@pytest.mark.parametrize("ratio", [1.0, 1e-3, 1e-6, 1e-9, 1e-10, 1e-12])
+def test_velocity_sums_in_flow_along_one_axis(sums, h, jitter, ratio):
+    pos, vel = _elements(1, 200, h, jitter, ratio=ratio)
+    for half_dt in (0.0, 1e-3 * h):
+        taken, _, fixed, fp64, size = sums(pos, vel, half_dt)
+        assert taken.all()
+        _no_further_off(fixed, fp64, size, range(5, 9))
