@@ -267,6 +267,17 @@ constexpr int kMinSpeed = 1023 - 400, kMaxSpeed = 1023 + 400;
 
 LULESH_FX unsigned umax(unsigned a, unsigned b) { return a > b ? a : b; }
 
+// The scales s (x = X 2^-s) of an element's three coordinates in place of their
+// extents' exponent fields, each its extent to [2^60, 2^61); an extent below
+// 2^-40 of the largest counts as that (no element that thin is taken). A largest
+// extent out of range shifts everything out.
+LULESH_FX void scales_of(int s[3]) {
+  const int top = imax(s[0], imax(s[1], s[2]));
+  const bool ok = top >= kMinExtent && top <= kMaxExtent;
+  LULESH_UNROLL
+  for (int j = 0; j < 3; ++j) s[j] = 1083 - (ok ? imax(s[j], top - 40) : 0x7ff);
+}
+
 // --- element geometry -----------------------------------------------------------
 // The 12 face diagonals in the FP64 code's order: d20 d31 d50 d14 d61 d25 d72
 // d36 d43 d07 d64 d57. Below 2^61.

@@ -25,24 +25,26 @@ enum : int {
 // sums over the coordinates
 enum : int {
   SUM_VOLUME = 0,  // 12 volume over 2^62
-  SUM_FACE = 1,    // 6: squared face vectors over 2^57, force order
-  SUM_AREA = 7,    // 3: squared cross products of the mean edges over 2^57
+  SUM_FACE = 1,    // 6: squared face vectors over 2^61, force order
+  SUM_AREA = 7,    // 3: squared cross products of the mean edges over 2^61
   SUM_FLOW = 10,   // 3: those cross products times velocity differences
   SUM_RATE = 13,   // cofactors times velocity differences
   SUM_JAC = 14,    // half-step determinant over 2^59
-  SUM_EXPO = 15,   // (16 bits each) exponents of the three flows and the rate
-  kSums = 16
+  SUM_EXPO = 15,   // (16 bits each) exponents of the three flows, the rate and the three areas
+  kSums = 17
 };
 // exponent of a term that is exactly zero
 constexpr int kNoTerm = -16384;
 static_assert(3 * kSums <= 54, "the sums overlay the diagonals");
 
 // What a thread keeps over the phases: its components (unscaled integers) of
-// the face vectors, the volume's V x W, the edges' cross products (over
-// 2^(64 - up)), the cofactors (over 2^62), and its velocity differences and edges.
+// the face vectors (over 2^62), the volume's V x W, the edges' cross products
+// (over 2^(64 - up)), the cofactors (over 2^62), and its velocity differences and
+// edges. A component of a cross product is in the other two coordinates' units,
+// a triple product in all three, whichever the component.
 struct KinLane {
   double x[8], v[8];
-  int s, sv;  // scales of the positions and of this coordinate's velocities
+  int s, sv, all;  // scales of this coordinate's positions and velocities; sum of the three positions'
   int up[3];
   bool ok_x, ok;  // positions taken; positions and velocities taken
   i64 g[12], w[3], vw[3];
@@ -50,12 +52,26 @@ struct KinLane {
   Num half_eta;
 };
 
-// a^2 over 2^57; all four limb products, as the squares of the low limbs do
+// a^2 over 2^61; all four limb products, as the squares of the low limbs do
 // not average out
 LULESH_FX i64 square(Num a) {
   const i64 h = mulw(a.hi, a.hi), m = mulw(a.hi, a.lo);
   const u64 l = (u64)mulw(a.lo, a.lo);
-  return shl(h, 7) + ((m + (i64)(l >> 33)) >> 24);
+  return shl(h, 3) + ((m + (i64)(l >> 33)) >> 28);
+}
+
+// The positions' scales.
+struct Scales {
+  int s[3];
+  LULESH_FX int thin() const { return imax(s[0], imax(s[1], s[2])); }
+  LULESH_FX int wide() const { return imin(s[0], imin(s[1], s[2])); }
+};
+LULESH_FX Scales kin_scales(Slots sh) {
+  Scales r;
+  LULESH_UNROLL
+  for (int j = 0; j < 3; ++j) r.s[j] = exponent_field((unsigned)sh[KS_EXT + j].lo);
+  scales_of(r.s);
+  return r;
 }
 
 // 1: r.x and r.v hold coordinate k's corner values.
@@ -67,33 +83,39 @@ LULESH_FX void kin_extents(int k, Slots sh, const KinLane& r) {
 }
 
 // 2: diagonals, mean edges, velocity differences and half-step edges (edge -
-// dt/2 velocity difference, half_dt = dt/2). Each coordinate's velocities have
-// their own scale: in flow along one axis the others' differences, which alone
-// make up the monotonic-Q gradients across it, are as small as they please.
+// dt/2 velocity difference, half_dt = dt/2). Each coordinate's positions and
+// velocities have their own scale: a thin element keeps its thin direction's
+// bits, and in flow along one axis the others' differences, which alone make up
+// the monotonic-Q gradients across it, are as small as they please.
 LULESH_FX void kin_edges(int k, Slots sh, double half_dt, KinLane& r) {
   const Num m0 = sh[KS_EXT], m1 = sh[KS_EXT + 1], m2 = sh[KS_EXT + 2];
   const int ex = exponent_field(umax(umax((unsigned)m0.lo, (unsigned)m1.lo), (unsigned)m2.lo));
-  const int fastest = exponent_field(umax(umax((unsigned)m0.hi, (unsigned)m1.hi), (unsigned)m2.hi));
   r.ok_x = ex >= kMinExtent && ex <= kMaxExtent;
-  const Float T = to_float(half_dt);
-  const bool wild = fastest > kMaxSpeed;  // not finite, or far beyond any flow
-  const int ev = wild ? 0x7ff : imax(exponent_field((unsigned)(k == 0 ? m0 : k == 1 ? m1 : m2).hi), kMinSpeed);
-  const int exs = r.ok_x ? ex : 0x7ff;
-  r.s = 1083 - exs;
-  r.sv = 1083 - ev;
+  const Scales s = kin_scales(sh);
+  r.s = k == 0 ? s.s[0] : k == 1 ? s.s[1] : s.s[2];
+  r.all = s.s[0] + s.s[1] + s.s[2];
+  int ev[3] = {exponent_field((unsigned)m0.hi), exponent_field((unsigned)m1.hi), exponent_field((unsigned)m2.hi)};
+  const bool wild = imax(ev[0], imax(ev[1], ev[2])) > kMaxSpeed;  // not finite, or far beyond any flow
+  int fastest = kNoExponent;
+  LULESH_UNROLL
+  for (int j = 0; j < 3; ++j) {
+    ev[j] = wild ? 0x7ff : imax(ev[j], kMinSpeed);
+    fastest = imax(fastest, s.s[j] - 1083 + ev[j]);
+  }
+  r.sv = 1083 - (k == 0 ? ev[0] : k == 1 ? ev[1] : ev[2]);
   // dt/2 in units of the edges over those of the velocities, T.m 2^tx: taken
   // while corners move less than an eighth of the scale's 2^61
+  const Float T = to_float(half_dt);
   const int tx = T.k + r.s - r.sv;
-  r.ok = r.ok_x && !wild && T.k + r.s - 1083 + imax(fastest, kMinSpeed) <= -64 &&
-         exponent_field((unsigned)hi_word(half_dt)) != 0x7ff;
+  r.ok = r.ok_x && !wild && T.k + fastest <= -64 && exponent_field((unsigned)hi_word(half_dt)) != 0x7ff;
   const Num tau = limbs(T.m >> (r.ok ? imin(-64 - tx, 63) : 63));
   i64 c[8];
   LULESH_UNROLL
-  for (int i = 0; i < 8; ++i) c[i] = to_fixed(r.x[i], 8 - exs);
+  for (int i = 0; i < 8; ++i) c[i] = to_fixed(r.x[i], r.s - 1075);
   diagonals(c, r.g);
   walsh(c, r.w, nullptr);
   LULESH_UNROLL
-  for (int i = 0; i < 8; ++i) c[i] = to_fixed(r.v[i], 8 - ev);
+  for (int i = 0; i < 8; ++i) c[i] = to_fixed(r.v[i], r.sv - 1075);
   walsh(c, r.vw, nullptr);
   const int at = KS_GEO + 18 * k;
   LULESH_UNROLL
@@ -115,7 +137,8 @@ LULESH_FX void kin_products(int k, Slots sh, KinLane& r) {
     return take<0>(mul_minus(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]));
   };
   LULESH_UNROLL
-  for (int f = 0; f < 6; ++f) r.n[f] = cross_k(2 * f, 2 * f + 1);
+  for (int f = 0; f < 6; ++f)
+    r.n[f] = take<2>(mul_minus(sh[i1 + 2 * f], sh[i2 + 2 * f + 1], sh[i2 + 2 * f], sh[i1 + 2 * f + 1]));
   // V x W of the three products: (-g7, g0), (g10, -g9), (g4, g2)
   r.gU[0] = cross_k(0, 7);
   r.gU[1] = cross_k(9, 10);
@@ -140,23 +163,26 @@ LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
     mac_full(a, limbs(r.g[3] + r.g[5]), limbs(r.gU[2]));
     sh.put(at + SUM_VOLUME, take<2>(a));
   }
+  // (of the faces only the largest counts: they take the largest unit)
+  const int thinner = imin(kin_scales(sh).thin() - r.s, 63), two = r.all - r.s;
   LULESH_UNROLL
-  for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square(limbs(r.n[f])));
-  // The terms of a sum with velocities differ in scale by coordinate: each is
-  // brought to 2^60 and carries its exponent, and the sum takes the largest's.
-  int e[4];
+  for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square(limbs(r.n[f] >> thinner)));
+  // The terms of the other sums differ in scale by coordinate: each is brought
+  // to 2^60 and carries its exponent, and the sum takes the largest's.
+  int e[7];
   auto put_term = [&](int i, i64 t, int shift, int& expo) {
     const int c = room(t);
     sh.put(at + i, shl(t, c));
-    expo = t != 0 ? -(r.sv + shift + c) : kNoTerm;
+    expo = t != 0 ? -(r.sv + two + shift + c) : kNoTerm;
   };
   Acc rate = {0, 0};
   LULESH_UNROLL
   for (int d = 0; d < 3; ++d) {
-    const Num u = limbs(r.vw[d]), c = limbs(r.C[d]);
-    sh.put(at + SUM_AREA + d, square(limbs(r.A[d] >> r.up[d])));
+    const Num a = limbs(r.A[d]), u = limbs(r.vw[d]), c = limbs(r.C[d]);
+    sh.put(at + SUM_AREA + d, square(a));
+    e[4 + d] = r.A[d] != 0 ? -2 * (two + r.up[d]) : kNoTerm;
     Acc flow = {0, 0};
-    mac_full(flow, limbs(r.A[d]), u);
+    mac_full(flow, a, u);
     put_term(SUM_FLOW + d, take<3>(flow), r.up[d], e[d]);
     mac_full(rate, c, u);
   }
@@ -165,6 +191,9 @@ LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
   x.lo = (e[0] & 0xffff) | (int)((unsigned)e[1] << 16);
   x.hi = (e[2] & 0xffff) | (int)((unsigned)e[3] << 16);
   sh[at + SUM_EXPO] = x;
+  x.lo = (e[4] & 0xffff) | (int)((unsigned)e[5] << 16);
+  x.hi = e[6];
+  sh[at + SUM_EXPO + 1] = x;
   Acc jac = {0, 0};
   mac_full(jac, r.half_eta, limbs(r.C[1]));
   sh.put(at + SUM_JAC, take<3>(jac));
@@ -174,10 +203,10 @@ LULESH_FX i64 kin_sum(Slots sh, int i) {
   return add(add(sh.get(KS_SUM + i), sh.get(KS_SUM + kSums + i)), sh.get(KS_SUM + 2 * kSums + i));
 }
 
-// the exponent of coordinate j's term of flow i, or of the rate (i = 3)
+// the exponent of coordinate j's term of flow i, of the rate (i = 3) or of area i - 4
 LULESH_FX int kin_expo(Slots sh, int j, int i) {
-  const Num x = sh[KS_SUM + kSums * j + SUM_EXPO];
-  const int w = i < 2 ? x.lo : x.hi;
+  const Num x = sh[KS_SUM + kSums * j + SUM_EXPO + (i >> 2)];
+  const int w = i & 2 ? x.hi : x.lo;
   return i & 1 ? w >> 16 : (int)(short)w;
 }
 // the sum of those terms, times 2^k
@@ -191,14 +220,19 @@ LULESH_FX double kin_aligned(Slots sh, int sum, int i, int k) {
 
 LULESH_FX i64 kin_determinant(Slots sh) { return sh.get(KS_DET) + sh.get(KS_DET + 1) + sh.get(KS_DET + 2); }
 
-// 5: whether the element is taken (by its determinant and volume too), and the
-// sums in FP64 with their true scales.
-LULESH_FX void kin_accept(Slots sh, KinLane& r) {
-  const bool det = kin_determinant(sh) >= kMinDet;
-  r.ok_x = r.ok_x && det;
-  r.ok = r.ok && det && kin_sum(sh, SUM_VOLUME) >= kMinDet << 4;
+// 5: whether the element is taken (by its determinant and volume too, over the
+// cube of its largest extent), and the sums in FP64 with their true scales.
+LULESH_FX i64 kin_least(Slots sh, const KinLane& r) {
+  return shl(kMinDet, imin(r.all - 3 * kin_scales(sh).wide(), 11));  // (no determinant reaches 2^58)
 }
-LULESH_FX double kin_volume12(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_VOLUME), 126 - 3 * r.s); }
+LULESH_FX bool kin_positions_taken(Slots sh, const KinLane& r) {
+  return r.ok_x && kin_determinant(sh) >= kin_least(sh, r);
+}
+LULESH_FX void kin_accept(Slots sh, KinLane& r) {
+  r.ok_x = kin_positions_taken(sh, r);
+  r.ok = r.ok && r.ok_x && kin_sum(sh, SUM_VOLUME) >= shl(kin_least(sh, r), 4);
+}
+LULESH_FX double kin_volume12(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_VOLUME), 126 - r.all); }
 // the largest squared face vector and its place in the reference's face order
 // (0, 5, 1, 2, 3, 4 of the force order)
 LULESH_FX double kin_largest_face(Slots sh, const KinLane& r, int& place) {
@@ -212,20 +246,16 @@ LULESH_FX double kin_largest_face(Slots sh, const KinLane& r, int& place) {
       place = q;
     }
   }
-  return to_double(best, 185 - 4 * r.s);
+  return to_double(best, 185 - 2 * (r.all - kin_scales(sh).thin()));
 }
-LULESH_FX double kin_area(Slots sh, const KinLane& r, int d) {
-  return to_double(kin_sum(sh, SUM_AREA + d), 193 - 4 * r.s);
-}
-LULESH_FX double kin_flow(Slots sh, const KinLane& r, int d) {
-  return kin_aligned(sh, SUM_FLOW + d, d, 131 - 2 * r.s);
-}
-LULESH_FX double kin_rate(Slots sh, const KinLane& r) { return kin_aligned(sh, SUM_RATE, 3, 131 - 2 * r.s); }
+LULESH_FX double kin_area(Slots sh, const KinLane&, int d) { return kin_aligned(sh, SUM_AREA + d, 4 + d, 197); }
+LULESH_FX double kin_flow(Slots sh, const KinLane&, int d) { return kin_aligned(sh, SUM_FLOW + d, d, 131); }
+LULESH_FX double kin_rate(Slots sh, const KinLane&) { return kin_aligned(sh, SUM_RATE, 3, 131); }
 // coordinate k's part of it
-LULESH_FX double kin_own_rate(Slots sh, const KinLane& r, int k) {
-  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 131 - 2 * r.s + kin_expo(sh, k, 3));
+LULESH_FX double kin_own_rate(Slots sh, const KinLane&, int k) {
+  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 131 + kin_expo(sh, k, 3));
 }
-LULESH_FX double kin_jacobian(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_JAC), 129 - 3 * r.s); }
+LULESH_FX double kin_jacobian(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_JAC), 129 - r.all); }
 
 }  // namespace fx
 }  // namespace lulesh

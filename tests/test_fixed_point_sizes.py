@@ -63,3 +63,13 @@ def test_velocity_sums_in_flow_along_one_axis(sums, h, jitter, ratio):
         taken, _, fixed, fp64, size = sums(pos, vel, half_dt)
         assert taken.all()
         _no_further_off(fixed, fp64, size, range(5, 9))
+
+
+@pytest.mark.parametrize("h", [1.125 / 30, 1.125 / 150, 2.0 ** -7])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("squash", [1.0, 0.5, 0.2, 0.09, 1 / 25, 1 / 32])
+def test_sums_of_thin_elements(sums, h, axis, squash):
+    pos, vel = _elements(2, 400, h, 0.02, squash, axis)
+    taken, _, fixed, fp64, size = sums(pos, vel, 1e-4 * h)
+    assert taken.all() if squash > 0.1 else taken.any()
+    _no_further_off(fixed[taken], fp64[taken], size[taken], range(10))
