@@ -368,11 +368,6 @@ __device__ __forceinline__ void walsh_modes_t(const T t[4], T out[8]) {
   out[4] = cp - s; out[5] = -d - cp; out[6] = s + cp; out[7] = d - cp;
 }
 
-// to_fixed rounded towards zero, so that zeros of both signs give zero: where no
-// adjoint has come to an element yet, its sums stay exact zeros.
-__device__ __forceinline__ fx::i64 to_fixed0(double x, int bias) {
-  return fx::sub(fx::to_fixed(x, bias), (fx::i64)(fx::hi_word(x) >> 31));
-}
 // A coefficient's mantissa in the unit 2^u of a sum, its own unit being 2^e.
 __device__ __forceinline__ fx::i64 in_unit(const fx::Float& f, int e, int u) { return f.m >> fx::imin(u - e, 63); }
 // Whether a sum is in range: coefficients at most 2^400 (so not infinities or
@@ -612,8 +607,8 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       if (ok_edges) {
-        num(own + KA_LA + d) = fx::limbs(to_fixed0(LA[d], sg + cA - 1075));
-        num(own + KA_LC + d) = fx::limbs(to_fixed0(LC[d], sg + cC - 1075));
+        num(own + KA_LA + d) = fx::limbs(fx::to_fixed0(LA[d], sg + cA - 1075));
+        num(own + KA_LC + d) = fx::limbs(fx::to_fixed0(LC[d], sg + cC - 1075));
       } else {
         sh(own + KA_LA + d) = LA[d];
         sh(own + KA_LC + d) = LC[d];
@@ -632,7 +627,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     uc = 61 - (s0 + s1 + s2 - sg + common);
     if (ok)
 #pragma unroll
-      for (int q = KA_DV; q < KA_LA; ++q) num(own + q) = fx::limbs(to_fixed0(sh(own + q), sg + common - 1075));
+      for (int q = KA_DV; q < KA_LA; ++q) num(own + q) = fx::limbs(fx::to_fixed0(sh(own + q), sg + common - 1075));
   }
   // component k of sums of (slot i) x (slot j)
   struct Cross { fx::Acc p, n; };
@@ -1029,9 +1024,9 @@ __device__ __forceinline__ void corner_differences(const double u[8], Put put) {
   x.lo = 1081 - ev;
   x.hi = ok;
   put(0, x);
-  const fx::i64 u0 = to_fixed0(u[0], 6 - ev);
+  const fx::i64 u0 = fx::to_fixed0(u[0], 6 - ev);
 #pragma unroll
-  for (int c = 1; c < 8; ++c) put(c, fx::limbs(fx::sub(to_fixed0(u[c], 6 - ev), u0)));
+  for (int c = 1; c < 8; ++c) put(c, fx::limbs(fx::sub(fx::to_fixed0(u[c], 6 - ev), u0)));
 }
 
 template <int MODE>

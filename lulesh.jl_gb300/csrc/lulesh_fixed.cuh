@@ -226,6 +226,12 @@ LULESH_FX i64 to_fixed(double x, int bias) {
   return (i64)r ^ (i64)(h >> 31);
 }
 
+// The same rounded towards zero: zeros of both signs give zero, and x and -x
+// opposite numbers, so that what cancels in doubles that fit cancels here. (A
+// velocity divergence that is exactly zero sets no time constraint, and where no
+// adjoint has come to an element yet, its sums stay exact zeros.)
+LULESH_FX i64 to_fixed0(double x, int bias) { return sub(to_fixed(x, bias), (i64)(hi_word(x) >> 31)); }
+
 // v 2^k, rounded once; the caller keeps the result's exponent in range
 LULESH_FX double to_double(i64 v, int k) {
   const double d = (double)v;

@@ -115,7 +115,7 @@ LULESH_FX void kin_edges(int k, Slots sh, double half_dt, KinLane& r) {
   diagonals(c, r.g);
   walsh(c, r.w, nullptr);
   LULESH_UNROLL
-  for (int i = 0; i < 8; ++i) c[i] = to_fixed(r.v[i], r.sv - 1075);
+  for (int i = 0; i < 8; ++i) c[i] = to_fixed0(r.v[i], r.sv - 1075);
   walsh(c, r.vw, nullptr);
   const int at = KS_GEO + 18 * k;
   LULESH_UNROLL

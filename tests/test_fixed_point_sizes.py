@@ -73,3 +73,29 @@ def test_sums_of_thin_elements(sums, h, axis, squash):
     taken, _, fixed, fp64, size = sums(pos, vel, 1e-4 * h)
     assert taken.all() if squash > 0.1 else taken.any()
     _no_further_off(fixed[taken], fp64[taken], size[taken], range(10))
+
+
+def test_exact_zeros_stay_zeros(sums):
+    """Velocities of zeros of both signs, and a flow whose divergence is exactly
+    zero in doubles (compression along one axis as expansion along another, on
+    either side of rest): the sums are zeros, as in FP64. A divergence that is not
+    would set a time constraint (src/domain.jl:2964-3014)."""
+    h = 0.125
+    pos = np.ascontiguousarray(h * (np.array([[[2.0], [3.0], [5.0]]]) + CUBE))
+    r = np.random.default_rng(3)
+    vel = np.where(r.random((200, 3, 8)) < 0.5, 0.0, -0.0)
+    many = np.ascontiguousarray(np.broadcast_to(pos, (200, 3, 8)))
+    taken, want, fixed, _, _ = sums(many, np.ascontiguousarray(vel), 1e-6)
+    assert taken.all() and not want[:, 5:9].any() and not fixed[:, 5:9].any()
+    for i in range(3):
+        j, k = (i + 1) % 3, (i + 2) % 3
+        for a, b in ((1.0, 0.0), (0.75, 0.25), (0.1, 0.2)):
+            v = np.zeros((1, 3, 8))
+            v[0, i] = np.where(CUBE[i] > 0, a, -a)  # a - (-a)
+            v[0, j] = np.where(CUBE[j] > 0, b, b + 2 * a)
+            v[0, k] = -0.0
+            taken, want, fixed, fp64, _ = sums(pos, v, 0.0)
+            assert taken.all()
+            if (b + 2 * a) - b == 2 * a:
+                assert want[0, 8] == 0 and fp64[0, 8] == 0 and fixed[0, 8] == 0, (i, a, b)
+            assert fixed[0, 5 + k] == 0
