@@ -6,13 +6,13 @@
 // integer add 237; double<->integer conversions take an FP64 slot each. So
 // sums and products of quantities that share one scale run on the integer
 // pipes at about six (products) to thirty times (sums) the FP64 rate. What an
-// element kernel forms from its eight corners is such a set: differences of
-// positions or velocities within one element.
+// element kernel forms from its eight corners is such a set: differences of one
+// coordinate's positions or velocities within one element.
 //
-// Numbers are integers X with an element-wide exponent: x = X 2^-s. The scale
-// puts the element's largest coordinate extent in [2^60, 2^61), so a
-// difference of corners keeps 60 bits below the extent where a double keeps
-// 52 below the (larger) coordinate itself. Conversion is modulo 2^64: a corner
+// Numbers are integers X with an exponent for each coordinate of an element:
+// x = X 2^-s. The scale puts the coordinate's extent over the corners in [2^60,
+// 2^61), so a difference of corners keeps 60 bits below the extent where a double
+// keeps 52 below the (larger) coordinate itself. Conversion is modulo 2^64: a corner
 // far from the origin wraps, and the differences, which is all that is used,
 // are exact. A product keeps the upper 64 of its 128 bits.
 //
@@ -21,11 +21,12 @@
 // (below a quarter of the last kept bit, of either sign) is dropped. Sums of
 // products share one pair of accumulators and one rounding.
 //
-// Error: a difference 2^-61 of the extent, a cross product about 2^-57 of the
-// extent's square, the volume about 2^-56 of the extent's cube, each at or
-// below what the FP64 expressions leave. Elements whose Jacobian determinant
-// is below kMinDet of the scaled box (thin, inverted, not finite, or of a size
-// no mesh here has) are left to the FP64 expressions by the callers.
+// Error: a difference 2^-61 of the coordinate's extent, a cross product's component
+// about 2^-57 of the product of the other two's, the volume about 2^-56 of the
+// product of all three, each at or below what the FP64 expressions leave (tested
+// beside them). Elements whose Jacobian determinant is below kMinDet of the cube of
+// the largest extent (thin, inverted, not finite, or of a size no mesh here has)
+// are left to the FP64 expressions by the callers.
 //
 // Everything here also compiles for the host, where the tests compare it with
 // exact rational arithmetic.
@@ -273,15 +274,24 @@ constexpr int kMinSpeed = 1023 - 400, kMaxSpeed = 1023 + 400;
 
 LULESH_FX unsigned umax(unsigned a, unsigned b) { return a > b ? a : b; }
 
-// The scales s (x = X 2^-s) of an element's three coordinates in place of their
-// extents' exponent fields, each its extent to [2^60, 2^61); an extent below
-// 2^-40 of the largest counts as that (no element that thin is taken). A largest
-// extent out of range shifts everything out.
-LULESH_FX void scales_of(int s[3]) {
-  const int top = imax(s[0], imax(s[1], s[2]));
+// The scales s (x = X 2^-s) of an element's three coordinates, each its extent to
+// [2^60, 2^61); an extent below 2^-40 of the largest counts as that (no element
+// that thin is taken). A largest extent out of range shifts everything out.
+struct Scales {
+  int s[3];
+  LULESH_FX int thin() const { return imax(s[0], imax(s[1], s[2])); }
+  LULESH_FX int wide() const { return imin(s[0], imin(s[1], s[2])); }
+  // kMinDet, which is over the cube of the largest extent, in the determinant's
+  // units (none reaches 2^58)
+  LULESH_FX i64 least_determinant() const { return shl(kMinDet, imin(s[0] + s[1] + s[2] - 3 * wide(), 11)); }
+};
+LULESH_FX Scales scales_of(unsigned hi0, unsigned hi1, unsigned hi2) {  // high words of the extents
+  Scales r = {{exponent_field(hi0), exponent_field(hi1), exponent_field(hi2)}};
+  const int top = imax(r.s[0], imax(r.s[1], r.s[2]));
   const bool ok = top >= kMinExtent && top <= kMaxExtent;
   LULESH_UNROLL
-  for (int j = 0; j < 3; ++j) s[j] = 1083 - (ok ? imax(s[j], top - 40) : 0x7ff);
+  for (int j = 0; j < 3; ++j) r.s[j] = 1083 - (ok ? imax(r.s[j], top - 40) : 0x7ff);
+  return r;
 }
 
 // --- element geometry -----------------------------------------------------------

@@ -59,7 +59,7 @@ enum : int {
 struct ForceLane {
   double x[8];
   Num V[8];
-  int ev, s, q;
+  int ev, s, all, q;  // (s: this coordinate's scale, all: the sum of the three)
   bool ok;
   i64 w1;
   Num B[4], B0;
@@ -105,12 +105,12 @@ LULESH_FX void force_diagonals(int k, Slots sh, ForceLane& r, i64 hm[4]) {
   const int ex = exponent_field(umax(umax((unsigned)m0.lo, (unsigned)m1.lo), (unsigned)m2.lo));
   r.ok = ex >= kMinExtent && ex <= kMaxExtent && (m0.hi | m1.hi | m2.hi) == 0 && sh[FS_EXPO].hi != 1 << 20 &&
          sh[FS_EXPO + 1].hi != 0;
-  // (an element not taken shifts everything out)
-  const int exs = r.ok ? ex : 0x7ff;
-  r.s = 1083 - exs;
+  const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo);
+  r.s = k == 0 ? s.s[0] : k == 1 ? s.s[1] : s.s[2];
+  r.all = s.s[0] + s.s[1] + s.s[2];
   i64 v[8], g[12], w[3];
   LULESH_UNROLL
-  for (int c = 0; c < 8; ++c) v[c] = to_fixed(r.x[c], 8 - exs);
+  for (int c = 0; c < 8; ++c) v[c] = to_fixed(r.x[c], r.s - 1075);
   diagonals(v, g);
   walsh(v, w, &hm[3]);
   even_modes(g, hm);
@@ -140,6 +140,11 @@ LULESH_FX void force_diagonals(int k, Slots sh, ForceLane& r, i64 hm[4]) {
 // minus corners 0, 1, 2, 3), volume derivatives in the reference's slots (node
 // 3's in slot 1 and node 1's in slot 3 unless MODE bit 1), the determinant of
 // the mean edges, and the scaled modes.
+//
+// Each coordinate's positions have their own scale: a cross product's component
+// is in the other two's units, derivative * mode and the determinant in all
+// three, whichever the component. A thin element's forces along its thin
+// direction, and across it, keep their bits.
 //
 // The modes are scaled by 1/(12 determ) so that derivative * mode is in units
 // 2^(q - 58) of the base vectors. The scale's exponent L is taken as a left
@@ -178,14 +183,14 @@ LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Ta
     for (int n = 0; n < 8; ++n) {
       const int src = (MODE & 2) ? n : (n == 1 ? 3 : n == 3 ? 1 : n);
       sh[FS_DV + 12 * k + n] = limbs(d[src]);
-      if (Tape::on) tape.derivative(k, n, to_double(d[src], 64 - 2 * r.s));
+      if (Tape::on) tape.derivative(k, n, to_double(d[src], 64 - (r.all - r.s)));
     }
   }
   sh.put(FS_DET + k, product(limbs(r.w1), limbs(cross_k(17, 15))));
 
   const Num expo = sh[FS_EXPO];
   const unsigned used = (unsigned)(sh[FS_USED].lo | sh[FS_USED + 1].lo | sh[FS_USED + 2].lo);
-  const int room = leading_zeros(used) - 3, L = expo.lo + 252 - 3 * r.s;
+  const int room = leading_zeros(used) - 3, L = expo.lo + 252 - r.all;
   r.q = imax(L - (room + 4), 0);
   r.ok = r.ok && L >= 0 && r.q <= 4;
   r.q = r.ok ? r.q : 0;
@@ -195,13 +200,14 @@ LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Ta
   for (int m = 0; m < 4; ++m) {
     const i64 h = shl(product(limbs(shl(hm[m], left)), kl), rest);
     sh[FS_DV + 12 * k + 8 + m] = limbs(h);
-    if (Tape::on) tape.mode(k, m, to_double(h, 2 * r.s - 186 + r.q));
+    if (Tape::on) tape.mode(k, m, to_double(h, r.all - r.s - 186 + r.q));
   }
 }
 
 // 4: every third entry of the base vectors, gamma - sum_k derivative_k mode_k.
 LULESH_FX void force_base(int k, Slots sh, ForceLane& r) {
-  r.ok = r.ok && sh.get(FS_DET) + sh.get(FS_DET + 1) + sh.get(FS_DET + 2) >= kMinDet;
+  const Scales s = scales_of((unsigned)sh[FS_EXT].lo, (unsigned)sh[FS_EXT + 1].lo, (unsigned)sh[FS_EXT + 2].lo);
+  r.ok = r.ok && sh.get(FS_DET) + sh.get(FS_DET + 1) + sh.get(FS_DET + 2) >= s.least_determinant();
   const i64 one = 1ll << (58 - r.q);
   LULESH_UNROLL
   for (int j = 0; j < 11; ++j) {
@@ -240,7 +246,7 @@ LULESH_FX void force_corners(int k, Slots sh, const ForceLane& r, Out out, Tape 
   const int Ck = sh[FS_EXPO].hi, Sk = sh[FS_EXPO + 1].lo;
   // both parts of the force in the larger of their units, 2^u
   const int uh = Cm != 0 && (used | low) != 0u ? 67 + 2 * r.q - room - sv + Ck : kNoExponent;
-  const int us = Sm != 0 ? 125 - 2 * r.s + Sk : kNoExponent;
+  const int us = Sm != 0 ? 125 - (r.all - r.s) + Sk : kNoExponent;
   const int u = imax(uh, us);
   const Num Cl = limbs(Cm >> imin(u - uh, 63)), Sl = limbs(Sm >> imin(u - us, 63));
   Num H[4];

@@ -61,17 +61,8 @@ LULESH_FX i64 square(Num a) {
 }
 
 // The positions' scales.
-struct Scales {
-  int s[3];
-  LULESH_FX int thin() const { return imax(s[0], imax(s[1], s[2])); }
-  LULESH_FX int wide() const { return imin(s[0], imin(s[1], s[2])); }
-};
 LULESH_FX Scales kin_scales(Slots sh) {
-  Scales r;
-  LULESH_UNROLL
-  for (int j = 0; j < 3; ++j) r.s[j] = exponent_field((unsigned)sh[KS_EXT + j].lo);
-  scales_of(r.s);
-  return r;
+  return scales_of((unsigned)sh[KS_EXT].lo, (unsigned)sh[KS_EXT + 1].lo, (unsigned)sh[KS_EXT + 2].lo);
 }
 
 // 1: r.x and r.v hold coordinate k's corner values.
@@ -222,15 +213,12 @@ LULESH_FX i64 kin_determinant(Slots sh) { return sh.get(KS_DET) + sh.get(KS_DET 
 
 // 5: whether the element is taken (by its determinant and volume too, over the
 // cube of its largest extent), and the sums in FP64 with their true scales.
-LULESH_FX i64 kin_least(Slots sh, const KinLane& r) {
-  return shl(kMinDet, imin(r.all - 3 * kin_scales(sh).wide(), 11));  // (no determinant reaches 2^58)
-}
 LULESH_FX bool kin_positions_taken(Slots sh, const KinLane& r) {
-  return r.ok_x && kin_determinant(sh) >= kin_least(sh, r);
+  return r.ok_x && kin_determinant(sh) >= kin_scales(sh).least_determinant();
 }
 LULESH_FX void kin_accept(Slots sh, KinLane& r) {
   r.ok_x = kin_positions_taken(sh, r);
-  r.ok = r.ok && r.ok_x && kin_sum(sh, SUM_VOLUME) >= shl(kin_least(sh, r), 4);
+  r.ok = r.ok && r.ok_x && kin_sum(sh, SUM_VOLUME) >= shl(kin_scales(sh).least_determinant(), 4);
 }
 LULESH_FX double kin_volume12(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_VOLUME), 126 - r.all); }
 // the largest squared face vector and its place in the reference's face order

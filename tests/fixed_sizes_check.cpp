@@ -1,23 +1,10 @@
-// Host harness of the kinematics' fixed-point sums (lulesh_fixed_kin.cuh) beside
-// the FP64 expressions the kernels had and still have for the elements the
-// fixed-point form does not take (kin_fp64 in lulesh_element_fp64.cuh), both
-// against 113-bit floating point.
-#include "../lulesh.jl_gb300/csrc/lulesh_fixed_kin.cuh"
-
-#include <cmath>
-#include <cstdlib>
-
-#if defined(__x86_64__)
-typedef __float128 Q;
-#else
-typedef long double Q;  // binary128 on aarch64
-#endif
+// Host harness of the fixed-point kinematics sums and forces (lulesh_fixed_kin.cuh,
+// lulesh_fixed_force.cuh) beside the FP64 expressions the kernels had and still
+// have for the elements the fixed-point form does not take (kin_fp64 and force_fp64
+// in lulesh_element_fp64.cuh), both against 113-bit floating point.
+#include "fixed_check.cpp"
 
 namespace {
-using namespace lulesh::fx;
-
-Q qabs(Q a) { return a < 0 ? -a : a; }
-
 // kin_fp64's sums: 12 volume, the largest squared face vector, areas, flows,
 // rate, determinant.
 void fp64_sums(const double p[3][8], const double v[3][8], double half_dt, double out[10]) {
@@ -59,6 +46,55 @@ void fp64_sums(const double p[3][8], const double v[3][8], double half_dt, doubl
   out[1] = 0;
   for (int f = 0; f < 6; ++f) out[1] = std::fmax(out[1], sum(1 + f));
   for (int j = 2; j < 10; ++j) out[j] = sum(5 + j);
+}
+
+// force_fp64's corner forces (mode 3: no defects).
+void fp64_forces(const double p[3][8], const double v[3][8], double vi12, double coef, double s8, double f[3][8]) {
+  static const int pa[12] = {2, 3, 5, 1, 6, 2, 7, 3, 4, 0, 6, 5}, pb[12] = {0, 1, 0, 4, 1, 5, 2, 6, 3, 7, 4, 7};
+  double g[3][15], B[3][8], dv[3][8], hm[3][4], hg[8][4];
+  for (int k = 0; k < 3; ++k) {
+    const double* x = p[k];
+    for (int q = 0; q < 12; ++q) g[k][q] = x[pa[q]] - x[pb[q]];
+    g[k][12] = g[k][1] + g[k][6];
+    g[k][13] = g[k][8] + g[k][11];
+    g[k][14] = g[k][3] + g[k][5];
+    const double a = x[6] - x[0], b = x[5] - x[3], c = x[7] - x[1], d = x[4] - x[2];
+    const double pp = g[k][9] + g[k][4], qq = g[k][8] + g[k][5];
+    const double h[4] = {(g[k][10] - g[k][11]) - (g[k][0] + g[k][1]), pp - qq, pp + qq, (a - b) - (c - d)};
+    for (int m = 0; m < 4; ++m) hm[k][m] = h[m] * vi12;
+  }
+  for (int k = 0; k < 3; ++k) {
+    const int i = (k + 1) % 3, j = (k + 2) % 3;
+    auto cr = [&](int a, int b) { return std::fma(g[i][a], g[j][b], -g[j][a] * g[i][b]); };
+    double n[5];
+    for (int q = 0; q < 5; ++q) n[q] = cr(2 * q, 2 * q + 1);
+    const double p01 = n[0] + n[1];
+    B[k][0] = p01 + n[4];
+    B[k][1] = p01 + n[2];
+    B[k][2] = (n[0] + n[2]) + n[3];
+    B[k][3] = (n[0] + n[3]) + n[4];
+    static const int opposite[4] = {6, 7, 4, 5};
+    for (int c = 0; c < 4; ++c) B[k][opposite[c]] = -B[k][c];
+    const double u0 = cr(0, 7), v0 = cr(0, 12), w0 = cr(7, 12), u1 = cr(9, 10), v1 = cr(13, 9), w1 = cr(13, 10);
+    const double u2 = cr(4, 2), v2 = cr(2, 14), w2 = cr(14, 4), t12 = u2 - u0, t37 = u0 - u1, t45 = u1 - u2;
+    const double d[8] = {-((w0 + w1) + w2), t12 - v2, t12 + w0, t37 - v0, t45 - v1, t45 + w2, (v0 + v1) + v2, t37 + w1};
+    for (int c = 0; c < 8; ++c) dv[k][c] = d[c];
+  }
+  for (int c = 0; c < 8; ++c)
+    for (int m = 0; m < 4; ++m)
+      hg[c][m] = std::fma(-dv[2][c], hm[2][m], std::fma(-dv[1][c], hm[1][m], std::fma(-dv[0][c], hm[0][m], gamma_negative(c, m) ? -1.0 : 1.0)));
+  for (int k = 0; k < 3; ++k) {
+    double h[4];
+    for (int m = 0; m < 4; ++m) {
+      double s = hg[0][m] * v[k][0];
+      for (int c = 1; c < 8; ++c) s = std::fma(hg[c][m], v[k][c], s);
+      h[m] = coef * s;
+    }
+    for (int c = 0; c < 8; ++c) {
+      f[k][c] = s8 * B[k][c];
+      for (int m = 3; m >= 0; --m) f[k][c] = std::fma(hg[c][m], h[m], f[k][c]);
+    }
+  }
 }
 
 // c = a x b, and p the sums of its products' magnitudes
@@ -181,6 +217,49 @@ void check_sizes(int n, const double* pos, const double* vel, double half_dt, in
       fixed[10 * i + j] = (double)qabs((Q)got[j] - w[j]);
       fp64[10 * i + j] = (double)qabs((Q)plain[j] - w[j]);
       size[10 * i + j] = (double)s[j];
+    }
+  }
+}
+
+// Corner forces (mode 3) of n elements (scal: [n][3] = vi12, coef, s8): per element
+// taken, and for coordinate k the largest errors over the corners of the two forms,
+// and the size: |s8| times the magnitudes of the products of a corner's three
+// faces, plus |coef| times the coordinate's velocity extent.
+void check_force_sizes(int n, const double* pos, const double* vel, const double* scal, int* taken, double* fixed,
+                       double* fp64, double* size) {
+  static const int fd[6][4] = {{2, 0, 3, 1}, {5, 0, 1, 4}, {6, 1, 2, 5}, {7, 2, 3, 6}, {4, 3, 0, 7}, {6, 4, 5, 7}};
+  for (int i = 0; i < n; ++i) {
+    const double(*p)[8] = reinterpret_cast<const double(*)[8]>(pos + 24 * i);
+    const double(*v)[8] = reinterpret_cast<const double(*)[8]>(vel + 24 * i);
+    const double vi12 = scal[3 * i], coef = scal[3 * i + 1], s8 = scal[3 * i + 2];
+    double f[3][8], plain[3][8];
+    taken[i] = fixed_forces<3>(p, v, vi12, coef, s8, f, NoTape{});
+    if (!taken[i]) continue;
+    Q qf[3][8], qdv[3][8], qh[3][4], qS[3][4];
+    exact_forces(p, v, vi12, coef, s8, 3, qf, qdv, qh, qS);
+    fp64_forces(p, v, vi12, coef, s8, plain);
+    Q most[3] = {0, 0, 0};
+    for (int q = 0; q < 6; ++q) {
+      Q a[3], b[3], c[3], m[3];
+      for (int k = 0; k < 3; ++k) {
+        a[k] = (Q)p[k][fd[q][0]] - p[k][fd[q][1]];
+        b[k] = (Q)p[k][fd[q][2]] - p[k][fd[q][3]];
+      }
+      cross(a, b, c, m);
+      for (int k = 0; k < 3; ++k)
+        if (m[k] > most[k]) most[k] = m[k];
+    }
+    for (int k = 0; k < 3; ++k) {
+      double dV = 0;
+      Q e = 0, g = 0;
+      for (int c = 0; c < 8; ++c) {
+        for (int b = 0; b < 8; ++b) dV = std::fmax(dV, v[k][c] - v[k][b]);
+        if (qabs(f[k][c] - qf[k][c]) > e) e = qabs(f[k][c] - qf[k][c]);
+        if (qabs(plain[k][c] - qf[k][c]) > g) g = qabs(plain[k][c] - qf[k][c]);
+      }
+      fixed[3 * i + k] = (double)e;
+      fp64[3 * i + k] = (double)g;
+      size[3 * i + k] = (double)(3 * std::fabs(s8) * most[k]) + std::fabs(coef) * dV;
     }
   }
 }

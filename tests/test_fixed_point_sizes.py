@@ -1,5 +1,5 @@
-"""The kinematics' fixed-point sums (lulesh_fixed_kin.cuh) beside the FP64
-expressions they took the place of, both against 113-bit floating point: over a
+"""The kinematics' fixed-point sums (lulesh_fixed_kin.cuh) and the corner forces
+(lulesh_fixed_force.cuh) beside the FP64 expressions they took the place of, both against 113-bit floating point: over a
 group of elements the largest error, relative to the sum of the magnitudes of the
 sum's products, may not be larger than that of the FP64 expressions by more than
 2^-52 (a result rounded to a double, 2^-53 of the sum, and as much again for
@@ -20,13 +20,16 @@ CUBE = np.array([[0, 1, 1, 0, 0, 1, 1, 0], [0, 0, 1, 1, 0, 0, 1, 1], [0, 0, 0, 0
 
 
 @pytest.fixture(scope="module")
-def sums(tmp_path_factory):
+def lib(tmp_path_factory):
     cxx = os.environ.get("CXX") or shutil.which("g++")
     so = str(tmp_path_factory.mktemp("sizes") / "sizes.so")
     subprocess.run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off",
                     os.path.join(ROOT, "tests", "fixed_sizes_check.cpp"), "-o", so], check=True)
-    lib = ctypes.CDLL(so)
+    return ctypes.CDLL(so)
 
+
+@pytest.fixture(scope="module")
+def sums(lib):
     def run(pos, vel, half_dt):
         n = len(pos)
         taken = np.zeros(n, np.int32)
@@ -34,6 +37,17 @@ def sums(tmp_path_factory):
         lib.check_sizes(n, *(a.ctypes.data_as(ctypes.c_void_p) for a in (pos, vel)), ctypes.c_double(half_dt),
                         *(a.ctypes.data_as(ctypes.c_void_p) for a in (taken, *out)))
         return taken.astype(bool), *out  # want, errors of the fixed-point and the FP64 form, size
+    return run
+
+
+@pytest.fixture(scope="module")
+def forces(lib):
+    def run(pos, vel, scal):
+        n = len(pos)
+        taken = np.zeros(n, np.int32)
+        out = [np.zeros((n, 3)) for _ in range(3)]
+        lib.check_force_sizes(n, *(a.ctypes.data_as(ctypes.c_void_p) for a in (pos, vel, np.ascontiguousarray(scal), taken, *out)))
+        return taken.astype(bool), *out  # errors of the fixed-point and the FP64 form, size
     return run
 
 
@@ -99,3 +113,18 @@ def test_exact_zeros_stay_zeros(sums):
             if (b + 2 * a) - b == 2 * a:
                 assert want[0, 8] == 0 and fp64[0, 8] == 0 and fixed[0, 8] == 0, (i, a, b)
             assert fixed[0, 5 + k] == 0
+
+
+@pytest.mark.parametrize("h", [1.125 / 30, 1.125 / 150, 2.0 ** -7])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("squash", [1.0, 0.5, 0.2, 0.09, 1 / 25, 1 / 32])
+def test_forces_of_thin_elements(forces, h, axis, squash):
+    """The pure stress, the hourglass forces, and both."""
+    pos, vel = _elements(4, 400, h, 0.02, squash, axis)
+    r = np.random.default_rng(5)
+    vi12 = 1 / (12 * h ** 3 * squash * r.uniform(0.95, 1.05, 400))
+    for coef, s8 in ((0.0, -100.0), (-30.0 * h * h, 0.0), (-30.0 * h * h, -10.0)):
+        scal = np.stack([vi12, np.full(400, coef), np.full(400, s8)], 1)
+        taken, fixed, fp64, size = forces(pos, vel, scal)
+        assert taken.all() if squash > 0.1 else taken.any()
+        _no_further_off(fixed[taken], fp64[taken], size[taken], range(3))
