@@ -281,9 +281,9 @@ struct Scales {
   int s[3];
   LULESH_FX int thin() const { return imax(s[0], imax(s[1], s[2])); }
   LULESH_FX int wide() const { return imin(s[0], imin(s[1], s[2])); }
-  // kMinDet, which is over the cube of the largest extent, in the determinant's
-  // units (none reaches 2^58)
-  LULESH_FX i64 least_determinant() const { return shl(kMinDet, imin(s[0] + s[1] + s[2] - 3 * wide(), 11)); }
+  // kMinDet, which is over the cube of the largest extent, is kMinDet 2^least() in
+  // the determinant's units (none reaches 2^58)
+  LULESH_FX int least() const { return imin(s[0] + s[1] + s[2] - 3 * wide(), 11); }
 };
 LULESH_FX Scales scales_of(unsigned hi0, unsigned hi1, unsigned hi2) {  // high words of the extents
   Scales r = {{exponent_field(hi0), exponent_field(hi1), exponent_field(hi2)}};

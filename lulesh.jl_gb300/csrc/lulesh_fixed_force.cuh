@@ -60,6 +60,7 @@ struct ForceLane {
   double x[8];
   Num V[8];
   int ev, s, all, q;  // (s: this coordinate's scale, all: the sum of the three)
+  int least;          // the least determinant is kMinDet 2^least
   bool ok;
   i64 w1;
   Num B[4], B0;
@@ -108,6 +109,7 @@ LULESH_FX void force_diagonals(int k, Slots sh, ForceLane& r, i64 hm[4]) {
   const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo);
   r.s = k == 0 ? s.s[0] : k == 1 ? s.s[1] : s.s[2];
   r.all = s.s[0] + s.s[1] + s.s[2];
+  r.least = s.least();
   i64 v[8], g[12], w[3];
   LULESH_UNROLL
   for (int c = 0; c < 8; ++c) v[c] = to_fixed(r.x[c], r.s - 1075);
@@ -206,8 +208,7 @@ LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Ta
 
 // 4: every third entry of the base vectors, gamma - sum_k derivative_k mode_k.
 LULESH_FX void force_base(int k, Slots sh, ForceLane& r) {
-  const Scales s = scales_of((unsigned)sh[FS_EXT].lo, (unsigned)sh[FS_EXT + 1].lo, (unsigned)sh[FS_EXT + 2].lo);
-  r.ok = r.ok && sh.get(FS_DET) + sh.get(FS_DET + 1) + sh.get(FS_DET + 2) >= s.least_determinant();
+  r.ok = r.ok && sh.get(FS_DET) + sh.get(FS_DET + 1) + sh.get(FS_DET + 2) >= shl(kMinDet, r.least);
   const i64 one = 1ll << (58 - r.q);
   LULESH_UNROLL
   for (int j = 0; j < 11; ++j) {

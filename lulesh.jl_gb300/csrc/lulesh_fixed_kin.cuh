@@ -17,34 +17,35 @@ namespace fx {
 enum : int {
   KS_GEO = 0,    // 18 k + q: limbs of diagonal q (12), mean edge (3), half-step edge (3) of coordinate k
   KS_SUM = 0,    // kSums k + i: coordinate k's terms, over the diagonals once those are read
-  KS_DET = 54,   // k: a term of the Jacobian determinant
-  KS_EXT = 57,   // k: high words of the position and velocity extents
-  KS_MID = 60,   // 1/(64 volume), then the divergence's factor and the divergence
-  KS_COUNT = 63
+  KS_DET = 57,   // k: a term of the Jacobian determinant
+  KS_EXT = 60,   // k: high words of the position and velocity extents
+  KS_MID = 63,   // 1/(64 volume), then the divergence's factor and the divergence
+  KS_COUNT = 66
 };
 // sums over the coordinates
 enum : int {
   SUM_VOLUME = 0,  // 12 volume over 2^62
-  SUM_FACE = 1,    // 6: squared face vectors over 2^61, force order
+  SUM_FACE = 1,    // 6: squared face vectors over 2^57, force order
   SUM_AREA = 7,    // 3: squared cross products of the mean edges over 2^61
   SUM_FLOW = 10,   // 3: those cross products times velocity differences
   SUM_RATE = 13,   // cofactors times velocity differences
   SUM_JAC = 14,    // half-step determinant over 2^59
-  SUM_EXPO = 15,   // (16 bits each) exponents of the three flows, the rate and the three areas
-  kSums = 17
+  SUM_EXPO = 15,   // 4: exponents of flow d (low word) and area d (high word), the last the rate's
+  kSums = 19
 };
 // exponent of a term that is exactly zero
 constexpr int kNoTerm = -16384;
-static_assert(3 * kSums <= 54, "the sums overlay the diagonals");
+static_assert(3 * kSums <= KS_DET, "the sums overlay the diagonals");
 
 // What a thread keeps over the phases: its components (unscaled integers) of
-// the face vectors (over 2^62), the volume's V x W, the edges' cross products
-// (over 2^(64 - up)), the cofactors (over 2^62), and its velocity differences and
-// edges. A component of a cross product is in the other two coordinates' units,
+// the face vectors, the volume's V x W, the edges' cross products (over
+// 2^(64 - up)), the cofactors, and its velocity differences and edges. A component of a cross product is in the other two coordinates' units,
 // a triple product in all three, whichever the component.
 struct KinLane {
   double x[8], v[8];
   int s, sv, all;  // scales of this coordinate's positions and velocities; sum of the three positions'
+  int thinner;     // the thinnest coordinate's scale over this one's, up to 63
+  int least;       // the least determinant is kMinDet 2^least
   int up[3];
   bool ok_x, ok;  // positions taken; positions and velocities taken
   i64 g[12], w[3], vw[3];
@@ -52,17 +53,13 @@ struct KinLane {
   Num half_eta;
 };
 
-// a^2 over 2^61; all four limb products, as the squares of the low limbs do
+// a^2 over 2^B; all four limb products, as the squares of the low limbs do
 // not average out
+template <int B>
 LULESH_FX i64 square(Num a) {
   const i64 h = mulw(a.hi, a.hi), m = mulw(a.hi, a.lo);
   const u64 l = (u64)mulw(a.lo, a.lo);
-  return shl(h, 3) + ((m + (i64)(l >> 33)) >> 28);
-}
-
-// The positions' scales.
-LULESH_FX Scales kin_scales(Slots sh) {
-  return scales_of((unsigned)sh[KS_EXT].lo, (unsigned)sh[KS_EXT + 1].lo, (unsigned)sh[KS_EXT + 2].lo);
+  return shl(h, 64 - B) + ((m + (i64)(l >> 33)) >> (B - 33));
 }
 
 // 1: r.x and r.v hold coordinate k's corner values.
@@ -82,9 +79,11 @@ LULESH_FX void kin_edges(int k, Slots sh, double half_dt, KinLane& r) {
   const Num m0 = sh[KS_EXT], m1 = sh[KS_EXT + 1], m2 = sh[KS_EXT + 2];
   const int ex = exponent_field(umax(umax((unsigned)m0.lo, (unsigned)m1.lo), (unsigned)m2.lo));
   r.ok_x = ex >= kMinExtent && ex <= kMaxExtent;
-  const Scales s = kin_scales(sh);
+  const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo);
   r.s = k == 0 ? s.s[0] : k == 1 ? s.s[1] : s.s[2];
   r.all = s.s[0] + s.s[1] + s.s[2];
+  r.thinner = imin(s.thin() - r.s, 63);
+  r.least = s.least();
   int ev[3] = {exponent_field((unsigned)m0.hi), exponent_field((unsigned)m1.hi), exponent_field((unsigned)m2.hi)};
   const bool wild = imax(ev[0], imax(ev[1], ev[2])) > kMaxSpeed;  // not finite, or far beyond any flow
   int fastest = kNoExponent;
@@ -128,8 +127,7 @@ LULESH_FX void kin_products(int k, Slots sh, KinLane& r) {
     return take<0>(mul_minus(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]));
   };
   LULESH_UNROLL
-  for (int f = 0; f < 6; ++f)
-    r.n[f] = take<2>(mul_minus(sh[i1 + 2 * f], sh[i2 + 2 * f + 1], sh[i2 + 2 * f], sh[i1 + 2 * f + 1]));
+  for (int f = 0; f < 6; ++f) r.n[f] = cross_k(2 * f, 2 * f + 1);
   // V x W of the three products: (-g7, g0), (g10, -g9), (g4, g2)
   r.gU[0] = cross_k(0, 7);
   r.gU[1] = cross_k(9, 10);
@@ -139,7 +137,7 @@ LULESH_FX void kin_products(int k, Slots sh, KinLane& r) {
   for (int d = 0; d < 3; ++d) {
     const int a = 12 + (d + 1) % 3, b = 12 + (d + 2) % 3;
     r.A[d] = take_all(mul_minus_full(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]), r.up[d]);
-    r.C[d] = take<2>(mul_minus(sh[i1 + a + 3], sh[i2 + b + 3], sh[i2 + a + 3], sh[i1 + b + 3]));
+    r.C[d] = cross_k(a + 3, b + 3);
   }
   sh.put(KS_DET + k, product(limbs(r.w[1]), limbs(r.A[1] >> r.up[1])));
 }
@@ -155,70 +153,61 @@ LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
     sh.put(at + SUM_VOLUME, take<2>(a));
   }
   // (of the faces only the largest counts: they take the largest unit)
-  const int thinner = imin(kin_scales(sh).thin() - r.s, 63), two = r.all - r.s;
   LULESH_UNROLL
-  for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square(limbs(r.n[f] >> thinner)));
+  for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square<57>(limbs(r.n[f] >> r.thinner)));
   // The terms of the other sums differ in scale by coordinate: each is brought
   // to 2^60 and carries its exponent, and the sum takes the largest's.
-  int e[7];
-  auto put_term = [&](int i, i64 t, int shift, int& expo) {
+  const int two = r.all - r.s;
+  auto put_term = [&](int i, i64 t, int shift) {
     const int c = room(t);
     sh.put(at + i, shl(t, c));
-    expo = t != 0 ? -(r.sv + two + shift + c) : kNoTerm;
+    return t != 0 ? -(r.sv + two + shift + c) : kNoTerm;
   };
   Acc rate = {0, 0};
   LULESH_UNROLL
   for (int d = 0; d < 3; ++d) {
     const Num a = limbs(r.A[d]), u = limbs(r.vw[d]), c = limbs(r.C[d]);
-    sh.put(at + SUM_AREA + d, square(a));
-    e[4 + d] = r.A[d] != 0 ? -2 * (two + r.up[d]) : kNoTerm;
+    sh.put(at + SUM_AREA + d, square<61>(a));
+    Num e;
+    e.hi = r.A[d] != 0 ? -2 * (two + r.up[d]) : kNoTerm;
     Acc flow = {0, 0};
     mac_full(flow, a, u);
-    put_term(SUM_FLOW + d, take<3>(flow), r.up[d], e[d]);
+    e.lo = put_term(SUM_FLOW + d, take<3>(flow), r.up[d]);
+    sh[at + SUM_EXPO + d] = e;
     mac_full(rate, c, u);
   }
-  put_term(SUM_RATE, take<1>(rate), 0, e[3]);
-  Num x;
-  x.lo = (e[0] & 0xffff) | (int)((unsigned)e[1] << 16);
-  x.hi = (e[2] & 0xffff) | (int)((unsigned)e[3] << 16);
-  sh[at + SUM_EXPO] = x;
-  x.lo = (e[4] & 0xffff) | (int)((unsigned)e[5] << 16);
-  x.hi = e[6];
-  sh[at + SUM_EXPO + 1] = x;
+  Num e;
+  e.lo = put_term(SUM_RATE, take<3>(rate), 0);
+  e.hi = 0;
+  sh[at + SUM_EXPO + 3] = e;
   Acc jac = {0, 0};
   mac_full(jac, r.half_eta, limbs(r.C[1]));
-  sh.put(at + SUM_JAC, take<3>(jac));
+  sh.put(at + SUM_JAC, take<5>(jac));
 }
 
 LULESH_FX i64 kin_sum(Slots sh, int i) {
   return add(add(sh.get(KS_SUM + i), sh.get(KS_SUM + kSums + i)), sh.get(KS_SUM + 2 * kSums + i));
 }
 
-// the exponent of coordinate j's term of flow i, of the rate (i = 3) or of area i - 4
-LULESH_FX int kin_expo(Slots sh, int j, int i) {
-  const Num x = sh[KS_SUM + kSums * j + SUM_EXPO + (i >> 2)];
-  const int w = i & 2 ? x.hi : x.lo;
-  return i & 1 ? w >> 16 : (int)(short)w;
-}
-// the sum of those terms, times 2^k
-LULESH_FX double kin_aligned(Slots sh, int sum, int i, int k) {
-  const int e0 = kin_expo(sh, 0, i), e1 = kin_expo(sh, 1, i), e2 = kin_expo(sh, 2, i);
+// the sum of the terms with exponents e, times 2^k
+LULESH_FX double kin_aligned(Slots sh, int sum, int e0, int e1, int e2, int k) {
   const int top = imax(e0, imax(e1, e2));
   const i64 t = (sh.get(KS_SUM + sum) >> imin(top - e0, 63)) + (sh.get(KS_SUM + kSums + sum) >> imin(top - e1, 63)) +
                 (sh.get(KS_SUM + 2 * kSums + sum) >> imin(top - e2, 63));
   return to_double(t, k + top);
 }
+LULESH_FX Num kin_expo(Slots sh, int j, int d) { return sh[KS_SUM + kSums * j + SUM_EXPO + d]; }
 
 LULESH_FX i64 kin_determinant(Slots sh) { return sh.get(KS_DET) + sh.get(KS_DET + 1) + sh.get(KS_DET + 2); }
 
 // 5: whether the element is taken (by its determinant and volume too, over the
 // cube of its largest extent), and the sums in FP64 with their true scales.
 LULESH_FX bool kin_positions_taken(Slots sh, const KinLane& r) {
-  return r.ok_x && kin_determinant(sh) >= kin_scales(sh).least_determinant();
+  return r.ok_x && kin_determinant(sh) >= shl(kMinDet, r.least);
 }
 LULESH_FX void kin_accept(Slots sh, KinLane& r) {
   r.ok_x = kin_positions_taken(sh, r);
-  r.ok = r.ok && r.ok_x && kin_sum(sh, SUM_VOLUME) >= shl(kin_scales(sh).least_determinant(), 4);
+  r.ok = r.ok && r.ok_x && kin_sum(sh, SUM_VOLUME) >= shl(kMinDet, r.least + 4);
 }
 LULESH_FX double kin_volume12(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_VOLUME), 126 - r.all); }
 // the largest squared face vector and its place in the reference's face order
@@ -234,14 +223,20 @@ LULESH_FX double kin_largest_face(Slots sh, const KinLane& r, int& place) {
       place = q;
     }
   }
-  return to_double(best, 185 - 2 * (r.all - kin_scales(sh).thin()));
+  return to_double(best, 185 - 2 * (r.all - r.s - r.thinner));
 }
-LULESH_FX double kin_area(Slots sh, const KinLane&, int d) { return kin_aligned(sh, SUM_AREA + d, 4 + d, 197); }
-LULESH_FX double kin_flow(Slots sh, const KinLane&, int d) { return kin_aligned(sh, SUM_FLOW + d, d, 131); }
-LULESH_FX double kin_rate(Slots sh, const KinLane&) { return kin_aligned(sh, SUM_RATE, 3, 131); }
+LULESH_FX double kin_area(Slots sh, const KinLane&, int d) {
+  return kin_aligned(sh, SUM_AREA + d, kin_expo(sh, 0, d).hi, kin_expo(sh, 1, d).hi, kin_expo(sh, 2, d).hi, 197);
+}
+LULESH_FX double kin_flow(Slots sh, const KinLane&, int d) {
+  return kin_aligned(sh, SUM_FLOW + d, kin_expo(sh, 0, d).lo, kin_expo(sh, 1, d).lo, kin_expo(sh, 2, d).lo, 131);
+}
+LULESH_FX double kin_rate(Slots sh, const KinLane&) {
+  return kin_aligned(sh, SUM_RATE, kin_expo(sh, 0, 3).lo, kin_expo(sh, 1, 3).lo, kin_expo(sh, 2, 3).lo, 131);
+}
 // coordinate k's part of it
 LULESH_FX double kin_own_rate(Slots sh, const KinLane&, int k) {
-  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 131 + kin_expo(sh, k, 3));
+  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 131 + kin_expo(sh, k, 3).lo);
 }
 LULESH_FX double kin_jacobian(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_JAC), 129 - r.all); }
 

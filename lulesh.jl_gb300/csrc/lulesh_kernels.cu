@@ -364,11 +364,11 @@ struct FixedTaped {
   const fx::KinLane& r;
   __device__ double w(int a) const { return fx::to_double(r.w[a], 2 - r.s); }
   __device__ double vw(int a) const { return fx::to_double(r.vw[a], 2 - r.sv); }
-  __device__ double C(int a) const { return fx::to_double(r.C[a], 66 - (r.all - r.s)); }
+  __device__ double C(int a) const { return fx::to_double(r.C[a], 68 - (r.all - r.s)); }
   __device__ double A(int a) const { return fx::to_double(r.A[a], 68 - r.up[a] - (r.all - r.s)); }
   __device__ double gU(int a) const { return fx::to_double(r.gU[a], 64 - (r.all - r.s)); }
   __device__ double g(int q) const { return fx::to_double(r.g[q], -r.s); }
-  __device__ double n(int f) const { return fx::to_double(r.n[f], 62 - (r.all - r.s)); }
+  __device__ double n(int f) const { return fx::to_double(r.n[f], 64 - (r.all - r.s)); }
 };
 struct RealSums {
   const KinSums& s;
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(3 * kFixedElems) k_tape_geometry(const __grid_
 #pragma unroll
   for (int q = 0; q < 12; ++q) g[q] = fx::to_double(r.g[q], -r.s);
 #pragma unroll
-  for (int f = 0; f < 5; ++f) n[f] = fx::to_double(r.n[f], 62 - (r.all - r.s));
+  for (int f = 0; f < 5; ++f) n[f] = fx::to_double(r.n[f], 64 - (r.all - r.s));
   if (__syncthreads_or(live && !taken)) {
     KinSums sums;
     KinTaped t;
