@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     }
     const int eg = fx::exponent_field(top);
     top = 0;
-    ok = eg >= fx::kMinExtent && eg <= fx::kMaxExtent;
+    ok = eg >= fx::wide().least_extent && eg <= 1023 + 40;
     sg = 1081 - eg;  // below 2^59
 #pragma unroll
     for (int d = 0; d < 3; ++d) {

@@ -24,9 +24,8 @@
 // Error: a difference 2^-61 of the coordinate's extent, a cross product's component
 // about 2^-57 of the product of the other two's, the volume about 2^-56 of the
 // product of all three, each at or below what the FP64 expressions leave (tested
-// beside them). Elements whose Jacobian determinant is below kMinDet of the cube of
-// the largest extent (thin, inverted, not finite, or of a size no mesh here has)
-// are left to the FP64 expressions by the callers.
+// beside them). What is inverted, flat, not finite or of a size no mesh has is left
+// to the FP64 expressions by the callers (Range).
 //
 // Everything here also compiles for the host, where the tests compare it with
 // exact rational arithmetic.
@@ -42,8 +41,10 @@
 #endif
 #ifdef __CUDA_ARCH__
 #define LULESH_UNROLL _Pragma("unroll")
+#define LULESH_ROLLED _Pragma("unroll 1")
 #else
 #define LULESH_UNROLL
+#define LULESH_ROLLED
 #endif
 
 namespace lulesh {
@@ -183,11 +184,12 @@ LULESH_FX int room(i64 x) {
   const int h = (int)(x >> 32);
   return imax(leading_zeros((unsigned)(h ^ (h >> 31))) - 3, 0);
 }
+LULESH_FX i64 take_up(Acc a, int B) { return shl(a.h, B) + (a.m >> (32 - B)); }
 // The accumulated sum over 2^(64 - B), B as large as it stays below 2^61 with:
 // a component far below the others of its vector keeps its bits.
 LULESH_FX i64 take_all(Acc a, int& B) {
   B = room(take<0>(a));
-  return shl(a.h, B) + (a.m >> (32 - B));
+  return take_up(a, B);
 }
 // --- conversions ------------------------------------------------------------
 // Exponent field of a bound on the extent of eight doubles, from their high
@@ -259,38 +261,53 @@ LULESH_FX Float to_float(double x) {
 }
 
 // --- scale of an element ------------------------------------------------------
-// kMinDet: the Jacobian determinant (of the mean edges, which are the extents
-// of an undistorted element) over the cube of the scale's 2^61. An undistorted
-// cube has 2^52 to 2^55 by where its extent lies in [2^60, 2^61); the bound is
-// a volume of 1/32 to 1/256 of the element's bounding box. There the
-// fixed-point volume's error (0.2 units of 12 * 2^47) meets that of the FP64
-// expressions, 2^-53. A blast's shocked elements hold 0.09 of their boxes.
-constexpr i64 kMinDet = 1ll << 47;
-// extents from 2^-12 (where the guards 1e-36 added to squared areas and to
-// volumes are still below half a unit of them) to 2^40
-constexpr int kMinExtent = 1023 - 12, kMaxExtent = 1023 + 40;
+// Which elements the fixed-point form takes. Extents: exponent fields of the
+// least and most an element's largest extent may be. det: the least Jacobian
+// determinant (of the mean edges, which are the extents of an undistorted element;
+// an undistorted box has 2^52 to 2^55 of its scale, by where its extents lie in
+// [2^60, 2^61)), over the box or over the cube of the largest extent. distortion: the
+// powers of two the hourglass base vectors may outgrow their scale by.
+struct Range {
+  int least_extent, most_extent;
+  int det;
+  bool over_cube;
+  int distortion;
+};
+// Where every sum is within a few units of 2^-47 of its own size: extents for
+// which the guards 1e-36 added to squared areas and to volumes are below half a
+// unit, volumes above 1/32 to 1/256 of the cube.
+LULESH_FX constexpr Range narrow() { return {1023 - 12, 1023 + 40, 47, true, 4}; }
+// Where every sum is at least as good as the FP64 expressions leave it, whose errors
+// are relative to products over the box too. The kernels add the guards. Below
+// 2^-30 of its box not even FP64 tells a volume from its rounding; those elements
+// (and inverted, flat or non-finite ones) are left to the FP64 form, whose
+// errors the step reports. Plates and needles of aspect 1:100 and meshes of edges
+// below 2^-12, which the narrow range refuses, take 0.66 ms per cycle at 100^3 so;
+// both forms one after the other took 2.32, the FP64 kernels 1.81.
+LULESH_FX constexpr Range wide() { return {1023 - 100, 1023 + 100, 24, false, 31}; }
 // velocity extents below 2^-400 are taken as that: they move nothing
 constexpr int kMinSpeed = 1023 - 400, kMaxSpeed = 1023 + 400;
 
 LULESH_FX unsigned umax(unsigned a, unsigned b) { return a > b ? a : b; }
 
 // The scales s (x = X 2^-s) of an element's three coordinates, each its extent to
-// [2^60, 2^61); an extent below 2^-40 of the largest counts as that (no element
-// that thin is taken). A largest extent out of range shifts everything out.
+// [2^60, 2^61); an extent below 2^-60 of the largest counts as that. A largest
+// extent out of range shifts everything out.
 struct Scales {
   int s[3];
-  LULESH_FX int thin() const { return imax(s[0], imax(s[1], s[2])); }
+  bool ok;
   LULESH_FX int wide() const { return imin(s[0], imin(s[1], s[2])); }
-  // kMinDet, which is over the cube of the largest extent, is kMinDet 2^least() in
-  // the determinant's units (none reaches 2^58)
-  LULESH_FX int least() const { return imin(s[0] + s[1] + s[2] - 3 * wide(), 11); }
+  // the least determinant is 2^least(), in its own units (none reaches 2^58)
+  LULESH_FX int least(Range range) const {
+    return imin(range.det + (range.over_cube ? s[0] + s[1] + s[2] - 3 * wide() : 0), 58);
+  }
 };
-LULESH_FX Scales scales_of(unsigned hi0, unsigned hi1, unsigned hi2) {  // high words of the extents
-  Scales r = {{exponent_field(hi0), exponent_field(hi1), exponent_field(hi2)}};
+LULESH_FX Scales scales_of(unsigned hi0, unsigned hi1, unsigned hi2, Range range) {  // high words of the extents
+  Scales r = {{exponent_field(hi0), exponent_field(hi1), exponent_field(hi2)}, false};
   const int top = imax(r.s[0], imax(r.s[1], r.s[2]));
-  const bool ok = top >= kMinExtent && top <= kMaxExtent;
+  r.ok = top >= range.least_extent && top <= range.most_extent;
   LULESH_UNROLL
-  for (int j = 0; j < 3; ++j) r.s[j] = 1083 - (ok ? imax(r.s[j], top - 40) : 0x7ff);
+  for (int j = 0; j < 3; ++j) r.s[j] = 1083 - (r.ok ? imax(r.s[j], top - 60) : 0x7ff);
   return r;
 }
 

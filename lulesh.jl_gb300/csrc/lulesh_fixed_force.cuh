@@ -52,7 +52,8 @@ enum : int {
   FS_S = 98,
   FS_EXPO = 99,    // K.k and C.k; Sg.k and whether the scalars are in range
   FS_DET = 101,    // k: a term of the Jacobian determinant
-  FS_COUNT = 104
+  FS_SMALL = 104,  // k: bits used by the derivatives' high words, where the base vectors outgrow their scale
+  FS_COUNT = 107
 };
 
 // What a thread keeps over the phases.
@@ -60,7 +61,7 @@ struct ForceLane {
   double x[8];
   Num V[8];
   int ev, s, all, q;  // (s: this coordinate's scale, all: the sum of the three)
-  int least;          // the least determinant is kMinDet 2^least
+  int least;          // the least determinant is 2^least
   bool ok;
   i64 w1;
   Num B[4], B0;
@@ -101,15 +102,13 @@ LULESH_FX void force_stress(Slots sh, double s8) {
 }
 
 // 2: the coordinate's diagonals, U vectors, mean edges and hourglass modes.
-LULESH_FX void force_diagonals(int k, Slots sh, ForceLane& r, i64 hm[4]) {
+LULESH_FX void force_diagonals(int k, Slots sh, ForceLane& r, i64 hm[4], Range range = narrow()) {
   const Num m0 = sh[FS_EXT], m1 = sh[FS_EXT + 1], m2 = sh[FS_EXT + 2];
-  const int ex = exponent_field(umax(umax((unsigned)m0.lo, (unsigned)m1.lo), (unsigned)m2.lo));
-  r.ok = ex >= kMinExtent && ex <= kMaxExtent && (m0.hi | m1.hi | m2.hi) == 0 && sh[FS_EXPO].hi != 1 << 20 &&
-         sh[FS_EXPO + 1].hi != 0;
-  const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo);
+  const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo, range);
+  r.ok = s.ok && (m0.hi | m1.hi | m2.hi) == 0 && sh[FS_EXPO].hi != 1 << 20 && sh[FS_EXPO + 1].hi != 0;
   r.s = k == 0 ? s.s[0] : k == 1 ? s.s[1] : s.s[2];
   r.all = s.s[0] + s.s[1] + s.s[2];
-  r.least = s.least();
+  r.least = s.least(range);
   i64 v[8], g[12], w[3];
   LULESH_UNROLL
   for (int c = 0; c < 8; ++c) v[c] = to_fixed(r.x[c], r.s - 1075);
@@ -152,11 +151,13 @@ LULESH_FX void force_diagonals(int k, Slots sh, ForceLane& r, i64 hm[4]) {
 // 2^(q - 58) of the base vectors. The scale's exponent L is taken as a left
 // shift of the modes as far as they leave room (below 2^61) and, up to 4
 // places, of the product; q is 0 unless the distortion needs more, and more
-// than 4 is left to the FP64 form. A derivative is at most 3 E^2 (its bilinear
+// than the range has is left to the FP64 form. A derivative is at most 3 E^2 (its bilinear
 // form over the corners of a box), below 2^59.6, so the base vectors stay
-// below 2^59.8.
+// below 2^59.8. Where q is not 0, what the derivatives leave of that is taken off it
+// in phase 4: a slender element's are as far below its box's areas as its base
+// vectors' terms are above their scale.
 template <int MODE, class Tape>
-LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Tape tape) {
+LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Tape tape, Range range = narrow()) {
   const int i1 = FS_GEO + 18 * (k == 2 ? 0 : k + 1), i2 = FS_GEO + 18 * (k == 0 ? 2 : k - 1);
   auto cross_k = [&](int a, int b) {
     return take<0>(mul_minus(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]));
@@ -191,12 +192,20 @@ LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Ta
   sh.put(FS_DET + k, product(limbs(r.w1), limbs(cross_k(17, 15))));
 
   const Num expo = sh[FS_EXPO];
-  const unsigned used = (unsigned)(sh[FS_USED].lo | sh[FS_USED + 1].lo | sh[FS_USED + 2].lo);
-  const int room = leading_zeros(used) - 3, L = expo.lo + 252 - r.all;
+  const unsigned modes_used = (unsigned)(sh[FS_USED].lo | sh[FS_USED + 1].lo | sh[FS_USED + 2].lo);
+  const int room = leading_zeros(modes_used) - 3, L = expo.lo + 252 - r.all;
   r.q = imax(L - (room + 4), 0);
-  r.ok = r.ok && L >= 0 && r.q <= 4;
+  r.ok = r.ok && L >= 0 && r.q <= range.distortion;
   r.q = r.ok ? r.q : 0;
   const int Lq = r.ok ? L - r.q : 0, left = imin(Lq, room), rest = Lq - left;
+  if (r.q > 0) {
+    Num small = {0, 0};
+    for (int n = 0; n < 8; ++n) {
+      const int h = sh[FS_DV + 12 * k + n].hi;
+      small.lo |= h ^ (h >> 31);
+    }
+    sh[FS_SMALL + k] = small;
+  }
   const Num kl = limbs(sh.get(FS_K));
   LULESH_UNROLL
   for (int m = 0; m < 4; ++m) {
@@ -208,16 +217,28 @@ LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Ta
 
 // 4: every third entry of the base vectors, gamma - sum_k derivative_k mode_k.
 LULESH_FX void force_base(int k, Slots sh, ForceLane& r) {
-  r.ok = r.ok && sh.get(FS_DET) + sh.get(FS_DET + 1) + sh.get(FS_DET + 2) >= shl(kMinDet, r.least);
+  r.ok = r.ok && sh.get(FS_DET) + sh.get(FS_DET + 1) + sh.get(FS_DET + 2) >= shl(1, r.least);
+  int up = 0;
+  if (r.q > 0) {
+    const int used = sh[FS_SMALL].lo | sh[FS_SMALL + 1].lo | sh[FS_SMALL + 2].lo;
+    up = imin(imax(leading_zeros((unsigned)used) - 3, 0), r.q);
+    r.q -= up;
+  }
   const i64 one = 1ll << (58 - r.q);
-  LULESH_UNROLL
-  for (int j = 0; j < 11; ++j) {
-    const int i = 3 * j + k, n = (i >> 2) & 7, m = i & 3;
+  auto entry = [&](int i, auto take_sum) {
+    const int n = (i >> 2) & 7, m = i & 3;
     Acc a = mul(sh[FS_DV + n], sh[FS_DV + 8 + m]);
     mac(a, sh[FS_DV + 12 + n], sh[FS_DV + 20 + m]);
     mac(a, sh[FS_DV + 24 + n], sh[FS_DV + 32 + m]);
-    const Num g = limbs(((kGammaSigns >> (i & 31)) & 1u ? -one : one) - take<0>(a));
+    const Num g = limbs(((kGammaSigns >> (i & 31)) & 1u ? -one : one) - take_sum(a));
     if (i < 32) sh[FS_HG + i] = g;
+  };
+  if (up == 0) {
+    LULESH_UNROLL
+    for (int j = 0; j < 11; ++j) entry(3 * j + k, [](const Acc& a) { return take<0>(a); });
+  } else {
+    LULESH_ROLLED
+    for (int j = 0; j < 11; ++j) entry(3 * j + k, [&](const Acc& a) { return take_up(a, up); });
   }
 }
 

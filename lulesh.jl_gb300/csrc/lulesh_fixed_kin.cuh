@@ -25,41 +25,44 @@ enum : int {
 // sums over the coordinates
 enum : int {
   SUM_VOLUME = 0,  // 12 volume over 2^62
-  SUM_FACE = 1,    // 6: squared face vectors over 2^57, force order
+  SUM_FACE = 1,    // 6: squared face vectors over 2^61, force order
   SUM_AREA = 7,    // 3: squared cross products of the mean edges over 2^61
   SUM_FLOW = 10,   // 3: those cross products times velocity differences
   SUM_RATE = 13,   // cofactors times velocity differences
-  SUM_JAC = 14,    // half-step determinant over 2^59
-  SUM_EXPO = 15,   // 4: exponents of flow d (low word) and area d (high word), the last the rate's
+  SUM_JAC = 14,    // half-step determinant
+  SUM_EXPO = 15,   // 4: exponents of flow d (low word) and area d (high word), then the rate's and the faces'
   kSums = 19
 };
 // exponent of a term that is exactly zero
 constexpr int kNoTerm = -16384;
+// places the largest cofactor may leave free above it (of the 60 that hold it)
+constexpr int kFewBits = 5;
 static_assert(3 * kSums <= KS_DET, "the sums overlay the diagonals");
 
 // What a thread keeps over the phases: its components (unscaled integers) of
 // the face vectors, the volume's V x W, the edges' cross products (over
-// 2^(64 - up)), the cofactors, and its velocity differences and edges. A component of a cross product is in the other two coordinates' units,
+// 2^(64 - up)), the cofactors (over 2^(64 - cup)), and its velocity differences and
+// edges. A component of a cross product is in the other two coordinates' units,
 // a triple product in all three, whichever the component.
 struct KinLane {
   double x[8], v[8];
   int s, sv, all;  // scales of this coordinate's positions and velocities; sum of the three positions'
-  int thinner;     // the thinnest coordinate's scale over this one's, up to 63
-  int least;       // the least determinant is kMinDet 2^least
-  int up[3];
+  int least;       // the least determinant is 2^least
+  int up[3], cup;
+  i64 eta;  // the eta cofactor by itself; with half_eta 2^eup times the determinant's term
+  int eup;
   bool ok_x, ok;  // positions taken; positions and velocities taken
   i64 g[12], w[3], vw[3];
   i64 n[6], gU[3], A[3], C[3];
   Num half_eta;
 };
 
-// a^2 over 2^B; all four limb products, as the squares of the low limbs do
+// a^2 over 2^61; all four limb products, as the squares of the low limbs do
 // not average out
-template <int B>
 LULESH_FX i64 square(Num a) {
   const i64 h = mulw(a.hi, a.hi), m = mulw(a.hi, a.lo);
   const u64 l = (u64)mulw(a.lo, a.lo);
-  return shl(h, 64 - B) + ((m + (i64)(l >> 33)) >> (B - 33));
+  return shl(h, 3) + ((m + (i64)(l >> 33)) >> 28);
 }
 
 // 1: r.x and r.v hold coordinate k's corner values.
@@ -75,15 +78,13 @@ LULESH_FX void kin_extents(int k, Slots sh, const KinLane& r) {
 // velocities have their own scale: a thin element keeps its thin direction's
 // bits, and in flow along one axis the others' differences, which alone make up
 // the monotonic-Q gradients across it, are as small as they please.
-LULESH_FX void kin_edges(int k, Slots sh, double half_dt, KinLane& r) {
+LULESH_FX void kin_edges(int k, Slots sh, double half_dt, KinLane& r, Range range = narrow()) {
   const Num m0 = sh[KS_EXT], m1 = sh[KS_EXT + 1], m2 = sh[KS_EXT + 2];
-  const int ex = exponent_field(umax(umax((unsigned)m0.lo, (unsigned)m1.lo), (unsigned)m2.lo));
-  r.ok_x = ex >= kMinExtent && ex <= kMaxExtent;
-  const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo);
+  const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo, range);
+  r.ok_x = s.ok;
   r.s = k == 0 ? s.s[0] : k == 1 ? s.s[1] : s.s[2];
   r.all = s.s[0] + s.s[1] + s.s[2];
-  r.thinner = imin(s.thin() - r.s, 63);
-  r.least = s.least();
+  r.least = s.least(range);
   int ev[3] = {exponent_field((unsigned)m0.hi), exponent_field((unsigned)m1.hi), exponent_field((unsigned)m2.hi)};
   const bool wild = imax(ev[0], imax(ev[1], ev[2])) > kMaxSpeed;  // not finite, or far beyond any flow
   int fastest = kNoExponent;
@@ -137,8 +138,26 @@ LULESH_FX void kin_products(int k, Slots sh, KinLane& r) {
   for (int d = 0; d < 3; ++d) {
     const int a = 12 + (d + 1) % 3, b = 12 + (d + 2) % 3;
     r.A[d] = take_all(mul_minus_full(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]), r.up[d]);
-    r.C[d] = cross_k(a + 3, b + 3);
+    if (d != 1) r.C[d] = cross_k(a + 3, b + 3);
   }
+  // The determinant's factors keep all their bits; of the cofactors only the
+  // largest count, but a slender element's are far below its box's areas.
+  r.eta = take_all(mul_minus_full(sh[i1 + 17], sh[i2 + 15], sh[i2 + 17], sh[i1 + 15]), r.eup);
+  r.cup = imin(r.eup, imin(room(r.C[0]), room(r.C[2])));
+  if (r.cup <= kFewBits) {
+    r.cup = 0;
+  } else {
+    LULESH_UNROLL
+    for (int d = 0; d < 3; d += 2) {
+      const int a = 15 + (d + 1) % 3, b = 15 + (d + 2) % 3;
+      r.C[d] = take_up(mul_minus_full(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]), r.cup);
+    }
+  }
+  r.C[1] = r.eta >> (r.eup - r.cup);
+  const i64 h = add(shl((i64)r.half_eta.hi, 32), (i64)r.half_eta.lo);
+  const int thin = room(h);
+  r.half_eta = limbs(shl(h, thin));
+  r.eup += thin;
   sh.put(KS_DET + k, product(limbs(r.w[1]), limbs(r.A[1] >> r.up[1])));
 }
 
@@ -152,12 +171,23 @@ LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
     mac_full(a, limbs(r.g[3] + r.g[5]), limbs(r.gU[2]));
     sh.put(at + SUM_VOLUME, take<2>(a));
   }
-  // (of the faces only the largest counts: they take the largest unit)
-  LULESH_UNROLL
-  for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square<57>(limbs(r.n[f] >> r.thinner)));
   // The terms of the other sums differ in scale by coordinate: each is brought
-  // to 2^60 and carries its exponent, and the sum takes the largest's.
+  // to 2^60 and carries its exponent, and the sum takes the largest's. (Of the
+  // faces only the largest counts: a coordinate's six share an exponent.)
   const int two = r.all - r.s;
+  Num last;
+  {
+    unsigned used = 0;
+    LULESH_UNROLL
+    for (int f = 0; f < 6; ++f) {
+      const int h = (int)(r.n[f] >> 32);
+      used |= (unsigned)(h ^ (h >> 31));
+    }
+    const int c = imax(leading_zeros(used) - 3, 0);
+    LULESH_UNROLL
+    for (int f = 0; f < 6; ++f) sh.put(at + SUM_FACE + f, square(limbs(shl(r.n[f], c))));
+    last.hi = -2 * (two + c);
+  }
   auto put_term = [&](int i, i64 t, int shift) {
     const int c = room(t);
     sh.put(at + i, shl(t, c));
@@ -167,7 +197,7 @@ LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
   LULESH_UNROLL
   for (int d = 0; d < 3; ++d) {
     const Num a = limbs(r.A[d]), u = limbs(r.vw[d]), c = limbs(r.C[d]);
-    sh.put(at + SUM_AREA + d, square<61>(a));
+    sh.put(at + SUM_AREA + d, square(a));
     Num e;
     e.hi = r.A[d] != 0 ? -2 * (two + r.up[d]) : kNoTerm;
     Acc flow = {0, 0};
@@ -176,13 +206,12 @@ LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
     sh[at + SUM_EXPO + d] = e;
     mac_full(rate, c, u);
   }
-  Num e;
-  e.lo = put_term(SUM_RATE, take<3>(rate), 0);
-  e.hi = 0;
-  sh[at + SUM_EXPO + 3] = e;
+  last.lo = put_term(SUM_RATE, take<1>(rate), r.cup);
+  last.hi = (int)((unsigned)last.hi << 8) | r.eup;
+  sh[at + SUM_EXPO + 3] = last;
   Acc jac = {0, 0};
-  mac_full(jac, r.half_eta, limbs(r.C[1]));
-  sh.put(at + SUM_JAC, take<5>(jac));
+  mac_full(jac, r.half_eta, limbs(r.eta));
+  sh.put(at + SUM_JAC, take<3>(jac));
 }
 
 LULESH_FX i64 kin_sum(Slots sh, int i) {
@@ -200,30 +229,34 @@ LULESH_FX Num kin_expo(Slots sh, int j, int d) { return sh[KS_SUM + kSums * j + 
 
 LULESH_FX i64 kin_determinant(Slots sh) { return sh.get(KS_DET) + sh.get(KS_DET + 1) + sh.get(KS_DET + 2); }
 
-// 5: whether the element is taken (by its determinant and volume too, over the
-// cube of its largest extent), and the sums in FP64 with their true scales.
+// 5: whether the element is taken (by its determinant and volume too), and the
+// sums in FP64 with their true scales.
 LULESH_FX bool kin_positions_taken(Slots sh, const KinLane& r) {
-  return r.ok_x && kin_determinant(sh) >= shl(kMinDet, r.least);
+  return r.ok_x && kin_determinant(sh) >= shl(1, r.least);
 }
 LULESH_FX void kin_accept(Slots sh, KinLane& r) {
   r.ok_x = kin_positions_taken(sh, r);
-  r.ok = r.ok && r.ok_x && kin_sum(sh, SUM_VOLUME) >= shl(kMinDet, r.least + 4);
+  r.ok = r.ok && r.ok_x && kin_sum(sh, SUM_VOLUME) >= shl(1, r.least + 4);
 }
 LULESH_FX double kin_volume12(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_VOLUME), 126 - r.all); }
 // the largest squared face vector and its place in the reference's face order
 // (0, 5, 1, 2, 3, 4 of the force order)
 LULESH_FX double kin_largest_face(Slots sh, const KinLane& r, int& place) {
-  i64 best = kin_sum(sh, SUM_FACE);
+  const int e0 = kin_expo(sh, 0, 3).hi >> 8, e1 = kin_expo(sh, 1, 3).hi >> 8, e2 = kin_expo(sh, 2, 3).hi >> 8;
+  const int top = imax(e0, imax(e1, e2));
+  const int d0 = imin(top - e0, 63), d1 = imin(top - e1, 63), d2 = imin(top - e2, 63);
+  i64 best = -1;
   place = 0;
   LULESH_UNROLL
-  for (int q = 1; q < 6; ++q) {
-    const i64 a = kin_sum(sh, SUM_FACE + (q == 1 ? 5 : q - 1));
+  for (int q = 0; q < 6; ++q) {
+    const int f = SUM_FACE + (q == 0 ? 0 : q == 1 ? 5 : q - 1);
+    const i64 a = (sh.get(KS_SUM + f) >> d0) + (sh.get(KS_SUM + kSums + f) >> d1) + (sh.get(KS_SUM + 2 * kSums + f) >> d2);
     if (a > best) {
       best = a;
       place = q;
     }
   }
-  return to_double(best, 185 - 2 * (r.all - r.s - r.thinner));
+  return to_double(best, 189 + top);
 }
 LULESH_FX double kin_area(Slots sh, const KinLane&, int d) {
   return kin_aligned(sh, SUM_AREA + d, kin_expo(sh, 0, d).hi, kin_expo(sh, 1, d).hi, kin_expo(sh, 2, d).hi, 197);
@@ -232,13 +265,16 @@ LULESH_FX double kin_flow(Slots sh, const KinLane&, int d) {
   return kin_aligned(sh, SUM_FLOW + d, kin_expo(sh, 0, d).lo, kin_expo(sh, 1, d).lo, kin_expo(sh, 2, d).lo, 131);
 }
 LULESH_FX double kin_rate(Slots sh, const KinLane&) {
-  return kin_aligned(sh, SUM_RATE, kin_expo(sh, 0, 3).lo, kin_expo(sh, 1, 3).lo, kin_expo(sh, 2, 3).lo, 131);
+  return kin_aligned(sh, SUM_RATE, kin_expo(sh, 0, 3).lo, kin_expo(sh, 1, 3).lo, kin_expo(sh, 2, 3).lo, 133);
 }
 // coordinate k's part of it
 LULESH_FX double kin_own_rate(Slots sh, const KinLane&, int k) {
-  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 131 + kin_expo(sh, k, 3).lo);
+  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 133 + kin_expo(sh, k, 3).lo);
 }
-LULESH_FX double kin_jacobian(Slots sh, const KinLane& r) { return to_double(kin_sum(sh, SUM_JAC), 129 - r.all); }
+LULESH_FX double kin_jacobian(Slots sh, const KinLane& r) {
+  auto e = [&](int j) { return -(kin_expo(sh, j, 3).hi & 0xff); };
+  return kin_aligned(sh, SUM_JAC, e(0), e(1), e(2), 131 - r.all);
+}
 
 }  // namespace fx
 }  // namespace lulesh

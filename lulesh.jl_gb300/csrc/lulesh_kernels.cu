@@ -173,9 +173,9 @@ __global__ void __launch_bounds__(3 * kFixedElems, 7)
   }
   long long hm[4];
   __syncthreads();
-  fx::force_diagonals(k, sh, r, hm);
+  fx::force_diagonals(k, sh, r, hm, fx::wide());
   __syncthreads();
-  fx::force_products<MODE>(k, sh, r, hm, tape);
+  fx::force_products<MODE>(k, sh, r, hm, tape, fx::wide());
   __syncthreads();
   fx::force_base(k, sh, r);
   const int others = __syncthreads_or(live && !r.ok);
@@ -353,8 +353,7 @@ struct FixedSums {
   const fx::KinLane& r;
   __device__ double volume12() const { return fx::kin_volume12(sh, r); }
   __device__ double face(int& place) const { return fx::kin_largest_face(sh, r, place); }
-  // (of the size the fixed-point form takes, |A|^2 is far above 256*ptiny)
-  __device__ double area(int k) const { return fx::kin_area(sh, r, k); }
+  __device__ double area(int k) const { return fx::kin_area(sh, r, k) + 256.e-36; }
   __device__ double flow(int k) const { return fx::kin_flow(sh, r, k); }
   __device__ double rate() const { return fx::kin_rate(sh, r); }
   __device__ double jacobian() const { return fx::kin_jacobian(sh, r); }
@@ -364,7 +363,7 @@ struct FixedTaped {
   const fx::KinLane& r;
   __device__ double w(int a) const { return fx::to_double(r.w[a], 2 - r.s); }
   __device__ double vw(int a) const { return fx::to_double(r.vw[a], 2 - r.sv); }
-  __device__ double C(int a) const { return fx::to_double(r.C[a], 68 - (r.all - r.s)); }
+  __device__ double C(int a) const { return fx::to_double(r.C[a], 68 - r.cup - (r.all - r.s)); }
   __device__ double A(int a) const { return fx::to_double(r.A[a], 68 - r.up[a] - (r.all - r.s)); }
   __device__ double gU(int a) const { return fx::to_double(r.gU[a], 64 - (r.all - r.s)); }
   __device__ double g(int q) const { return fx::to_double(r.g[q], -r.s); }
@@ -453,7 +452,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 8)
   }
   fx::kin_extents(k, sh, r);
   __syncthreads();
-  fx::kin_edges(k, sh, 0.5 * dt, r);
+  fx::kin_edges(k, sh, 0.5 * dt, r, fx::wide());
   __syncthreads();
   fx::kin_products(k, sh, r);
   __syncthreads();
@@ -491,7 +490,7 @@ __global__ void __launch_bounds__(3 * kFixedElems) k_tape_geometry(const __grid_
   }
   fx::kin_extents(k, sh, r);
   __syncthreads();
-  fx::kin_edges(k, sh, 0.0, r);
+  fx::kin_edges(k, sh, 0.0, r, fx::wide());
   __syncthreads();
   fx::kin_products(k, sh, r);
   __syncthreads();

@@ -104,9 +104,9 @@ __global__ void __launch_bounds__(3 * kFixedElems) k_static_corner_forces(lulesh
   fx::force_load(k, sh, v, r);
   long long hm[4];
   __syncthreads();
-  fx::force_diagonals(k, sh, r, hm);
+  fx::force_diagonals(k, sh, r, hm, fx::wide());
   __syncthreads();
-  fx::force_products<MODE>(k, sh, r, hm, NoTape{});
+  fx::force_products<MODE>(k, sh, r, hm, NoTape{}, fx::wide());
   __syncthreads();
   fx::force_base(k, sh, r);
   const int others = __syncthreads_or(live && !r.ok);

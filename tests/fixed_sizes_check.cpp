@@ -97,6 +97,27 @@ void fp64_forces(const double p[3][8], const double v[3][8], double vi12, double
   }
 }
 
+// fixed_forces over either range
+bool ranged_forces(const double p[3][8], const double vel[3][8], double vi12, double coef, double s8, Range range,
+                   double f[3][8]) {
+  Num column[FS_COUNT];
+  const Slots sh{column, 1};
+  ForceLane r[3];
+  i64 hm[3][4];
+  for (int k = 0; k < 3; ++k) {
+    for (int c = 0; c < 8; ++c) r[k].x[c] = p[k][c];
+    force_load(k, sh, vel[k], r[k]);
+  }
+  force_scales(sh, vi12, coef);
+  force_stress(sh, s8);
+  for (int k = 0; k < 3; ++k) force_diagonals(k, sh, r[k], hm[k], range);
+  for (int k = 0; k < 3; ++k) force_products<3>(k, sh, r[k], hm[k], NoTape{}, range);
+  for (int k = 0; k < 3; ++k) force_base(k, sh, r[k]);
+  if (r[0].ok != r[1].ok || r[0].ok != r[2].ok) std::abort();
+  for (int k = 0; k < 3 && r[0].ok; ++k) force_corners(k, sh, r[k], [&](int n, double v) { f[k][n] = v; }, NoTape{});
+  return r[0].ok;
+}
+
 // c = a x b, and p the sums of its products' magnitudes
 void cross(const Q a[3], const Q b[3], Q c[3], Q p[3]) {
   for (int k = 0; k < 3; ++k) {
@@ -115,8 +136,8 @@ extern "C" {
 // cofactor sum, the half-step determinant) want[10 i + j], the errors of the fixed-point
 // form and of the FP64 form, and the sum of the magnitudes of its products.
 // (Sums with velocities take 4 of the coordinate's velocity extent for a
-// difference, the size of its four body diagonals.)
-void check_sizes(int n, const double* pos, const double* vel, double half_dt, int* taken, double* want, double* fixed,
+// difference, the size of its four body diagonals.) kernels: over the kernels' range.
+void check_sizes(int kernels, int n, const double* pos, const double* vel, double half_dt, int* taken, double* want, double* fixed,
                  double* fp64, double* size) {
   for (int i = 0; i < n; ++i) {
     const double(*p)[8] = reinterpret_cast<const double(*)[8]>(pos + 24 * i);
@@ -131,7 +152,7 @@ void check_sizes(int n, const double* pos, const double* vel, double half_dt, in
       }
       kin_extents(k, sh, r[k]);
     }
-    for (int k = 0; k < 3; ++k) kin_edges(k, sh, half_dt, r[k]);
+    for (int k = 0; k < 3; ++k) kin_edges(k, sh, half_dt, r[k], kernels ? wide() : narrow());
     for (int k = 0; k < 3; ++k) kin_products(k, sh, r[k]);
     for (int k = 0; k < 3; ++k) kin_terms(k, sh, r[k]);
     for (int k = 0; k < 3; ++k) kin_accept(sh, r[k]);
@@ -225,7 +246,7 @@ void check_sizes(int n, const double* pos, const double* vel, double half_dt, in
 // taken, and for coordinate k the largest errors over the corners of the two forms,
 // and the size: |s8| times the magnitudes of the products of a corner's three
 // faces, plus |coef| times the coordinate's velocity extent.
-void check_force_sizes(int n, const double* pos, const double* vel, const double* scal, int* taken, double* fixed,
+void check_force_sizes(int kernels, int n, const double* pos, const double* vel, const double* scal, int* taken, double* fixed,
                        double* fp64, double* size) {
   static const int fd[6][4] = {{2, 0, 3, 1}, {5, 0, 1, 4}, {6, 1, 2, 5}, {7, 2, 3, 6}, {4, 3, 0, 7}, {6, 4, 5, 7}};
   for (int i = 0; i < n; ++i) {
@@ -233,7 +254,7 @@ void check_force_sizes(int n, const double* pos, const double* vel, const double
     const double(*v)[8] = reinterpret_cast<const double(*)[8]>(vel + 24 * i);
     const double vi12 = scal[3 * i], coef = scal[3 * i + 1], s8 = scal[3 * i + 2];
     double f[3][8], plain[3][8];
-    taken[i] = fixed_forces<3>(p, v, vi12, coef, s8, f, NoTape{});
+    taken[i] = ranged_forces(p, v, vi12, coef, s8, kernels ? wide() : narrow(), f);
     if (!taken[i]) continue;
     Q qf[3][8], qdv[3][8], qh[3][4], qS[3][4];
     exact_forces(p, v, vi12, coef, s8, 3, qf, qdv, qh, qS);

@@ -30,11 +30,11 @@ def lib(tmp_path_factory):
 
 @pytest.fixture(scope="module")
 def sums(lib):
-    def run(pos, vel, half_dt):
+    def run(pos, vel, half_dt, wide=False):
         n = len(pos)
         taken = np.zeros(n, np.int32)
         out = [np.zeros((n, 10)) for _ in range(4)]
-        lib.check_sizes(n, *(a.ctypes.data_as(ctypes.c_void_p) for a in (pos, vel)), ctypes.c_double(half_dt),
+        lib.check_sizes(int(wide), n, *(a.ctypes.data_as(ctypes.c_void_p) for a in (pos, vel)), ctypes.c_double(half_dt),
                         *(a.ctypes.data_as(ctypes.c_void_p) for a in (taken, *out)))
         return taken.astype(bool), *out  # want, errors of the fixed-point and the FP64 form, size
     return run
@@ -42,11 +42,11 @@ def sums(lib):
 
 @pytest.fixture(scope="module")
 def forces(lib):
-    def run(pos, vel, scal):
+    def run(pos, vel, scal, wide=False):
         n = len(pos)
         taken = np.zeros(n, np.int32)
         out = [np.zeros((n, 3)) for _ in range(3)]
-        lib.check_force_sizes(n, *(a.ctypes.data_as(ctypes.c_void_p) for a in (pos, vel, np.ascontiguousarray(scal), taken, *out)))
+        lib.check_force_sizes(int(wide), n, *(a.ctypes.data_as(ctypes.c_void_p) for a in (pos, vel, np.ascontiguousarray(scal), taken, *out)))
         return taken.astype(bool), *out  # errors of the fixed-point and the FP64 form, size
     return run
 
@@ -128,3 +128,53 @@ def test_forces_of_thin_elements(forces, h, axis, squash):
         taken, fixed, fp64, size = forces(pos, vel, scal)
         assert taken.all() if squash > 0.1 else taken.any()
         _no_further_off(fixed[taken], fp64[taken], size[taken], range(3))
+
+
+def _slender(seed, n, size, thin, rotated):
+    """Plates and needles (edges size and size * thin), jittered in their own
+    coordinates, some distance from the origin, along the axes or turned."""
+    r = np.random.default_rng(seed)
+    e = CUBE + 0.03 * r.uniform(-1, 1, (n, 3, 8)) + np.floor(r.uniform(0, 50, (n, 3, 1)))
+    few = r.integers(0, 3, n)
+    many = r.random(n) < 0.5
+    for i in range(n):
+        for k in range(3):
+            if (k == few[i]) == many[i]:
+                e[i, k] *= thin
+    if rotated:
+        q = np.linalg.qr(r.standard_normal((n, 3, 3)))[0]
+        q *= np.sign(np.linalg.det(q))[:, None, None]
+        e = q @ e
+    return np.ascontiguousarray(size * e), np.ascontiguousarray(r.uniform(-1, 1, (n, 3, 8)))
+
+
+@pytest.mark.parametrize("size", [2.0 ** -90, 1e-9, 1e-5, 0.01, 1e13, 2.0 ** 90])
+@pytest.mark.parametrize("thin", [1.0, 0.1, 1e-2, 1e-3])
+@pytest.mark.parametrize("rotated", [False, True])
+def test_the_kernels_range(sums, forces, size, thin, rotated):
+    """Plates, needles, and elements of any size are taken."""
+    pos, vel = _slender(6, 300, size, thin, rotated)
+    ext = (pos.max(2) - pos.min(2)).min(1)
+    taken, want, fixed, fp64, size_ = sums(pos, vel, 1e-3 * ext.min(), wide=True)
+    assert taken.all()
+    _no_further_off(fixed, fp64, size_, range(10))
+    scal = np.stack([1 / want[:, 0], np.full(300, -1.0), np.full(300, -1 / size / size)], 1)
+    taken, fixed, fp64, size_ = forces(pos, vel, scal, wide=True)
+    assert taken.all()
+    _no_further_off(fixed, fp64, size_, range(3))
+
+
+def test_what_the_kernels_range_refuses(sums, forces):
+    """Inverted, flat and non-finite elements, and extents beyond 2^100."""
+    pos, vel = _slender(7, 8, 0.01, 1.0, True)
+    pos[0] = pos[0, :, [4, 5, 6, 7, 0, 1, 2, 3]].T
+    pos[1, :, 4:] = pos[1, :, :4]
+    pos[2, 1, 3] = np.nan
+    pos[3, 0, 7] = np.inf
+    pos[4] *= 1e35
+    pos[5] *= 1e-35
+    vel[6, 2, 1] = np.inf
+    scal = np.tile([1.0, -1.0, -1.0], (8, 1))
+    assert sums(pos, vel, 1e-9, wide=True)[0].tolist() == [False] * 7 + [True]
+    scal[:, 0] = 1 / 12e-6
+    assert forces(pos, vel, scal, wide=True)[0].tolist() == [False] * 7 + [True]
