@@ -119,7 +119,7 @@ __device__ __noinline__ void force_fallback(const DevDomain& d, DevState* st, un
 // with the flags read in one load (one by one, past the first-level cache,
 // k_node's third flag cost 12 us at 150^3).
 template <int MODE, bool ENS, bool TAPE, bool TIME>
-__global__ void __launch_bounds__(3 * kFixedElems, 7)
+__global__ void __launch_bounds__(3 * kFixedElems, 8)
     k_force(const __grid_constant__ DevDomain d, const __grid_constant__ Params prm) {
   __shared__ fx::Num column[fx::FS_COUNT * kFixedElems];
   const int E = d.E;
@@ -423,7 +423,7 @@ __device__ __noinline__ void kin_fallback(const DevDomain& d, DevState* st, fx::
 // geometry). Eight blocks per SM, 80 registers: six (96) 0.67 ms, five (128)
 // 0.77 ms.
 template <bool AUX, bool ENS, bool TAPE>
-__global__ void __launch_bounds__(3 * kFixedElems, 8)
+__global__ void __launch_bounds__(3 * kFixedElems, 7)
     k_kinematics(const __grid_constant__ DevDomain d, const __grid_constant__ Params prm) {
   __shared__ fx::Num column[fx::KS_COUNT * kFixedElems];
   const int E = d.E;
