@@ -370,6 +370,19 @@ __device__ __forceinline__ void walsh_modes_t(const T t[4], T out[8]) {
 
 // A coefficient's mantissa in the unit 2^u of a sum, its own unit being 2^e.
 __device__ __forceinline__ fx::i64 in_unit(const fx::Float& f, int e, int u) { return f.m >> fx::imin(u - e, 63); }
+// The unit 2^k of a cross product's component whose two products have scales of
+// their own (2^-61 of their bounds): how far each is shifted to it.
+struct Unit {
+  int k, dp, dn;
+  __device__ __forceinline__ Unit() {}
+  // edge and vector scales of the positive and of the negative product
+  __device__ __forceinline__ Unit(int ep, int vp, int en, int vn) {
+    const int p = 61 - (ep + vp), n = 61 - (en + vn);
+    k = fx::imax(p, n);
+    dp = fx::imin(k - p, 63);
+    dn = fx::imin(k - n, 63);
+  }
+};
 // Whether a sum is in range: coefficients at most 2^400 (so not infinities or
 // NaN, top their largest exponent), and a unit whose values are doubles or none.
 __device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && (u < -2000 || u >= -950); }
@@ -392,8 +405,7 @@ __device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && 
 // The crosses onto the edges and the face diagonals, all of an edge, a diagonal
 // (or a sum of two) and an adjoint vector, and the sums onto the position corners
 // run on the integer pipes. Edges and diagonals are scaled by their coordinate's
-// extent 2^-sg[k], adjoint vectors by 2^-(sg[k] + common), so that both products
-// of a cross have one unit; what else joins the corners (edges, modes, V x W)
+// extent, adjoint vectors by their coordinate's largest; what else joins the corners (edges, modes, V x W)
 // enters as mantissas in the largest term's unit. Elements of sizes or adjoints
 // out of range take the crosses in doubles, the positions' part from the tape.
 // Bound by FP64 issue (350 slots per element, the pipe 71 % busy; ALU 29 %,
@@ -406,7 +418,7 @@ __device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && 
 // the edges' crosses there too: 95 us, 18.61 -> 18.29, 2.60 -> 2.60.
 enum : int {
   // per coordinate: mean edges, half-step edges, 12 diagonals, U vectors (limbs),
-  // the differences of dL/ddv along V and W, the faces' terms (by the face's
+  // the differences of dL/ddv along V and -W, the faces' terms (by the face's
   // first diagonal), Lv12 U + dU; then the adjoints of the edges' cross products
   // and of the cofactors (doubles, then limbs)
   KA_W = 0, KA_F = 3, KA_D = 6, KA_U = 18, KA_DV = 21, KA_DW = 24, KA_LN = 27, KA_A = 33,
@@ -518,9 +530,9 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     put(KA_DV, G[6] - G[3]);
     put(KA_DV + 1, G[6] - G[4]);
     put(KA_DV + 2, G[6] - G[1]);
-    put(KA_DW, G[2] - G[0]);
-    put(KA_DW + 1, G[7] - G[0]);
-    put(KA_DW + 2, G[5] - G[0]);
+    put(KA_DW, G[0] - G[2]);
+    put(KA_DW + 1, G[0] - G[7]);
+    put(KA_DW + 2, G[0] - G[5]);
     // The next cycle's stress force: face f's normal d1 x d2 with LN = s8 LU_f
     // gives d1 the adjoint d2 x LN and d2 the adjoint LN x d1; s8 from this
     // cycle's end state. Faces (d20, d31) (d50, d14) (d61, d25) (d72, d36) (d43,
@@ -589,26 +601,25 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     ok = ok && (top == 0 || (ea >= fx::kMinSpeed && ea <= fx::kMaxSpeed));
     num(KA_EXP + k).hi = ok ? 1081 - fx::imax(ea, fx::kMinSpeed) : fx::kNoExponent;  // below 2^59
   }
-  // the edges' adjoints in their units
+  // The edges' adjoints in their units. Each coordinate's adjoint vectors have a
+  // scale of their own: what a component's two coordinates hold may be far below
+  // what the third does.
+  const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
   bool ok_edges;
-  int uA, uC;
+  Unit unit_A, unit_C;
   {
     const int x0 = num(KA_EXP).lo, x1 = num(KA_EXP + 1).lo, x2 = num(KA_EXP + 2).lo;
-    auto least = [&](int shift) {
-      const int a0 = (x0 >> shift) & 0xfff, a1 = (x1 >> shift) & 0xfff, a2 = (x2 >> shift) & 0xfff;
-      return fx::imin(a0, fx::imin(a1, a2)) == 0
-                 ? fx::kNoExponent
-                 : fx::imin(a0 - (x0 & 0xff), fx::imin(a1 - (x1 & 0xff), a2 - (x2 & 0xff))) - 512;
-    };
-    const int cA = least(8), cC = least(20), both = (x0 & 0xff) + (x1 & 0xff) + (x2 & 0xff) - sg;
-    ok_edges = fx::imin(cA, cC) != fx::kNoExponent;
-    uA = 61 - (both + cA);
-    uC = 61 - (both + cC);
+    const int here = num(KA_EXP + k).lo, xp = num(KA_EXP + k1).lo, xq = num(KA_EXP + k2).lo;
+    auto scale = [](int x, int shift) { return ((x >> shift) & 0xfff) - 512; };
+    auto all = [&](int shift) { return (x0 >> shift & 0xfff) != 0 && (x1 >> shift & 0xfff) != 0 && (x2 >> shift & 0xfff) != 0; };
+    ok_edges = all(8) && all(20);
+    unit_A = Unit(xp & 0xff, scale(xq, 8), xq & 0xff, scale(xp, 8));
+    unit_C = Unit(xp & 0xff, scale(xq, 20), xq & 0xff, scale(xp, 20));
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       if (ok_edges) {
-        num(own + KA_LA + d) = fx::limbs(fx::to_fixed0(LA[d], sg + cA - 1075));
-        num(own + KA_LC + d) = fx::limbs(fx::to_fixed0(LC[d], sg + cC - 1075));
+        num(own + KA_LA + d) = fx::limbs(fx::to_fixed0(LA[d], scale(here, 8) - 1075));
+        num(own + KA_LC + d) = fx::limbs(fx::to_fixed0(LC[d], scale(here, 20) - 1075));
       } else {
         sh(own + KA_LA + d) = LA[d];
         sh(own + KA_LC + d) = LC[d];
@@ -616,20 +627,19 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     }
   }
   __syncthreads();
-  // scales: of an adjoint vector's component j sg[j] + common, of a cross's
-  // component k uc
-  int uc;
+  Unit unit;
   {
     const fx::Num x0 = num(KA_EXP), x1 = num(KA_EXP + 1), x2 = num(KA_EXP + 2);
+    const fx::Num mine = num(KA_EXP + k), xp = num(KA_EXP + k1), xq = num(KA_EXP + k2);
     ok = fx::imin(x0.hi, fx::imin(x1.hi, x2.hi)) != fx::kNoExponent;
-    const int s0 = x0.lo & 0xff, s1 = x1.lo & 0xff, s2 = x2.lo & 0xff;
-    const int common = fx::imin(x0.hi - s0, fx::imin(x1.hi - s1, x2.hi - s2));
-    uc = 61 - (s0 + s1 + s2 - sg + common);
+    unit = Unit(xp.lo & 0xff, xq.hi, xq.lo & 0xff, xp.hi);
     if (ok)
 #pragma unroll
-      for (int q = KA_DV; q < KA_LA; ++q) num(own + q) = fx::limbs(fx::to_fixed0(sh(own + q), sg + common - 1075));
+      for (int q = KA_DV; q < KA_LA; ++q) num(own + q) = fx::limbs(fx::to_fixed0(sh(own + q), mine.hi - 1075));
   }
-  // component k of sums of (slot i) x (slot j)
+  // component k of sums of crosses of an edge or diagonal (slot i) and an adjoint
+  // vector (slot j), or (minus) the other way round: the products of the edge's
+  // next component and the vector's after it have one scale, the others another
   struct Cross { fx::Acc p, n; };
   auto first = [&](int i, int j) {
     Cross r;
@@ -641,14 +651,12 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     fx::mac(r.p, num(c1 + i), num(c2 + j));
     fx::mac(r.n, num(c2 + i), num(c1 + j));
   };
-  auto value = [&](const Cross& r) {
-    fx::Acc d;
-    d.h = r.p.h - r.n.h;
-    d.m = r.p.m - r.n.m;
-    return fx::take<3>(d);
+  auto minus = [&](Cross& r, int i, int j) {
+    fx::msub(r.p, num(c1 + i), num(c2 + j));
+    fx::msub(r.n, num(c2 + i), num(c1 + j));
   };
+  auto value = [](const Cross& r, const Unit& u) { return (fx::take<3>(r.p) >> u.dp) - (fx::take<3>(r.n) >> u.dn); };
   // the same in doubles, the positions' slots from the tape
-  const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
   auto at = [&](int j, int i) {
     if (i >= KA_DV) return sh(KA_COMP * j + i);
     auto t = [&](int q) { return a.kin[row(q, E, e)]; };
@@ -666,11 +674,11 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
     const int b = (i + 1) % 3, c = (i + 2) % 3;  // P of c, Q of b
     if (ok_edges) {
       Cross r = first(KA_W + b, KA_LA + c);
-      plus(r, KA_LA + b, KA_W + c);
-      LW[i] = fx::to_double(value(r), uA);
+      minus(r, KA_W + c, KA_LA + b);
+      LW[i] = fx::to_double(value(r, unit_A), unit_A.k);
       r = first(KA_F + b, KA_LC + c);
-      plus(r, KA_LC + b, KA_F + c);
-      LF[i] = fx::to_double(value(r), uC);
+      minus(r, KA_F + c, KA_LC + b);
+      LF[i] = fx::to_double(value(r, unit_C), unit_C.k);
     } else {
       LW[i] = add_cross(add_cross(0.0, KA_W + b, KA_LA + c), KA_LA + b, KA_W + c);
       LF[i] = add_cross(add_cross(0.0, KA_F + b, KA_LC + c), KA_LC + b, KA_F + c);
@@ -739,19 +747,20 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
       const int v = iv[t], w = iw[t];
-      Cross r = first(KA_DV + t, KA_D + w);
+      // (the slots of dW hold -dW)
+      Cross r = first(KA_D + w, KA_DV + t);
       plus(r, KA_D + v, KA_DW + t);
-      const fx::i64 gU = value(r);
+      const fx::i64 gU = value(r, unit);
 #pragma unroll
-      for (int q = 6 + 2 * t; q < 8 + 2 * t; ++q) onto(q, gU + value(first(KA_LN + partner[q], KA_D + partner[q])));
+      for (int q = 6 + 2 * t; q < 8 + 2 * t; ++q) onto(q, -(gU + value(first(KA_D + partner[q], KA_LN + partner[q]), unit)));
       r = first(KA_D + w, KA_A + t);
-      plus(r, KA_DW + t, KA_U + t);
+      plus(r, KA_U + t, KA_DW + t);
       plus(r, KA_D + partner[v], KA_LN + v);
-      onto(v, value(r));
-      r = first(KA_A + t, KA_D + v);
-      plus(r, KA_U + t, KA_DV + t);
+      onto(v, value(r, unit));
+      r = first(KA_U + t, KA_DV + t);
+      minus(r, KA_D + v, KA_A + t);
       plus(r, KA_D + partner[w], KA_LN + w);
-      onto(w, value(r));
+      onto(w, value(r, unit));
     }
     // the other terms' mantissas below 2^58, ten to a corner
     fx::Float f[10];
@@ -761,7 +770,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
       f[q] = fx::to_float(q < 3 ? vw[q] : q < 6 ? LW[q - 3] : tm[q - 6]);
       top = fx::imax(top, f[q].k);
     }
-    const int u = fx::imax(uc, top + 3);
+    const int u = fx::imax(unit.k, top + 3);
     summed = good_sum(top, u);
     if (summed) {
       fx::i64 i[10], y[8];
@@ -772,12 +781,12 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
       walsh1_t(w, y);
 #pragma unroll
       for (int q = 6; q < 12; ++q) { y[pp[q]] += i[(q - 6) / 2]; y[pq[q]] -= i[(q - 6) / 2]; }
-      const int down = fx::imin(u - uc, 63);
+      const int down = fx::imin(u - unit.k, 63);
 #pragma unroll
       for (int c = 0; c < 8; ++c) LX[c] = fx::to_double((X[c] >> down) + y[c], u);
     } else {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) LX[c] = fx::to_double(X[c], uc);
+      for (int c = 0; c < 8; ++c) LX[c] = fx::to_double(X[c], unit.k);
     }
   } else {
 #pragma unroll
@@ -786,10 +795,10 @@ __global__ void __launch_bounds__(3 * kFixedElems, 6) ka_kinematics(AdjDev a, co
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
       const int v = iv[t], w = iw[t];
-      const double gU = add_cross(add_cross(0.0, KA_DV + t, KA_D + w), KA_D + v, KA_DW + t);
+      const double gU = add_cross(add_cross(0.0, KA_DV + t, KA_D + w), KA_DW + t, KA_D + v);
 #pragma unroll
       for (int q = 6 + 2 * t; q < 8 + 2 * t; ++q) onto(q, add_cross(gU, KA_LN + partner[q], KA_D + partner[q]));
-      onto(v, add_cross(add_cross(add_cross(0.0, KA_D + w, KA_A + t), KA_DW + t, KA_U + t), KA_D + partner[v], KA_LN + v));
+      onto(v, add_cross(add_cross(add_cross(0.0, KA_D + w, KA_A + t), KA_U + t, KA_DW + t), KA_D + partner[v], KA_LN + v));
       onto(w, add_cross(add_cross(add_cross(0.0, KA_A + t, KA_D + v), KA_U + t, KA_DV + t), KA_D + partner[w], KA_LN + w));
     }
   }

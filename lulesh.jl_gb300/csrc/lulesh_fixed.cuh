@@ -152,6 +152,10 @@ LULESH_FX void mac(Acc& r, Num a, Num b) {
   r.h = mad(a.hi, b.hi, r.h);
   r.m = mad(a.lo, b.hi, mad(a.hi, b.lo, r.m));
 }
+LULESH_FX void msub(Acc& r, Num a, Num b) {
+  r.h -= mulw(a.hi, b.hi);
+  r.m -= mad(a.lo, b.hi, mulw(a.hi, b.lo));
+}
 // with lo*lo too, for sums whose terms cancel or are far below their scale
 LULESH_FX void mac_full(Acc& r, Num a, Num b) {
   mac(r, a, b);
