@@ -163,9 +163,7 @@ __global__ void __launch_bounds__(3 * kFixedElems, 8)
       const double vol = d.v[e];
       const double rc = inv_cbrt(LDG(&d.volo[e]) * vol);
       const double coef = gt_zero(hgcoef) ? ((-hgcoef * 0.01) * d.ss[e]) * LDG(&d.elemMass[e]) * rc : 0.0;
-      // (a taped element without hourglass forces leaves its tape as it is)
-      const bool take = gt_zero(vol) && !(TAPE && !gt_zero(hgcoef));
-      fx::force_scales(sh, take ? (rc * rc) * (rc * (1.0 / 12.0)) : 0.0, coef);
+      fx::force_scales(sh, gt_zero(vol) ? (rc * rc) * (rc * (1.0 / 12.0)) : 0.0, coef);
     } else if (k == 1) {
       fx::force_stress(sh, ((-d.p[e]) - d.q[e]) * 0.125);
     }
