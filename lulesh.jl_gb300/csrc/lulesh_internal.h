@@ -6,6 +6,8 @@
 #include <cstring>
 #include <cuda_runtime.h>
 
+#include "lulesh_courant.cuh"
+
 namespace lulesh {
 
 // Boundary-condition masks, src/bc.jl:3-30.
@@ -65,12 +67,12 @@ struct Params {
   double u_cut, hgcoef, qstop, monoq_max_slope, monoq_limiter_mult, e_cut, p_cut, q_cut, v_cut;
   double qlc_monoq, qqc_monoq, qqc, eosvmax, eosvmin, pmin, emin, dvovmax, refdens;
   double dtfixed, deltatimemultlb, deltatimemultub, stoptime, dtmax;
-  // formed once on the host by finish_params: 1 / refdens, 64 qqc^2 (also as a
-  // float), twice the limiter's multiplier, the comparison
-  // keys (fkey) of the thresholds the element kernels test against, and
+  // formed once on the host by finish_params: 1 / refdens, 64 qqc^2, 8 |qqc| for the
+  // coarse comparison of Courant candidates, twice the limiter's multiplier, the
+  // comparison keys (fkey) of the thresholds the element kernels test against, and
   // whether eosvmin / eosvmax are set (nonzero)
   double inv_refdens, qqc2x64, monoq_mult2;
-  float qqc2x64f;
+  float qqc8;
   long long k_qstop, k_max_slope, k_eosvmin, k_eosvmax, k_pmin, k_emin;
   int has_eosvmin, has_eosvmax;
 };
@@ -91,7 +93,7 @@ inline long long fkey_host(double x) {
 inline void finish_params(Params& p) {
   p.inv_refdens = 1.0 / p.refdens;
   p.qqc2x64 = (64.0 * p.qqc) * p.qqc;
-  p.qqc2x64f = (float)p.qqc2x64;
+  p.qqc8 = coarse_qqc8(p.qqc);
   p.monoq_mult2 = 2.0 * p.monoq_limiter_mult;
   p.k_qstop = fkey_host(p.qstop);
   p.k_max_slope = fkey_host(p.monoq_max_slope);

@@ -16,6 +16,7 @@
 //                (src/domain.jl:2322-3064)
 // plus timeIncrement! (src/domain.jl:920-961) for the device-resident run loop,
 // in blocks of k_force or as k_time_increment.
+#include "lulesh_courant.cuh"
 #include "lulesh_device.cuh"
 #include "lulesh_element_fp64.cuh"
 #include "lulesh_fixed_force.cuh"
@@ -624,15 +625,6 @@ __device__ __forceinline__ void warp_limits_by_instance(Limits a, int inst, DevS
   }
 }
 
-// A non-negative double as a float, rounded down; 0 below the float range and
-// infinity above it. On the integer pipe (a conversion takes an FP64 slot).
-__device__ __forceinline__ float coarse(double x) {
-  const int h = __double2hiint(x);
-  if (h < 0x38100000) return 0.f;
-  if (h >= 0x47f00000) return __int_as_float(0x7f800000);
-  return __int_as_float(((h - 0x38000000) << 3) | (int)((unsigned)__double2loint(x) >> 29));
-}
-
 // An empty register move the compiler cannot see through: a value passed
 // through it must be recomputed from it.
 __device__ __forceinline__ void opaque(double& x) { asm volatile("" : "+d"(x)); }
@@ -898,9 +890,8 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
     if (le_zero(tmpV)) err |= ST_UPDATE;
 
     // ---- Courant and hydro constraints, src/domain.jl:2964-3054 ----
-    // A candidate that is certainly above the least so far is not formed: the
-    // estimate, in FP32 from rounded-down operands, is good to 1e-6, and what it
-    // compares with only falls. (dtf below 1e-30 leaves the float range.)
+    // A candidate that is certainly above the least so far is not formed (what it
+    // compares with only falls).
     double dtc = __longlong_as_double((long long)kInfBits), dth = dtc;
     if (!is_zero(vdov)) {
       const double arealg = d.arealg[i];
@@ -908,11 +899,8 @@ __global__ void __launch_bounds__(kMaxElemBlock) k_material(DevDomain d, Params 
       if (rate <= kInfBits) limits.rate = rate;  // (a NaN constrains nothing)
       bool skip = false;
       if (!TAPE) {
-        const float fa = coarse(arealg), fs = coarse(ss_new), fv = coarse(fabs(vdov));
-        float f = fs * fs;
-        if (lt_zero(vdov)) f = fmaf((prm.qqc2x64f * fa) * fa, fv * fv, f);
         const double least = __longlong_as_double((long long)*(volatile unsigned long long*)&st->acc_courant);
-        skip = f > 1e-30f && fa > coarse(least) * (sqrtf(f) * 1.0001f);
+        skip = courant_above(arealg, ss_new, vdov, least, prm.qqc8);
       }
       if (!skip) {
         double dtf = ss_new * ss_new;
