@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(3 * kFixedElems) k_static_corner_forces(lulesh
 
 // fx = sum of the node's corner forces in nodeElemCornerList order
 // (src/domain.jl:1112-1127).
-// It also hands the status word over and clears it for the next call.
+// It also hands the status word over and clears it for the next call (a call whose
+// gather is not launched clears it itself).
 __global__ void __launch_bounds__(256) k_static_gather(lulesh_force_args a, double* scratch, int64_t max_elems) {
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n == 0) {
@@ -180,7 +181,14 @@ extern "C" int lulesh_calc_force_for_nodes_static(const lulesh_force_args* args,
     default: k_static_corner_forces<3><<<eg, bs, 0, s>>>(a, scratch, kStaticMaxElems); break;
   }
   k_static_gather<<<(int)((a.num_node + 255) / 256), 256, 0, s>>>(a, scratch, kStaticMaxElems);
-  if (cudaGetLastError() != cudaSuccess) return LULESH_ERR_CUDA;
+  if (cudaGetLastError() != cudaSuccess) {
+    // one of the two was not launched: what the first may have found is no
+    // one's to report
+    cudaMemsetAsync(scratch + 24 * kStaticMaxElems, 0, sizeof(double), s);
+    cudaStreamSynchronize(s);
+    cudaGetLastError();
+    return LULESH_ERR_CUDA;
+  }
   unsigned bits = 0;
   if (cudaMemcpyAsync(&bits, status, sizeof(unsigned), cudaMemcpyDeviceToHost, s) != cudaSuccess)
     return LULESH_ERR_CUDA;
