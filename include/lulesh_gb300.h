@@ -227,12 +227,14 @@ int lulesh_block_plan(int32_t nx, int32_t blocks_per_edge, int32_t mode, int32_t
  * state. No choice changes any result (bitwise). k_force and k_kinematics run
  * three threads per element in blocks of 96 and form their geometry
  * themselves: force_block, kin_block and geometry are checked and handed back
- * by lulesh_get_tuning, and change nothing. */
+ * by lulesh_get_tuning, and change nothing. The defaults of node_block (256) and
+ * mat_block (128) are upper bounds: on meshes with fewer than eight blocks per SM
+ * the kernels take smaller ones. Other values are used as they are. */
 typedef struct {
   int32_t force_block;   /* 64, 128 or 256 (no effect) */
-  int32_t node_block;    /* k_node: 128, 256 or 512 */
+  int32_t node_block;    /* k_node: 128, 256 (by mesh size up to that) or 512 */
   int32_t kin_block;     /* 64, 128 or 256 (no effect) */
-  int32_t mat_block;     /* k_material: 64, 128 or 256 */
+  int32_t mat_block;     /* k_material: 64, 128 (by mesh size up to that) or 256 */
   int32_t geometry;      /* 0 or 1 (no effect) */
 } lulesh_tuning;
 

@@ -950,7 +950,7 @@ int lulesh_autotune(lulesh_domain* d, int32_t cycles, lulesh_tuning* chosen) {
     err = cudaMemcpyAsync(dd.st, d->hst, sizeof(DevState), cudaMemcpyHostToDevice, s);
   }
   if (err == cudaSuccess) {
-      err = autotune_blocks(dd, make_params(d), d->params.keep_aux != 0, 1, s, cycles, d->tuning);
+    err = autotune_blocks(dd, make_params(d), d->params.keep_aux != 0, 1, s, cycles, d->tuning);
   }
   if (err == cudaSuccess) err = copy_all(false);
   if (err == cudaSuccess) err = cudaStreamSynchronize(s);

@@ -961,15 +961,6 @@ __global__ void k_time_increment(DevState* st, int n, Params prm) {
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-// Threads per block of a kernel with one thread per unit: the tuned size, halved
-// down to a warp until there are eight blocks per SM. A small mesh then spreads
-// over the SMs evenly: 41.2 -> 39.9 us per cycle at 30^3, nothing from 64^3 up.
-static int spread(int units, int block) {
-  constexpr int kSMs = 152;
-  while (block > 32 && (units + block - 1) / block < 8 * kSMs) block /= 2;
-  return block;
-}
-
 void launch_tape_geometry(const DevDomain& d, cudaStream_t s) {
   k_tape_geometry<<<(d.E + kFixedElems - 1) / kFixedElems, 3 * kFixedElems, 0, s>>>(d);
 }
@@ -998,7 +989,7 @@ void launch_node(const DevDomain& d, const Params& prm, bool aux, const Tuning& 
     const int n = d.nCornerSlot - 8 * d.E;
     launch(k_halo_corners, (n + 255) / 256, 256, s, d);
   }
-  const int bs = spread(d.N, t.node);
+  const int bs = threads_per_block(d.N, t.node, kNodeBlock);
   const int grid = (d.N + bs - 1) / bs;
   if (d.nodeInst) launch(k_node<false, true>, grid, bs, s, d, prm);
   else if (aux) launch(k_node<true, false>, grid, bs, s, d, prm);
@@ -1019,7 +1010,7 @@ void launch_material(const DevDomain& d, const Params& prm, bool aux, const Tuni
     const int n = d.Eg - d.E;
     launch(k_halo_delv, (n + 255) / 256, 256, s, d);
   }
-  const int bs = spread(d.E, t.mat);
+  const int bs = threads_per_block(d.E, t.mat, kMatBlock);
   const int grid = (d.E + bs - 1) / bs;
   const bool fix = (d.mode & 4) != 0;
   const bool region = d.regOrder != nullptr;
