@@ -681,7 +681,7 @@ int lulesh_adj_gradient(lulesh_adjoint* a, int64_t num_cycles, lulesh_adj_result
   // segments k >= first_taped are taped by the forward sweep itself
   const int first_taped = nplan - (plan == kTwo ? std::min(2, nplan) : 1);
   if (nplan > 1 && (!a->fwd_graph || std::memcmp(&a->fwd_prm, &prm, sizeof(Params)) != 0 ||
-                    std::memcmp(&a->fwd_tuning, &d->tuning, sizeof(Tuning)) != 0 || a->fwd_aux != aux)) {
+                    !same_launches(a->fwd_tuning, d->tuning) || a->fwd_aux != aux)) {
     if (a->fwd_graph) cudaGraphExecDestroy(a->fwd_graph);
     a->fwd_graph = nullptr;
     cudaGraph_t g;
@@ -738,7 +738,7 @@ int lulesh_adj_gradient(lulesh_adjoint* a, int64_t num_cycles, lulesh_adj_result
     return LULESH_OK;
   };
   const int nsets = plan == kTwo ? 2 : 1;
-  if (std::memcmp(&a->rev_prm, &prm, sizeof(Params)) != 0 || std::memcmp(&a->rev_tuning, &d->tuning, sizeof(Tuning)) != 0) {
+  if (std::memcmp(&a->rev_prm, &prm, sizeof(Params)) != 0 || !same_launches(a->rev_tuning, d->tuning)) {
     for (int x = 0; x < 2; ++x) {
       if (a->rec_graph[x]) { cudaGraphExecDestroy(a->rec_graph[x]); a->rec_graph[x] = nullptr; }
       if (a->tr_graph[x]) { cudaGraphExecDestroy(a->tr_graph[x]); a->tr_graph[x] = nullptr; }

@@ -909,12 +909,13 @@ int lulesh_set_tuning(lulesh_domain* d, const lulesh_tuning* t) {
       !(t->node_block == 128 || t->node_block == 256 || t->node_block == 512) ||
       !(t->geometry == 0 || t->geometry == 1))
     return LULESH_ERR_ARGUMENT;
+  const Tuning before = d->tuning;
   d->tuning.force = t->force_block;
   d->tuning.node = t->node_block;
   d->tuning.kin = t->kin_block;
   d->tuning.mat = t->mat_block;
   d->tuning.geo = t->geometry;
-  drop_graph(d);
+  if (!same_launches(before, d->tuning)) drop_graph(d);
   return LULESH_OK;
 }
 

@@ -475,12 +475,13 @@ static bool valid_tuning(const lulesh_tuning* t) {
 
 int lulesh_ens_set_tuning(lulesh_ensemble* s, const lulesh_tuning* t) {
   if (!s || !valid_tuning(t)) return LULESH_ERR_ARGUMENT;
+  const Tuning before = s->tuning;
   s->tuning.force = t->force_block;
   s->tuning.node = t->node_block;
   s->tuning.kin = t->kin_block;
   s->tuning.mat = t->mat_block;
   s->tuning.geo = t->geometry;
-  drop_graph(s);
+  if (!same_launches(before, s->tuning)) drop_graph(s);
   return LULESH_OK;
 }
 

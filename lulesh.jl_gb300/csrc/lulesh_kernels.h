@@ -31,6 +31,9 @@ struct Tuning {
   int geo = 0;
 };
 
+// Whether two configurations launch the same kernels.
+inline bool same_launches(const Tuning& a, const Tuning& b) { return a.node == b.node && a.mat == b.mat; }
+
 // Threads per block of a kernel with one thread per unit. A block size the caller
 // set is used as it is; the default is halved, down to a warp, until there are
 // eight blocks per SM. A small mesh then spreads over the SMs evenly: 41.2 -> 39.9 us
