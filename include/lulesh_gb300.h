@@ -379,6 +379,8 @@ typedef struct {
   int32_t reserved;
 } lulesh_adj_result;
 
+/* (An adjoint may be destroyed after its domain: until then its last gradient can
+ * be read, other calls return LULESH_ERR_ARGUMENT.) */
 int lulesh_adj_create(lulesh_domain* dom, double radius, int32_t checkpoint_every, lulesh_adjoint** out);
 int lulesh_adj_destroy(lulesh_adjoint* adj);
 /* Linear objective weights for one state field (replaces the energy

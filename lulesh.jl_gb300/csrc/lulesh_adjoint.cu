@@ -90,7 +90,8 @@ struct TapeSet {
 };
 
 struct lulesh_adjoint {
-  lulesh_domain* dom = nullptr;
+  lulesh_domain* dom = nullptr;  // null once the domain is destroyed
+  int device = 0;
   double radius = 0.3;
   int K = 20;
   int E = 0, N = 0;
@@ -249,6 +250,12 @@ static bool ensure_slot_events(lulesh_adjoint* a) {
     a->ev_slot.push_back(e);
   }
   return true;
+}
+
+void lulesh::detach_adjoint(lulesh_adjoint* a) {
+  if (a->rstream) cudaStreamSynchronize(a->rstream);
+  if (a->tstream) cudaStreamSynchronize(a->tstream);
+  a->dom = nullptr;
 }
 
 static StateSet domain_set(lulesh_adjoint* a) {
@@ -457,6 +464,7 @@ int lulesh_adj_create(lulesh_domain* dom, double radius, int32_t checkpoint_ever
   lulesh_adjoint* a = new (std::nothrow) lulesh_adjoint();
   if (!a) return LULESH_ERR_MEMORY;
   a->dom = dom;
+  a->device = dom->params.device;
   a->radius = radius;
   a->K = checkpoint_every;
   a->E = (int)dom->E;
@@ -567,14 +575,23 @@ int lulesh_adj_create(lulesh_domain* dom, double radius, int32_t checkpoint_ever
         cudaMemcpy(a->wn, v.data(), N * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
       return fail(LULESH_ERR_CUDA);
   }
+  try {
+    dom->adjoints.push_back(a);
+  } catch (const std::bad_alloc&) {
+    return fail(LULESH_ERR_MEMORY);
+  }
   *out = a;
   return LULESH_OK;
 }
 
 int lulesh_adj_destroy(lulesh_adjoint* a) {
   if (!a) return LULESH_ERR_ARGUMENT;
-  cudaSetDevice(a->dom->params.device);
-  cudaStreamSynchronize(a->dom->stream);
+  cudaSetDevice(a->device);
+  if (a->dom) {
+    cudaStreamSynchronize(a->dom->stream);
+    std::vector<lulesh_adjoint*>& live = a->dom->adjoints;
+    live.erase(std::remove(live.begin(), live.end(), a), live.end());
+  }
   if (a->fwd_graph) cudaGraphExecDestroy(a->fwd_graph);
   if (a->rec_graph[0]) cudaGraphExecDestroy(a->rec_graph[0]);
   if (a->tr_graph[0]) cudaGraphExecDestroy(a->tr_graph[0]);
@@ -592,8 +609,8 @@ int lulesh_adj_destroy(lulesh_adjoint* a) {
 }
 
 int lulesh_adj_set_overlap(lulesh_adjoint* a, int32_t mode) {
-  if (!a || mode < 0 || mode > 2) return LULESH_ERR_ARGUMENT;
-  ACK(cudaSetDevice(a->dom->params.device));
+  if (!a || !a->dom || mode < 0 || mode > 2) return LULESH_ERR_ARGUMENT;
+  ACK(cudaSetDevice(a->device));
   ACK(cudaStreamSynchronize(a->dom->stream));
   if (a->rstream) ACK(cudaStreamSynchronize(a->rstream));
   if (a->tstream) ACK(cudaStreamSynchronize(a->tstream));
@@ -623,13 +640,13 @@ int lulesh_adj_clear_seeds(lulesh_adjoint* a) {
 }
 
 int lulesh_adj_loss(lulesh_adjoint* a, double* loss) {
-  if (!a || !loss) return LULESH_ERR_ARGUMENT;
-  ACK(cudaSetDevice(a->dom->params.device));
+  if (!a || !a->dom || !loss) return LULESH_ERR_ARGUMENT;
+  ACK(cudaSetDevice(a->device));
   return objective(a, false, loss);
 }
 
 int lulesh_adj_gradient(lulesh_adjoint* a, int64_t num_cycles, lulesh_adj_result* res) {
-  if (!a || num_cycles < 1) return LULESH_ERR_ARGUMENT;
+  if (!a || !a->dom || num_cycles < 1) return LULESH_ERR_ARGUMENT;
   TraceRange trace("lulesh_adj_gradient");
   lulesh_domain* d = a->dom;
   ACK(cudaSetDevice(d->params.device));
@@ -893,7 +910,7 @@ int lulesh_adj_get_gradient(lulesh_adjoint* a, int32_t field, double* host, int6
   if (!a || !host) return LULESH_ERR_ARGUMENT;
   const int k = field_index(field);
   if (k < 0 || count != (k < 6 ? a->N : a->E)) return LULESH_ERR_ARGUMENT;
-  ACK(cudaSetDevice(a->dom->params.device));
+  ACK(cudaSetDevice(a->device));
   ACK(cudaMemcpy(host, adj_field(a, field), count * sizeof(double), cudaMemcpyDeviceToHost));
   return LULESH_OK;
 }

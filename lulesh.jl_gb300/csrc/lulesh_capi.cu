@@ -480,6 +480,7 @@ int lulesh_destroy(lulesh_domain* d) {
   if (!d) return LULESH_ERR_ARGUMENT;
   cudaSetDevice(d->params.device);
   if (d->stream) cudaStreamSynchronize(d->stream);
+  for (lulesh_adjoint* a : d->adjoints) detach_adjoint(a);
   drop_graph(d);
   for (auto& ev : d->ring) if (ev) cudaEventDestroy(ev);
   if (d->hst) cudaFreeHost(d->hst);

@@ -41,10 +41,14 @@ struct lulesh_domain {
   int ring_used = 0;
   lulesh::Tuning tuning;
   double kernel_ms[lulesh::kNumKernels] = {};
+  std::vector<lulesh_adjoint*> adjoints;  // live adjoints of this domain
   int64_t cycle_i() const { return (int64_t)sc[LULESH_S_CYCLE]; }
 };
 
 namespace lulesh {
+// The domain is about to be destroyed (its stream has been waited for): its adjoint
+// takes no more of it.
+void detach_adjoint(lulesh_adjoint* a);
 // Kernel parameters from the handle's Domain scalars.
 Params make_params(const lulesh_domain* d);
 // Status bits of a step -> (lulesh_status, lulesh_site) in the reference's order.
