@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kMaxNodeBlock) k_node(DevDomain d, Params prm)
   const int s = LDG(&d.nodeElemStart[i]);
   int t = LDG(&d.nodeElemStart[i + 1]);
   const double im = LDG(&d.inv_nodalMass[i]);
-  const int first = s < t ? LDG(&d.cornerList[s]) : 0;
+  const int first = s < t ? LDG(&d.cornerList[LULESH_IDX(s, d.nCornerList, st)]) : 0;
   wait_for_last_kernel();
   const uint4 flags = __ldcv(reinterpret_cast<const uint4*>(&st->status));  // status, done, force_status
   const double dt = st->deltatime;
