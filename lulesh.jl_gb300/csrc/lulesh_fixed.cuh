@@ -269,49 +269,50 @@ LULESH_FX Float to_float(double x) {
 // least and most an element's largest extent may be. det: the least Jacobian
 // determinant (of the mean edges, which are the extents of an undistorted element;
 // an undistorted box has 2^52 to 2^55 of its scale, by where its extents lie in
-// [2^60, 2^61)), over the box or over the cube of the largest extent. distortion: the
-// powers of two the hourglass base vectors may outgrow their scale by.
+// [2^60, 2^61)) that k_force and k_kinematics take, over the box or over the cube of
+// the largest extent. distortion: the powers of two the hourglass base vectors may
+// outgrow their scale by.
 struct Range {
   int least_extent, most_extent;
-  int det;
+  int force_det, kin_det;
   bool over_cube;
   int distortion;
 };
 // Where every sum is within a few units of 2^-47 of its own size: extents for
 // which the guards 1e-36 added to squared areas and to volumes are below half a
 // unit, volumes above 1/32 to 1/256 of the cube.
-LULESH_FX constexpr Range narrow() { return {1023 - 12, 1023 + 40, 47, true, 4}; }
-// Where every sum is at least as good as the FP64 expressions leave it, whose errors
-// are relative to products over the box too. The kernels add the guards. Below
-// 2^-30 of its box not even FP64 tells a volume from its rounding; those elements
-// (and inverted, flat or non-finite ones) are left to the FP64 form, whose
-// errors the step reports. Plates and needles of aspect 1:100 and meshes of edges
-// below 2^-12, which the narrow range refuses, take 0.66 ms per cycle at 100^3 so;
-// both forms one after the other took 2.32, the FP64 kernels 1.81.
-LULESH_FX constexpr Range wide() { return {1023 - 100, 1023 + 100, 24, false, 31}; }
+LULESH_FX constexpr Range narrow() { return {1023 - 12, 1023 + 40, 47, 47, true, 4}; }
+// Where every sum is at least as good as the FP64 expressions leave it. The kernels
+// add the guards. Plates and needles along the axes are boxes; of turned ones the
+// kinematics takes those above 1/32 to 1/256 of their box (the cofactors of others
+// are too far below its areas), the forces down to 2^-30. What is inverted, flat or
+// not finite is the FP64 form's, whose errors the step reports. A cycle at 100^3 of
+// plates or needles 1:100, or of edges below 2^-12: 0.81 ms, as of cubes (in a calm
+// state), turned plates 1:500 1.38; over the narrow range, both forms one after the
+// other, 2.32; the FP64 kernels alone 1.81.
+LULESH_FX constexpr Range wide() { return {1023 - 100, 1023 + 100, 24, 47, false, 31}; }
 // velocity extents below 2^-400 are taken as that: they move nothing
 constexpr int kMinSpeed = 1023 - 400, kMaxSpeed = 1023 + 400;
 
 LULESH_FX unsigned umax(unsigned a, unsigned b) { return a > b ? a : b; }
 
 // The scales s (x = X 2^-s) of an element's three coordinates, each its extent to
-// [2^60, 2^61); an extent below 2^-60 of the largest counts as that. A largest
-// extent out of range shifts everything out.
+// [2^60, 2^61); an extent below 2^-28 of the largest counts as that.
 struct Scales {
   int s[3];
-  bool ok;
+  bool ok;  // the largest extent is in range
   LULESH_FX int wide() const { return imin(s[0], imin(s[1], s[2])); }
-  // the least determinant is 2^least(), in its own units (none reaches 2^58)
-  LULESH_FX int least(Range range) const {
-    return imin(range.det + (range.over_cube ? s[0] + s[1] + s[2] - 3 * wide() : 0), 58);
+  // the least determinant is 2^least, in its own units (none reaches 2^58)
+  LULESH_FX int least(int det, Range range) const {
+    return range.over_cube ? imin(det + s[0] + s[1] + s[2] - 3 * wide(), 58) : det;
   }
 };
-LULESH_FX Scales scales_of(unsigned hi0, unsigned hi1, unsigned hi2, Range range) {  // high words of the extents
-  Scales r = {{exponent_field(hi0), exponent_field(hi1), exponent_field(hi2)}, false};
-  const int top = imax(r.s[0], imax(r.s[1], r.s[2]));
+LULESH_FX Scales scales_of(int ex0, int ex1, int ex2, Range range) {  // exponent fields of the extents
+  Scales r = {{ex0, ex1, ex2}, false};
+  const int top = imax(ex0, imax(ex1, ex2));
   r.ok = top >= range.least_extent && top <= range.most_extent;
   LULESH_UNROLL
-  for (int j = 0; j < 3; ++j) r.s[j] = 1083 - (r.ok ? imax(r.s[j], top - 60) : 0x7ff);
+  for (int j = 0; j < 3; ++j) r.s[j] = 1083 - imax(r.s[j], top - 28);
   return r;
 }
 

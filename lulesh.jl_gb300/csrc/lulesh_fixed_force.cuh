@@ -45,7 +45,7 @@ enum : int {
   FS_GEO = 0,      // 18 k + q: limbs of diagonal q (12), U vector (3), mean edge (3) of coordinate k
   FS_HG = 0,       // 4 n + m: limbs of the base vectors, over the diagonals once those are read
   FS_DV = 54,      // 12 k + n: limbs of the volume derivatives (8) and scaled modes (4)
-  FS_EXT = 90,     // k: extent's high word; whether the velocities are out of range
+  FS_EXT = 90,     // k: extent's exponent field; whether the velocities are out of range
   FS_USED = 93,    // k: bits used by the modes' high words
   FS_K = 96,       // mantissas of 1/(12 determ), the coefficient and the stress, then their exponents
   FS_C = 97,
@@ -55,6 +55,9 @@ enum : int {
   FS_SMALL = 104,  // k: bits used by the derivatives' high words, where the base vectors outgrow their scale
   FS_COUNT = 107
 };
+
+// places the base vectors may outgrow their scale by at the cost of their last bits
+constexpr int kFewPlaces = 1;
 
 // What a thread keeps over the phases.
 struct ForceLane {
@@ -76,7 +79,7 @@ LULESH_FX void force_load(int k, Slots sh, const double v[8], ForceLane& r) {
   LULESH_UNROLL
   for (int n = 1; n < 8; ++n) r.V[n] = limbs(sub(to_fixed(v[n], 7 - r.ev), v0));
   Num m;
-  m.lo = (int)extent_hi(r.x);
+  m.lo = exponent_field(extent_hi(r.x));
   m.hi = wild;
   sh[FS_EXT + k] = m;
 }
@@ -104,11 +107,11 @@ LULESH_FX void force_stress(Slots sh, double s8) {
 // 2: the coordinate's diagonals, U vectors, mean edges and hourglass modes.
 LULESH_FX void force_diagonals(int k, Slots sh, ForceLane& r, i64 hm[4], Range range = narrow()) {
   const Num m0 = sh[FS_EXT], m1 = sh[FS_EXT + 1], m2 = sh[FS_EXT + 2];
-  const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo, range);
+  const Scales s = scales_of(m0.lo, m1.lo, m2.lo, range);
   r.ok = s.ok && (m0.hi | m1.hi | m2.hi) == 0 && sh[FS_EXPO].hi != 1 << 20 && sh[FS_EXPO + 1].hi != 0;
   r.s = k == 0 ? s.s[0] : k == 1 ? s.s[1] : s.s[2];
   r.all = s.s[0] + s.s[1] + s.s[2];
-  r.least = s.least(range);
+  r.least = s.least(range.force_det, range);
   i64 v[8], g[12], w[3];
   LULESH_UNROLL
   for (int c = 0; c < 8; ++c) v[c] = to_fixed(r.x[c], r.s - 1075);
@@ -153,8 +156,8 @@ LULESH_FX void force_diagonals(int k, Slots sh, ForceLane& r, i64 hm[4], Range r
 // places, of the product; q is 0 unless the distortion needs more, and more
 // than the range has is left to the FP64 form. A derivative is at most 3 E^2 (its bilinear
 // form over the corners of a box), below 2^59.6, so the base vectors stay
-// below 2^59.8. Where q is not 0, what the derivatives leave of that is taken off it
-// in phase 4: a slender element's are as far below its box's areas as its base
+// below 2^59.8. Where q is more than a few places, what the derivatives leave of that
+// is taken off it in phase 4: a slender element's are as far below its box's areas as its base
 // vectors' terms are above their scale.
 template <int MODE, class Tape>
 LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Tape tape, Range range = narrow()) {
@@ -198,7 +201,7 @@ LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Ta
   r.ok = r.ok && L >= 0 && r.q <= range.distortion;
   r.q = r.ok ? r.q : 0;
   const int Lq = r.ok ? L - r.q : 0, left = imin(Lq, room), rest = Lq - left;
-  if (r.q > 0) {
+  if (r.q > kFewPlaces) {
     Num small = {0, 0};
     for (int n = 0; n < 8; ++n) {
       const int h = sh[FS_DV + 12 * k + n].hi;
@@ -219,7 +222,7 @@ LULESH_FX void force_products(int k, Slots sh, ForceLane& r, const i64 hm[4], Ta
 LULESH_FX void force_base(int k, Slots sh, ForceLane& r) {
   r.ok = r.ok && sh.get(FS_DET) + sh.get(FS_DET + 1) + sh.get(FS_DET + 2) >= shl(1, r.least);
   int up = 0;
-  if (r.q > 0) {
+  if (r.q > kFewPlaces) {
     const int used = sh[FS_SMALL].lo | sh[FS_SMALL + 1].lo | sh[FS_SMALL + 2].lo;
     up = imin(imax(leading_zeros((unsigned)used) - 3, 0), r.q);
     r.q -= up;

@@ -18,7 +18,7 @@ enum : int {
   KS_GEO = 0,    // 18 k + q: limbs of diagonal q (12), mean edge (3), half-step edge (3) of coordinate k
   KS_SUM = 0,    // kSums k + i: coordinate k's terms, over the diagonals once those are read
   KS_DET = 57,   // k: a term of the Jacobian determinant
-  KS_EXT = 60,   // k: high words of the position and velocity extents
+  KS_EXT = 60,   // k: exponent fields of the position and velocity extents
   KS_MID = 63,   // 1/(64 volume), then the divergence's factor and the divergence
   KS_COUNT = 66
 };
@@ -30,27 +30,24 @@ enum : int {
   SUM_FLOW = 10,   // 3: those cross products times velocity differences
   SUM_RATE = 13,   // cofactors times velocity differences
   SUM_JAC = 14,    // half-step determinant
-  SUM_EXPO = 15,   // 4: exponents of flow d (low word) and area d (high word), then the rate's and the faces'
+  SUM_EXPO = 15,   // 4: exponents of flow d (low word) and area d (high word); the rate's, and over 2^8 the faces', with the
+                   // determinant's below
   kSums = 19
 };
 // exponent of a term that is exactly zero
 constexpr int kNoTerm = -16384;
-// places the largest cofactor may leave free above it (of the 60 that hold it)
-constexpr int kFewBits = 5;
 static_assert(3 * kSums <= KS_DET, "the sums overlay the diagonals");
 
 // What a thread keeps over the phases: its components (unscaled integers) of
 // the face vectors, the volume's V x W, the edges' cross products (over
-// 2^(64 - up)), the cofactors (over 2^(64 - cup)), and its velocity differences and
+// 2^(64 - up)), the cofactors (over 2^62), and its velocity differences and
 // edges. A component of a cross product is in the other two coordinates' units,
 // a triple product in all three, whichever the component.
 struct KinLane {
   double x[8], v[8];
   int s, sv, all;  // scales of this coordinate's positions and velocities; sum of the three positions'
   int least;       // the least determinant is 2^least
-  int up[3], cup;
-  i64 eta;  // the eta cofactor by itself; with half_eta 2^eup times the determinant's term
-  int eup;
+  int up[3];
   bool ok_x, ok;  // positions taken; positions and velocities taken
   i64 g[12], w[3], vw[3];
   i64 n[6], gU[3], A[3], C[3];
@@ -68,8 +65,8 @@ LULESH_FX i64 square(Num a) {
 // 1: r.x and r.v hold coordinate k's corner values.
 LULESH_FX void kin_extents(int k, Slots sh, const KinLane& r) {
   Num m;
-  m.lo = (int)extent_hi(r.x);
-  m.hi = (int)extent_hi(r.v);
+  m.lo = exponent_field(extent_hi(r.x));
+  m.hi = exponent_field(extent_hi(r.v));
   sh[KS_EXT + k] = m;
 }
 
@@ -80,17 +77,17 @@ LULESH_FX void kin_extents(int k, Slots sh, const KinLane& r) {
 // the monotonic-Q gradients across it, are as small as they please.
 LULESH_FX void kin_edges(int k, Slots sh, double half_dt, KinLane& r, Range range = narrow()) {
   const Num m0 = sh[KS_EXT], m1 = sh[KS_EXT + 1], m2 = sh[KS_EXT + 2];
-  const Scales s = scales_of((unsigned)m0.lo, (unsigned)m1.lo, (unsigned)m2.lo, range);
+  const Scales s = scales_of(m0.lo, m1.lo, m2.lo, range);
   r.ok_x = s.ok;
   r.s = k == 0 ? s.s[0] : k == 1 ? s.s[1] : s.s[2];
   r.all = s.s[0] + s.s[1] + s.s[2];
-  r.least = s.least(range);
-  int ev[3] = {exponent_field((unsigned)m0.hi), exponent_field((unsigned)m1.hi), exponent_field((unsigned)m2.hi)};
+  r.least = s.least(range.kin_det, range);
+  int ev[3] = {m0.hi, m1.hi, m2.hi};
   const bool wild = imax(ev[0], imax(ev[1], ev[2])) > kMaxSpeed;  // not finite, or far beyond any flow
   int fastest = kNoExponent;
   LULESH_UNROLL
   for (int j = 0; j < 3; ++j) {
-    ev[j] = wild ? 0x7ff : imax(ev[j], kMinSpeed);
+    ev[j] = imax(ev[j], kMinSpeed);
     fastest = imax(fastest, s.s[j] - 1083 + ev[j]);
   }
   r.sv = 1083 - (k == 0 ? ev[0] : k == 1 ? ev[1] : ev[2]);
@@ -138,26 +135,8 @@ LULESH_FX void kin_products(int k, Slots sh, KinLane& r) {
   for (int d = 0; d < 3; ++d) {
     const int a = 12 + (d + 1) % 3, b = 12 + (d + 2) % 3;
     r.A[d] = take_all(mul_minus_full(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]), r.up[d]);
-    if (d != 1) r.C[d] = cross_k(a + 3, b + 3);
+    r.C[d] = take<2>(mul_minus(sh[i1 + a + 3], sh[i2 + b + 3], sh[i2 + a + 3], sh[i1 + b + 3]));
   }
-  // The determinant's factors keep all their bits; of the cofactors only the
-  // largest count, but a slender element's are far below its box's areas.
-  r.eta = take_all(mul_minus_full(sh[i1 + 17], sh[i2 + 15], sh[i2 + 17], sh[i1 + 15]), r.eup);
-  r.cup = imin(r.eup, imin(room(r.C[0]), room(r.C[2])));
-  if (r.cup <= kFewBits) {
-    r.cup = 0;
-  } else {
-    LULESH_UNROLL
-    for (int d = 0; d < 3; d += 2) {
-      const int a = 15 + (d + 1) % 3, b = 15 + (d + 2) % 3;
-      r.C[d] = take_up(mul_minus_full(sh[i1 + a], sh[i2 + b], sh[i2 + a], sh[i1 + b]), r.cup);
-    }
-  }
-  r.C[1] = r.eta >> (r.eup - r.cup);
-  const i64 h = add(shl((i64)r.half_eta.hi, 32), (i64)r.half_eta.lo);
-  const int thin = room(h);
-  r.half_eta = limbs(shl(h, thin));
-  r.eup += thin;
   sh.put(KS_DET + k, product(limbs(r.w[1]), limbs(r.A[1] >> r.up[1])));
 }
 
@@ -199,19 +178,20 @@ LULESH_FX void kin_terms(int k, Slots sh, const KinLane& r) {
     const Num a = limbs(r.A[d]), u = limbs(r.vw[d]), c = limbs(r.C[d]);
     sh.put(at + SUM_AREA + d, square(a));
     Num e;
-    e.hi = r.A[d] != 0 ? -2 * (two + r.up[d]) : kNoTerm;
+    e.hi = -2 * (two + r.up[d]);  // (with up 29 and scales within 2^28 of one another, zeros stay below the rest)
     Acc flow = {0, 0};
     mac_full(flow, a, u);
     e.lo = put_term(SUM_FLOW + d, take<3>(flow), r.up[d]);
     sh[at + SUM_EXPO + d] = e;
     mac_full(rate, c, u);
   }
-  last.lo = put_term(SUM_RATE, take<1>(rate), r.cup);
-  last.hi = (int)((unsigned)last.hi << 8) | r.eup;
-  sh[at + SUM_EXPO + 3] = last;
+  last.lo = put_term(SUM_RATE, take<1>(rate), 0);
   Acc jac = {0, 0};
-  mac_full(jac, r.half_eta, limbs(r.eta));
-  sh.put(at + SUM_JAC, take<3>(jac));
+  mac_full(jac, r.half_eta, limbs(r.C[1]));
+  int c;
+  sh.put(at + SUM_JAC, take_all(jac, c));
+  last.hi = (int)((unsigned)last.hi << 8) | c;
+  sh[at + SUM_EXPO + 3] = last;
 }
 
 LULESH_FX i64 kin_sum(Slots sh, int i) {
@@ -265,15 +245,15 @@ LULESH_FX double kin_flow(Slots sh, const KinLane&, int d) {
   return kin_aligned(sh, SUM_FLOW + d, kin_expo(sh, 0, d).lo, kin_expo(sh, 1, d).lo, kin_expo(sh, 2, d).lo, 131);
 }
 LULESH_FX double kin_rate(Slots sh, const KinLane&) {
-  return kin_aligned(sh, SUM_RATE, kin_expo(sh, 0, 3).lo, kin_expo(sh, 1, 3).lo, kin_expo(sh, 2, 3).lo, 133);
+  return kin_aligned(sh, SUM_RATE, kin_expo(sh, 0, 3).lo, kin_expo(sh, 1, 3).lo, kin_expo(sh, 2, 3).lo, 131);
 }
 // coordinate k's part of it
 LULESH_FX double kin_own_rate(Slots sh, const KinLane&, int k) {
-  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 133 + kin_expo(sh, k, 3).lo);
+  return to_double(sh.get(KS_SUM + kSums * k + SUM_RATE), 131 + kin_expo(sh, k, 3).lo);
 }
 LULESH_FX double kin_jacobian(Slots sh, const KinLane& r) {
   auto e = [&](int j) { return -(kin_expo(sh, j, 3).hi & 0xff); };
-  return kin_aligned(sh, SUM_JAC, e(0), e(1), e(2), 131 - r.all);
+  return kin_aligned(sh, SUM_JAC, e(0), e(1), e(2), 132 - r.all);
 }
 
 }  // namespace fx

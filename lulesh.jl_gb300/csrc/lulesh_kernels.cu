@@ -352,7 +352,11 @@ struct FixedSums {
   const fx::KinLane& r;
   __device__ double volume12() const { return fx::kin_volume12(sh, r); }
   __device__ double face(int& place) const { return fx::kin_largest_face(sh, r, place); }
-  __device__ double area(int k) const { return fx::kin_area(sh, r, k) + 256.e-36; }
+  // (from 2^-54 up the guard is below half a unit)
+  __device__ double area(int k) const {
+    const double a = fx::kin_area(sh, r, k);
+    return fx::hi_word(a) < (1023 - 54) << 20 ? a + 256.e-36 : a;
+  }
   __device__ double flow(int k) const { return fx::kin_flow(sh, r, k); }
   __device__ double rate() const { return fx::kin_rate(sh, r); }
   __device__ double jacobian() const { return fx::kin_jacobian(sh, r); }
@@ -362,7 +366,7 @@ struct FixedTaped {
   const fx::KinLane& r;
   __device__ double w(int a) const { return fx::to_double(r.w[a], 2 - r.s); }
   __device__ double vw(int a) const { return fx::to_double(r.vw[a], 2 - r.sv); }
-  __device__ double C(int a) const { return fx::to_double(r.C[a], 68 - r.cup - (r.all - r.s)); }
+  __device__ double C(int a) const { return fx::to_double(r.C[a], 66 - (r.all - r.s)); }
   __device__ double A(int a) const { return fx::to_double(r.A[a], 68 - r.up[a] - (r.all - r.s)); }
   __device__ double gU(int a) const { return fx::to_double(r.gU[a], 64 - (r.all - r.s)); }
   __device__ double g(int q) const { return fx::to_double(r.g[q], -r.s); }
