@@ -1,6 +1,7 @@
 // The force and kinematics phases of lulesh_fixed_force.cuh and
 // lulesh_fixed_kin.cuh in FP64, for the elements the fixed-point form does not
-// take: thin, inverted or not finite ones, whose volume errors these record.
+// take: inverted, flat or not finite ones, whose volume errors these record, turned
+// slender ones (kinematics), and numbers outside 2^-400..2^400.
 //
 // The same three threads, slots and barriers: a thread's component takes about
 // 190 FP64 slots (forces) or 110 (kinematics), 6 and 4 us for a block that has

@@ -104,12 +104,11 @@ __device__ __noinline__ void force_fallback(const DevDomain& d, DevState* st, un
 
 // Three threads per element, one per coordinate and each in a warp of its own:
 // a block is 32 elements (lulesh_fixed_force.cuh). Bound by the integer pipes
-// (multiply-adds, shifts and logic issue every other cycle and share them:
-// counters 59 % and 46 % of the cycles, no other pipe above 25 %): 0.91 ms per
-// cycle at 150^3, where FP64 took 1.98 ms with the geometry stored by
-// k_kinematics (0.87 ms of that kernel). Seven blocks per SM, 80 registers:
-// six (96 registers) 1.02 ms, five (128) 1.12 ms; below 45^3 the three are
-// alike.
+// (multiply-adds, shifts and logic issue every other cycle and share them: ALU 52 %
+// and FMA-heavy 40 % of the cycles, FP64 28 %): 0.92 ms per cycle at 150^3, where
+// FP64 took 1.98 ms with the geometry stored by k_kinematics (0.87 ms of that
+// kernel). Eight blocks per SM, 80 registers: seven 0.94 ms, six (96 registers)
+// 1.02; below 45^3 alike.
 //
 // TIME: the cycle's timeIncrement! runs here too, by blocks of its own after
 // the elements'; the forces need neither dt nor time. The element blocks may
@@ -422,9 +421,10 @@ __device__ __noinline__ void kin_fallback(const DevDomain& d, DevState* st, fx::
 }
 
 // Three threads per element as in k_force (lulesh_fixed_kin.cuh). Bound by the
-// integer pipes: 0.58 ms per cycle at 150^3 (FP64: 1.93 ms without the force
-// geometry). Eight blocks per SM, 80 registers: six (96) 0.67 ms, five (128)
-// 0.77 ms.
+// integer pipes (ALU 60 %, FMA-heavy 34 %) and FP64 (59 %): 0.65 ms per cycle at
+// 150^3 (FP64: 1.93 ms without the force geometry), of which the scales by
+// coordinate and the terms' exponents are 0.09. Seven blocks per SM, 80 registers:
+// eight 0.66 ms, six (96) 0.79.
 template <bool AUX, bool ENS, bool TAPE>
 __global__ void __launch_bounds__(3 * kFixedElems, 7)
     k_kinematics(const __grid_constant__ DevDomain d, const __grid_constant__ Params prm) {

@@ -33,7 +33,4 @@ void launch(void (*kernel)(P...), int grid, int block, cudaStream_t s, const A&.
   cudaLaunchKernelEx(&c, kernel, args...);
 }
 
-// An ensemble (d.elemInst set) runs the ENS instantiations, which read each
-// element's or node's instance; the plain path runs ENS = false.
-
 }  // namespace lulesh
