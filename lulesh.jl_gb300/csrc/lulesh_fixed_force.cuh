@@ -224,7 +224,7 @@ LULESH_FX void force_base(int k, Slots sh, ForceLane& r) {
   int up = 0;
   if (r.q > kFewPlaces) {
     const int used = sh[FS_SMALL].lo | sh[FS_SMALL + 1].lo | sh[FS_SMALL + 2].lo;
-    up = imin(imax(leading_zeros((unsigned)used) - 3, 0), r.q);
+    up = imin(imax(leading_zeros((unsigned)used) - 4, 0), r.q);  // (derivatives stay below 2^60)
     r.q -= up;
   }
   const i64 one = 1ll << (58 - r.q);

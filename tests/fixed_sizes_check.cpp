@@ -99,7 +99,7 @@ void fp64_forces(const double p[3][8], const double v[3][8], double vi12, double
 
 // fixed_forces over either range
 bool ranged_forces(const double p[3][8], const double vel[3][8], double vi12, double coef, double s8, Range range,
-                   double f[3][8]) {
+                   double f[3][8], double* largest_base = nullptr) {
   Num column[FS_COUNT];
   const Slots sh{column, 1};
   ForceLane r[3];
@@ -114,6 +114,9 @@ bool ranged_forces(const double p[3][8], const double vel[3][8], double vi12, do
   for (int k = 0; k < 3; ++k) force_products<3>(k, sh, r[k], hm[k], NoTape{}, range);
   for (int k = 0; k < 3; ++k) force_base(k, sh, r[k]);
   if (r[0].ok != r[1].ok || r[0].ok != r[2].ok) std::abort();
+  if (largest_base)
+    for (int i = *largest_base = 0; i < 32; ++i)
+      *largest_base = std::fmax(*largest_base, std::fabs(sh[FS_HG + i].hi * 4294967296.0 + sh[FS_HG + i].lo));
   for (int k = 0; k < 3 && r[0].ok; ++k) force_corners(k, sh, r[k], [&](int n, double v) { f[k][n] = v; }, NoTape{});
   return r[0].ok;
 }
@@ -282,6 +285,17 @@ void check_force_sizes(int kernels, int n, const double* pos, const double* vel,
       fp64[3 * i + k] = (double)g;
       size[3 * i + k] = (double)(3 * std::fabs(s8) * most[k]) + std::fabs(coef) * dV;
     }
+  }
+}
+
+// The largest entry of the hourglass base vectors, in their units, over the kernels'
+// range (0 for an element that is not taken).
+void check_base(int n, const double* pos, const double* vel, const double* scal, double* largest) {
+  for (int i = 0; i < n; ++i) {
+    double f[3][8];
+    if (!ranged_forces(reinterpret_cast<const double(*)[8]>(pos + 24 * i), reinterpret_cast<const double(*)[8]>(vel + 24 * i),
+                       scal[3 * i], scal[3 * i + 1], scal[3 * i + 2], wide(), f, largest + i))
+      largest[i] = 0;
   }
 }
 

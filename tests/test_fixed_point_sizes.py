@@ -187,3 +187,26 @@ def test_what_the_kernels_range_refuses(sums, forces):
     assert sums(pos, vel, 1e-9, wide=True)[0].tolist() == [False] * 7 + [True]
     scal[:, 0] = 1 / 12e-6
     assert forces(pos, vel, scal, wide=True)[0].tolist() == [False] * 7 + [True]
+
+
+def test_base_vectors_stay_in_bounds(lib):
+    """Elements as distorted as they come, with volumes of state far from their own:
+    three products of derivatives below 2^60 and modes below 2^62 over 2^64, and 2^58
+    for gamma, are below 2^60; the sums over corners hold seven times that and no more."""
+    r = np.random.default_rng(8)
+    n = 40000
+    e = CUBE + r.uniform(0, 0.5, (n, 1, 1)) * r.choice([-1, 1], (n, 3, 8)) * r.uniform(0.5, 1, (n, 3, 8))
+    e[:, 2] *= 10 ** r.uniform(-3, 0, (n, 1))
+    q = np.linalg.qr(r.standard_normal((n, 3, 3)))[0]
+    q *= np.sign(np.linalg.det(q))[:, None, None]
+    turned = r.random(n) < 0.6
+    e[turned] = (q @ e)[turned]
+    pos = np.ascontiguousarray(0.01 * e)
+    w = _volume12(pos)
+    pos, w = np.ascontiguousarray(pos[w > 0]), w[w > 0]
+    n = len(w)
+    vel = np.ascontiguousarray(r.choice([-1.0, 1.0, 0.99], (n, 3, 8)))
+    scal = np.ascontiguousarray(np.stack([10 ** r.uniform(-1, 3, n) / w, np.full(n, -1.0), np.zeros(n)], 1))
+    largest = np.zeros(n)
+    lib.check_base(n, *(a.ctypes.data_as(ctypes.c_void_p) for a in (pos, vel, scal, largest)))
+    assert (largest > 0).mean() > 0.5 and largest.max() < 2.0 ** 60
