@@ -408,14 +408,15 @@ __device__ __forceinline__ bool good_sum(int top, int u) { return top <= 340 && 
 // extent, adjoint vectors by their coordinate's largest; what else joins the corners (edges, modes, V x W)
 // enters as mantissas in the largest term's unit. Elements of sizes or adjoints
 // out of range take the crosses in doubles, the positions' part from the tape.
-// Bound by FP64 issue (350 slots per element, the pipe 71 % busy; ALU 29 %,
-// multiply-adds 16 %). At 48^3 173 us with the crosses and corner sums on the FP64
+// Bound by FP64 issue (350 slots per element, the pipe 69 % busy; ALU 32 %,
+// multiply-adds 15 %). At 48^3 173 us with the crosses and corner sums on the FP64
 // pipe (87 % busy), 116 us so; a gradient of 40 cycles at 48^3 21.7 -> 20.0 ms, of
 // 24 cycles at 15^3 2.81 -> 2.73. Six blocks per SM (96 registers; 148 slots are
 // the most six can have) against five and seven: 20.04, 20.37, 20.18 ms. The
 // volume's scalars in one thread instead of all three (a barrier more) and the
 // velocity corners on the integer pipes: 101 us, 19.52 -> 18.91 ms, 2.65 -> 2.61;
-// the edges' crosses there too: 95 us, 18.61 -> 18.29, 2.60 -> 2.60.
+// the edges' crosses there too: 95 us, 18.61 -> 18.29, 2.60 -> 2.60; a scale for each
+// coordinate's adjoint vectors, 96 us.
 enum : int {
   // per coordinate: mean edges, half-step edges, 12 diagonals, U vectors (limbs),
   // the differences of dL/ddv along V and -W, the faces' terms (by the face's
