@@ -1026,7 +1026,7 @@ enum : int {
 // place of corner 0 their scale's exponent and whether they are in range.
 template <class Put>
 __device__ __forceinline__ void corner_differences(const double u[8], Put put) {
-  int ev = fx::exponent_field(fx::extent_hi(u));
+  int ev = fx::extent_field(u);
   // (all zero, or in range)
   const bool ok = ev == 0 || (ev >= fx::kMinSpeed && ev <= fx::kMaxSpeed);
   ev = ok ? fx::imax(ev, fx::kMinSpeed) : 0x7ff;

@@ -72,14 +72,14 @@ struct ForceLane {
 
 // 1: positions x and velocities v of coordinate k.
 LULESH_FX void force_load(int k, Slots sh, const double v[8], ForceLane& r) {
-  int ev = exponent_field(extent_hi(v));
+  int ev;
+  Num m;
+  extent_fields(v, r.x, ev, m.lo);
   const bool wild = ev > kMaxSpeed;  // not finite, or far beyond any flow
   r.ev = wild ? 0x7ff : imax(ev, kMinSpeed);
   const i64 v0 = to_fixed(v[0], 7 - r.ev);
   LULESH_UNROLL
   for (int n = 1; n < 8; ++n) r.V[n] = limbs(sub(to_fixed(v[n], 7 - r.ev), v0));
-  Num m;
-  m.lo = exponent_field(extent_hi(r.x));
   m.hi = wild;
   sh[FS_EXT + k] = m;
 }

@@ -65,8 +65,7 @@ LULESH_FX i64 square(Num a) {
 // 1: r.x and r.v hold coordinate k's corner values.
 LULESH_FX void kin_extents(int k, Slots sh, const KinLane& r) {
   Num m;
-  m.lo = exponent_field(extent_hi(r.x));
-  m.hi = exponent_field(extent_hi(r.v));
+  extent_fields(r.x, r.v, m.lo, m.hi);
   sh[KS_EXT + k] = m;
 }
 

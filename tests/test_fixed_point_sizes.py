@@ -89,6 +89,43 @@ def test_sums_of_thin_elements(sums, h, axis, squash):
     _no_further_off(fixed[taken], fp64[taken], size[taken], range(10))
 
 
+@pytest.mark.parametrize("boost", [1.0, 1e3, 1e6])
+@pytest.mark.parametrize("step", [1e-3, 1e-6, 1e-9])
+@pytest.mark.parametrize("wide", [False, True])
+def test_a_fast_uniform_motion(sums, forces, boost, step, wide):
+    """Differences far below the velocities themselves, down to what the velocities
+    still resolve."""
+    h = 1.125 / 150
+    pos, vel = _elements(9, 200, h, 0.05)
+    vel = np.ascontiguousarray(boost * (1 + np.arange(3)[None, :, None]) + step * vel)
+    for half_dt in (0.0, 1e-3 * h / boost):
+        taken, _, fixed, fp64, size = sums(pos, vel, half_dt, wide)
+        assert taken.all()
+        _no_further_off(fixed, fp64, size, range(10))
+    scal = np.tile([1 / (12 * h ** 3), -30 * h * h, -10.0], (200, 1))
+    taken, fixed, fp64, size = forces(pos, vel, scal, wide)
+    assert taken.all()
+    _no_further_off(fixed, fp64, size, range(3))
+
+
+@pytest.mark.parametrize("away", [12, 20, 24, 28, 32, 40])
+@pytest.mark.parametrize("axes", [(0,), (1, 2), (0, 1, 2)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_a_mesh_far_from_the_origin(sums, forces, away, axes, wide):
+    """2^away spacings from it, along some axes; the extents are known exactly there too."""
+    h = 1.125 / 150
+    pos, vel = _elements(10, 200, h, 0.05)
+    pos -= h * np.floor(pos[:, :, :1] / h)
+    pos[:, list(axes)] += h * 2.0 ** away
+    taken, _, fixed, fp64, size = sums(pos, vel, 1e-4 * h, wide)
+    assert taken.all()
+    _no_further_off(fixed, fp64, size, range(10))
+    scal = np.stack([1 / _volume12(pos), np.full(200, -30 * h * h), np.full(200, -10.0)], 1)
+    taken, fixed, fp64, size = forces(pos, vel, scal, wide)
+    assert taken.all()
+    _no_further_off(fixed, fp64, size, range(3))
+
+
 def test_exact_zeros_stay_zeros(sums):
     """Velocities of zeros of both signs, and a flow whose divergence is exactly
     zero in doubles (compression along one axis as expansion along another, on
